@@ -3,24 +3,33 @@
 The library is built in-tree by ``build()`` with a plain ``nvcc`` command (no JIT cache, no
 torch extension machinery) and loaded lazily.  There is no fallback: if the library is missing
 or cannot be loaded, every operator of this package raises.
+
+Beside it stands ``_host.so`` (csrc/host.cpp, built with ``g++``): the native host path of the
+Python operators, a CPython extension that links the library.
 """
 from __future__ import annotations
 
 import ctypes
 import fcntl
 import glob
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import subprocess
+import sysconfig
 import threading
+
+import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libfa4_nvfp4.so")
 CSRC = os.path.join(_HERE, "csrc")
+HOST_PATH = os.path.join(_HERE, "_host.so")
 LOCK_PATH = os.path.join(_HERE, ".build.lock")
 SOURCES = ["api.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "--shared", "-Xcompiler", "-fPIC"]
+              "--shared", "-Xcompiler", "-fPIC", "-Xlinker", "-soname=libfa4_nvfp4.so"]
 
 ERROR_NAMES = {1: "null pointer", 2: "unsupported shape", 3: "bad stride", 4: "misaligned pointer",
                5: "unknown variant", 6: "tensor map rejected", 7: "struct size mismatch",
@@ -75,17 +84,29 @@ class Varlen(ctypes.Structure):
 
 
 def _dependencies():
-    """Every file the library is compiled from: all of csrc/ and the public header."""
+    """Every file the library is compiled from: the CUDA files of csrc/ and the public header."""
     deps = sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
     deps.append(os.path.join(_HERE, "..", "include", "fa4_nvfp4.h"))
     return deps
 
 
-def _needs_build() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _host_dependencies():
+    return [os.path.join(CSRC, "host.cpp"), os.path.join(_HERE, "..", "include", "fa4_nvfp4.h")]
+
+
+def _stale(path: str, deps) -> bool:
+    if not os.path.exists(path):
         return True
-    t = os.path.getmtime(LIB_PATH)
-    return any(os.path.exists(d) and os.path.getmtime(d) > t for d in _dependencies())
+    t = os.path.getmtime(path)
+    return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps)
+
+
+def _needs_build() -> bool:
+    return _stale(LIB_PATH, _dependencies())
+
+
+def _host_needs_build() -> bool:
+    return _stale(HOST_PATH, _host_dependencies())
 
 
 class _BuildLock:
@@ -102,26 +123,47 @@ class _BuildLock:
         self.f.close()
 
 
-def _compile(verbose: bool) -> None:
-    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-    tmp = f"{LIB_PATH}.{os.getpid()}.tmp"
-    cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + \
-          ["-o", tmp] + [os.path.join(CSRC, s) for s in SOURCES]
-    res = subprocess.run(cmd, capture_output=True, text=True)
+def _run_compiler(cmd, path: str, verbose: bool) -> None:
+    tmp = f"{path}.{os.getpid()}.tmp"
+    res = subprocess.run(cmd + ["-o", tmp], capture_output=True, text=True)
     if res.returncode != 0:
         if os.path.exists(tmp):
             os.unlink(tmp)
-        raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-    os.replace(tmp, LIB_PATH)       # readers see the old file or the complete new one
+        raise RuntimeError(f"{os.path.basename(cmd[0])} failed:\n" + res.stdout + res.stderr)
+    os.replace(tmp, path)           # readers see the old file or the complete new one
     if verbose:
         print(res.stderr)
 
 
+def _nvcc():
+    return shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+
+
+def _compile(verbose: bool) -> None:
+    _run_compiler([_nvcc()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) +
+                  [os.path.join(CSRC, s) for s in SOURCES], LIB_PATH, verbose)
+
+
+def _compile_host(verbose: bool) -> None:
+    torch_dir = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    includes = [sysconfig.get_paths()["include"], os.path.join(torch_dir, "include"),
+                os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
+    libs = os.path.join(torch_dir, "lib")
+    _run_compiler([shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+                   f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] +
+                  [f"-I{i}" for i in includes] + [os.path.join(CSRC, "host.cpp"), f"-L{libs}", "-ltorch_python",
+                   "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", LIB_PATH, f"-Wl,-rpath,{libs}",
+                   "-Wl,-rpath,$ORIGIN"], HOST_PATH, verbose)
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the CUDA library for sm_100a (cross-compiles without a GPU)."""
+    """Compile the CUDA library for sm_100a (cross-compiles without a GPU) and the host extension."""
     with _BuildLock():
         if force or _needs_build():
             _compile(verbose)
+        if force or _host_needs_build():
+            _compile_host(verbose)
     return LIB_PATH
 
 
@@ -188,6 +230,32 @@ def lib() -> ctypes.CDLL:
             L.fa4_nvfp4_fwd_linear_sf_noalloc.restype = ctypes.c_int
             _lib = L
         return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/host.cpp), built on demand like the library."""
+    global _host
+    if _host is None:
+        lib()                           # the extension links the library: build and load that first
+        with _lock:
+            if _host is None:
+                with _BuildLock():
+                    if _host_needs_build():
+                        if shutil.which("g++"):
+                            _compile_host(False)
+                        elif not os.path.exists(HOST_PATH):
+                            raise RuntimeError(f"{HOST_PATH} is missing and g++ is not available; "
+                                               "run flash_attention_b200.build() first")
+                    name = __package__ + "._host"
+                    loader = importlib.machinery.ExtensionFileLoader(name, HOST_PATH)
+                    spec = importlib.util.spec_from_file_location(name, HOST_PATH, loader=loader)
+                    mod = importlib.util.module_from_spec(spec)
+                    loader.exec_module(mod)
+                _host = mod
+    return _host
 
 
 EXPORTS = ["fa4_nvfp4_fwd", "fa4_nvfp4_sf_linear_to_tiled", "fa4_nvfp4_query",

@@ -1,0 +1,564 @@
+// Native host path of the Python operators: argument checks, output and scratch allocation, the
+// parameter block and the launch of one attention call, as a CPython extension over the C ABI of
+// include/fa4_nvfp4.h.
+//
+// Why it exists: a decode step is 5-10 us of GPU time, and the same checks, attribute reads and
+// ctypes assignments written in Python took 35-60 us per call (B200 box, 76 us per pass of a
+// one-token call with linear scales), so the GPU waited for the host.  Here they take 5-8 us.
+//
+// The functions take their arguments positionally (METH_FASTCALL); interface.py and varlen.py own
+// the signatures, defaults and documentation.  Error types and messages are those of the
+// reference's host code (flash_attn/cute/interface.py:231-236, 384-398): AssertionError for
+// malformed tensors, NotImplementedError for what is not built, ValueError for bad numbers.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Device.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstdarg>
+#include <cstdio>
+#include <string>
+
+#include "../../include/fa4_nvfp4.h"
+
+namespace {
+
+// A Python exception that has been set (PyErr_SetString) travels to the boundary as this.
+struct PyErrorSet {};
+
+[[noreturn]] __attribute__((format(printf, 2, 3))) void fail(PyObject* type, const char* fmt, ...) {
+  char msg[512];
+  va_list ap;
+  va_start(ap, fmt);
+  vsnprintf(msg, sizeof msg, fmt, ap);
+  va_end(ap);
+  PyErr_SetString(type, msg);
+  throw PyErrorSet();
+}
+#define FA4_ASSERT(cond, ...) \
+  do { if (!(cond)) fail(PyExc_AssertionError, __VA_ARGS__); } while (0)
+
+std::string dims_of(at::IntArrayRef s) {
+  std::string r = "(";
+  for (size_t i = 0; i < s.size(); ++i) r += (i ? ", " : "") + std::to_string(s[i]);
+  return r + ")";
+}
+
+const at::Tensor& tensor_of(PyObject* o, const char* name) {
+  if (!THPVariable_Check(o)) fail(PyExc_TypeError, "%s must be a torch.Tensor, got %s", name, Py_TYPE(o)->tp_name);
+  return THPVariable_Unpack(o);
+}
+bool is_none(PyObject* o) { return o == nullptr || o == Py_None; }
+
+// packed bytes arrive as uint8, float8_e4m3fn or float4_e2m1fn_x2
+at::Tensor as_u8(PyObject* o, const char* name) {
+  const at::Tensor& t = tensor_of(o, name);
+  const auto st = t.scalar_type();
+  if (st == at::kByte) return t;
+  if (st == at::ScalarType::Float8_e4m3fn || st == at::ScalarType::Float4_e2m1fn_x2) return t.view(at::kByte);
+  fail(PyExc_AssertionError, "%s must be uint8 / float8_e4m3fn / float4_e2m1fn_x2, got %s", name,
+       c10::toString(st));
+}
+
+void validate(const at::Tensor& t, const char* name, at::IntArrayRef shape, at::ScalarType dtype,
+              const at::Device& device) {
+  FA4_ASSERT(t.sizes() == shape, "%s shape %s != expected %s", name, dims_of(t.sizes()).c_str(), dims_of(shape).c_str());
+  FA4_ASSERT(t.scalar_type() == dtype, "%s dtype %s != expected %s", name, c10::toString(t.scalar_type()),
+             c10::toString(dtype));
+  FA4_ASSERT(t.device() == device, "%s device %s != expected %s", name, t.device().str().c_str(), device.str().c_str());
+  FA4_ASSERT(t.is_cuda(), "%s must be on CUDA", name);
+}
+
+at::Tensor inner_contiguous(at::Tensor t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
+
+double number_of(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw PyErrorSet();
+  return v;
+}
+long integer_of(PyObject* o) {
+  PyObject* n = PyNumber_Long(o);
+  if (n == nullptr) throw PyErrorSet();
+  const long v = PyLong_AsLong(n);
+  Py_DECREF(n);
+  if (v == -1 && PyErr_Occurred()) throw PyErrorSet();
+  return v;
+}
+bool truth_of(PyObject* o) {
+  if (o == Py_True) return true;
+  if (o == Py_False) return false;
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw PyErrorSet();
+  return v != 0;
+}
+// a per-tensor scale: a number, or a one-element tensor whose value is read (synchronises if it
+// lives on the device)
+float scalar_of(PyObject* o, const char* name) {
+  if (THPVariable_Check(o)) {
+    const at::Tensor& t = THPVariable_Unpack(o);
+    FA4_ASSERT(t.numel() == 1, "%s must be a python float or a 1-element tensor", name);
+    return static_cast<float>(t.item<double>());
+  }
+  return static_cast<float>(number_of(o));
+}
+
+// The status word of a device (see DeviceStatus in interface.py, which owns it): address kept here.
+uint32_t* status_word(const at::Device& device) {
+  static PyObject* kept[64] = {};
+  static uint32_t* ptr[64] = {};
+  const int idx = device.index();
+  TORCH_CHECK(idx >= 0 && idx < 64, "device index out of range");
+  if (ptr[idx] == nullptr) {
+    PyObject* mod = PyImport_ImportModule("flash_attention_b200.interface");
+    if (mod == nullptr) throw PyErrorSet();
+    PyObject* cls = PyObject_GetAttrString(mod, "DeviceStatus");
+    Py_DECREF(mod);
+    if (cls == nullptr) throw PyErrorSet();
+    PyObject* dev = THPDevice_New(device);
+    PyObject* w = dev ? PyObject_CallMethod(cls, "word", "O", dev) : nullptr;
+    Py_XDECREF(dev);
+    Py_DECREF(cls);
+    if (w == nullptr) throw PyErrorSet();
+    kept[idx] = w;   // never freed: one word per device
+    ptr[idx] = static_cast<uint32_t*>(THPVariable_Unpack(w).data_ptr());
+  }
+  return ptr[idx];
+}
+
+// Turns a return code of the C ABI into the exception _lib.check raises for it.
+void check_rc(int rc, const char* what) {
+  if (rc == 0) return;
+  PyObject* mod = PyImport_ImportModule("flash_attention_b200._lib");
+  if (mod == nullptr) throw PyErrorSet();
+  PyObject* r = PyObject_CallMethod(mod, "check", "is", rc, what);
+  Py_DECREF(mod);
+  Py_XDECREF(r);
+  throw PyErrorSet();
+}
+
+// ---- rules on sizes (interface.py documents them) ------------------------------------------------
+
+// Causal and window arguments after the reference's rules (flash_attn/cute/interface.py:256-276).
+struct Window {
+  bool causal = false;
+  int left = -1, right = -1;      // -1: no limit
+};
+Window resolve_window(bool causal, PyObject* left_o, PyObject* right_o) {
+  bool has_l = !is_none(left_o), has_r = !is_none(right_o);
+  long l = has_l ? integer_of(left_o) : 0, r = has_r ? integer_of(right_o) : 0;
+  if (causal) { has_r = true; r = 0; }
+  if (has_l && has_r && l + r < 0) has_l = has_r = false;
+  if ((has_l && l < 0) || (has_r && r < 0))
+    fail(PyExc_NotImplementedError, "negative window limits (a band shifted off the diagonal) are not built");
+  Window w;
+  w.left = has_l ? static_cast<int>(std::min<long>(l, 0x7fffffff)) : -1;
+  w.right = has_r ? static_cast<int>(std::min<long>(r, 0x7fffffff)) : -1;
+  w.causal = has_r && r == 0 && !has_l;
+  return w;
+}
+
+int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+int64_t decode_splits(int64_t B, int64_t Hkv, int64_t Sk, int64_t sms) {
+  const int64_t blocks = cdiv(Sk, 128), units = std::max<int64_t>(1, B * Hkv);
+  if (units > 3 * sms) {
+    int64_t best = 1, best_cost = -1;
+    for (int64_t ns = 1; ns < 5 && ns <= std::max<int64_t>(1, blocks / 2); ++ns) {
+      const int64_t cost = cdiv(ns * units, 3 * sms) * (cdiv(blocks, ns) + 4);
+      if (best_cost < 0 || cost < best_cost) { best = ns; best_cost = cost; }
+    }
+    return best;
+  }
+  const int64_t want = std::max<int64_t>(1, (2 * sms + units / 2) / units);
+  return std::max<int64_t>(1, std::min({int64_t{128}, want, std::max<int64_t>(1, blocks / 2)}));
+}
+
+int64_t prefill_splits(int64_t B, int64_t Sq, int64_t Sk, int64_t Hq, int64_t sms) {
+  const int64_t tiles = B * Hq * cdiv(Sq, 128), blocks = cdiv(Sk, 128);
+  if (tiles * 2 > sms || blocks < 8) return 1;
+  int64_t best = 1, best_cost = -1;
+  for (int64_t n = 1; n <= std::min<int64_t>(blocks / 4, 128); ++n) {
+    const int64_t per = cdiv(blocks, n);
+    if (n > 1 && per * (n - 1) >= blocks) continue;   // the last split would be empty
+    const int64_t cost = cdiv(tiles * n, sms) * (per + 2);
+    if (best_cost < 0 || cost < best_cost) { best = n; best_cost = cost; }
+  }
+  return best;
+}
+
+int64_t sm_count(const at::Device& d) { return at::cuda::getDeviceProperties(d.index())->multiProcessorCount; }
+
+bool head_dims_built(int64_t D, int64_t Dv) {
+  return (D == Dv && (D == 64 || D == 128)) || (D == 192 && Dv == 128);
+}
+
+// The learnable sink as Hq contiguous fp32 values on the device.
+at::Tensor sink_of(PyObject* o, int64_t Hq, const at::Device& device) {
+  if (is_none(o)) return {};
+  const at::Tensor& t = tensor_of(o, "learnable_sink");
+  FA4_ASSERT(t.dim() == 1 && t.size(0) == Hq, "learnable_sink must have one entry per query head");
+  if (t.device() == device && t.scalar_type() == at::kFloat && t.is_contiguous()) return t;
+  return t.to(device, at::kFloat).contiguous();
+}
+
+// Linear scales (outer, inner, rows, cols; any strides but the last) -> the tiled layout.
+at::Tensor tile_scales(const at::Tensor& sf, int rows_dim, int head_dim, int64_t mult, void* stream) {
+  const int64_t B = sf.size(0), H = sf.size(head_dim), R = sf.size(rows_dim), C = sf.size(3);
+  const int64_t ct = cdiv(cdiv(C, 4), mult) * mult;
+  at::Tensor out = at::empty({B, H, cdiv(R, 128), ct, 512}, sf.options());
+  check_rc(fa4_nvfp4_sf_linear_to_tiled(sf.data_ptr(), out.data_ptr(), (int)B, (int)H, (int)R, (int)C, sf.stride(0),
+                                        sf.stride(head_dim), sf.stride(rows_dim), (int)mult, stream),
+           "fa4_nvfp4_sf_linear_to_tiled");
+  return out;
+}
+
+PyObject* pair_of(PyObject* out_o, const at::Tensor& out, PyObject* lse_o, const at::Tensor& lse) {
+  PyObject* a;
+  if (!is_none(out_o)) { a = out_o; Py_INCREF(a); } else a = THPVariable_Wrap(out);
+  PyObject* b;
+  if (!is_none(lse_o)) { b = lse_o; Py_INCREF(b); }
+  else if (lse.defined()) b = THPVariable_Wrap(lse);
+  else { b = Py_None; Py_INCREF(b); }
+  PyObject* r = PyTuple_New(2);
+  PyTuple_SET_ITEM(r, 0, a);
+  PyTuple_SET_ITEM(r, 1, b);
+  return r;
+}
+
+// ---- flash_attn_fp4_func ------------------------------------------------------------------------
+// q k v q_sf k_sf v_sf q_scale k_scale v_scale softmax_scale causal return_lse out lse sf_layout
+// variant num_splits window_left window_right learnable_sink softcap seqused_k page_table
+PyObject* fwd(PyObject* const* a) {
+  at::Tensor q = as_u8(a[0], "q"), k = as_u8(a[1], "k"), v = as_u8(a[2], "v");
+  at::Tensor q_sf = as_u8(a[3], "q_sf"), k_sf = as_u8(a[4], "k_sf"), v_sf = as_u8(a[5], "v_sf");
+  PyObject *out_o = a[12], *lse_o = a[13], *used_o = a[21], *table_o = a[22];
+  FA4_ASSERT(q.dim() == 4 && k.dim() == 4 && v.dim() == 4, "q, k, v must be 4-D");
+  FA4_ASSERT(q.is_cuda() && k.is_cuda() && v.is_cuda(), "inputs must be on CUDA");
+  q = inner_contiguous(std::move(q));
+  k = inner_contiguous(std::move(k));
+  v = inner_contiguous(std::move(v));
+  const int64_t B = q.size(0), Sq = q.size(1), Hq = q.size(2), D = 2 * q.size(3);
+  const int64_t B_kv = k.size(0), Sk_kv = k.size(1), Hkv = k.size(2), Dv = v.size(2);
+  const at::Device device = q.device();
+  const bool paged = !is_none(table_o);
+  int64_t Sk = Sk_kv, pages_per_seq = 0;
+  at::Tensor table, used;
+  if (paged) {
+    // k / v are a pool of B_kv pages of Sk_kv (= page_size) keys; Sk is the logical key length
+    const at::Tensor& t = tensor_of(table_o, "page_table");
+    FA4_ASSERT(t.dim() == 2 && t.size(0) == B && t.scalar_type() == at::kInt && t.is_cuda(),
+               "page_table must be a (B, pages_per_seq) int32 CUDA tensor");
+    FA4_ASSERT(v.size(0) == B_kv, "k and v pools differ in their number of pages");
+    if (Sk_kv % 128 != 0)
+      fail(PyExc_NotImplementedError, "page_size must be a multiple of 128 (whole K/V blocks per page)");
+    table = t.contiguous();
+    pages_per_seq = t.size(1);
+    Sk = pages_per_seq * Sk_kv;
+  } else {
+    FA4_ASSERT(B_kv == B && v.size(0) == B, "batch size mismatch");
+  }
+  if (!is_none(used_o)) {
+    const at::Tensor& t = tensor_of(used_o, "seqused_k");
+    FA4_ASSERT(t.dim() == 1 && t.size(0) == B && t.scalar_type() == at::kInt && t.is_cuda(),
+               "seqused_k must be a (B,) int32 CUDA tensor");
+    used = t.contiguous();
+  }
+  FA4_ASSERT(2 * k.size(3) == D, "q and k head dims differ");
+  const int64_t Sk_pad = cdiv(Sk_kv, 32) * 32;   // V's key axis is padded to whole 32-key groups (zeros)
+  FA4_ASSERT(v.size(1) == Hkv && 2 * v.size(3) == Sk_pad,
+             "v must be (B, Hkv, Dv, Skp/2) with Skp = seqlen_k rounded up to a multiple of 32, got %s",
+             dims_of(v.sizes()).c_str());
+  FA4_ASSERT(Hkv > 0 && Hq % Hkv == 0, "num_head must be divisible by num_head_kv");
+  if (!head_dims_built(D, Dv))
+    fail(PyExc_NotImplementedError,
+         "head dims (D=%lld, Dv=%lld) not built; supported: (128, 128), (64, 64) and (192, 128)", (long long)D,
+         (long long)Dv);
+  const double softmax_scale = is_none(a[9]) ? 1.0 / std::sqrt((double)D) : number_of(a[9]);
+
+  c10::cuda::OptionalCUDAGuard guard;
+  if (device.index() != c10::cuda::current_device()) guard.set_device(device);
+  void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
+
+  const char* layout = PyUnicode_Check(a[14]) ? PyUnicode_AsUTF8(a[14]) : nullptr;
+  if (layout != nullptr && !strcmp(layout, "linear")) {
+    validate(q_sf, "q_sf", {B, Sq, Hq, D / 16}, at::kByte, device);
+    validate(k_sf, "k_sf", {B_kv, Sk_kv, Hkv, D / 16}, at::kByte, device);
+    validate(v_sf, "v_sf", {B_kv, Hkv, Dv, Sk_pad / 16}, at::kByte, device);
+    q_sf = tile_scales(inner_contiguous(std::move(q_sf)), 1, 2, 1, stream);
+    k_sf = tile_scales(inner_contiguous(std::move(k_sf)), 1, 2, 1, stream);
+    v_sf = tile_scales(inner_contiguous(std::move(v_sf)), 2, 1, 2, stream);
+  } else if (layout != nullptr && !strcmp(layout, "tiled")) {
+    validate(q_sf, "q_sf", {B, Hq, cdiv(Sq, 128), D / 64, 512}, at::kByte, device);
+    validate(k_sf, "k_sf", {B_kv, Hkv, cdiv(Sk_kv, 128), D / 64, 512}, at::kByte, device);
+    validate(v_sf, "v_sf", {B_kv, Hkv, cdiv(Dv, 128), 2 * cdiv(Sk_kv, 128), 512}, at::kByte, device);
+    FA4_ASSERT(q_sf.is_contiguous() && k_sf.is_contiguous() && v_sf.is_contiguous(),
+               "tiled scale factors must be contiguous");
+  } else {
+    PyErr_Format(PyExc_ValueError, "sf_layout must be 'linear' or 'tiled', got %R", a[14]);
+    throw PyErrorSet();
+  }
+
+  at::Tensor out, lse;
+  if (is_none(out_o)) {
+    out = at::empty({B, Sq, Hq, Dv}, q.options().dtype(at::kBFloat16));
+  } else {
+    out = tensor_of(out_o, "out");
+    validate(out, "out", {B, Sq, Hq, Dv}, at::kBFloat16, device);
+    FA4_ASSERT(out.stride(-1) == 1, "out's last dimension must be contiguous");
+  }
+  if (!is_none(lse_o)) {
+    lse = tensor_of(lse_o, "lse");
+    validate(lse, "lse", {B, Hq, Sq}, at::kFloat, device);
+    FA4_ASSERT(lse.is_contiguous(), "lse must be contiguous");
+  } else if (truth_of(a[11])) {
+    lse = at::empty({B, Hq, Sq}, q.options().dtype(at::kFloat));
+  }
+
+  fa4_nvfp4_params p = {};
+  p.struct_size = sizeof p;
+  p.variant = (int32_t)integer_of(a[15]);
+  p.q = q.data_ptr();
+  p.k = k.data_ptr();
+  p.v = v.data_ptr();
+  p.q_sf = q_sf.data_ptr();
+  p.k_sf = k_sf.data_ptr();
+  p.v_sf = v_sf.data_ptr();
+  p.out = out.data_ptr();
+  p.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
+  p.status = status_word(device);
+  p.q_stride_b = q.stride(0); p.q_stride_s = q.stride(1); p.q_stride_h = q.stride(2);
+  p.k_stride_b = k.stride(0); p.k_stride_s = k.stride(1); p.k_stride_h = k.stride(2);
+  p.v_stride_b = v.stride(0); p.v_stride_h = v.stride(1); p.v_stride_d = v.stride(2);
+  p.o_stride_b = out.stride(0); p.o_stride_s = out.stride(1); p.o_stride_h = out.stride(2);
+  p.B = (int32_t)B; p.Sq = (int32_t)Sq; p.Sk = (int32_t)Sk; p.Hq = (int32_t)Hq; p.Hkv = (int32_t)Hkv;
+  p.D = (int32_t)D; p.Dv = (int32_t)Dv;
+  p.q_scale = scalar_of(a[6], "q_scale");
+  p.k_scale = scalar_of(a[7], "k_scale");
+  p.v_scale = scalar_of(a[8], "v_scale");
+  p.softmax_scale = (float)softmax_scale;
+
+  long num_splits = integer_of(a[16]);
+  if (num_splits < 0 || num_splits > 128) fail(PyExc_ValueError, "num_splits must be in 0..128");
+  const bool auto_splits = num_splits == 0;
+  const Window win = resolve_window(truth_of(a[10]), a[17], a[18]);
+  p.causal = win.causal ? 1 : 0;
+  const double softcap = is_none(a[20]) ? 0.0 : number_of(a[20]);
+  if (!(softcap >= 0.0) || !std::isfinite(softcap)) fail(PyExc_ValueError, "softcap must be a finite number >= 0");
+  const at::Tensor sink = sink_of(a[19], Hq, device);
+  // A handful of query rows per kv head (decode, append): the transposed kernel, which always
+  // splits the keys over CTAs and merges with the combine kernel.
+  const bool decode_ok = D == 128 && Dv == 128 && Sq * (Hq / Hkv) <= 32 && win.left < 0 && win.right <= 0 &&
+                         !sink.defined() && softcap == 0.0;
+  if (p.variant == FA4_VARIANT_DECODE && !decode_ok)
+    fail(PyExc_NotImplementedError,
+         "the decode kernel takes D = Dv = 128, Sq * (Hq / Hkv) <= 32, no window / sink / softcap");
+  if (p.variant == FA4_VARIANT_AUTO && decode_ok) p.variant = FA4_VARIANT_DECODE;
+  const bool decode = p.variant == FA4_VARIANT_DECODE;
+  if (auto_splits)
+    num_splits = decode ? decode_splits(B, Hkv, Sk, sm_count(device)) : prefill_splits(B, Sq, Sk, Hq, sm_count(device));
+
+  if (num_splits == 1 && !sink.defined() && win.left < 0 && win.right <= 0 && softcap == 0.0 && !used.defined() &&
+      !paged && !decode) {
+    check_rc(fa4_nvfp4_fwd(&p, stream), "fa4_nvfp4_fwd");
+  } else {
+    fa4_nvfp4_ext x = {};
+    x.struct_size = sizeof x;
+    x.num_splits = (int32_t)num_splits;
+    x.window_left = win.left;
+    x.window_right = win.right;
+    x.sink = sink.defined() ? sink.data_ptr<float>() : nullptr;
+    x.softcap = (float)softcap;
+    x.seqused_k = used.defined() ? used.data_ptr<int32_t>() : nullptr;
+    if (paged) {
+      x.page_table = table.data_ptr<int32_t>();
+      x.page_size = (int32_t)Sk_kv;
+      x.pages_per_seq = (int32_t)pages_per_seq;
+      x.num_pages = (int32_t)B_kv;
+    }
+    at::Tensor workspace;   // stream-ordered scratch
+    if (num_splits > 1 || decode) {
+      const int64_t bytes = fa4_nvfp4_splitkv_workspace_bytes(&p, (int32_t)std::max(2l, num_splits));
+      if (bytes < 0) check_rc((int)bytes, "fa4_nvfp4_splitkv_workspace_bytes");
+      workspace = at::empty({bytes}, q.options());
+      x.workspace = workspace.data_ptr();
+      x.workspace_bytes = (uint64_t)bytes;
+    }
+    check_rc(fa4_nvfp4_fwd_ex(&p, &x, stream), "fa4_nvfp4_fwd_ex");
+  }
+  return pair_of(out_o, out, lse_o, lse);
+}
+
+// ---- flash_attn_varlen_fp4_func -------------------------------------------------------------------
+// Packed scales -> per-sequence tiles, padded to the longest sequence.
+at::Tensor tile_packed(const at::Tensor& sf, const at::Tensor& cu, int64_t seqs, int64_t inner, int64_t max_rows,
+                       int64_t max_cols, int64_t stride_inner, int64_t stride_row, int64_t mult, bool packed_rows,
+                       void* stream) {
+  const int64_t ct = cdiv(cdiv(max_cols, 4), mult) * mult;
+  at::Tensor out = at::empty({seqs, inner, cdiv(max_rows, 128), ct, 512}, sf.options());
+  check_rc(fa4_nvfp4_sf_linear_to_tiled_packed(sf.data_ptr(), out.data_ptr(), cu.data_ptr<int32_t>(), (int)seqs,
+                                               (int)inner, (int)max_rows, (int)max_cols, stride_inner, stride_row,
+                                               (int)mult, packed_rows ? 1 : 0, stream),
+           "fa4_nvfp4_sf_linear_to_tiled_packed");
+  return out;
+}
+
+at::Tensor offsets_of(PyObject* o, const char* name, const at::Device& device) {
+  if (is_none(o)) return {};
+  const at::Tensor& t = tensor_of(o, name);
+  FA4_ASSERT(t.dim() == 1, "%s must be one-dimensional", name);
+  if (t.device() == device && t.scalar_type() == at::kInt && t.is_contiguous()) return t;
+  return t.to(device, at::kInt).contiguous();
+}
+
+// the longest sequence of a packed batch: one synchronising read
+int64_t longest_of(const at::Tensor& cu) { return cu.diff().max().item<int64_t>(); }
+
+// q k v q_sf k_sf v_sf q_scale k_scale v_scale cu_q cu_k seqused_k cu_v max_q max_k softmax_scale causal
+// window_left window_right learnable_sink softcap return_lse
+PyObject* varlen_fwd(PyObject* const* a) {
+  at::Tensor q = as_u8(a[0], "q"), k = as_u8(a[1], "k"), v = as_u8(a[2], "v");
+  at::Tensor q_sf = as_u8(a[3], "q_sf"), k_sf = as_u8(a[4], "k_sf"), v_sf = as_u8(a[5], "v_sf");
+  FA4_ASSERT(q.dim() == 3 && k.dim() == 3 && v.dim() == 3, "packed operands are 3-D");
+  FA4_ASSERT(q.is_cuda() && k.is_cuda() && v.is_cuda(), "inputs must be on CUDA");
+  q = inner_contiguous(std::move(q));
+  k = inner_contiguous(std::move(k));
+  v = inner_contiguous(std::move(v));
+  const at::Device device = q.device();
+  c10::cuda::OptionalCUDAGuard guard;
+  if (device.index() != c10::cuda::current_device()) guard.set_device(device);
+  void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
+  q_sf = q_sf.contiguous();
+  k_sf = k_sf.contiguous();
+  v_sf = v_sf.contiguous();
+  const int64_t total_q = q.size(0), Hq = q.size(1), D = 2 * q.size(2);
+  const int64_t total_k = k.size(0), Hkv = k.size(1), Dv = v.size(1);
+  const bool has_cu_v = !is_none(a[12]);
+  const int64_t total_kp = has_cu_v ? 2 * v.size(2) : cdiv(total_k, 32) * 32;
+  FA4_ASSERT(2 * k.size(2) == D && v.size(0) == Hkv && Hkv > 0 && Hq % Hkv == 0,
+             "head counts / head dims of q, k, v do not fit");
+  FA4_ASSERT(2 * v.size(2) == total_kp && total_kp % 32 == 0 && total_kp >= total_k,
+             "v must be (Hkv, Dv, total_kp/2) with total_kp = %lld, got %s", (long long)total_kp,
+             dims_of(v.sizes()).c_str());
+  FA4_ASSERT(q_sf.sizes() == at::IntArrayRef({total_q, Hq, D / 16}) &&
+                 k_sf.sizes() == at::IntArrayRef({total_k, Hkv, D / 16}) &&
+                 v_sf.sizes() == at::IntArrayRef({Hkv, Dv, total_kp / 16}),
+             "scale factors must be the packed linear layouts");
+  if (!head_dims_built(D, Dv))
+    fail(PyExc_NotImplementedError, "head dims (D=%lld, Dv=%lld) not built", (long long)D, (long long)Dv);
+  const at::Tensor cu_q = offsets_of(a[9], "cu_seqlens_q", device), cu_k = offsets_of(a[10], "cu_seqlens_k", device);
+  FA4_ASSERT(cu_q.numel() == cu_k.numel() && cu_q.numel() >= 2, "cu_seqlens_q / cu_seqlens_k describe different batches");
+  const int64_t seqs = cu_q.numel() - 1;
+  const at::Tensor cu_v = offsets_of(a[12], "cu_seqlens_v", device), used = offsets_of(a[11], "seqused_k", device);
+  FA4_ASSERT(!cu_v.defined() || cu_v.numel() == seqs + 1, "cu_seqlens_v has another batch size");
+  FA4_ASSERT(!used.defined() || used.numel() == seqs, "seqused_k has another batch size");
+  // without both maxima one synchronising read; pass them to stay asynchronous, as the reference's callers do
+  const bool known = !is_none(a[13]) && !is_none(a[14]);
+  int64_t max_q = known ? integer_of(a[13]) : longest_of(cu_q), max_k = known ? integer_of(a[14]) : longest_of(cu_k);
+  max_q = std::min(std::max<int64_t>(1, max_q), total_q);
+  max_k = std::min(std::max<int64_t>(1, max_k), total_k);
+  const double softmax_scale = is_none(a[15]) ? 1.0 / std::sqrt((double)D) : number_of(a[15]);
+  const Window win = resolve_window(truth_of(a[16]), a[17], a[18]);
+  const at::Tensor sink = sink_of(a[19], Hq, device);
+
+  const at::Tensor q_t = tile_packed(q_sf, cu_q, seqs, Hq, max_q, D / 16, D / 16, Hq * (D / 16), 1, true, stream);
+  const at::Tensor k_t = tile_packed(k_sf, cu_k, seqs, Hkv, max_k, D / 16, D / 16, Hkv * (D / 16), 1, true, stream);
+  const at::Tensor v_t = tile_packed(v_sf, cu_v.defined() ? cu_v : cu_k, seqs, Hkv, Dv, cdiv(max_k, 16),
+                                     Dv * (total_kp / 16), total_kp / 16, 2, false, stream);
+  at::Tensor out = at::empty({total_q, Hq, Dv}, q.options().dtype(at::kBFloat16)), lse;
+  if (truth_of(a[21])) lse = at::empty({Hq, total_q}, q.options().dtype(at::kFloat));
+
+  fa4_nvfp4_params p = {};
+  p.struct_size = sizeof p;
+  p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr();
+  p.q_sf = q_t.data_ptr(); p.k_sf = k_t.data_ptr(); p.v_sf = v_t.data_ptr();
+  p.out = out.data_ptr();
+  p.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
+  p.status = status_word(device);
+  p.q_stride_s = q.stride(0); p.q_stride_h = q.stride(1); p.q_stride_b = q.stride(0) * std::max<int64_t>(1, total_q);
+  p.k_stride_s = k.stride(0); p.k_stride_h = k.stride(1); p.k_stride_b = k.stride(0) * std::max<int64_t>(1, total_k);
+  p.v_stride_h = v.stride(0); p.v_stride_d = v.stride(1); p.v_stride_b = v.stride(0) * Hkv;
+  p.o_stride_s = out.stride(0); p.o_stride_h = out.stride(1); p.o_stride_b = out.stride(0) * std::max<int64_t>(1, total_q);
+  p.B = (int32_t)seqs; p.Sq = (int32_t)max_q; p.Sk = (int32_t)max_k; p.Hq = (int32_t)Hq; p.Hkv = (int32_t)Hkv;
+  p.D = (int32_t)D; p.Dv = (int32_t)Dv;
+  p.causal = win.causal ? 1 : 0;
+  p.q_scale = scalar_of(a[6], "q_scale");
+  p.k_scale = scalar_of(a[7], "k_scale");
+  p.v_scale = scalar_of(a[8], "v_scale");
+  p.softmax_scale = (float)softmax_scale;
+
+  fa4_nvfp4_varlen x = {};
+  x.struct_size = sizeof x;
+  x.num_seqs = (int32_t)seqs;
+  x.cu_seqlens_q = cu_q.data_ptr<int32_t>();
+  x.cu_seqlens_k = cu_k.data_ptr<int32_t>();
+  x.seqused_k = used.defined() ? used.data_ptr<int32_t>() : nullptr;
+  x.total_q = (int32_t)total_q;
+  x.total_k = (int32_t)total_k;
+  x.max_seqlen_q = (int32_t)max_q;
+  x.max_seqlen_k = (int32_t)max_k;
+  x.window_left = win.left;
+  x.window_right = win.right;
+  x.sink = sink.defined() ? sink.data_ptr<float>() : nullptr;
+  x.softcap = is_none(a[20]) ? 0.f : (float)number_of(a[20]);
+  x.cu_seqlens_v = cu_v.defined() ? cu_v.data_ptr<int32_t>() : nullptr;
+  x.total_v = cu_v.defined() ? (int32_t)total_kp : 0;
+  check_rc(fa4_nvfp4_fwd_varlen(&p, &x, stream), "fa4_nvfp4_fwd_varlen");
+  return pair_of(nullptr, out, nullptr, lse);
+}
+
+// ---- the module -----------------------------------------------------------------------------------
+PyObject* choose_decode_splits(PyObject* const* a) {
+  return PyLong_FromLongLong(decode_splits(integer_of(a[0]), integer_of(a[1]), integer_of(a[2]), integer_of(a[3])));
+}
+PyObject* choose_num_splits(PyObject* const* a) {
+  return PyLong_FromLongLong(
+      prefill_splits(integer_of(a[0]), integer_of(a[1]), integer_of(a[2]), integer_of(a[3]), integer_of(a[4])));
+}
+PyObject* window_of(PyObject* const* a) {
+  const Window w = resolve_window(truth_of(a[0]), a[1], a[2]);
+  PyObject *t = w.causal ? Py_True : Py_False, *l = w.left < 0 ? nullptr : PyLong_FromLong(w.left),
+           *r = w.right < 0 ? nullptr : PyLong_FromLong(w.right);
+  PyObject* res = PyTuple_Pack(3, t, l ? l : Py_None, r ? r : Py_None);
+  Py_XDECREF(l);
+  Py_XDECREF(r);
+  return res;
+}
+
+template <PyObject* (*fn)(PyObject* const*), int kArgs>
+PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != kArgs) {
+    PyErr_Format(PyExc_TypeError, "expected %d positional arguments, got %zd", kArgs, n);
+    return nullptr;
+  }
+  HANDLE_TH_ERRORS
+  try {
+    return fn(args);
+  } catch (const PyErrorSet&) {
+    return nullptr;
+  }
+  END_HANDLE_TH_ERRORS
+}
+template <PyObject* (*fn)(PyObject* const*), int kArgs>
+PyMethodDef method(const char* name) {
+  return {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&entry<fn, kArgs>)), METH_FASTCALL, nullptr};
+}
+PyMethodDef methods[] = {method<fwd, 23>("fwd"),
+                         method<varlen_fwd, 22>("varlen_fwd"),
+                         method<choose_decode_splits, 4>("choose_decode_splits"),
+                         method<choose_num_splits, 5>("choose_num_splits"),
+                         method<window_of, 3>("resolve_window"),
+                         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "Native host path of flash_attention_b200.", -1, methods,
+                          nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module_def); }
