@@ -201,25 +201,56 @@ extern "C" int fa4_nvfp4_fwd_varlen(const fa4_nvfp4_params* p, const fa4_nvfp4_v
   return launch_fwd(&q, 1, nullptr, 0, v->window_left, v->window_right, v->sink, v->softcap, cache, cuda_stream);
 }
 
+extern "C" int fa4_nvfp4_sf_tile_jobs(const fa4_nvfp4_sf_job* jobs, int32_t n, void* cuda_stream) {
+  if (jobs == nullptr) return -FA4_E_NULL;
+  if (n < 1 || n > 3) return -FA4_E_SHAPE;
+  SfTileJobs k;
+  k.n = n;
+  int64_t blocks = 0;
+  for (int i = 0; i < n; ++i) {
+    const fa4_nvfp4_sf_job& a = jobs[i];
+    SfTileJob& j = k.job[i];
+    if (!a.src || !a.dst) return -FA4_E_NULL;
+    if (a.n_outer <= 0 || a.n_inner <= 0 || a.rows <= 0 || a.cols <= 0 || a.col_tile_multiple <= 0) return -FA4_E_SHAPE;
+    if (!aligned16(a.dst)) return -FA4_E_ALIGN;
+    j.src = static_cast<const uint8_t*>(a.src);
+    j.dst = static_cast<uint8_t*>(a.dst);
+    j.cu = a.cu_seqlens;
+    j.packed_rows = a.packed_rows ? 1 : 0;
+    j.stride_outer = a.stride_outer;
+    j.stride_inner = a.stride_inner;
+    j.stride_row = a.stride_row;
+    j.n_inner = a.n_inner;
+    j.rows = a.rows;
+    j.cols = a.cols;
+    j.row_tiles = (a.rows + 127) / 128;
+    j.col_tiles = ((a.cols + 3) / 4 + a.col_tile_multiple - 1) / a.col_tile_multiple * a.col_tile_multiple;
+    const int64_t combos = (int64_t)a.n_inner * j.col_tiles;
+    const int64_t warps = (int64_t)a.n_outer * j.row_tiles * ((combos + 7) / 8) * 8;
+    if (combos > 0x7fffffffll || warps > 0x7fffffffll) return -FA4_E_TOO_LARGE;
+    j.combos = (int)combos;
+    j.warps = (uint32_t)warps;
+    j.first_block = (int)blocks;
+    j.div_combo8 = make_fastdiv((uint32_t)((combos + 7) / 8));
+    j.div_row_tiles = make_fastdiv((uint32_t)j.row_tiles);
+    j.div_col_tiles = make_fastdiv((uint32_t)j.col_tiles);
+    blocks += (warps + 7) / 8;
+  }
+  if (blocks > 0x7fffffffll) return -FA4_E_TOO_LARGE;
+  sf_tile_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(k);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : (int)e;
+}
+
 extern "C" int fa4_nvfp4_sf_linear_to_tiled_packed(const void* src, void* dst, const int32_t* cu_seqlens,
                                                    int32_t num_seqs, int32_t n_inner, int32_t max_rows,
                                                    int32_t max_cols, int64_t stride_inner, int64_t stride_row,
                                                    int32_t col_tile_multiple, int32_t packed_rows,
                                                    void* cuda_stream) {
-  if (!src || !dst || !cu_seqlens) return -FA4_E_NULL;
-  if (num_seqs <= 0 || n_inner <= 0 || max_rows <= 0 || max_cols <= 0 || col_tile_multiple <= 0)
-    return -FA4_E_SHAPE;
-  if (!aligned16(dst)) return -FA4_E_ALIGN;
-  const int64_t ct = ((max_cols + 3) / 4 + col_tile_multiple - 1) / col_tile_multiple * col_tile_multiple;
-  const int64_t total = (int64_t)num_seqs * n_inner * ((max_rows + 127) / 128) * ct * 32;
-  int64_t blocks = (total + 255) / 256;
-  const int64_t cap = 148 * 16;
-  if (blocks > cap) blocks = cap;
-  sf_linear_to_tiled_packed_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
-      static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), cu_seqlens, num_seqs, n_inner, max_rows,
-      max_cols, stride_inner, stride_row, col_tile_multiple, packed_rows ? 1 : 0);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : (int)e;
+  if (!cu_seqlens) return -FA4_E_NULL;
+  const fa4_nvfp4_sf_job j = {src, dst, cu_seqlens, num_seqs, n_inner, max_rows, max_cols, 0, stride_inner, stride_row,
+                              col_tile_multiple, packed_rows};
+  return fa4_nvfp4_sf_tile_jobs(&j, 1, cuda_stream);
 }
 
 extern "C" int64_t fa4_nvfp4_splitkv_workspace_bytes(const fa4_nvfp4_params* p, int32_t num_splits) {
@@ -530,20 +561,9 @@ extern "C" int fa4_nvfp4_sf_linear_to_tiled(const void* src, void* dst, int32_t 
                                             int64_t stride_outer, int64_t stride_inner,
                                             int64_t stride_row, int32_t col_tile_multiple,
                                             void* cuda_stream) {
-  if (!src || !dst) return -FA4_E_NULL;
-  if (n_outer <= 0 || n_inner <= 0 || rows <= 0 || cols <= 0 || col_tile_multiple <= 0)
-    return -FA4_E_SHAPE;
-  if (!aligned16(dst)) return -FA4_E_ALIGN;
-  const int64_t ct = ((cols + 3) / 4 + col_tile_multiple - 1) / col_tile_multiple * col_tile_multiple;
-  const int64_t total = (int64_t)n_outer * n_inner * ((rows + 127) / 128) * ct * 32;
-  int64_t blocks = (total + 255) / 256;
-  const int64_t cap = 148 * 16;  // grid-stride beyond a few waves
-  if (blocks > cap) blocks = cap;
-  sf_linear_to_tiled_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
-      static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), n_outer, n_inner, rows, cols,
-      stride_outer, stride_inner, stride_row, col_tile_multiple);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : (int)e;
+  const fa4_nvfp4_sf_job j = {src, dst, nullptr, n_outer, n_inner, rows, cols, stride_outer, stride_inner, stride_row,
+                              col_tile_multiple, 0};
+  return fa4_nvfp4_sf_tile_jobs(&j, 1, cuda_stream);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -719,20 +739,13 @@ extern "C" int fa4_nvfp4_fwd_linear_sf_noalloc(const fa4_nvfp4_params* p, void* 
   uint8_t* v_t = k_t + k_bytes;
 
   const int64_t cq = p->D / 16, cv = skp / 16;
-  // q_sf (B, Sq, Hq, D/16) and k_sf (B, Sk, Hkv, D/16): matrix (b, h) has row stride H * D/16
-  if (int e = fa4_nvfp4_sf_linear_to_tiled(p->q_sf, q_t, p->B, p->Hq, p->Sq, (int)cq,
-                                           (int64_t)p->Sq * p->Hq * cq, cq, (int64_t)p->Hq * cq, 1,
-                                           cuda_stream))
-    return e;
-  if (int e = fa4_nvfp4_sf_linear_to_tiled(p->k_sf, k_t, p->B, p->Hkv, p->Sk, (int)cq,
-                                           (int64_t)p->Sk * p->Hkv * cq, cq, (int64_t)p->Hkv * cq, 1,
-                                           cuda_stream))
-    return e;
+  // q_sf (B, Sq, Hq, D/16) and k_sf (B, Sk, Hkv, D/16): matrix (b, h) has row stride H * D/16;
   // v_sf (B, Hkv, Dv, Sk/16): matrix (b, h) is contiguous
-  if (int e = fa4_nvfp4_sf_linear_to_tiled(p->v_sf, v_t, p->B, p->Hkv, p->Dv, (int)cv,
-                                           (int64_t)p->Hkv * p->Dv * cv, (int64_t)p->Dv * cv, cv, 2,
-                                           cuda_stream))
-    return e;
+  const fa4_nvfp4_sf_job jobs[3] = {
+      {p->q_sf, q_t, nullptr, p->B, p->Hq, p->Sq, (int32_t)cq, p->Sq * p->Hq * cq, cq, p->Hq * cq, 1, 0},
+      {p->k_sf, k_t, nullptr, p->B, p->Hkv, p->Sk, (int32_t)cq, p->Sk * p->Hkv * cq, cq, p->Hkv * cq, 1, 0},
+      {p->v_sf, v_t, nullptr, p->B, p->Hkv, p->Dv, (int32_t)cv, p->Hkv * p->Dv * cv, p->Dv * cv, cv, 2, 0}};
+  if (int e = fa4_nvfp4_sf_tile_jobs(jobs, 3, cuda_stream)) return e;
   fa4_nvfp4_params tiled = *p;
   tiled.q_sf = q_t;
   tiled.k_sf = k_t;

@@ -6,96 +6,89 @@
 namespace fa4 {
 
 // ---------------------------------------------------------------------------------------------
-// Scale factors, linear (rows x cols bytes, row stride given) -> 128 x 4 tiles of 512 bytes.
-// One thread writes one 16-byte row of a tile chunk: destination offset (r % 32) * 16 holds
-// the scales of rows r, r + 32, r + 64, r + 96 (4 bytes each = 4 consecutive columns).
-// Grid: x = 32-row-group index over all tiles of all matrices; HBM-bound byte shuffling,
-// reads are 4-byte per row (the linear layout offers no more), writes are 16-byte coalesced.
+// Scale factors, linear -> 128 x 4 tiles of 512 bytes, up to three tensors (q, k, v) in one launch.
+//
+// A tile chunk holds element (r, c) at (r % 32) * 16 + (r / 32) * 4 + c % 4, so one thread writes one
+// 16-byte piece: rows l, l + 32, l + 64, l + 96 of four neighbouring columns.  A warp takes eight
+// neighbouring column tiles (of one matrix, or of neighbouring heads where their columns follow one
+// another in memory, as in (B, S, H, D/16)) times four neighbouring l: eight 4-byte reads fill a
+// 32-byte sector, four 16-byte writes 64 bytes.  (One warp = 32 values of l read 4 bytes of every
+// sector it touched, byte by byte: the three tensors of B=8, S=2048, H=16, D=192 took 3 x 11 us.)
+//
+// Dense: (n_outer, n_inner) matrices of rows x cols bytes at outer * stride_outer + inner *
+// stride_inner + r * stride_row.
+// Packed batch (cu != null): sequence `outer` owns rows cu[outer] .. cu[outer + 1] (packed_rows) or the
+// columns cu[outer] / 16 .. ceil(cu[outer + 1] / 16) (V: the key axis, sequence starts are multiples of
+// 16 keys), and tiles wholly past its end are left alone: no kernel reads them.
+// dst: (n_outer, n_inner, row_tiles, col_tiles, 512); rows and columns past the end are zero.
 // ---------------------------------------------------------------------------------------------
-__global__ void sf_linear_to_tiled_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
-                                          int n_outer, int n_inner, int rows, int cols,
-                                          int64_t stride_outer, int64_t stride_inner,
-                                          int64_t stride_row, int col_tile_multiple) {
-  const int row_tiles = (rows + 127) / 128;
-  const int col_tiles = ((cols + 3) / 4 + col_tile_multiple - 1) / col_tile_multiple * col_tile_multiple;
-  const int64_t total = (int64_t)n_outer * n_inner * row_tiles * col_tiles * 32;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int l = (int)(idx & 31);
-    int64_t tile = idx >> 5;
-    const int ct = (int)(tile % col_tiles);
-    tile /= col_tiles;
-    const int rt = (int)(tile % row_tiles);
-    tile /= row_tiles;
-    const int mi = (int)(tile % n_inner);
-    const int mo = (int)(tile / n_inner);
-    const uint8_t* m = src + mo * stride_outer + mi * stride_inner;
-    uint32_t w[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int r = rt * 128 + c * 32 + l;
-      uint32_t v = 0;
-      if (r < rows) {
-        const uint8_t* pr = m + (int64_t)r * stride_row + ct * 4;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (ct * 4 + k < cols) v |= (uint32_t)pr[k] << (8 * k);
-        }
-      }
-      w[c] = v;
-    }
-    reinterpret_cast<uint4*>(dst)[idx] = make_uint4(w[0], w[1], w[2], w[3]);
-  }
-}
+struct SfTileJob {
+  const uint8_t* src;
+  uint8_t* dst;
+  const int32_t* cu;
+  int64_t stride_outer, stride_inner, stride_row;
+  int n_inner, rows, cols, row_tiles, col_tiles, packed_rows;
+  int combos;              // n_inner * col_tiles
+  int first_block;         // of this job in the grid
+  uint32_t warps;          // work items: outer x row tile x (eight column tiles) x (four l)
+  FastDiv div_combo8, div_row_tiles, div_col_tiles;
+};
+struct SfTileJobs {
+  SfTileJob job[3];
+  int n;
+};
 
-// ---------------------------------------------------------------------------------------------
-// The same conversion for a PACKED batch (sequences concatenated along the token axis, bounds in
-// cu_seqlens on the device): every sequence gets its own tiles, padded with zeros to the longest
-// sequence, so that a tile never mixes two sequences.
-//   packed_rows = 1: the packed axis is the row axis (q / k scales, (total, H, cols)): matrix
-//       (b, h) has rows cu[b] .. cu[b+1] at src + row * stride_row + h * stride_inner
-//   packed_rows = 0: the packed axis is the column axis (v scales, (H, rows, total / 16)): matrix
-//       (b, h) has `rows` rows at src + h * stride_inner + r * stride_row and the columns
-//       cu[b] / 16 .. ceil(cu[b+1] / 16) (sequence starts are multiples of 16 keys)
-// dst: (num_seqs, n_inner, ceil(max_rows / 128), col tiles of max_cols, 512).
-// ---------------------------------------------------------------------------------------------
-__global__ void sf_linear_to_tiled_packed_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
-                                                 const int32_t* __restrict__ cu, int num_seqs, int n_inner,
-                                                 int max_rows, int max_cols, int64_t stride_inner,
-                                                 int64_t stride_row, int col_tile_multiple, int packed_rows) {
-  const int row_tiles = (max_rows + 127) / 128;
-  const int col_tiles = ((max_cols + 3) / 4 + col_tile_multiple - 1) / col_tile_multiple * col_tile_multiple;
-  const int64_t total = (int64_t)num_seqs * n_inner * row_tiles * col_tiles * 32;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int l = (int)(idx & 31);
-    int64_t tile = idx >> 5;
-    const int ct = (int)(tile % col_tiles);
-    tile /= col_tiles;
-    const int rt = (int)(tile % row_tiles);
-    tile /= row_tiles;
-    const int mi = (int)(tile % n_inner);
-    const int mo = (int)(tile / n_inner);
-    const int c0 = cu[mo], c1 = cu[mo + 1];
-    const int rows = packed_rows ? (c1 - c0) : max_rows;
-    const int cols = packed_rows ? max_cols : ((c1 - c0 + 15) >> 4);
-    const uint8_t* m = src + mi * stride_inner + (packed_rows ? (int64_t)c0 * stride_row : (int64_t)(c0 >> 4));
-    uint32_t w[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int r = rt * 128 + c * 32 + l;
-      uint32_t v = 0;
-      if (r < rows) {
-        const uint8_t* pr = m + (int64_t)r * stride_row + ct * 4;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (ct * 4 + k < cols) v |= (uint32_t)pr[k] << (8 * k);
-        }
-      }
-      w[c] = v;
+__global__ void __launch_bounds__(256)
+sf_tile_kernel(const __grid_constant__ SfTileJobs jobs) {
+  int ji = 0;
+  while (ji + 1 < jobs.n && (int)blockIdx.x >= jobs.job[ji + 1].first_block) ++ji;
+  const SfTileJob& j = jobs.job[ji];
+  const uint32_t w = (blockIdx.x - j.first_block) * 8u + (threadIdx.x >> 5);
+  if (w >= j.warps) return;
+  const int lane = threadIdx.x & 31;
+  const int l = (int)(w & 7u) * 4 + (lane >> 3);
+  const int u = (int)(w >> 3);
+  const int v = fast_div(u, j.div_combo8);
+  const int combo = (u - v * ((j.combos + 7) >> 3)) * 8 + (lane & 7);
+  const int outer = fast_div(v, j.div_row_tiles), rt = v - outer * j.row_tiles;
+  if (combo >= j.combos) return;
+  const int inner = fast_div(combo, j.div_col_tiles), ct = combo - inner * j.col_tiles;
+  const uint8_t* m = j.src + inner * j.stride_inner + 4 * ct;
+  int rows = j.rows, cols = j.cols;
+  if (j.cu != nullptr) {
+    const int c0 = j.cu[outer], len = j.cu[outer + 1] - c0;
+    if (j.packed_rows) {
+      rows = len;
+      m += c0 * j.stride_row;
+      if (rt * 128 >= len) return;
+    } else {
+      cols = (len + 15) >> 4;
+      m += c0 >> 4;
+      if ((ct & ~1) * 64 >= len) return;
     }
-    reinterpret_cast<uint4*>(dst)[idx] = make_uint4(w[0], w[1], w[2], w[3]);
+  } else {
+    m += outer * j.stride_outer;
   }
+  const int left = cols - 4 * ct;                    // columns of this tile that exist
+  const bool word = left >= 4 && ((reinterpret_cast<uintptr_t>(m) | (uintptr_t)j.stride_row) & 3u) == 0;
+  uint32_t out[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int r = rt * 128 + c * 32 + l;
+    const uint8_t* pr = m + r * j.stride_row;
+    out[c] = 0u;
+    if (r < rows) {
+      if (word) {
+        out[c] = *reinterpret_cast<const uint32_t*>(pr);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (k < left) out[c] |= (uint32_t)pr[k] << (8 * k);
+      }
+    }
+  }
+  const int64_t chunk = (((int64_t)outer * j.n_inner + inner) * j.row_tiles + rt) * j.col_tiles + ct;
+  *reinterpret_cast<uint4*>(j.dst + chunk * 512 + l * 16) = make_uint4(out[0], out[1], out[2], out[3]);
 }
 
 // ---------------------------------------------------------------------------------------------

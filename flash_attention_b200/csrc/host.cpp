@@ -209,14 +209,34 @@ at::Tensor sink_of(PyObject* o, int64_t Hq, const at::Device& device) {
   return t.to(device, at::kFloat).contiguous();
 }
 
-// Linear scales (outer, inner, rows, cols; any strides but the last) -> the tiled layout.
-at::Tensor tile_scales(const at::Tensor& sf, int rows_dim, int head_dim, int64_t mult, void* stream) {
-  const int64_t B = sf.size(0), H = sf.size(head_dim), R = sf.size(rows_dim), C = sf.size(3);
-  const int64_t ct = cdiv(cdiv(C, 4), mult) * mult;
-  at::Tensor out = at::empty({B, H, cdiv(R, 128), ct, 512}, sf.options());
-  check_rc(fa4_nvfp4_sf_linear_to_tiled(sf.data_ptr(), out.data_ptr(), (int)B, (int)H, (int)R, (int)C, sf.stride(0),
-                                        sf.stride(head_dim), sf.stride(rows_dim), (int)mult, stream),
-           "fa4_nvfp4_sf_linear_to_tiled");
+// ---- linear scales -> the tiled layout, the three tensors of a call in one launch ------------------
+// One job: (outer, inner) matrices of rows x cols bytes.
+fa4_nvfp4_sf_job sf_job(const at::Tensor& sf, int64_t outer, int64_t inner, int64_t rows, int64_t cols,
+                        int64_t stride_outer, int64_t stride_inner, int64_t stride_row, int64_t mult) {
+  fa4_nvfp4_sf_job j = {};
+  j.src = sf.data_ptr();
+  j.n_outer = (int32_t)outer; j.n_inner = (int32_t)inner; j.rows = (int32_t)rows; j.cols = (int32_t)cols;
+  j.stride_outer = stride_outer; j.stride_inner = stride_inner; j.stride_row = stride_row;
+  j.col_tile_multiple = (int32_t)mult;
+  return j;
+}
+fa4_nvfp4_sf_job sf_job(const at::Tensor& sf, int rows_dim, int head_dim, int64_t mult) {
+  return sf_job(sf, sf.size(0), sf.size(head_dim), sf.size(rows_dim), sf.size(3), sf.stride(0), sf.stride(head_dim),
+                sf.stride(rows_dim), mult);
+}
+// Allocates the tiles of all jobs as one buffer and launches; the tiles of job i are at jobs[i].dst.
+at::Tensor tile_scales(fa4_nvfp4_sf_job (&jobs)[3], const at::Tensor& like, void* stream) {
+  int64_t bytes[3], total = 0;
+  for (int i = 0; i < 3; ++i) {
+    const fa4_nvfp4_sf_job& j = jobs[i];
+    const int64_t ct = cdiv(cdiv(j.cols, 4), j.col_tile_multiple) * j.col_tile_multiple;
+    bytes[i] = (int64_t)j.n_outer * j.n_inner * cdiv(j.rows, 128) * ct * 512;
+    total += bytes[i];
+  }
+  at::Tensor out = at::empty({total}, like.options());
+  uint8_t* at_byte = out.data_ptr<uint8_t>();
+  for (int i = 0; i < 3; at_byte += bytes[i++]) jobs[i].dst = at_byte;
+  check_rc(fa4_nvfp4_sf_tile_jobs(jobs, 3, stream), "fa4_nvfp4_sf_tile_jobs");
   return out;
 }
 
@@ -287,20 +307,28 @@ PyObject* fwd(PyObject* const* a) {
   if (device.index() != c10::cuda::current_device()) guard.set_device(device);
   void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
 
+  at::Tensor tiles;                       // scratch for tiled copies of linear scales
+  const void* sf_ptr[3];
   const char* layout = PyUnicode_Check(a[14]) ? PyUnicode_AsUTF8(a[14]) : nullptr;
   if (layout != nullptr && !strcmp(layout, "linear")) {
     validate(q_sf, "q_sf", {B, Sq, Hq, D / 16}, at::kByte, device);
     validate(k_sf, "k_sf", {B_kv, Sk_kv, Hkv, D / 16}, at::kByte, device);
     validate(v_sf, "v_sf", {B_kv, Hkv, Dv, Sk_pad / 16}, at::kByte, device);
-    q_sf = tile_scales(inner_contiguous(std::move(q_sf)), 1, 2, 1, stream);
-    k_sf = tile_scales(inner_contiguous(std::move(k_sf)), 1, 2, 1, stream);
-    v_sf = tile_scales(inner_contiguous(std::move(v_sf)), 2, 1, 2, stream);
+    q_sf = inner_contiguous(std::move(q_sf));
+    k_sf = inner_contiguous(std::move(k_sf));
+    v_sf = inner_contiguous(std::move(v_sf));
+    fa4_nvfp4_sf_job jobs[3] = {sf_job(q_sf, 1, 2, 1), sf_job(k_sf, 1, 2, 1), sf_job(v_sf, 2, 1, 2)};
+    tiles = tile_scales(jobs, q, stream);
+    for (int i = 0; i < 3; ++i) sf_ptr[i] = jobs[i].dst;
   } else if (layout != nullptr && !strcmp(layout, "tiled")) {
     validate(q_sf, "q_sf", {B, Hq, cdiv(Sq, 128), D / 64, 512}, at::kByte, device);
     validate(k_sf, "k_sf", {B_kv, Hkv, cdiv(Sk_kv, 128), D / 64, 512}, at::kByte, device);
     validate(v_sf, "v_sf", {B_kv, Hkv, cdiv(Dv, 128), 2 * cdiv(Sk_kv, 128), 512}, at::kByte, device);
     FA4_ASSERT(q_sf.is_contiguous() && k_sf.is_contiguous() && v_sf.is_contiguous(),
                "tiled scale factors must be contiguous");
+    sf_ptr[0] = q_sf.data_ptr();
+    sf_ptr[1] = k_sf.data_ptr();
+    sf_ptr[2] = v_sf.data_ptr();
   } else {
     PyErr_Format(PyExc_ValueError, "sf_layout must be 'linear' or 'tiled', got %R", a[14]);
     throw PyErrorSet();
@@ -328,9 +356,9 @@ PyObject* fwd(PyObject* const* a) {
   p.q = q.data_ptr();
   p.k = k.data_ptr();
   p.v = v.data_ptr();
-  p.q_sf = q_sf.data_ptr();
-  p.k_sf = k_sf.data_ptr();
-  p.v_sf = v_sf.data_ptr();
+  p.q_sf = sf_ptr[0];
+  p.k_sf = sf_ptr[1];
+  p.v_sf = sf_ptr[2];
   p.out = out.data_ptr();
   p.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
   p.status = status_word(device);
@@ -397,19 +425,6 @@ PyObject* fwd(PyObject* const* a) {
 }
 
 // ---- flash_attn_varlen_fp4_func -------------------------------------------------------------------
-// Packed scales -> per-sequence tiles, padded to the longest sequence.
-at::Tensor tile_packed(const at::Tensor& sf, const at::Tensor& cu, int64_t seqs, int64_t inner, int64_t max_rows,
-                       int64_t max_cols, int64_t stride_inner, int64_t stride_row, int64_t mult, bool packed_rows,
-                       void* stream) {
-  const int64_t ct = cdiv(cdiv(max_cols, 4), mult) * mult;
-  at::Tensor out = at::empty({seqs, inner, cdiv(max_rows, 128), ct, 512}, sf.options());
-  check_rc(fa4_nvfp4_sf_linear_to_tiled_packed(sf.data_ptr(), out.data_ptr(), cu.data_ptr<int32_t>(), (int)seqs,
-                                               (int)inner, (int)max_rows, (int)max_cols, stride_inner, stride_row,
-                                               (int)mult, packed_rows ? 1 : 0, stream),
-           "fa4_nvfp4_sf_linear_to_tiled_packed");
-  return out;
-}
-
 at::Tensor offsets_of(PyObject* o, const char* name, const at::Device& device) {
   if (is_none(o)) return {};
   const at::Tensor& t = tensor_of(o, name);
@@ -468,17 +483,23 @@ PyObject* varlen_fwd(PyObject* const* a) {
   const Window win = resolve_window(truth_of(a[16]), a[17], a[18]);
   const at::Tensor sink = sink_of(a[19], Hq, device);
 
-  const at::Tensor q_t = tile_packed(q_sf, cu_q, seqs, Hq, max_q, D / 16, D / 16, Hq * (D / 16), 1, true, stream);
-  const at::Tensor k_t = tile_packed(k_sf, cu_k, seqs, Hkv, max_k, D / 16, D / 16, Hkv * (D / 16), 1, true, stream);
-  const at::Tensor v_t = tile_packed(v_sf, cu_v.defined() ? cu_v : cu_k, seqs, Hkv, Dv, cdiv(max_k, 16),
-                                     Dv * (total_kp / 16), total_kp / 16, 2, false, stream);
+  // per-sequence tiles of the packed scales, padded to the longest sequence
+  const int64_t c = D / 16, ckp = total_kp / 16;
+  fa4_nvfp4_sf_job jobs[3] = {sf_job(q_sf, seqs, Hq, max_q, c, 0, c, Hq * c, 1),
+                              sf_job(k_sf, seqs, Hkv, max_k, c, 0, c, Hkv * c, 1),
+                              sf_job(v_sf, seqs, Hkv, Dv, cdiv(max_k, 16), 0, Dv * ckp, ckp, 2)};
+  jobs[0].cu_seqlens = cu_q.data_ptr<int32_t>();
+  jobs[1].cu_seqlens = cu_k.data_ptr<int32_t>();
+  jobs[2].cu_seqlens = (cu_v.defined() ? cu_v : cu_k).data_ptr<int32_t>();
+  jobs[0].packed_rows = jobs[1].packed_rows = 1;
+  const at::Tensor tiles = tile_scales(jobs, q, stream);
   at::Tensor out = at::empty({total_q, Hq, Dv}, q.options().dtype(at::kBFloat16)), lse;
   if (truth_of(a[21])) lse = at::empty({Hq, total_q}, q.options().dtype(at::kFloat));
 
   fa4_nvfp4_params p = {};
   p.struct_size = sizeof p;
   p.q = q.data_ptr(); p.k = k.data_ptr(); p.v = v.data_ptr();
-  p.q_sf = q_t.data_ptr(); p.k_sf = k_t.data_ptr(); p.v_sf = v_t.data_ptr();
+  p.q_sf = jobs[0].dst; p.k_sf = jobs[1].dst; p.v_sf = jobs[2].dst;
   p.out = out.data_ptr();
   p.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
   p.status = status_word(device);

@@ -275,6 +275,24 @@ int fa4_nvfp4_sf_linear_to_tiled(const void* src, void* dst,
                                  void* cuda_stream);
 
 /*
+ * One to three such conversions (the q, k and v scales of one call) in ONE launch.  cu_seqlens
+ * NULL: fa4_nvfp4_sf_linear_to_tiled of the same fields; else fa4_nvfp4_sf_linear_to_tiled_packed
+ * (n_outer = number of sequences, rows / cols = the longest ones, stride_outer unused), whose
+ * tiles past the end of a sequence are left unwritten (the attention kernels do not read them).
+ * No counterpart in the reference (it has no scale factors).
+ */
+typedef struct fa4_nvfp4_sf_job {
+  const void* src;
+  void* dst;                  /* 16-byte aligned */
+  const int32_t* cu_seqlens;  /* device, n_outer + 1, or NULL */
+  int32_t n_outer, n_inner, rows, cols;
+  int64_t stride_outer, stride_inner, stride_row;
+  int32_t col_tile_multiple;
+  int32_t packed_rows;
+} fa4_nvfp4_sf_job;
+int fa4_nvfp4_sf_tile_jobs(const fa4_nvfp4_sf_job* jobs, int32_t n, void* cuda_stream);
+
+/*
  * Version / capability query (host only, never touches a GPU).
  *   what = 0: ABI version; 1: number of supported head dims; 2+i: i-th supported
  *   head dim; 100: default dynamic shared memory per CTA of the WS variant; 101: which of the 8
