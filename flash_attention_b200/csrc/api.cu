@@ -71,7 +71,7 @@ uint32_t next_launch_epoch() {
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Per-kernel launch preparation, done once per (kernel, device) and remembered: the opt-in to
-// `smem_bytes` of dynamic shared memory and -- for the warp-specialised kernels, which re-partition
+// `smem_bytes` of dynamic shared memory, the carve-out (see launch_pdl) and -- for the warp-specialised kernels, which re-partition
 // registers with setmaxnreg -- the check that the build kept the register count the budget in the
 // source assumes (an increase blocks for ever when the CTA was launched with fewer registers per
 // thread; such a build is refused with -FA4_E_BUILD instead of being launched).
@@ -88,6 +88,8 @@ int prepare_kernel(const void* kernel, uint32_t smem_bytes, int expected_regs) {
   if (it != seen.end()) return it->second;
   int rc = 0;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return (int)e;          // not remembered: the caller may retry
   if (expected_regs > 0) {
     cudaFuncAttributes attr;
@@ -105,6 +107,26 @@ int ensure_smem(Kernel kernel, uint32_t bytes) {
 template <class Kernel>
 int ensure_kernel(Kernel kernel, uint32_t bytes, int expected_regs) {
   return prepare_kernel(reinterpret_cast<const void*>(kernel), bytes, expected_regs);
+}
+
+// Launch as a programmatic dependent of whatever precedes it in the stream (see pdl_wait in
+// ptx.cuh): launch latency and set-up overlap the end of the kernel before.
+// Every kernel asks for the largest shared-memory carve-out, also those that use none: an SM changes
+// its carve-out only while it is empty, which would take the overlap away again.
+template <class... KArgs, class... Args>
+int launch_pdl(void (*kernel)(KArgs...), dim3 grid, unsigned threads, uint32_t smem, cudaStream_t stream, Args&&... args) {
+  if (int e = prepare_kernel(reinterpret_cast<const void*>(kernel), smem, 0)) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 }  // namespace
@@ -237,9 +259,7 @@ extern "C" int fa4_nvfp4_sf_tile_jobs(const fa4_nvfp4_sf_job* jobs, int32_t n, v
     blocks += (warps + 7) / 8;
   }
   if (blocks > 0x7fffffffll) return -FA4_E_TOO_LARGE;
-  sf_tile_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(k);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : (int)e;
+  return launch_pdl(sf_tile_kernel, dim3((unsigned)blocks), 256, 0, static_cast<cudaStream_t>(cuda_stream), k);
 }
 
 extern "C" int fa4_nvfp4_sf_linear_to_tiled_packed(const void* src, void* dst, const int32_t* cu_seqlens,
@@ -459,10 +479,8 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     dp.o_partial = kp.o_partial;
     dp.lse_partial = kp.lse_partial;
     auto launch_dec = [&](auto kernel, uint32_t smem) -> int {
-      if (int e = ensure_smem(kernel, smem)) return e;
-      kernel<<<dim3((unsigned)num_splits, (unsigned)p->Hkv, (unsigned)p->B), dec::kThreads, smem, stream>>>(
-          tm_k, tm_v, kp, dp);
-      return 0;
+      return launch_pdl(kernel, dim3((unsigned)num_splits, (unsigned)p->Hkv, (unsigned)p->B), dec::kThreads, smem, stream,
+                        tm_k, tm_v, kp, dp);
     };
     const int rc = dec_rows <= 4    ? launch_dec(attn_decode_kernel<4>, dec::kSmemRequest)
                    : dec_rows <= 8  ? launch_dec(attn_decode_kernel<8>, dec::kSmemRequest)
@@ -487,15 +505,13 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     }
     auto launch = [&](auto kernel) -> int {
       if (int e = ensure_kernel(kernel, ws::kSmemRequest, ws::kRegsLaunch)) return e;
-      kernel<<<grid, ws::kThreads, ws::kSmemRequest, stream>>>(tm_q, tm_k, tm_v, tm_o, kp);
-      return 0;
+      return launch_pdl(kernel, dim3(grid), ws::kThreads, ws::kSmemRequest, stream, tm_q, tm_k, tm_v, tm_o, kp);
     };
     int rc;
     if (variant == FA4_VARIANT_WS64) {
       auto launch64 = [&](auto kernel) -> int {
         if (int e = ensure_kernel(kernel, ws64::kSmemRequest, ws64::kRegsLaunch)) return e;
-        kernel<<<grid, ws64::kThreads, ws64::kSmemRequest, stream>>>(tm_q, tm_k, tm_v, tm_o, kp);
-        return 0;
+        return launch_pdl(kernel, dim3(grid), ws64::kThreads, ws64::kSmemRequest, stream, tm_q, tm_k, tm_v, tm_o, kp);
       };
       if (general && local) {   // window (with or without sink / softcap / cache view)
         rc = p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, true>)
@@ -522,37 +538,14 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     }
     if (rc != 0) return rc;
   }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return (int)e;
   if (num_splits > 1 || decode) {
     const int64_t items = (int64_t)p->B * p->Sq * p->Hq * (p->Dv / 4);
     int64_t blocks = (items + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    if (decode) {
-      // programmatic dependent launch: the launch latency of the combine kernel overlaps the
-      // decode kernel (the combine CTAs wait on griddepcontrol.wait)
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)blocks);
-      cfg.blockDim = dim3(256);
-      cfg.dynamicSmemBytes = 0;
-      cfg.stream = stream;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[0].val.programmaticStreamSerializationAllowed = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      const cudaError_t le = cudaLaunchKernelEx(
-          &cfg, combine_splits_kernel, (const float*)kp.o_partial, (const float*)kp.lse_partial, kp.out, kp.lse,
-          num_splits, p->B, p->Sq, p->Hq, p->Dv, kp.o_stride_b, kp.o_stride_s, kp.o_stride_h);
-      if (le != cudaSuccess) return (int)le;
-    } else {
-      combine_splits_kernel<<<(unsigned)blocks, 256, 0, stream>>>(
-          kp.o_partial, kp.lse_partial, kp.out, kp.lse, num_splits, p->B, p->Sq, p->Hq, p->Dv,
-          kp.o_stride_b, kp.o_stride_s, kp.o_stride_h);
-    }
-    e = cudaGetLastError();
+    return launch_pdl(combine_splits_kernel, dim3((unsigned)blocks), 256, 0, stream, kp.o_partial, kp.lse_partial, kp.out,
+                      kp.lse, num_splits, p->B, p->Sq, p->Hq, p->Dv, kp.o_stride_b, kp.o_stride_s, kp.o_stride_h);
   }
-  return e == cudaSuccess ? 0 : (int)e;
+  return 0;
 }
 }  // namespace
 
@@ -584,11 +577,9 @@ extern "C" int fa4_nvfp4_amax_bf16(const void* x, int64_t n0, int32_t n1, int32_
   if (rows_per_group > rows) rows_per_group = rows;
   const int groups = (rows + rows_per_group - 1) / rows_per_group;
   const int grid = groups < 148 * 8 ? groups : 148 * 8;
-  amax_bf16_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+  return launch_pdl(amax_bf16_kernel, dim3(grid), 256, 0, static_cast<cudaStream_t>(cuda_stream),
       static_cast<const __nv_bfloat16*>(x), n1, n2, inner / 8, s0, s1, s2, rows, rows_per_group,
       make_fastdiv(per_row), make_fastdiv(inner / 8), make_fastdiv(n1), amax);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : (int)e;
 }
 
 extern "C" int fa4_nvfp4_quantize_qk_bf16(const void* x, int32_t B, int32_t S, int32_t H, int32_t D,
@@ -610,13 +601,11 @@ extern "C" int fa4_nvfp4_quantize_qk_bf16(const void* x, int32_t B, int32_t S, i
   int rows_per_group = per_row >= 2048 ? 1 : 2048 / per_row;
   const int64_t groups = (rows64 + rows_per_group - 1) / rows_per_group;
   if (groups > 0x7fffffffll) return -FA4_E_TOO_LARGE;
-  quantize_rows_kernel<<<(unsigned)groups, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+  return launch_pdl(quantize_rows_kernel, dim3((unsigned)groups), 256, 0, static_cast<cudaStream_t>(cuda_stream),
       static_cast<const __nv_bfloat16*>(x), B, S, H, D, stride_b, stride_s, stride_h, amax,
       static_cast<uint8_t*>(packed), static_cast<uint8_t*>(sf_linear),
       static_cast<uint8_t*>(sf_tiled), scale_out, rows_per_group, make_fastdiv(per_row),
       make_fastdiv(D / 16), make_fastdiv(((S + 127) / 128) * 128));
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : (int)e;
 }
 
 extern "C" int fa4_nvfp4_quantize_v_bf16(const void* x, int32_t B, int32_t Sk, int32_t H, int32_t Dv,
@@ -631,12 +620,10 @@ extern "C" int fa4_nvfp4_quantize_v_bf16(const void* x, int32_t B, int32_t Sk, i
       (sf_tiled && !aligned16(sf_tiled)))
     return -FA4_E_ALIGN;
   const dim3 grid((Sk + 127) / 128, (Dv + 127) / 128, B * H);
-  quantize_v_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
+  return launch_pdl(quantize_v_kernel, grid, 256, 0, static_cast<cudaStream_t>(cuda_stream),
       static_cast<const __nv_bfloat16*>(x), B, Sk, H, Dv, stride_b, stride_s, stride_h, amax,
       static_cast<uint8_t*>(packed), static_cast<uint8_t*>(sf_linear),
       static_cast<uint8_t*>(sf_tiled), scale_out);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : (int)e;
 }
 
 extern "C" int fa4_nvfp4_debug_qk_tile(const void* q, const void* k, const void* q_sf,

@@ -224,9 +224,34 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   const WaitCtx wc{s_abort, p.status, p.budget_ns, p.epoch};
   const int R = p.Sq * p.group;  // live query rows (<= kR)
 
-  // The query rows and their scale words go to registers first thing: their latency (a trip to
-  // HBM while every CTA of the grid starts its K / V stream) then overlaps the set-up below
-  // instead of following it.  Threads 0-127: row tid / 4, 16-byte chunk tid % 4; threads 0-63
+  if (tid == 0) {
+    *s_abort = 0u;
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(bars.at(Bars::kKFull + s), 1);
+      mbar_init(bars.at(Bars::kVFull + s), 1);
+      mbar_init(bars.at(Bars::kKFree + s), 1);
+      mbar_init(bars.at(Bars::kVFree + s), 1);
+      mbar_init(bars.at(Bars::kSFull + s), 1);
+      mbar_init(bars.at(Bars::kSFree + s), 128);
+      mbar_init(bars.at(Bars::kPFull + s), 128);
+      mbar_init(bars.at(Bars::kPvDone + s), 1);
+    }
+    mbar_init(bars.at(Bars::kQReady), 128);
+    mbar_init(bars.at(Bars::kSync), 128);
+    mbar_init(bars.at(Bars::kDrain), 1);
+    fence_barrier_init();
+  }
+  if (warp == 4 && lane == 0) tma_prefetch_desc(&tm_k);
+  if (warp == 6 && lane == 0) tma_prefetch_desc(&tm_v);
+  if (warp == 5) {
+    tmem_alloc(base + kOffMisc, TM::kCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  pdl_wait();
+  // The query rows and their scale words go to registers before anything else is read: their
+  // latency (a trip to HBM while every CTA of the grid starts its K / V stream) then overlaps the
+  // rendezvous below.  Threads 0-127: row tid / 4, 16-byte chunk tid % 4; threads 0-63
   // also: row tid / 2, the scale word of 64-element step tid % 2.
   uint4 q_pref = make_uint4(0u, 0u, 0u, 0u);
   uint32_t qsf_pref = 0u;
@@ -260,36 +285,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   const int i0 = split * per < n_total ? split * per : n_total;
   const int i1 = i0 + per < n_total ? i0 + per : n_total;
   const int n = i1 - i0;
-
-  if (tid == 0) {
-    *s_abort = 0u;
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(bars.at(Bars::kKFull + s), 1);
-      mbar_init(bars.at(Bars::kVFull + s), 1);
-      mbar_init(bars.at(Bars::kKFree + s), 1);
-      mbar_init(bars.at(Bars::kVFree + s), 1);
-      mbar_init(bars.at(Bars::kSFull + s), 1);
-      mbar_init(bars.at(Bars::kSFree + s), 128);
-      mbar_init(bars.at(Bars::kPFull + s), 128);
-      mbar_init(bars.at(Bars::kPvDone + s), 1);
-    }
-    mbar_init(bars.at(Bars::kQReady), 128);
-    mbar_init(bars.at(Bars::kSync), 128);
-    mbar_init(bars.at(Bars::kDrain), 1);
-    fence_barrier_init();
-  }
-  if (warp == 4 && lane == 0) tma_prefetch_desc(&tm_k);
-  if (warp == 6 && lane == 0) tma_prefetch_desc(&tm_v);
-  if (warp == 5) {
-    tmem_alloc(base + kOffMisc, TM::kCols);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  // the combine kernel is launched as a programmatic dependent: let its CTAs be scheduled while
-  // this grid still runs (they wait for its completion before they read the partials)
-  asm volatile("griddepcontrol.launch_dependents;");
+  pdl_trigger();
   const uint32_t tmem = *tmem_slot;
   constexpr uint32_t idesc = make_idesc_nvf4(128, kN);
   bool ok = true;

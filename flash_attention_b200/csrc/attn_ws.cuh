@@ -343,8 +343,10 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_relinquish();
   }
   tc_fence_before_sync();
+  pdl_wait();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_trigger();
   const uint32_t tmem = *tmem_slot;
   static_assert(kD == 128 || kD == 64, "head dimensions built: 128 and 64");
   constexpr uint32_t idesc_qk = make_idesc_nvf4(128, 128);

@@ -207,8 +207,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_relinquish();
   }
   tc_fence_before_sync();
+  pdl_wait();
   __syncthreads();
   tc_fence_after_sync();
+  pdl_trigger();
   const uint32_t tmem = *tmem_slot;
   static_assert(kD == 128 || kD == 64 || kD == 192, "head dimensions built: 128, 64 and (192, 128)");
   constexpr int kDv = kD == 192 ? 128 : kD;            // head dim of V and O

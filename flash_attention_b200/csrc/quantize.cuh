@@ -153,6 +153,7 @@ amax_bf16_kernel(const __nv_bfloat16* __restrict__ x, int n1, int n2, int inner8
                  int64_t s1, int64_t s2, int rows, int rows_per_group, FastDiv div_per_row,
                  FastDiv div_inner8, FastDiv div_n1, float* __restrict__ amax) {
   __shared__ float warp_max[8];
+  pdl_wait();
   const int per_row = n2 * inner8;
   const int per_group = rows_per_group * per_row;
   const int groups = (rows + rows_per_group - 1) / rows_per_group;
@@ -206,6 +207,7 @@ quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int B, int S, int H, i
                      uint8_t* __restrict__ packed, uint8_t* __restrict__ sf_lin,
                      uint8_t* __restrict__ sf_tiled, float* __restrict__ scale_out,
                      int rows_per_group, FastDiv div_per_row, FastDiv div_nb, FastDiv div_spad) {
+  pdl_wait();
   const TensorScale g = make_tensor_scale(*amax);
   if (scale_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *scale_out = g.g;
   const int nb = D / 16, ct = D / 64;
@@ -287,6 +289,7 @@ quantize_v_kernel(const __nv_bfloat16* __restrict__ x, int B, int Sk, int H, int
                   uint8_t* __restrict__ packed, uint8_t* __restrict__ sf_lin,
                   uint8_t* __restrict__ sf_tiled, float* __restrict__ scale_out) {
   __shared__ __align__(16) uint8_t tile[128 * 256];  // [key][16 chunks of 16 B], chunk ^ (key/16)
+  pdl_wait();
   const TensorScale g = make_tensor_scale(*amax);
   if (scale_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 &&
       threadIdx.x == 0)
