@@ -163,14 +163,15 @@ struct CacheView {
 };
 int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint64_t workspace_bytes,
                int win_left, int win_right, const float* sink, float softcap, const CacheView& cache,
-               void* cuda_stream);
+               void* cuda_stream, const float* const* scales = nullptr);
 }  // namespace
 
 extern "C" int fa4_nvfp4_fwd(const fa4_nvfp4_params* p, void* cuda_stream) {
   return launch_fwd(p, 1, nullptr, 0, -1, -1, nullptr, 0.f, CacheView{}, cuda_stream);
 }
 
-extern "C" int fa4_nvfp4_fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, void* cuda_stream) {
+namespace {
+int fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, const float* const* scales, void* cuda_stream) {
   if (x == nullptr) return -FA4_E_NULL;
   if (x->struct_size != sizeof(fa4_nvfp4_ext)) return -FA4_E_STRUCT;
   const int splits = x->num_splits == 0 ? 1 : x->num_splits;
@@ -189,7 +190,21 @@ extern "C" int fa4_nvfp4_fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* 
     cache.num_pages = x->num_pages;
   }
   return launch_fwd(p, splits, x->workspace, x->workspace_bytes, x->window_left, x->window_right,
-                    x->sink, x->softcap, cache, cuda_stream);
+                    x->sink, x->softcap, cache, cuda_stream, scales);
+}
+}  // namespace
+
+extern "C" int fa4_nvfp4_fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, void* cuda_stream) {
+  return fwd_ex(p, x, nullptr, cuda_stream);
+}
+
+extern "C" int fa4_nvfp4_fwd_device_scales(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, const float* q_scale,
+                                           const float* k_scale, const float* v_scale, void* cuda_stream) {
+  if (p == nullptr || !q_scale || !k_scale || !v_scale) return -FA4_E_NULL;
+  fa4_nvfp4_params q = *p;
+  q.q_scale = q.k_scale = q.v_scale = 1.f;      // not read
+  const float* const scales[3] = {q_scale, k_scale, v_scale};
+  return fwd_ex(&q, x, scales, cuda_stream);
 }
 
 extern "C" int fa4_nvfp4_fwd_varlen(const fa4_nvfp4_params* p, const fa4_nvfp4_varlen* v, void* cuda_stream) {
@@ -366,7 +381,7 @@ int validate_fwd(const fa4_nvfp4_params* p, int num_splits, const void* workspac
 
 int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint64_t workspace_bytes,
                int win_left, int win_right, const float* sink, float softcap, const CacheView& cache,
-               void* cuda_stream) {
+               void* cuda_stream, const float* const* scales) {
   FwdPlan plan;
   if (int e = validate_fwd(p, num_splits, workspace, workspace_bytes, win_left, win_right, sink, softcap, cache,
                            false, &plan))
@@ -458,6 +473,11 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     kp.sl2 = softcap * 1.4426950408889634f;
   }
   kp.out_scale = p->v_scale;
+  kp.q_scale = scales ? scales[0] : nullptr;
+  kp.k_scale = scales ? scales[1] : nullptr;
+  kp.v_scale = scales ? scales[2] : nullptr;
+  kp.softmax_scale = p->softmax_scale;
+  kp.softcap = softcap;
   kp.budget_ns = p->wait_budget_ns ? p->wait_budget_ns : kDefaultBudgetNs;
   kp.num_splits = num_splits;
   kp.Dv = p->Dv;
@@ -562,68 +582,175 @@ extern "C" int fa4_nvfp4_sf_linear_to_tiled(const void* src, void* dst, int32_t 
 // ---------------------------------------------------------------------------------------------
 // Fused NVFP4 quantiser (bf16 operands in the reference layout -> what fa4_nvfp4_fwd reads)
 // ---------------------------------------------------------------------------------------------
+namespace {
+constexpr int64_t kMaxQuantUnits = 0x7fffffffll;
+
+// Number of CTAs of a tensor that has `units` of `total` units of work, at most one per `per_cta` units.
+int share_of(int64_t ctas, int64_t units, int64_t total, int64_t per_cta) {
+  const int64_t want = (ctas * units + total - 1) / total, most = (units + per_cta - 1) / per_cta;
+  return (int)(want < 1 ? 1 : (want < most ? want : most));
+}
+
+// Shape, strides and alignment of one tensor; the fields of the amax pass.
+int describe_tensor(QuantJob* j, const void* x, int64_t B, int64_t S, int64_t H, int64_t D, int64_t sb, int64_t ss,
+                    int64_t sh) {
+  if (!x) return -FA4_E_NULL;
+  if (B <= 0 || S <= 0 || H <= 0 || D <= 0 || D % 8 != 0) return -FA4_E_SHAPE;
+  if (sb % 8 != 0 || ss % 8 != 0 || sh % 8 != 0) return -FA4_E_STRIDE;
+  if (!aligned16(x)) return -FA4_E_ALIGN;
+  if (B > 0x7fffffffll || S > 0x7fffffffll || H > 0x7fffffffll || D > 0x7fffffffll) return -FA4_E_TOO_LARGE;
+  *j = QuantJob{};
+  j->x = static_cast<const __nv_bfloat16*>(x);
+  j->sb = sb; j->ss = ss; j->sh = sh;
+  j->B = (int)B; j->S = (int)S; j->H = (int)H; j->D = (int)D;
+  j->wide = ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(2 * (sb | ss | sh | D))) & 31u) == 0;
+  // the tensor as runs of contiguous elements, merged as far as the strides allow
+  int64_t inner = D, n0 = B, n1 = S, n2 = H, r0 = sb, r1 = ss, r2 = sh;
+  auto merge = [&](int64_t n, int64_t stride) { return n == 1 || stride == inner; };
+  if (merge(H, sh)) {
+    inner *= H; n0 = 1; n1 = B; n2 = S; r0 = 0; r1 = sb; r2 = ss;
+    if (merge(S, ss)) {
+      inner *= S; n1 = 1; n2 = B; r1 = 0; r2 = sb;
+      if (merge(B, sb)) { inner *= B; n2 = 1; r2 = 0; }
+    }
+  }
+  j->unit = inner % 16 == 0 ? 16 : 8;
+  const int64_t units = n0 * n1 * n2 * (inner / j->unit);
+  if (units > kMaxQuantUnits) return -FA4_E_TOO_LARGE;
+  j->units = (uint32_t)units;
+  j->inner_units = (int)(inner / j->unit);
+  j->n1 = (int)n1; j->n2 = (int)n2;
+  j->r0 = r0; j->r1 = r1; j->r2 = r2;
+  j->div_inner = make_fastdiv((uint32_t)j->inner_units);
+  j->div_n2 = make_fastdiv((uint32_t)n2);
+  j->div_n1 = make_fastdiv((uint32_t)n1);
+  return 0;
+}
+
+// The fields of the quantise pass.
+int describe_outputs(QuantJob* j, bool is_v, int64_t s_out, void* packed, void* sf_linear, void* sf_tiled, float* scale_out) {
+  if (!packed) return -FA4_E_NULL;
+  if (!aligned16(packed) || (sf_linear && !aligned16(sf_linear)) || (sf_tiled && !aligned16(sf_tiled))) return -FA4_E_ALIGN;
+  j->is_v = is_v;
+  j->packed = static_cast<uint8_t*>(packed);
+  j->lin = static_cast<uint8_t*>(sf_linear);
+  j->tiled = static_cast<uint8_t*>(sf_tiled);
+  j->scale_out = scale_out;
+  int64_t items;
+  if (is_v) {
+    if (s_out < j->S || s_out % 16 != 0 || s_out > 0x7fffffffll) return -FA4_E_SHAPE;
+    j->s_out = (int)s_out;
+    j->rt = (int)((s_out + 127) / 128);
+    items = (int64_t)j->B * j->H * ((j->D + 127) / 128) * j->rt;
+    j->div_h = make_fastdiv((uint32_t)j->H);
+  } else {
+    if (j->D % 64 != 0) return -FA4_E_SHAPE;
+    j->nb = j->H * (j->D / 16);
+    j->rt = (j->S + 127) / 128;
+    items = (int64_t)j->B * j->rt * 32 * j->nb;
+    // four rows per item once that gives every SM its CTAs
+    j->single = items < 148 * kQuantizeCtas * 256;
+    if (j->single) items *= 4;
+    j->div_nb = make_fastdiv((uint32_t)j->nb);
+    j->div_h = make_fastdiv((uint32_t)(j->D / 16));
+  }
+  if (items > kMaxQuantUnits) return -FA4_E_TOO_LARGE;
+  j->items = (uint32_t)items;
+  j->div_rt = make_fastdiv((uint32_t)j->rt);
+  return 0;
+}
+
+int launch_amax(QuantJobs& q, cudaStream_t stream) {
+  int64_t total = 0;
+  int blocks = 0;
+  for (int i = 0; i < q.n; ++i) total += q.job[i].units;
+  for (int i = 0; i < q.n; ++i) {
+    QuantJob& j = q.job[i];
+    j.amax_block0 = blocks;
+    j.amax_blocks = share_of(148 * kAmaxCtas, j.units, total, kAmaxThreads);
+    j.parts = q.parts + blocks;
+    j.num_parts = j.amax_blocks;
+    blocks += j.amax_blocks;
+  }
+  return launch_pdl(amax_kernel, dim3(blocks), kAmaxThreads, 0, stream, q);
+}
+
+int launch_quantize(QuantJobs& q, cudaStream_t stream) {
+  // bytes, V's weighted by what its transpose costs more
+  auto weight = [](const QuantJob& j) { return (int64_t)j.units * j.unit * (j.is_v ? kQuantizeVWeight : 16); };
+  int64_t total = 0, blocks = 0;
+  for (int i = 0; i < q.n; ++i) total += weight(q.job[i]);
+  for (int i = 0; i < q.n; ++i) {
+    QuantJob& j = q.job[i];
+    const int64_t most = j.is_v ? j.items : ((int64_t)j.items + 255) / 256;
+    int64_t ctas = 148 * kQuantizeCtas * weight(j) / total;
+    if (ctas < 1) ctas = 1;
+    if (ctas > most || j.single) ctas = most;
+    j.block0 = (int)blocks;
+    j.blocks = (int)ctas;
+    blocks += ctas;
+  }
+  return launch_pdl(quantize_kernel, dim3((unsigned)blocks), 256, 0, stream, q);
+}
+}  // namespace
+
+extern "C" int fa4_nvfp4_quantize_jobs_bf16(const fa4_nvfp4_quant_job* jobs, int32_t n, float* scratch, void* cuda_stream) {
+  if (!jobs || !scratch) return -FA4_E_NULL;
+  if (n < 1 || n > 3) return -FA4_E_SHAPE;
+  QuantJobs q{};
+  q.n = n;
+  q.parts = scratch;
+  for (int i = 0; i < n; ++i) {
+    const fa4_nvfp4_quant_job& a = jobs[i];
+    if (int e = describe_tensor(&q.job[i], a.x, a.B, a.S, a.H, a.D, a.stride_b, a.stride_s, a.stride_h)) return e;
+    if (int e = describe_outputs(&q.job[i], a.is_v != 0, a.S_out, a.packed, a.sf_linear, a.sf_tiled, a.scale_out)) return e;
+    q.job[i].scale_host = a.scale_host;
+  }
+  const cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+  if (int e = launch_amax(q, stream)) return e;
+  return launch_quantize(q, stream);
+}
+
 extern "C" int fa4_nvfp4_amax_bf16(const void* x, int64_t n0, int32_t n1, int32_t n2, int32_t inner,
                                    int64_t s0, int64_t s1, int64_t s2, float* amax,
                                    void* cuda_stream) {
-  if (!x || !amax) return -FA4_E_NULL;
-  if (n0 <= 0 || n1 <= 0 || n2 <= 0 || inner <= 0 || inner % 8 != 0) return -FA4_E_SHAPE;
-  if (s0 % 8 != 0 || s1 % 8 != 0 || s2 % 8 != 0) return -FA4_E_STRIDE;
-  if (!aligned16(x)) return -FA4_E_ALIGN;
-  if (n0 * n1 > 0x7fffffffll || (int64_t)n2 * (inner / 8) > (1 << 24)) return -FA4_E_TOO_LARGE;
-  const int rows = (int)(n0 * n1);
-  const int per_row = n2 * (inner / 8);
-  // a group of rows gives every thread about 8 independent 16-byte loads
-  int rows_per_group = (256 * 8 + per_row - 1) / per_row;
-  if (rows_per_group > rows) rows_per_group = rows;
-  const int groups = (rows + rows_per_group - 1) / rows_per_group;
-  const int grid = groups < 148 * 8 ? groups : 148 * 8;
-  return launch_pdl(amax_bf16_kernel, dim3(grid), 256, 0, static_cast<cudaStream_t>(cuda_stream),
-      static_cast<const __nv_bfloat16*>(x), n1, n2, inner / 8, s0, s1, s2, rows, rows_per_group,
-      make_fastdiv(per_row), make_fastdiv(inner / 8), make_fastdiv(n1), amax);
+  if (!amax) return -FA4_E_NULL;
+  QuantJobs q{};
+  q.n = 1;
+  if (int e = describe_tensor(&q.job[0], x, n0, n1, n2, inner, s0, s1, s2)) return e;
+  q.job[0].amax_out = amax;
+  return launch_amax(q, static_cast<cudaStream_t>(cuda_stream));
 }
+
+namespace {
+int quantize_with_amax(const void* x, bool is_v, int32_t B, int32_t S, int32_t H, int32_t D, int64_t sb, int64_t ss,
+                       int64_t sh, const float* amax, void* packed, void* sf_linear, void* sf_tiled, float* scale_out,
+                       void* cuda_stream) {
+  if (!amax) return -FA4_E_NULL;
+  QuantJobs q{};
+  q.n = 1;
+  if (int e = describe_tensor(&q.job[0], x, B, S, H, D, sb, ss, sh)) return e;
+  if (int e = describe_outputs(&q.job[0], is_v, S, packed, sf_linear, sf_tiled, scale_out)) return e;
+  q.job[0].parts = amax;
+  q.job[0].num_parts = 1;
+  return launch_quantize(q, static_cast<cudaStream_t>(cuda_stream));
+}
+}  // namespace
 
 extern "C" int fa4_nvfp4_quantize_qk_bf16(const void* x, int32_t B, int32_t S, int32_t H, int32_t D,
                                           int64_t stride_b, int64_t stride_s, int64_t stride_h,
                                           const float* amax, void* packed, void* sf_linear,
                                           void* sf_tiled, float* scale_out, void* cuda_stream) {
-  if (!x || !amax || !packed) return -FA4_E_NULL;
-  if (B <= 0 || S <= 0 || H <= 0 || D <= 0 || D % 64 != 0) return -FA4_E_SHAPE;
-  if (stride_b % 8 != 0 || stride_s % 8 != 0 || stride_h % 8 != 0) return -FA4_E_STRIDE;
-  if (!aligned16(x) || !aligned16(packed) || (sf_linear && !aligned16(sf_linear)) ||
-      (sf_tiled && !aligned16(sf_tiled)))
-    return -FA4_E_ALIGN;
-  const int64_t rows64 = (int64_t)B * ((S + 127) / 128) * 128;
-  const int64_t per_row64 = (int64_t)H * (D / 16);
-  if (rows64 > 0x7fffffffll || per_row64 > (1 << 24)) return -FA4_E_TOO_LARGE;
-  const int per_row = (int)per_row64;
-  // about eight blocks of 16 per thread: the per-thread set-up (tensor scale and its reciprocal,
-  // index constants) is paid once per CTA, and a CTA streams 64 KB
-  int rows_per_group = per_row >= 2048 ? 1 : 2048 / per_row;
-  const int64_t groups = (rows64 + rows_per_group - 1) / rows_per_group;
-  if (groups > 0x7fffffffll) return -FA4_E_TOO_LARGE;
-  return launch_pdl(quantize_rows_kernel, dim3((unsigned)groups), 256, 0, static_cast<cudaStream_t>(cuda_stream),
-      static_cast<const __nv_bfloat16*>(x), B, S, H, D, stride_b, stride_s, stride_h, amax,
-      static_cast<uint8_t*>(packed), static_cast<uint8_t*>(sf_linear),
-      static_cast<uint8_t*>(sf_tiled), scale_out, rows_per_group, make_fastdiv(per_row),
-      make_fastdiv(D / 16), make_fastdiv(((S + 127) / 128) * 128));
+  return quantize_with_amax(x, false, B, S, H, D, stride_b, stride_s, stride_h, amax, packed, sf_linear, sf_tiled,
+                            scale_out, cuda_stream);
 }
 
 extern "C" int fa4_nvfp4_quantize_v_bf16(const void* x, int32_t B, int32_t Sk, int32_t H, int32_t Dv,
                                          int64_t stride_b, int64_t stride_s, int64_t stride_h,
                                          const float* amax, void* packed, void* sf_linear,
                                          void* sf_tiled, float* scale_out, void* cuda_stream) {
-  if (!x || !amax || !packed) return -FA4_E_NULL;
-  if (B <= 0 || Sk <= 0 || H <= 0 || Dv <= 0 || Sk % 16 != 0 || Dv % 8 != 0) return -FA4_E_SHAPE;
-  if ((int64_t)B * H > 65535) return -FA4_E_TOO_LARGE;
-  if (stride_b % 8 != 0 || stride_s % 8 != 0 || stride_h % 8 != 0) return -FA4_E_STRIDE;
-  if (!aligned16(x) || !aligned16(packed) || (sf_linear && !aligned16(sf_linear)) ||
-      (sf_tiled && !aligned16(sf_tiled)))
-    return -FA4_E_ALIGN;
-  const dim3 grid((Sk + 127) / 128, (Dv + 127) / 128, B * H);
-  return launch_pdl(quantize_v_kernel, grid, 256, 0, static_cast<cudaStream_t>(cuda_stream),
-      static_cast<const __nv_bfloat16*>(x), B, Sk, H, Dv, stride_b, stride_s, stride_h, amax,
-      static_cast<uint8_t*>(packed), static_cast<uint8_t*>(sf_linear),
-      static_cast<uint8_t*>(sf_tiled), scale_out);
+  return quantize_with_amax(x, true, B, Sk, H, Dv, stride_b, stride_s, stride_h, amax, packed, sf_linear, sf_tiled,
+                            scale_out, cuda_stream);
 }
 
 extern "C" int fa4_nvfp4_debug_qk_tile(const void* q, const void* k, const void* q_sf,

@@ -45,6 +45,12 @@ struct KernelParams {
   int causal;
   float sl2;        // softmax_scale * q_scale * k_scale * log2(e)
   float out_scale;  // v_scale
+  // per-tensor scales of q, k, v on the device (all three, or null: then the host folded them into
+  // sl2, out_scale and softcap_c1); see score_scales()
+  const float* q_scale;
+  const float* k_scale;
+  const float* v_scale;
+  float softmax_scale, softcap;
   uint64_t budget_ns;
   uint32_t epoch;   // launch epoch (0..255): a failure in the status word stops only the launch that recorded it
   // split-KV (num_splits > 1): every (tile, split) pair is a work item that visits a contiguous
@@ -88,6 +94,24 @@ struct KernelParams {
   const int32_t* cu_seqlens_v;   // starts of the sequences inside V (multiples of 32); null: cu_seqlens_k
   int total_q;
 };
+
+// The three numbers the scales of a call fold into.  With scales on the device every thread that needs
+// them reads the three words once (the quantiser's launch wrote them): a caller that quantises and
+// attends in one go never waits for them on the host.  The products are those of the host, in its
+// order, so the results are the same bits.
+struct ScoreScales {
+  float sl2, out_scale, softcap_c1;
+};
+__device__ __forceinline__ ScoreScales score_scales(const KernelParams& p) {
+  ScoreScales s{p.sl2, p.out_scale, p.softcap_c1};
+  if (p.q_scale != nullptr) {
+    const float qk = __fmul_rn(__fmul_rn(p.softmax_scale, *p.q_scale), *p.k_scale);
+    s.out_scale = *p.v_scale;
+    if (p.softcap > 0.f) s.softcap_c1 = __fdiv_rn(qk, p.softcap);   // sl2 = softcap * log2(e) needs no scale
+    else s.sl2 = __fmul_rn(qk, 1.4426950408889634f);
+  }
+  return s;
+}
 
 // Work tile of a CTA.  Tiles are ordered so that, for causal problems, the m-blocks with the
 // most K/V blocks come first (longest-processing-time-first, the idea of the reference's

@@ -289,6 +289,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   tc_fence_after_sync();
   pdl_trigger();
   const uint32_t tmem = *tmem_slot;
+  const ScoreScales sc = score_scales(p);
   constexpr uint32_t idesc = make_idesc_nvf4(128, kN);
   bool ok = true;
 
@@ -493,11 +494,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       // reference maximum of the row (CTA-uniform per row: every warp computes the same value)
       const float m_loc = fmaxf(fmaxf(red[my_row], red[kMaxRows + my_row]),
                                 fmaxf(red[2 * kMaxRows + my_row], red[3 * kMaxRows + my_row]));
-      const float m_new = next_reference(m_ref, m_loc, p.sl2);
+      const float m_new = next_reference(m_ref, m_loc, sc.sl2);
       float fac = 1.f;
       bool moved_row = false;
       if (m_new != m_ref) {
-        fac = reference_factor(m_ref, m_new, p.sl2);
+        fac = reference_factor(m_ref, m_new, sc.sl2);
         moved_row = m_ref != kNegInf;
         l_sum *= fac;
         m_ref = m_new;
@@ -516,11 +517,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         float pv[kR];
 #pragma unroll
         for (int q = 0; q < kB; ++q) {
-          block_exponent1(bm[q], m_ref, p.sl2, noff[q], ue[q]);
+          block_exponent1(bm[q], m_ref, sc.sl2, noff[q], ue[q]);
           float psum = 0.f;
 #pragma unroll
           for (int j = 0; j < kPer; ++j) {
-            pv[q * kPer + j] = ex2_approx(fmaf(x[q * kPer + j], p.sl2, noff[q]));
+            pv[q * kPer + j] = ex2_approx(fmaf(x[q * kPer + j], sc.sl2, noff[q]));
             psum += pv[q * kPer + j];
           }
           l_sum = fmaf(psum, __uint_as_float(ue[q] << 23), l_sum);
@@ -611,11 +612,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             // fixed order over the four warps: the sum of a row does not depend on timing
             const float l_tot = ((red[r] + red[kMaxRows + r]) + red[2 * kMaxRows + r]) + red[3 * kMaxRows + r];
             const int s = r / p.group, h = hk * p.group + r % p.group;
-            const float scale = (l_tot > 0.f && n > 0) ? p.out_scale / l_tot : 0.f;
+            const float scale = (l_tot > 0.f && n > 0) ? sc.out_scale / l_tot : 0.f;
             d.o_partial[((((int64_t)split * p.B + b) * p.Sq + s) * p.Hq + h) * 128 + tid] = o[r] * scale;
             if (tid == r) {   // thread r (warp 0, lane r) owns row r: its m_ref is the row's
               d.lse_partial[(((int64_t)split * p.B + b) * p.Hq + h) * p.Sq + s] =
-                  finish_lse(m_ref, l_tot, p.sl2);
+                  finish_lse(m_ref, l_tot, sc.sl2);
             }
           }
         }

@@ -348,6 +348,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
   tc_fence_after_sync();
   pdl_trigger();
   const uint32_t tmem = *tmem_slot;
+  const ScoreScales sc = score_scales(p);
   static_assert(kD == 128 || kD == 64, "head dimensions built: 128 and 64");
   constexpr uint32_t idesc_qk = make_idesc_nvf4(128, 128);
   constexpr uint32_t idesc_pv = make_idesc_nvf4(128, kD);
@@ -647,15 +648,15 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         mbar_arrive(bars.at(Bars::kSFree + b));
         if constexpr (kGeneral) {
           // tanh is monotone: capping the eight block maxima is capping every score under them
-          if (p.softcap_c1 != 0.f) {
+          if (sc.softcap_c1 != 0.f) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) bm[q] = soft_cap(bm[q], p.softcap_c1);
+            for (int q = 0; q < 8; ++q) bm[q] = soft_cap(bm[q], sc.softcap_c1);
           }
         }
         const float m01 = fmax3(bm[0], bm[1], bm[2]);
         const float m23 = fmax3(bm[3], bm[4], bm[5]);
         const float m_loc = fmax3(fmaxf(m01, m23), bm[6], bm[7]);
-        const float m_new = next_reference(m_run, m_loc, p.sl2);
+        const float m_new = next_reference(m_run, m_loc, sc.sl2);
         // the exponents themselves are derived by the softmax threads, each for its own four
         // blocks: this warpgroup is serial over all blocks of the CTA and publishes as early as
         // it can
@@ -734,16 +735,16 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
                               __uint_as_float(v_bm.w)};
         float noff4[4];
         uint32_t ue;
-        block_exponents4(bm4, m_new, p.sl2, noff4, ue);
-        if (m_new != m_ref) l_sum *= reference_factor(m_ref, m_new, p.sl2);
+        block_exponents4(bm4, m_new, sc.sl2, noff4, ue);
+        if (m_new != m_ref) l_sum *= reference_factor(m_ref, m_new, sc.sl2);
         m_ref = m_new;
         tc_wait_ld();
         tc_fence_before_sync();
         mbar_arrive(bars.at(Bars::kSFree + b));
         if constexpr (kGeneral) {
-          if (p.softcap_c1 != 0.f) {
+          if (sc.softcap_c1 != 0.f) {
 #pragma unroll
-            for (int x = 0; x < 64; ++x) s[x] = soft_cap(s[x], p.softcap_c1);
+            for (int x = 0; x < 64; ++x) s[x] = soft_cap(s[x], sc.softcap_c1);
           }
         }
 
@@ -754,10 +755,10 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         uint8_t* p_tile = gbase + kOffP + (G % kStagesP) * kTileBytes;
         uint4 chunk;
         l_sum += quantize_pair(&s[0], noff4[0], noff4[1],
-                               __byte_perm(ue, 0u, 0x4440u), __byte_perm(ue, 0u, 0x4441u), p.sl2, chunk);
+                               __byte_perm(ue, 0u, 0x4440u), __byte_perm(ue, 0u, 0x4441u), sc.sl2, chunk);
         *reinterpret_cast<uint4*>(p_tile + sw64_offset(row, 2 * half)) = chunk;
         l_sum += quantize_pair(&s[32], noff4[2], noff4[3],
-                               __byte_perm(ue, 0u, 0x4442u), __byte_perm(ue, 0u, 0x4443u), p.sl2, chunk);
+                               __byte_perm(ue, 0u, 0x4442u), __byte_perm(ue, 0u, 0x4443u), sc.sl2, chunk);
         *reinterpret_cast<uint4*>(p_tile + sw64_offset(row, 2 * half + 1)) = chunk;
         // scales of this half: one 64-key MMA step = scale word `half`
         *reinterpret_cast<uint32_t*>(gbase + kOffSFP + (G % kStagesP) * kSfBytes + 512 * half + (row & 31) * 16 +
@@ -771,7 +772,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
                                                  ((G - 1) / kStagesV) & 1, wc, kSitePvDone));
           if (!ok) break;
           tc_fence_after_sync();
-          const float f = (m_new != m_prev) ? reference_factor(m_prev, m_new, p.sl2) : 1.f;
+          const float f = (m_new != m_prev) ? reference_factor(m_prev, m_new, sc.sl2) : 1.f;
           rescale_accumulator(lane_addr + kTmO + (kD / 2) * half, f, kD / 64);
           tc_wait_st();
         }
@@ -802,13 +803,13 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
           m_fin = fmaxf(m_fin, mw[w]);
         }
 #pragma unroll
-        for (int w = 0; w < 4; ++w) l_tot += lw[w] * reference_factor(mw[w], m_fin, p.sl2);
+        for (int w = 0; w < 4; ++w) l_tot += lw[w] * reference_factor(mw[w], m_fin, sc.sl2);
         if (m_fin == kNegInf) l_tot = 0.f;
         if constexpr (kGeneral) {
           // the sink joins the row sum once (split 0), relative to the row's reference maximum
           if (p.sink != nullptr && t.split == 0 && m_fin != kNegInf) {
             l_tot += ex2_approx(static_cast<float>(kShift) + p.sink[t.h] * 1.4426950408889634f -
-                                m_fin * p.sl2);
+                                m_fin * sc.sl2);
           }
         }
         const uint32_t Gl = gb + n - 1;
@@ -816,7 +817,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
                         mbar_wait(bars.at(Bars::kPvDone + (Gl % kStagesV)), (Gl / kStagesV) & 1, wc, kSiteFinalO));
         if (!ok) break;
         tc_fence_after_sync();
-        scale = (l_tot > 0.f) ? p.out_scale / l_tot : 0.f;
+        scale = (l_tot > 0.f) ? sc.out_scale / l_tot : 0.f;
       }
       // warpgroup k stores output columns [32 k, 32 k + 32); with kD = 64 two of them only arrive
       if (kGeneral && p.num_splits > 1 && (kD == 128 || wg < kD / 32)) {
@@ -840,7 +841,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         mbar_arrive(bars.at(Bars::kOStaged));
       }
       if (wg == 0 && q_idx < p.Sq) {
-        float lse_v = finish_lse(m_fin, l_tot, p.sl2);
+        float lse_v = finish_lse(m_fin, l_tot, sc.sl2);
         if constexpr (kGeneral) {
           // a row without visible keys still has its sink: LSE = sink, output zero
           if (p.sink != nullptr && t.split == 0 && m_fin == kNegInf) lse_v = p.sink[t.h];

@@ -212,6 +212,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   tc_fence_after_sync();
   pdl_trigger();
   const uint32_t tmem = *tmem_slot;
+  const ScoreScales sc = score_scales(p);
   static_assert(kD == 128 || kD == 64 || kD == 192, "head dimensions built: 128, 64 and (192, 128)");
   constexpr int kDv = kD == 192 ? 128 : kD;            // head dim of V and O
   constexpr uint32_t idesc_qk = make_idesc_nvf4(128, 128);
@@ -283,12 +284,12 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
         mbar_arrive(bars.at(Bars::kFinFree + fb));
 #pragma unroll
-        for (int w = 0; w < 4; ++w) l_tot += lw[w] * reference_factor(mw[w], m_fin, p.sl2);
+        for (int w = 0; w < 4; ++w) l_tot += lw[w] * reference_factor(mw[w], m_fin, sc.sl2);
         if (m_fin == kNegInf) l_tot = 0.f;
         if constexpr (kGeneral) {
           // the sink joins the row sum, relative to the row's reference maximum
           if (p.sink != nullptr && m_fin != kNegInf) {
-            l_tot += ex2_approx(static_cast<float>(kShift) + p.sink[t.h] * 1.4426950408889634f - m_fin * p.sl2);
+            l_tot += ex2_approx(static_cast<float>(kShift) + p.sink[t.h] * 1.4426950408889634f - m_fin * sc.sl2);
           }
         }
         const uint32_t Jl = 2 * gb + 2 * n - 1;
@@ -296,7 +297,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
                         mbar_wait(bars.at(Bars::kPvDone + (Jl % kPSlots)), (Jl / kPSlots) & 1, wc, kS64FinalO));
         if (!ok) break;
         tc_fence_after_sync();
-        scale = (l_tot > 0.f) ? p.out_scale / l_tot : 0.f;
+        scale = (l_tot > 0.f) ? sc.out_scale / l_tot : 0.f;
       }
       // the staging tile is free once the previous store has read it
       if (it >= 1) {
@@ -354,7 +355,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         bulk_commit_group();
       }
       if (q_idx < sq && p.lse != nullptr) {
-        float lse_v = finish_lse(m_fin, l_tot, p.sl2);
+        float lse_v = finish_lse(m_fin, l_tot, sc.sl2);
         if constexpr (kGeneral) {
           // a row without visible keys still has its sink: LSE = sink, output zero
           if (p.sink != nullptr && m_fin == kNegInf) lse_v = p.sink[t.h];
@@ -660,9 +661,9 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         tc_fence_before_sync();
         mbar_arrive(bars.at(Bars::kSFree + wg));
         if constexpr (kGeneral) {
-          if (p.softcap_c1 != 0.f) {
+          if (sc.softcap_c1 != 0.f) {
 #pragma unroll
-            for (int x = 0; x < 64; ++x) s[x] = soft_cap(s[x], p.softcap_c1);
+            for (int x = 0; x < 64; ++x) s[x] = soft_cap(s[x], sc.softcap_c1);
           }
         }
 
@@ -680,24 +681,24 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           bm4[q] = fmaxf(m0, m1);
         }
         const float m_loc = fmaxf(fmaxf(bm4[0], bm4[1]), fmaxf(bm4[2], bm4[3]));
-        const float m_new = next_reference(m_prev, m_loc, p.sl2);
+        const float m_new = next_reference(m_prev, m_loc, sc.sl2);
         s_hand[wg * 128 + row] = m_new;
         mbar_arrive(bars.at(Bars::kHand + 4 * wg + (warp & 3)));
         float noff4[4];
         uint32_t sbits4[4], sf_bytes;
 #if FA4_P_SCALE_E4M3
-        block_scales4_e4m3(bm4, m_new, p.sl2, noff4, sf_bytes, sbits4);
+        block_scales4_e4m3(bm4, m_new, sc.sl2, noff4, sf_bytes, sbits4);
 #else
         {
           uint32_t ue;
-          block_exponents4(bm4, m_new, p.sl2, noff4, ue);
+          block_exponents4(bm4, m_new, sc.sl2, noff4, ue);
           sf_bytes = block_scale_bytes(ue);
 #pragma unroll
           for (int b4 = 0; b4 < 4; ++b4) sbits4[b4] = __byte_perm(ue, 0u, 0x4440u + b4) << 23;  // 2^e as fp32
         }
 #endif
         // own partial row sum follows the reference
-        if (m_new != m_ref) l_sum *= reference_factor(m_ref, m_new, p.sl2);
+        if (m_new != m_ref) l_sum *= reference_factor(m_ref, m_new, sc.sl2);
         m_ref = m_new;
 
         // 3. exponentials and quantisation; P slot J % 8 is free once P V of sub-block J - 8 has run
@@ -709,7 +710,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           float acc = 0.f;
 #pragma unroll
           for (int b4 = 0; b4 < 4; ++b4) {
-            const float bsum = quantize_block16(&s[16 * b4], noff4[b4], p.sl2, pk[2 * b4], pk[2 * b4 + 1]);
+            const float bsum = quantize_block16(&s[16 * b4], noff4[b4], sc.sl2, pk[2 * b4], pk[2 * b4 + 1]);
             acc = fmaf(bsum, __uint_as_float(sbits4[b4]), acc);   // times the block scale
           }
           l_sum += acc;
@@ -730,7 +731,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
                                                  (Jp / kPSlots) & 1, wc, kS64PvDone));
           if (!ok) break;
           tc_fence_after_sync();
-          const float f = fix ? reference_factor(m_prev, m_new, p.sl2) : 1.f;
+          const float f = fix ? reference_factor(m_prev, m_new, sc.sl2) : 1.f;
           rescale_accumulator(lane_addr + kTmO, f, kDv / 32);
           tc_wait_st();
         }

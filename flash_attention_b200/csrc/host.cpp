@@ -15,6 +15,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CachingHostAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Device.h>
@@ -25,6 +26,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <memory>
 #include <string>
 
 #include "../../include/fa4_nvfp4.h"
@@ -99,6 +101,66 @@ bool truth_of(PyObject* o) {
   if (v < 0) throw PyErrorSet();
   return v != 0;
 }
+// ---- per-tensor scales that are still on their way ------------------------------------------------
+// What quantize_qkv hands out for a scale: the quantiser writes it to the device and to pinned host
+// memory.  An attention call on the quantiser's stream reads the device copy, so quantising and
+// attending never wait on the host; float(scale) waits for the stream once, for all three tensors.
+struct ScaleState {
+  at::Tensor device, pinned;        // three floats each
+  cudaStream_t stream;
+  bool known = false;
+  float value[3];
+  void fetch() {
+    if (known) return;
+    cudaError_t e;
+    Py_BEGIN_ALLOW_THREADS
+    e = cudaStreamSynchronize(stream);
+    Py_END_ALLOW_THREADS
+    C10_CUDA_CHECK(e);
+    if (known) return;              // another thread was faster
+    std::copy_n(pinned.data_ptr<float>(), 3, value);
+    known = true;
+    pinned.reset();
+  }
+};
+struct LazyScale {
+  PyObject_HEAD
+  std::shared_ptr<ScaleState>* state;
+  int which;
+};
+PyObject* lazy_float(PyObject* self) {
+  HANDLE_TH_ERRORS
+  LazyScale* s = reinterpret_cast<LazyScale*>(self);
+  (*s->state)->fetch();
+  return PyFloat_FromDouble((*s->state)->value[s->which]);
+  END_HANDLE_TH_ERRORS
+}
+void lazy_dealloc(PyObject* self) {
+  delete reinterpret_cast<LazyScale*>(self)->state;
+  Py_TYPE(self)->tp_free(self);
+}
+PyNumberMethods lazy_number = {};
+PyTypeObject lazy_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+bool is_lazy(PyObject* o) { return Py_TYPE(o) == &lazy_type; }
+PyObject* new_lazy(const std::shared_ptr<ScaleState>& st, int which) {
+  PyObject* o = lazy_type.tp_alloc(&lazy_type, 0);
+  if (o == nullptr) throw PyErrorSet();
+  reinterpret_cast<LazyScale*>(o)->state = new std::shared_ptr<ScaleState>(st);
+  reinterpret_cast<LazyScale*>(o)->which = which;
+  return o;
+}
+// The device copies of three scales for a call on `stream`; false: take their values instead.
+bool device_scales(PyObject* const* o, const at::Device& device, cudaStream_t stream, const float** ptr) {
+  for (int i = 0; i < 3; ++i) {
+    if (!is_lazy(o[i])) return false;
+    const LazyScale* s = reinterpret_cast<const LazyScale*>(o[i]);
+    const ScaleState& st = **s->state;
+    if (st.known || st.stream != stream || st.device.device() != device) return false;
+    ptr[i] = st.device.data_ptr<float>() + s->which;
+  }
+  return true;
+}
+
 // a per-tensor scale: a number, or a one-element tensor whose value is read (synchronises if it
 // lives on the device)
 float scalar_of(PyObject* o, const char* name) {
@@ -368,9 +430,13 @@ PyObject* fwd(PyObject* const* a) {
   p.o_stride_b = out.stride(0); p.o_stride_s = out.stride(1); p.o_stride_h = out.stride(2);
   p.B = (int32_t)B; p.Sq = (int32_t)Sq; p.Sk = (int32_t)Sk; p.Hq = (int32_t)Hq; p.Hkv = (int32_t)Hkv;
   p.D = (int32_t)D; p.Dv = (int32_t)Dv;
-  p.q_scale = scalar_of(a[6], "q_scale");
-  p.k_scale = scalar_of(a[7], "k_scale");
-  p.v_scale = scalar_of(a[8], "v_scale");
+  const float* scales[3];
+  const bool lazy = device_scales(a + 6, device, static_cast<cudaStream_t>(stream), scales);
+  if (!lazy) {
+    p.q_scale = scalar_of(a[6], "q_scale");
+    p.k_scale = scalar_of(a[7], "k_scale");
+    p.v_scale = scalar_of(a[8], "v_scale");
+  }
   p.softmax_scale = (float)softmax_scale;
 
   long num_splits = integer_of(a[16]);
@@ -394,7 +460,7 @@ PyObject* fwd(PyObject* const* a) {
     num_splits = decode ? decode_splits(B, Hkv, Sk, sm_count(device)) : prefill_splits(B, Sq, Sk, Hq, sm_count(device));
 
   if (num_splits == 1 && !sink.defined() && win.left < 0 && win.right <= 0 && softcap == 0.0 && !used.defined() &&
-      !paged && !decode) {
+      !paged && !decode && !lazy) {
     check_rc(fa4_nvfp4_fwd(&p, stream), "fa4_nvfp4_fwd");
   } else {
     fa4_nvfp4_ext x = {};
@@ -419,7 +485,10 @@ PyObject* fwd(PyObject* const* a) {
       x.workspace = workspace.data_ptr();
       x.workspace_bytes = (uint64_t)bytes;
     }
-    check_rc(fa4_nvfp4_fwd_ex(&p, &x, stream), "fa4_nvfp4_fwd_ex");
+    if (lazy)
+      check_rc(fa4_nvfp4_fwd_device_scales(&p, &x, scales[0], scales[1], scales[2], stream), "fa4_nvfp4_fwd_device_scales");
+    else
+      check_rc(fa4_nvfp4_fwd_ex(&p, &x, stream), "fa4_nvfp4_fwd_ex");
   }
   return pair_of(out_o, out, lse_o, lse);
 }
@@ -535,6 +604,72 @@ PyObject* varlen_fwd(PyObject* const* a) {
   return pair_of(nullptr, out, nullptr, lse);
 }
 
+// ---- quantize_qkv_fused ----------------------------------------------------------------------------
+// q k v linear_sf -> (packed, linear scales or None, tiled scales, LazyScale) x 3
+PyObject* quantize_qkv(PyObject* const* a) {
+  static const char* names[3] = {"q", "k", "v"};
+  const bool linear = truth_of(a[3]);
+  const at::Device device = tensor_of(a[0], "q").device();
+  fa4_nvfp4_quant_job jobs[3] = {};
+  at::Tensor packed[3], lin[3], tiled[3], scratch, scales, pinned;
+  c10::cuda::OptionalCUDAGuard guard;
+  for (int i = 0; i < 3; ++i) {
+    const at::Tensor& x = tensor_of(a[i], names[i]);
+    FA4_ASSERT(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 4 && x.stride(-1) == 1 &&
+                   x.device() == device,
+               "quantize_qkv_fused takes CUDA bf16 (B, S, H, D) tensors, last dim contiguous");
+    if (i == 0) {
+      if (device.index() != c10::cuda::current_device()) guard.set_device(device);
+      scales = at::empty({3}, x.options().dtype(at::kFloat));
+      scratch = at::empty({FA4_QUANT_SCRATCH_FLOATS}, scales.options());
+      pinned = at::empty({3}, at::TensorOptions().dtype(at::kFloat).pinned_memory(true));
+    }
+    const auto bytes = x.options().dtype(at::kByte);
+    const int64_t B = x.size(0), S = x.size(1), H = x.size(2), D = x.size(3);
+    // V is blocked along its key axis, stored padded with zeros to whole 32-key groups
+    const int64_t s_out = i == 2 ? cdiv(S, 32) * 32 : S;
+    if (i == 2) {
+      packed[i] = at::empty({B, H, D, s_out / 2}, bytes);
+      if (linear) lin[i] = at::empty({B, H, D, s_out / 16}, bytes);
+      tiled[i] = at::empty({B, H, cdiv(D, 128), 2 * cdiv(s_out, 128), 512}, bytes);
+    } else {
+      packed[i] = at::empty({B, S, H, D / 2}, bytes);
+      if (linear) lin[i] = at::empty({B, S, H, D / 16}, bytes);
+      tiled[i] = at::empty({B, H, cdiv(S, 128), D / 64, 512}, bytes);
+    }
+    fa4_nvfp4_quant_job& j = jobs[2 - i];   // V first: its tiles take longest
+    j.x = x.data_ptr();
+    j.stride_b = x.stride(0); j.stride_s = x.stride(1); j.stride_h = x.stride(2);
+    j.B = (int32_t)B; j.S = (int32_t)S; j.H = (int32_t)H; j.D = (int32_t)D;
+    j.is_v = i == 2;
+    j.S_out = (int32_t)s_out;
+    j.packed = packed[i].data_ptr();
+    j.sf_linear = linear ? lin[i].data_ptr() : nullptr;
+    j.sf_tiled = tiled[i].data_ptr();
+    j.scale_out = scales.data_ptr<float>() + i;
+    j.scale_host = pinned.data_ptr<float>() + i;
+  }
+  const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(device.index());
+  check_rc(fa4_nvfp4_quantize_jobs_bf16(jobs, 3, scratch.data_ptr<float>(), stream.stream()), "fa4_nvfp4_quantize_jobs_bf16");
+  // the pinned words go back to their pool no earlier than the launch has written them
+  at::getHostAllocator(at::kCUDA)->record_event(pinned.data_ptr(), pinned.storage().data_ptr().get_context(), stream.unwrap());
+  auto state = std::make_shared<ScaleState>();
+  state->device = scales;
+  state->pinned = pinned;
+  state->stream = stream.stream();
+  PyObject* res = PyTuple_New(3);
+  for (int i = 0; i < 3; ++i) {
+    PyObject* t = PyTuple_New(4);
+    PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(packed[i]));
+    PyObject* l = linear ? THPVariable_Wrap(lin[i]) : (Py_INCREF(Py_None), Py_None);
+    PyTuple_SET_ITEM(t, 1, l);
+    PyTuple_SET_ITEM(t, 2, THPVariable_Wrap(tiled[i]));
+    PyTuple_SET_ITEM(t, 3, new_lazy(state, i));
+    PyTuple_SET_ITEM(res, i, t);
+  }
+  return res;
+}
+
 // ---- the module -----------------------------------------------------------------------------------
 PyObject* choose_decode_splits(PyObject* const* a) {
   return PyLong_FromLongLong(decode_splits(integer_of(a[0]), integer_of(a[1]), integer_of(a[2]), integer_of(a[3])));
@@ -575,6 +710,7 @@ PyMethodDef methods[] = {method<fwd, 23>("fwd"),
                          method<varlen_fwd, 22>("varlen_fwd"),
                          method<choose_decode_splits, 4>("choose_decode_splits"),
                          method<choose_num_splits, 5>("choose_num_splits"),
+                         method<quantize_qkv, 4>("quantize_qkv"),
                          method<window_of, 3>("resolve_window"),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "Native host path of flash_attention_b200.", -1, methods,
@@ -582,4 +718,16 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "Native host path of f
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module_def); }
+PyMODINIT_FUNC PyInit__host(void) {
+  lazy_number.nb_float = lazy_float;
+  lazy_type.tp_name = "flash_attention_b200._host.LazyScale";
+  lazy_type.tp_doc = "A per-tensor scale on its way from the quantiser; float() waits for it.";
+  lazy_type.tp_basicsize = sizeof(LazyScale);
+  lazy_type.tp_flags = Py_TPFLAGS_DEFAULT;
+  lazy_type.tp_as_number = &lazy_number;
+  lazy_type.tp_dealloc = lazy_dealloc;
+  if (PyType_Ready(&lazy_type) < 0) return nullptr;
+  PyObject* m = PyModule_Create(&module_def);
+  if (m != nullptr) PyModule_AddObjectRef(m, "LazyScale", reinterpret_cast<PyObject*>(&lazy_type));
+  return m;
+}

@@ -9,7 +9,10 @@
 //   element        = e2m1_rne(x / (float(block scale) * g)), no negative zero
 // every operation a correctly rounded fp32 one.
 //
-// All three kernels are HBM-bound byte movers: 2 B read per element in each pass, 9/16 B written.
+// Two launches for the q, k and v of a call (any one to three tensors): amax_kernel writes one partial
+// maximum per CTA, quantize_kernel reduces them and quantises.  2 B read per element in each pass,
+// 9/16 B (10/16 with both scale layouts) written: HBM-bound byte movers.  The second pass walks every
+// tensor from its end, where the first pass has just been, so that its first tens of MB come from L2.
 #pragma once
 #include "ptx.cuh"
 #include <cuda_bf16.h>
@@ -39,19 +42,6 @@ __device__ __forceinline__ uint32_t drop_negative_zero(uint32_t n) {
   return n & (0x77777777u | nz);
 }
 
-// Rare path of quantize_block16: sixteen correctly rounded divisions.  Out of line so that the
-// hot loop stays small (it was instruction-fetch bound with this inlined).
-struct Block16 {
-  float v[16];
-};
-__device__ __noinline__ uint2 quantize_block16_exact(Block16 x, float denom) {
-  float y[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) y[i] = denom > 0.f ? __fdiv_rn(x.v[i], denom) : 0.f;
-  return make_uint2(pack8_e2m1(y[0], y[1], y[2], y[3], y[4], y[5], y[6], y[7]),
-                    pack8_e2m1(y[8], y[9], y[10], y[11], y[12], y[13], y[14], y[15]));
-}
-
 // Correctly rounded a / b from the correctly rounded reciprocal rb = RN(1 / b) and nb = -b: the
 // product a rb is within 2 ulp of the quotient, one residual step (the residual a - y b is exact
 // in an FMA) makes it faithful and a second one correctly rounded (Markstein's division theorem).
@@ -63,14 +53,21 @@ __device__ __forceinline__ float div_rn_by(float a, float nb, float rb) {
   const float y1 = fmaf(fmaf(y0, nb, a), rb, y0);
   return fmaf(fmaf(y1, nb, a), rb, y1);
 }
-// The same for a pair (packed fp32 instructions: both lanes round like the scalar ones).
-__device__ __forceinline__ float2 div_rn_by2(float2 a, float2 nb, float2 rb) {
-  const float2 y0 = __fmul2_rn(a, rb);
-  const float2 y1 = __ffma2_rn(__ffma2_rn(y0, nb, a), rb, y0);
-  return __ffma2_rn(__ffma2_rn(y1, nb, a), rb, y1);
+
+// Rare path of quantize_block16 (denominators near the bottom of the fp32 range), out of line so
+// that the hot loop stays small.
+struct Block16 {
+  float v[16];
+};
+__device__ __noinline__ uint2 quantize_block16_exact(Block16 x, float denom) {
+  float y[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) y[i] = denom > 0.f ? __fdiv_rn(x.v[i], denom) : 0.f;
+  return make_uint2(pack8_e2m1(y[0], y[1], y[2], y[3], y[4], y[5], y[6], y[7]),
+                    pack8_e2m1(y[8], y[9], y[10], y[11], y[12], y[13], y[14], y[15]));
 }
 
-// Per-tensor constants of the quantisers: the tensor scale g, -g, RN(1 / g), and whether g is so
+// Per-tensor constants of the quantiser: the tensor scale g, -g, RN(1 / g), and whether g is so
 // small (below 1e-18) that the residual steps above could underflow where it matters: then the
 // block scales take the library division.
 struct TensorScale {
@@ -86,256 +83,334 @@ __device__ __forceinline__ TensorScale make_tensor_scale(float amax) {
   return t;
 }
 
-// One block of 16 values -> 8 packed bytes (two words) and its scale byte.
-__device__ __forceinline__ void quantize_block16(const float (&x)[16], const TensorScale& ts, uint32_t& lo,
-                                                 uint32_t& hi, uint32_t& sf_byte) {
-  const float g = ts.g;
-  // |x| maxima of the block (two chains)
-  float bm0 = fmaxf(fabsf(x[0]), fabsf(x[1])), bm1 = fmaxf(fabsf(x[2]), fabsf(x[3]));
-#pragma unroll
-  for (int i = 4; i < 16; i += 2) {
-    bm0 = fmaxf(bm0, fabsf(x[i]));
-    bm1 = fmaxf(bm1, fabsf(x[i + 1]));
-  }
-  const float bmax = fmaxf(bm0, bm1);
+// Scale byte and its value times g for a block with maximum bmax.
+__device__ __forceinline__ float block_scale_of(float bmax, const TensorScale& ts, uint32_t& sf_byte) {
   // block scale = e4m3_rne(min((bmax / 6) / g, 448)).  With g >= 1e-18 every quotient that can
   // reach the first rounding boundary of e4m3 (2^-10) has exact residuals; smaller quotients give
   // the zero byte whatever their last bits are.
   constexpr float kRcp6 = 0.16666667163372039794921875f;   // RN(1 / 6)
   float t;
   if (ts.tiny) {
-    t = __fdiv_rn(__fdiv_rn(bmax, 6.f), g);
+    t = __fdiv_rn(__fdiv_rn(bmax, 6.f), ts.g);
   } else {
     t = div_rn_by(div_rn_by(bmax, -6.f, kRcp6), ts.neg_g, ts.rcp_g);
   }
   sf_byte = e4m3_byte(fminf(t, 448.f));
-  const float denom = __fmul_rn(e4m3_value(sf_byte), g);
-  // The element codes are those of the correctly rounded quotients x / denom.  Denominators near
-  // the bottom of the fp32 range take the out-of-line exact path; quotients that small are far
-  // below the first rounding boundary (0.25) whatever the residuals do.
-  if (denom < 1e-30f) {
+  return __fmul_rn(e4m3_value(sf_byte), ts.g);
+}
+
+// One block of 16 values with maximum bmax -> 8 packed bytes (two words) and its scale byte.
+__device__ __forceinline__ void quantize_block16(const float (&x)[16], float bmax, const TensorScale& ts,
+                                                 uint32_t& lo, uint32_t& hi, uint32_t& sf_byte) {
+  const float denom = block_scale_of(bmax, ts, sf_byte);
+  // The element codes are those of the correctly rounded quotients x / denom.  One residual step is
+  // enough for them: only quotients within a few ulp of a rounding boundary of e2m1 (.25 .75 1.25
+  // 1.75 2.5 3.5 5) matter, x has eight significand bits, and for all 2^23 significands of denom and
+  // the values of x next to a boundary the steps below land on the same side of it (or on it) as
+  // the correctly rounded quotient (checked exhaustively on the GPU; without the step 257
+  // denominators fail).  Three instructions a pair where correctly rounded quotients take five.
+  if (denom >= 1e-30f) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(denom));
+    r = fmaf(fmaf(-denom, r, 1.f), r, r);
+    const float2 rr = make_float2(r, r), nd = make_float2(-denom, -denom);
+    float2 y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 v = make_float2(x[2 * i], x[2 * i + 1]), y0 = __fmul2_rn(v, rr);
+      y[i] = __ffma2_rn(__ffma2_rn(y0, nd, v), rr, y0);
+    }
+    lo = pack8_e2m1(y[0].x, y[0].y, y[1].x, y[1].y, y[2].x, y[2].y, y[3].x, y[3].y);
+    hi = pack8_e2m1(y[4].x, y[4].y, y[5].x, y[5].y, y[6].x, y[6].y, y[7].x, y[7].y);
+  } else {
     Block16 blk;
 #pragma unroll
     for (int i = 0; i < 16; ++i) blk.v[i] = x[i];
     const uint2 e = quantize_block16_exact(blk, denom);
     lo = e.x;
     hi = e.y;
-  } else {
-    const float r = __frcp_rn(denom);
-    const float2 rr = make_float2(r, r), nd = make_float2(-denom, -denom);
-    float2 y[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) y[i] = div_rn_by2(make_float2(x[2 * i], x[2 * i + 1]), nd, rr);
-    lo = pack8_e2m1(y[0].x, y[0].y, y[1].x, y[1].y, y[2].x, y[2].y, y[3].x, y[3].y);
-    hi = pack8_e2m1(y[4].x, y[4].y, y[5].x, y[5].y, y[6].x, y[6].y, y[7].x, y[7].y);
   }
   lo = drop_negative_zero(lo);
   hi = drop_negative_zero(hi);
 }
 
-__device__ __forceinline__ void unpack_bf16x8(const uint4& v, float* out) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    out[2 * i] = __uint_as_float(w[i] << 16);
-    out[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+
+// 32 consecutive bytes of global memory: one 256-bit load when the address allows it
+struct Words8 {
+  uint32_t w[8];
+};
+__device__ __forceinline__ Words8 load32(const void* p, bool wide) {
+  Words8 v;
+  if (wide) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]),
+                   "=r"(v.w[7])
+                 : "l"(p));
+  } else {
+    const uint4 a = *static_cast<const uint4*>(p), b = *(static_cast<const uint4*>(p) + 1);
+    v.w[0] = a.x; v.w[1] = a.y; v.w[2] = a.z; v.w[3] = a.w;
+    v.w[4] = b.x; v.w[5] = b.y; v.w[6] = b.z; v.w[7] = b.w;
   }
+  return v;
+}
+// max(|a|, |b|) of two bf16 pairs (a NaN loses to a number, like fmaxf); the result's signs are noise
+__device__ __forceinline__ uint32_t absmax2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ float max_of_pair(uint32_t m) {
+  return fmaxf(fabsf(__uint_as_float(m << 16)), fabsf(__uint_as_float(m & 0xffff0000u)));
+}
+__device__ __forceinline__ float absmax16(const Words8& v) {
+  return max_of_pair(absmax2(absmax2(absmax2(v.w[0], v.w[1]), absmax2(v.w[2], v.w[3])),
+                             absmax2(absmax2(v.w[4], v.w[5]), absmax2(v.w[6], v.w[7]))));
 }
 
+// One tensor of a launch: bf16 (B, S, H, D), last dimension contiguous.
+struct QuantJob {
+  const __nv_bfloat16* x;
+  int64_t sb, ss, sh;           // strides in elements
+  int B, S, H, D;
+  int s_out;                    // V: its key axis as stored (zeros from S on)
+  int is_v, wide;               // wide: every 32-byte piece is 32-byte aligned
+  // amax pass: units of 16 elements (8 where a run is no multiple of 16); the tensor as (n0, n1, n2)
+  // runs of inner_units
+  uint32_t units;
+  int unit;
+  int amax_block0, amax_blocks;
+  int64_t r0, r1, r2;           // strides of the runs
+  FastDiv div_inner, div_n2, div_n1;
+  int inner_units, n2, n1;
+  float* amax_out;              // atomic maximum of the tensor (then no partials), or null
+  // quantise pass
+  const float* parts;           // partial maxima of this tensor
+  int num_parts;
+  int block0, blocks;
+  int single;                   // Q / K: one row per work item instead of four (tensors too small to fill the GPU)
+  uint32_t items;               // Q / K: threads' work items; V: tiles
+  FastDiv div_nb, div_rt, div_h;
+  int nb, rt;                   // Q / K: blocks of a row of all heads; 128-row (V: 128-key) tiles
+  uint8_t *packed, *lin, *tiled;
+  float *scale_out, *scale_host;   // either may be null
+};
+struct QuantJobs {
+  QuantJob job[3];
+  float* parts;                 // amax pass: one float per CTA of the grid
+  int n;
+};
+
 // ---------------------------------------------------------------------------------------------
-// amax over a (n0, n1, n2, inner) bf16 tensor with contiguous last dimension.  A "row" is one
-// (i0, i1) pair = n2 * inner / 8 chunks of 16 bytes; a CTA walks groups of rows with a grid
-// stride, several independent 16-byte loads in flight per thread, and ends with ONE atomicMax on
-// the bit pattern (values >= 0).  *amax must be zero before the first launch that contributes.
+// Partial maxima of |x|, one per CTA (or an atomicMax into amax_out, bit patterns of values >= 0).
+// Two 32-byte loads in flight per thread, 1536 threads per SM: q, k, v of B=4, S=8192, Hq=32, Hkv=8, D=128
+// in 70 us (5.7 TB/s).  Four loads and 2048 threads in larger CTAs: 80; eight: 86 (the CTAs then
+// spread over too many DRAM pages at a time).  The three launches it replaced: 97.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-amax_bf16_kernel(const __nv_bfloat16* __restrict__ x, int n1, int n2, int inner8, int64_t s0,
-                 int64_t s1, int64_t s2, int rows, int rows_per_group, FastDiv div_per_row,
-                 FastDiv div_inner8, FastDiv div_n1, float* __restrict__ amax) {
-  __shared__ float warp_max[8];
+constexpr int kAmaxThreads = 256, kAmaxCtas = 6;   // CTAs per SM
+__global__ void __launch_bounds__(kAmaxThreads)
+amax_kernel(const __grid_constant__ QuantJobs jobs) {
+  __shared__ float warp_max[kAmaxThreads / 32];
   pdl_wait();
-  const int per_row = n2 * inner8;
-  const int per_group = rows_per_group * per_row;
-  const int groups = (rows + rows_per_group - 1) / rows_per_group;
-  float m = 0.f;
-  for (int grp = blockIdx.x; grp < groups; grp += gridDim.x) {
-    const int row0 = grp * rows_per_group;
-#pragma unroll 4
-    for (int item = threadIdx.x; item < per_group; item += 256) {
-      const int lr = fast_div(item, div_per_row), within = item - lr * per_row;
-      const int row = row0 + lr;
-      if (row < rows) {
-        const int i2 = fast_div(within, div_inner8), c = within - i2 * inner8;
-        const int i0 = fast_div(row, div_n1), i1 = row - i0 * n1;
-        const uint4 v = *reinterpret_cast<const uint4*>(x + i0 * s0 + i1 * s1 + i2 * s2 + c * 8);
-        // |bf16| maxima compare like their bit patterns with the sign cleared
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  int ji = 0;
+  while (ji + 1 < jobs.n && (int)blockIdx.x >= jobs.job[ji + 1].amax_block0) ++ji;
+  const QuantJob& j = jobs.job[ji];
+  const uint32_t stride = (uint32_t)j.amax_blocks * kAmaxThreads;
+  const bool flat = j.n1 * j.n2 == 1 && j.inner_units >= (int)j.units, wide = j.wide != 0;
+  auto at = [&](uint32_t u) -> const __nv_bfloat16* {
+    if (flat) return j.x + (int64_t)u * j.unit;
+    const int run = fast_div((int)u, j.div_inner), c = (int)u - run * j.inner_units;
+    const int i01 = fast_div(run, j.div_n2), i2 = run - i01 * j.n2;
+    const int i0 = fast_div(i01, j.div_n1), i1 = i01 - i0 * j.n1;
+    return j.x + i0 * j.r0 + i1 * j.r1 + i2 * j.r2 + (int64_t)c * j.unit;
+  };
+  const bool half = j.unit == 8;
+  auto load = [&](uint32_t i) -> Words8 {
+    if (!half) return load32(at(i), wide);
+    const uint4 a = *reinterpret_cast<const uint4*>(at(i));
+    return Words8{{a.x, a.y, a.z, a.w, 0u, 0u, 0u, 0u}};
+  };
+  uint32_t m2 = 0u;
+  uint32_t u = (blockIdx.x - j.amax_block0) * kAmaxThreads + threadIdx.x;
+  for (; u + (uint64_t)stride < j.units; u += 2 * stride) {
+    Words8 v[2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          m = fmaxf(m, __uint_as_float((w[i] << 16) & 0x7fffffffu));
-          m = fmaxf(m, __uint_as_float(w[i] & 0x7fff0000u));
-        }
-      }
-    }
+    for (int k = 0; k < 2; ++k) v[k] = load(u + k * stride);
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m2 = absmax2(m2, v[k].w[i]);
   }
+  for (; u < j.units; u += stride) {
+    const Words8 v = load(u);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m2 = absmax2(m2, v.w[i]);
+  }
+  float m = max_of_pair(m2);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
   __syncthreads();
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int w = 1; w < 8; ++w) m = fmaxf(m, warp_max[w]);
-    if (m > 0.f) atomicMax(reinterpret_cast<int*>(amax), __float_as_int(m));
+    for (int w = 1; w < kAmaxThreads / 32; ++w) m = fmaxf(m, warp_max[w]);
+    if (j.amax_out == nullptr) jobs.parts[blockIdx.x] = m;
+    else if (m > 0.f) atomicMax(reinterpret_cast<int*>(j.amax_out), __float_as_int(m));
   }
 }
 
 // ---------------------------------------------------------------------------------------------
-// Q / K: x (B, S, H, D) bf16, blocks along D.  One item = one block of 16 elements (two 16-byte
-// loads, one 8-byte store); a CTA takes a group of (b, s) rows, H * D/16 blocks each, about
-// eight items per thread.
-// The row index runs over S padded to a multiple of 128 so that the tiled scale layout gets its
-// zero padding from the same pass.
-//   packed    (B, S, H, D/2)  contiguous
-//   sf_lin    (B, S, H, D/16) contiguous, or null
-//   sf_tiled  (B, H, ceil(S/128), ceil(D/64), 512), or null
-// D is a multiple of 64 (four blocks = one 4-byte word of either scale layout); per_group is a
-// multiple of 4, so the four lanes that assemble a word always sit in one warp iteration.
+// Quantise.  CTAs are dealt to the tensors in proportion to their size and walk them from the end.
+//
+// Q / K, blocks along D: a work item is one block of 16 in the rows l, l + 32, l + 64, l + 96 of a
+// 128-row tile: their four scales share a 16-byte piece of the tiled layout.  Neighbouring threads take
+// neighbouring blocks, so a warp's reads (1 KB, the four rows in flight together) and packed writes
+// are contiguous.  (A thread with four neighbouring blocks of a row needs no exchange of scale bytes,
+// but its 128-byte stride filled the load/store pipe: 148 instead of 131 us.)
+//   packed (B, S, H, D/2), lin (B, S, H, D/16) or null, tiled (B, H, ceil(S/128), D/64, 512) or null
+//
+// V, blocks along the keys: a CTA transposes a tile of 128 keys x 128 d through shared memory (16-byte
+// chunks swizzled by the key block, so that the row-wise fill and the column-wise reads are both
+// conflict free); a thread takes two neighbouring d and one block of 16 keys.
+//   packed (B, H, Dv, s_out/2), lin (B, H, Dv, s_out/16) or null,
+//   tiled (B, H, ceil(Dv/128), 2 ceil(s_out/128), 512) or null
+//
+// Persistent: two CTAs per SM in all, dealt to the tensors in proportion to their bytes, and each
+// keeps the loads of its next item in flight behind the arithmetic of the current one.
+//
+// What bounds it: instruction issue and latency about equally, then HBM.  q, k, v of the sizes above,
+// quantise pass alone: 153 us as three kernels with correctly rounded divisions (274 instructions per
+// block), 117 us here (about 180).
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, int B, int S, int H, int D, int64_t sb,
-                     int64_t ss, int64_t sh, const float* __restrict__ amax,
-                     uint8_t* __restrict__ packed, uint8_t* __restrict__ sf_lin,
-                     uint8_t* __restrict__ sf_tiled, float* __restrict__ scale_out,
-                     int rows_per_group, FastDiv div_per_row, FastDiv div_nb, FastDiv div_spad) {
-  pdl_wait();
-  const TensorScale g = make_tensor_scale(*amax);
-  if (scale_out != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *scale_out = g.g;
-  const int nb = D / 16, ct = D / 64;
-  const int rt = (S + 127) / 128, s_pad = rt * 128;
-  const int rows = B * s_pad;
-  const int per_row = H * nb;
-  const int per_group = rows_per_group * per_row;
-  const int row0 = blockIdx.x * rows_per_group;
-  // Every lane of a warp runs the same number of iterations (shuffles below).  kBatch items per
-  // thread are loaded before any is processed (2 measured the same, 4 slower: the ALU and FMA
-  // pipes are 55-66 % busy and two thirds of the issue slots are used; loads in flight are not
-  // what limits it).
-  constexpr int kBatch = 1;
-  const int iters = (per_group + 256 * kBatch - 1) / (256 * kBatch);
-  for (int it = 0; it < iters; ++it) {
-    uint4 raw[kBatch][2];
-    int s_of[kBatch], b_of[kBatch], h_of[kBatch], c_of[kBatch];
-    bool in_range[kBatch];
-#pragma unroll
-    for (int k = 0; k < kBatch; ++k) {
-      const int item = (it * kBatch + k) * 256 + threadIdx.x;
-      const int lr = fast_div(item, div_per_row), within = item - lr * per_row;
-      const int row = row0 + lr;
-      h_of[k] = fast_div(within, div_nb);
-      c_of[k] = within - h_of[k] * nb;
-      b_of[k] = fast_div(row, div_spad);
-      s_of[k] = row - b_of[k] * s_pad;
-      in_range[k] = item < per_group && row < rows;
-      raw[k][0] = raw[k][1] = make_uint4(0u, 0u, 0u, 0u);
-      if (in_range[k] && s_of[k] < S) {
-        const __nv_bfloat16* src = x + b_of[k] * sb + s_of[k] * ss + h_of[k] * sh + c_of[k] * 16;
-        raw[k][0] = *reinterpret_cast<const uint4*>(src);
-        raw[k][1] = *reinterpret_cast<const uint4*>(src + 8);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < kBatch; ++k) {
-      const int s = s_of[k], b = b_of[k], h = h_of[k], c = c_of[k];
-      uint32_t lo = 0, hi = 0, sfb = 0;
-      if (in_range[k] && s < S) {
-        float v[16];
-        unpack_bf16x8(raw[k][0], v);
-        unpack_bf16x8(raw[k][1], v + 8);
-        quantize_block16(v, g, lo, hi, sfb);
-        const int64_t orow = ((int64_t)b * S + s) * H + h;
-        *reinterpret_cast<uint2*>(packed + (orow * nb + c) * 8) = make_uint2(lo, hi);
-      }
-      // four neighbouring lanes hold the four scale bytes of one word
-      uint32_t word = sfb << (8 * (c & 3));
-      word |= __shfl_xor_sync(0xffffffffu, word, 1);
-      word |= __shfl_xor_sync(0xffffffffu, word, 2);
-      if (in_range[k] && (c & 3) == 0) {
-        if (sf_lin != nullptr && s < S) {
-          const int64_t orow = ((int64_t)b * S + s) * H + h;
-          *reinterpret_cast<uint32_t*>(sf_lin + orow * nb + c) = word;
-        }
-        if (sf_tiled != nullptr) {
-          const int64_t chunk = (((int64_t)b * H + h) * rt + s / 128) * ct + c / 4;
-          const int rr = s % 128;
-          *reinterpret_cast<uint32_t*>(sf_tiled + chunk * 512 + (rr % 32) * 16 + (rr / 32) * 4) = word;
-        }
-      }
-    }
-  }
+
+// Where a Q / K work item lies.
+struct RowsItem {
+  const __nv_bfloat16* src;     // block (b, s0, h, c)
+  int b, rt, l, h, c, s0;
+};
+__device__ __forceinline__ RowsItem rows_item_at(const QuantJob& j, uint32_t item, int k0) {
+  RowsItem it;
+  const int rest = fast_div((int)item, j.div_nb), col = (int)item - rest * j.nb, bt = rest >> 5;
+  it.l = rest & 31;
+  it.b = fast_div(bt, j.div_rt);
+  it.rt = bt - it.b * j.rt;
+  it.h = fast_div(col, j.div_h);
+  it.c = col - it.h * (j.D >> 4);
+  it.s0 = it.rt * 128 + k0 * 32 + it.l;
+  it.src = j.x + it.b * j.sb + it.s0 * j.ss + it.h * j.sh + it.c * 16;
+  return it;
 }
 
-// ---------------------------------------------------------------------------------------------
-// V: x (B, Sk, H, Dv) bf16 -> key-contiguous packed (B, H, Dv, Sk/2), blocks along the keys.
-// One CTA transposes a tile of 128 keys x 128 d through shared memory (16-byte chunks swizzled
-// by the key block so that both the row-wise fill and the column-wise reads are conflict free).
-// One thread = two neighbouring d rows x one block of 16 keys.
-//   sf_lin    (B, H, Dv, Sk/16) contiguous, or null
-//   sf_tiled  (B, H, ceil(Dv/128), 2 * ceil(Sk/128), 512), or null
-// Sk is a multiple of 16 and Dv a multiple of 8.  grid = (ceil(Sk/128), ceil(Dv/128), B * H).
-// ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-quantize_v_kernel(const __nv_bfloat16* __restrict__ x, int B, int Sk, int H, int Dv, int64_t sb,
-                  int64_t ss, int64_t sh, const float* __restrict__ amax,
-                  uint8_t* __restrict__ packed, uint8_t* __restrict__ sf_lin,
-                  uint8_t* __restrict__ sf_tiled, float* __restrict__ scale_out) {
-  __shared__ __align__(16) uint8_t tile[128 * 256];  // [key][16 chunks of 16 B], chunk ^ (key/16)
-  pdl_wait();
-  const TensorScale g = make_tensor_scale(*amax);
-  if (scale_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 &&
-      threadIdx.x == 0)
-    *scale_out = g.g;
-  const int k0 = blockIdx.x * 128, d0 = blockIdx.y * 128;
-  const int b = blockIdx.z / H, h = blockIdx.z % H;
-  const int tid = threadIdx.x;
-
-  // fill: 128 keys x 16 chunks of 8 d values; zero outside the tensor
+// kRows = 4: the item's four rows; 1: row k0 of them (tensors too small to fill the GPU otherwise).
+// `raw` holds the item's rows; each is refilled with the row of the next item as soon as it has been
+// unpacked, so that its latency passes behind the arithmetic without a second set of registers.
+template <int kRows>
+__device__ __forceinline__ void quantize_rows_item(const QuantJob& j, const RowsItem& it, int k0, Words8 (&raw)[kRows],
+                                                   const RowsItem& next, bool has_next, const TensorScale& ts) {
+  const bool wide = j.wide != 0;
+  const int col = it.h * (j.D >> 4) + it.c;
+  uint8_t* dst = j.packed + (((int64_t)it.b * j.S + it.s0) * j.nb + col) * 8;
+  uint32_t bytes = 0u;          // byte k: the scale of row k
 #pragma unroll
-  for (int i = tid; i < 128 * 16; i += 256) {
-    const int key = i >> 4, ch = i & 15;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (k0 + key < Sk && d0 + ch * 8 < Dv)
-      v = *reinterpret_cast<const uint4*>(x + b * sb + (int64_t)(k0 + key) * ss + h * sh + d0 + ch * 8);
-    *reinterpret_cast<uint4*>(tile + key * 256 + ((ch ^ (key >> 4)) << 4)) = v;
+  for (int k = 0; k < kRows; ++k) {
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[2 * i] = __uint_as_float(raw[k].w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(raw[k].w[i] & 0xffff0000u);
+    }
+    const float bmax = absmax16(raw[k]);
+    if (has_next && next.s0 + 32 * k < j.S) raw[k] = load32(next.src + 32 * k * j.ss, wide);
+    if (it.s0 + 32 * k < j.S) {
+      uint32_t lo, hi, sfb;
+      quantize_block16(v, bmax, ts, lo, hi, sfb);
+      bytes |= sfb << (8 * k);
+      *reinterpret_cast<uint2*>(dst + (int64_t)(256 * k) * j.nb) = make_uint2(lo, hi);
+    }
+  }
+  // Four neighbouring lanes hold the four columns of a scale word.  kRows = 4: transpose the 4 x 4
+  // bytes between them, so that lane q ends up with the word of row q and all four store.
+  const int q = it.c & 3;
+  int row = k0;
+  bool mine = true;
+  if (kRows == 4) {
+    uint32_t p = __shfl_xor_sync(0xffffffffu, bytes, 1);
+    bytes = __byte_perm(bytes, p, (q & 1) ? 0x3715 : 0x6240);
+    p = __shfl_xor_sync(0xffffffffu, bytes, 2);
+    bytes = __byte_perm(bytes, p, (q & 2) ? 0x3276 : 0x5410);
+    row = q;
+  } else {
+    bytes <<= 8 * q;
+    bytes |= __shfl_xor_sync(0xffffffffu, bytes, 1);
+    bytes |= __shfl_xor_sync(0xffffffffu, bytes, 2);
+    mine = q == 0;
+  }
+  const int s = it.rt * 128 + row * 32 + it.l;
+  if (mine && j.lin != nullptr && s < j.S)
+    *reinterpret_cast<uint32_t*>(j.lin + ((int64_t)it.b * j.S + s) * j.nb + (col & ~3)) = bytes;
+  if (mine && j.tiled != nullptr)
+    *reinterpret_cast<uint32_t*>(j.tiled + ((((int64_t)it.b * j.H + it.h) * j.rt + it.rt) * (j.D >> 6) + (it.c >> 2)) * 512 +
+                                 it.l * 16 + row * 4) = bytes;
+}
+
+// Where a V tile lies, and this thread's eight 16-byte pieces of it (128 keys x 16 chunks of 8 d).
+struct VTile {
+  int hd, kb0, bh, d0;
+};
+__device__ __forceinline__ VTile v_tile_at(const QuantJob& j, int tile_idx) {
+  VTile t;
+  const int dt = (j.D + 127) / 128;
+  t.hd = fast_div(tile_idx, j.div_rt);
+  t.kb0 = tile_idx - t.hd * j.rt;                  // key tile inside (b, h, d tile)
+  t.bh = t.hd / dt;
+  t.d0 = (t.hd - t.bh * dt) * 128;
+  return t;
+}
+__device__ __forceinline__ void load_v_tile(const QuantJob& j, const VTile& t, uint4 (&v)[8]) {
+  const int b = fast_div(t.bh, j.div_h), h = t.bh - b * j.H;
+  const __nv_bfloat16* src = j.x + b * j.sb + h * j.sh + t.d0;
+#pragma unroll
+  for (int n = 0; n < 8; ++n) {
+    const int i = threadIdx.x + 256 * n, key = t.kb0 * 128 + (i >> 4), ch = i & 15;
+    v[n] = make_uint4(0u, 0u, 0u, 0u);             // zero outside the tensor
+    if (key < j.S && t.d0 + ch * 8 < j.D) v[n] = *reinterpret_cast<const uint4*>(src + (int64_t)key * j.ss + ch * 8);
+  }
+}
+// `raw` is refilled with the CTA's next tile once it has been stored to shared memory.
+__device__ __forceinline__ void quantize_v_tile(const QuantJob& j, const VTile& t, uint4 (&raw)[8], const VTile& next,
+                                                bool has_next, const TensorScale& ts, uint8_t* tile) {
+  const int kt = j.rt, Sk = j.s_out, Dv = j.D, d0 = t.d0, k0 = t.kb0 * 128, tid = threadIdx.x;
+#pragma unroll
+  for (int n = 0; n < 8; ++n) {
+    const int i = tid + 256 * n, key = i >> 4, ch = i & 15;
+    *reinterpret_cast<uint4*>(tile + key * 256 + ((ch ^ (key >> 4)) << 4)) = raw[n];
   }
   __syncthreads();
-
+  if (has_next) load_v_tile(j, next, raw);
   const int n_kb_total = Sk / 16;
-  const int kt = (Sk + 127) / 128;  // 128-key tiles
-  const int dt = (Dv + 127) / 128;
 #pragma unroll 1
   for (int item = tid; item < 64 * 8; item += 256) {
     const int kb = item & 7, dp = item >> 3;  // key block inside the tile, d pair
     const int d = d0 + 2 * dp;
+    if (d0 + 2 * (dp & ~3) >= Dv && j.tiled == nullptr) continue;   // (whole groups of lanes: shuffles below)
     const int ch = dp >> 2, within = (dp & 3) * 4;  // chunk and byte offset of the d pair
     float v0[16], v1[16];
+    uint32_t m2 = 0u;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int key = 16 * kb + j;
-      const uint32_t w =
-          *reinterpret_cast<const uint32_t*>(tile + key * 256 + ((ch ^ kb) << 4) + within);
-      v0[j] = __uint_as_float(w << 16);
-      v1[j] = __uint_as_float(w & 0xffff0000u);
+    for (int i = 0; i < 16; ++i) {
+      const uint32_t w = *reinterpret_cast<const uint32_t*>(tile + (16 * kb + i) * 256 + ((ch ^ kb) << 4) + within);
+      v0[i] = __uint_as_float(w << 16);
+      v1[i] = __uint_as_float(w & 0xffff0000u);
+      m2 = absmax2(m2, w);
     }
     uint32_t lo0, hi0, sf0, lo1, hi1, sf1;
-    quantize_block16(v0, g, lo0, hi0, sf0);
-    quantize_block16(v1, g, lo1, hi1, sf1);
+    quantize_block16(v0, fabsf(__uint_as_float(m2 << 16)), ts, lo0, hi0, sf0);
+    quantize_block16(v1, fabsf(__uint_as_float(m2 & 0xffff0000u)), ts, lo1, hi1, sf1);
     const bool key_ok = k0 + 16 * kb < Sk;
-    const int64_t row0 = ((int64_t)b * H + h) * Dv + d;
+    const int64_t row0 = (int64_t)t.bh * Dv + d;
     if (key_ok && d < Dv)
-      *reinterpret_cast<uint2*>(packed + row0 * (Sk / 2) + (k0 + 16 * kb) / 2) = make_uint2(lo0, hi0);
+      *reinterpret_cast<uint2*>(j.packed + row0 * (Sk / 2) + (k0 + 16 * kb) / 2) = make_uint2(lo0, hi0);
     if (key_ok && d + 1 < Dv)
-      *reinterpret_cast<uint2*>(packed + (row0 + 1) * (Sk / 2) + (k0 + 16 * kb) / 2) =
-          make_uint2(lo1, hi1);
+      *reinterpret_cast<uint2*>(j.packed + (row0 + 1) * (Sk / 2) + (k0 + 16 * kb) / 2) = make_uint2(lo1, hi1);
     // scale bytes: lanes kb = 4 q .. 4 q + 3 hold one word of either layout
     if (!key_ok) sf0 = sf1 = 0;
     uint32_t w0 = sf0 << (8 * (kb & 3)), w1 = sf1 << (8 * (kb & 3));
@@ -345,9 +420,9 @@ quantize_v_kernel(const __nv_bfloat16* __restrict__ x, int B, int Sk, int H, int
     w1 |= __shfl_xor_sync(0xffffffffu, w1, 2);
     if ((kb & 3) == 0) {
       const int kb_global = k0 / 16 + kb;
-      if (sf_lin != nullptr && kb_global < n_kb_total) {
+      if (j.lin != nullptr && kb_global < n_kb_total) {
         // a word may run past the row's end when Sk/16 is not a multiple of 4: byte stores there
-        uint8_t* p0 = sf_lin + row0 * n_kb_total + kb_global;
+        uint8_t* p0 = j.lin + row0 * n_kb_total + kb_global;
         const int nvalid = n_kb_total - kb_global < 4 ? n_kb_total - kb_global : 4;
         if (nvalid == 4 && (n_kb_total & 3) == 0) {
           if (d < Dv) *reinterpret_cast<uint32_t*>(p0) = w0;
@@ -359,14 +434,95 @@ quantize_v_kernel(const __nv_bfloat16* __restrict__ x, int B, int Sk, int H, int
           }
         }
       }
-      if (sf_tiled != nullptr) {
+      if (j.tiled != nullptr) {
         // d rows past Dv inside the 128-row tile get their zero padding here as well
-        const int64_t chunk =
-            ((((int64_t)b * H + h) * dt + blockIdx.y) * (2 * kt) + 2 * blockIdx.x + kb / 4);
+        const int64_t chunk = (int64_t)t.hd * (2 * kt) + 2 * t.kb0 + kb / 4;
         const int r0 = 2 * dp, r1 = 2 * dp + 1;
-        uint8_t* base = sf_tiled + chunk * 512;
+        uint8_t* base = j.tiled + chunk * 512;
         *reinterpret_cast<uint32_t*>(base + (r0 % 32) * 16 + (r0 / 32) * 4) = d < Dv ? w0 : 0u;
         *reinterpret_cast<uint32_t*>(base + (r1 % 32) * 16 + (r1 / 32) * 4) = d + 1 < Dv ? w1 : 0u;
+      }
+    }
+  }
+}
+
+constexpr int kQuantizeCtas = 2;     // per SM
+constexpr int kQuantizeVWeight = 24; // cost of a byte of V, that of Q and K being 16
+__global__ void __launch_bounds__(256, kQuantizeCtas)
+quantize_kernel(const __grid_constant__ QuantJobs jobs) {
+  __shared__ __align__(16) uint8_t tile[128 * 256];  // [key][16 chunks of 16 B], chunk ^ (key/16)
+  __shared__ float warp_max[8];
+  int ji = 0;
+  while (ji + 1 < jobs.n && (int)blockIdx.x >= jobs.job[ji + 1].block0) ++ji;
+  const QuantJob& j = jobs.job[ji];
+  const int lane = threadIdx.x & 31;
+  pdl_wait();
+  // the first loads of the tensor go out before the partial maxima are read: one latency, not two
+  const int first = blockIdx.x - j.block0, per_round = j.blocks * 256;
+  const int quarter = (int)(j.items >> 2);
+  // Q / K: the CTA's item of the round (below zero: past the front of the tensor); V: its tile
+  int t = (int)j.items - (j.is_v ? first + 1 : 256 * (first + 1) - (int)threadIdx.x);
+  int k0 = 0;
+  VTile vt;
+  RowsItem it;
+  union {
+    uint4 v[8];
+    Words8 rows[4];
+  } raw;
+  if (j.is_v) {
+    vt = v_tile_at(j, t);
+    load_v_tile(j, vt, raw.v);
+  } else if (t >= 0) {
+    if (j.single) {
+      k0 = t / quarter;
+      t -= k0 * quarter;
+    }
+    it = rows_item_at(j, t, k0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if ((k == 0 || !j.single) && it.s0 + 32 * k < j.S) raw.rows[k] = load32(it.src + 32 * k * j.ss, j.wide != 0);
+  }
+  float m = 0.f;
+  for (int i = threadIdx.x; i < j.num_parts; i += 256) m = fmaxf(m, j.parts[i]);
+  if (j.num_parts > 1) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) warp_max[threadIdx.x >> 5] = m;
+    __syncthreads();
+    m = warp_max[0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) m = fmaxf(m, warp_max[w]);
+  } else {
+    m = j.parts[0];
+  }
+  const TensorScale ts = make_tensor_scale(m);
+  if (first == 0 && threadIdx.x == 0) {
+    if (j.scale_out != nullptr) *j.scale_out = ts.g;
+    if (j.scale_host != nullptr) *j.scale_host = ts.g;
+  }
+  if (j.is_v) {
+#pragma unroll 1
+    for (;;) {
+      const int tn = t - j.blocks;
+      const VTile next = v_tile_at(j, tn >= 0 ? tn : t);
+      quantize_v_tile(j, vt, raw.v, next, tn >= 0, ts, tile);
+      if (tn < 0) break;
+      __syncthreads();            // the transpose buffer is read out
+      vt = next;
+      t = tn;
+    }
+  } else if (t >= 0) {            // (items come in whole warps; lanes ascend with the blocks)
+    if (j.single) {
+      quantize_rows_item<1>(j, it, k0, *reinterpret_cast<Words8(*)[1]>(&raw.rows[0]), it, false, ts);
+    } else {
+#pragma unroll 1
+      for (;;) {
+        const int tn = t - per_round;
+        const RowsItem next = rows_item_at(j, tn >= 0 ? tn : t, 0);
+        quantize_rows_item<4>(j, it, 0, raw.rows, next, tn >= 0, ts);
+        if (tn < 0) break;
+        it = next;
+        t = tn;
       }
     }
   }

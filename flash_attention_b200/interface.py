@@ -189,14 +189,15 @@ def flash_attn_func(
     if mask_mod is not None or any(t is not None for t in (full_block_cnt, full_block_idx,
                                                            mask_block_cnt, mask_block_idx)):
         raise NotImplementedError("mask_mod / block sparsity is not built")
-    layouts = {t.tiled for t in (q, k, v)}
-    if len(layouts) != 1 or any(t.sf_tiled is not None for t in (q, k, v)):
-        q, k, v = (NVFP4Tensor(t.data, t.tiled_sf(), t.scale, True, t.is_v) for t in (q, k, v))
-    return flash_attn_fp4_func(
-        q.data, k.data, v.data, q.sf, k.sf, v.sf, q.scale, k.scale, v.scale,
-        softmax_scale=softmax_scale, causal=causal, return_lse=return_lse,
-        sf_layout="tiled" if q.tiled else "linear", num_splits=num_splits, window_size=tuple(window_size),
-        learnable_sink=learnable_sink, softcap=0.0 if softcap is None else softcap)
+    if q.tiled or k.tiled or v.tiled or q.sf_tiled is not None or k.sf_tiled is not None or v.sf_tiled is not None:
+        layout, q_sf, k_sf, v_sf = "tiled", q.tiled_sf(), k.tiled_sf(), v.tiled_sf()
+    else:
+        layout, q_sf, k_sf, v_sf = "linear", q.sf, k.sf, v.sf
+    win_left, win_right = window_size
+    # (_scale: a scale the quantiser has not delivered to the host yet is used where it is, on the device)
+    return _lib.host().fwd(q.data, k.data, v.data, q_sf, k_sf, v_sf, q._scale, k._scale, v._scale, softmax_scale, causal,
+                           return_lse, None, None, layout, VARIANT_AUTO, num_splits, win_left, win_right,
+                           learnable_sink, softcap, None, None)
 
 
 def measure_fp4_mma_rate(iters: int = 1 << 16, device=None, repeats: int = 3) -> dict:

@@ -194,6 +194,14 @@ typedef struct fa4_nvfp4_ext {
 int fa4_nvfp4_fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, void* cuda_stream);
 
 /*
+ * fa4_nvfp4_fwd_ex with the three per-tensor scales in DEVICE memory (p->q_scale, k_scale, v_scale
+ * are not read): for callers that quantise and attend on one stream without waiting for the scales
+ * on the host.  Every scale must be > 0 (the quantiser's are).  Same bits as with host scales.
+ */
+int fa4_nvfp4_fwd_device_scales(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, const float* q_scale,
+                                const float* k_scale, const float* v_scale, void* cuda_stream);
+
+/*
  * Packed variable-length batches in ONE launch: the reference's flash_attn_varlen_func
  * (flash_attn/cute/interface.py:1795-1840; its persistent varlen scheduler is
  * flash_attn/cute/tile_scheduler.py:755-1087).  q, k, v, out of `p` have no batch dimension:
@@ -336,6 +344,26 @@ int fa4_nvfp4_quantize_v_bf16(const void* x, int32_t B, int32_t Sk, int32_t H, i
                               int64_t stride_b, int64_t stride_s, int64_t stride_h,
                               const float* amax, void* packed, void* sf_linear, void* sf_tiled,
                               float* scale_out, void* cuda_stream);
+
+/*
+ * The two passes for one to three tensors (the q, k and v of a call) in two launches in all.  A job
+ * is one tensor; is_v: blocks along the key axis, which is stored S_out long (a multiple of 16, at
+ * least S; zeros from S on).  `scratch`: device memory for FA4_QUANT_SCRATCH_FLOATS floats, in use
+ * until the launches have run; *scale_out receives the tensor scale.  Outputs as above.
+ */
+#define FA4_QUANT_SCRATCH_FLOATS 1024
+typedef struct fa4_nvfp4_quant_job {
+  const void* x;
+  int64_t stride_b, stride_s, stride_h;
+  int32_t B, S, H, D;
+  int32_t is_v, S_out;
+  void* packed;
+  void* sf_linear;   /* or NULL */
+  void* sf_tiled;    /* or NULL */
+  float* scale_out;  /* device, or NULL */
+  float* scale_host; /* the same in device-accessible (pinned) host memory, or NULL */
+} fa4_nvfp4_quant_job;
+int fa4_nvfp4_quantize_jobs_bf16(const fa4_nvfp4_quant_job* jobs, int32_t n, float* scratch, void* cuda_stream);
 
 /*
  * Hardware-contract probe: one 128x128xD block-scaled tile S = A * B^T with
