@@ -531,7 +531,14 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     if (variant == FA4_VARIANT_WS64) {
       auto launch64 = [&](auto kernel) -> int {
         if (int e = ensure_kernel(kernel, ws64::kSmemRequest, ws64::kRegsLaunch)) return e;
-        return launch_pdl(kernel, dim3(grid), ws64::kThreads, ws64::kSmemRequest, stream, tm_q, tm_k, tm_v, tm_o, kp);
+        // as many launches as the per-CTA tile table asks for (one up to 113 664 tiles on 148 SMs)
+        for (uint32_t begin = 0; begin < tiles; begin += grid * ws64::kMaxTiles) {
+          kp.tile_begin = (int)begin;
+          kp.tile_end = (int)(tiles - begin < grid * ws64::kMaxTiles ? tiles : begin + grid * ws64::kMaxTiles);
+          if (int e = launch_pdl(kernel, dim3(grid), ws64::kThreads, ws64::kSmemRequest, stream, tm_q, tm_k, tm_v, tm_o, kp))
+            return e;
+        }
+        return 0;
       };
       if (general && local) {   // window (with or without sink / softcap / cache view)
         rc = p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, true>)

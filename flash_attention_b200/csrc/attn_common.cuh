@@ -42,6 +42,7 @@ struct KernelParams {
   FastDiv div_tiles_per_m;   // Hq * B
   FastDiv div_hq, div_group, div_splits;
   int num_m_blocks, num_n_blocks;
+  int tile_begin, tile_end;  // the part of the tile list this launch works on (64-key kernel)
   int causal;
   float sl2;        // softmax_scale * q_scale * k_scale * log2(e)
   float out_scale;  // v_scale
@@ -145,15 +146,7 @@ __device__ __forceinline__ int key_len(const KernelParams& p, const Tile& t) {
 // kGeneral = false: the work list is the tile list (num_splits == 1) and the only masks are
 // causal / key length; kept as a compile-time switch so that the common case carries none of the
 // split or window arithmetic or registers.
-// kFast: the three divisions of the tile index as multiply-high + shift instead of the hardware's
-// division sequence (about 35 instructions each).  Every warp decodes every tile, so for tiles of
-// a few K/V blocks the divisions are a visible share of the work: 1024-token sequences and
-// 1024-key windows run 8-20 % faster with them.  Measured as well: the single-lane service warps
-// of the 64-key kernel (producer, issuers, scale copier) are better left on the slow form in the
-// plain instantiation -- with the fast form there the long-tile workloads lose 1-2 % (the warps
-// reach their next wait sooner and spend the difference polling), while the softmax and epilogue
-// warps gain 1 % from it.
-template <bool kGeneral = false, bool kFast = true>
+template <bool kGeneral = false>
 __device__ __forceinline__ Tile decode_tile(const KernelParams& p, int tile_idx) {
   Tile t;
   t.split = 0;
@@ -163,11 +156,11 @@ __device__ __forceinline__ Tile decode_tile(const KernelParams& p, int tile_idx)
     tile_idx = whole;
   }
   const int per_m = p.Hq * p.B;
-  const int m_rev = kFast ? fast_div(tile_idx, p.div_tiles_per_m) : tile_idx / per_m;
+  const int m_rev = fast_div(tile_idx, p.div_tiles_per_m);
   const int rem = tile_idx - m_rev * per_m;
-  t.b = kFast ? fast_div(rem, p.div_hq) : rem / p.Hq;
+  t.b = fast_div(rem, p.div_hq);
   t.h = rem - t.b * p.Hq;
-  t.hk = kFast ? fast_div(t.h, p.div_group) : t.h / p.group;
+  t.hk = fast_div(t.h, p.div_group);
   t.m_blk = p.causal ? (p.num_m_blocks - 1 - m_rev) : m_rev;
   t.sk = p.Sk;
   t.sq = p.Sq;

@@ -66,7 +66,7 @@ struct Bars {
   __device__ __forceinline__ uint32_t at(uint32_t idx) const { return base + 8u * idx; }
 };
 constexpr uint32_t kOffMisc = kOffBar + 8 * Bars::kCount;
-constexpr uint32_t kSmemRequest = kOffMisc + 16 + 1024;
+constexpr uint32_t kSmemRequest = kOffMisc + 16 + sizeof(WaitCtx) + 1024;
 // The 32-row form allocates 256 tensor-memory columns: its request is padded so that only two CTAs
 // fit an SM (a third would sit inside tcgen05.alloc until one of them ends).
 constexpr uint32_t kSmemRequestWide = 100 * 1024;
@@ -221,11 +221,12 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-  const WaitCtx wc{s_abort, p.status, p.budget_ns, p.epoch};
+  WaitCtx& wc = *reinterpret_cast<WaitCtx*>(gbase + kOffMisc + 16);
   const int R = p.Sq * p.group;  // live query rows (<= kR)
 
   if (tid == 0) {
     *s_abort = 0u;
+    wc = WaitCtx{s_abort, p.status, p.budget_ns, p.epoch};
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bars.at(Bars::kKFull + s), 1);
       mbar_init(bars.at(Bars::kVFull + s), 1);

@@ -119,7 +119,7 @@ constexpr uint32_t kOffFin = kOffStats + 2 * 128 * 48;         // 2 tiles x 4 WG
 constexpr uint32_t kOffBar = kOffFin + 2 * 4 * 128 * 8;
 constexpr int kNumBars = 4 + 2 * kStagesK + 2 * kStagesV + 2 * 3 + kStagesP + 4 + 2;
 constexpr uint32_t kOffMisc = kOffBar + 8 * kNumBars;          // tmem slot, abort flag
-constexpr uint32_t kSmemUsed = kOffMisc + 16;
+constexpr uint32_t kSmemUsed = kOffMisc + 16 + sizeof(WaitCtx);
 constexpr uint32_t kSmemRequest = kSmemUsed + 1024;
 static_assert(kSmemRequest > 114 * 1024, "one CTA per SM: every CTA allocates all of tensor memory");
 
@@ -146,9 +146,9 @@ static_assert(Bars::kCount <= kNumBars, "barrier area too small");
 
 // Probe first, block (bounded) only if the probe failed; result is warp-uniform.
 __device__ __forceinline__ bool wait_probed(bool probed, uint32_t bar, uint32_t parity,
-                                            const WaitCtx& wc, uint32_t site) {
+                                            const volatile uint32_t* s_abort) {
   if (__all_sync(0xffffffffu, probed)) return true;
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, wc, site));
+  return __all_sync(0xffffffffu, mbar_wait_flag(bar, parity, s_abort));
 }
 
 // O[:, 32 * nchunks columns from taddr] *= f for this thread's row.  Rare (the reference maximum
@@ -308,12 +308,13 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const WaitCtx wc{s_abort, p.status, p.budget_ns, p.epoch};
+  WaitCtx& wc = *reinterpret_cast<WaitCtx*>(gbase + kOffMisc + 16);
   const int num_tiles = p.num_m_blocks * p.Hq * p.B * (kGeneral ? p.num_splits : 1);
   const int ncta = gridDim.x, cta = blockIdx.x;
 
   if (tid == 0) {
     *s_abort = 0u;
+    wc = WaitCtx{s_abort, p.status, p.budget_ns, p.epoch};
     for (int b = 0; b < 2; ++b) {
       mbar_init(bars.at(Bars::kQFull + b), 1);
       mbar_init(bars.at(Bars::kQEmpty + b), 1);
@@ -612,7 +613,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         const uint32_t bar_f = bars.at(Bars::kStFree + b), par_f = ((G - 2) >> 1) & 1;
         const bool r_s = mbar_test(bar_s, par_s);
         const bool r_f = (G >= 2) ? mbar_test(bar_f, par_f) : true;
-        ok = wait_probed(r_s, bar_s, par_s, wc, kSiteSFull);
+        ok = wait_probed(r_s, bar_s, par_s, s_abort);
         if (!ok) break;
         tc_fence_after_sync();
         const bool masked = block_needs_mask<kGeneral, kWindow>(p, t, nb);
@@ -663,7 +664,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         const float m_prev = m_run;
         m_run = m_new;
         // the slot is free once the softmax warpgroups of block G-2 have read it
-        ok = wait_probed(r_f, bar_f, par_f, wc, kSiteStFree);
+        ok = wait_probed(r_f, bar_f, par_f, s_abort);
         if (!ok) break;
         uint4* dst = reinterpret_cast<uint4*>(&s_stats[b * 128 + row]);
         dst[0] = make_uint4(__float_as_uint(bm[0]), __float_as_uint(bm[1]), __float_as_uint(bm[2]),
@@ -710,7 +711,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         // 1. the statistics of this block are published only after its Q K^T has completed and
         //    been read by the statistics warps (which waited on s_full and fenced), so this one
         //    wait covers the scores as well; it saves a barrier round trip per block
-        ok = wait_probed(mbar_test(bar_r, par_r), bar_r, par_r, wc, kSiteStReady);
+        ok = wait_probed(mbar_test(bar_r, par_r), bar_r, par_r, s_abort);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t s_addr = lane_addr + (b ? kTmS1 : kTmS0) + 64 * half;
@@ -750,7 +751,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
 
         // 3. exponentials and quantisation; P tile G % kStagesP is free once PV of block
         //    G - kStagesP has completed
-        ok = wait_probed(r_p, bar_p, par_p, wc, kSitePvDone);
+        ok = wait_probed(r_p, bar_p, par_p, s_abort);
         if (!ok) break;
         uint8_t* p_tile = gbase + kOffP + (G % kStagesP) * kTileBytes;
         uint4 chunk;
@@ -768,8 +769,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         //    0..i-1 relative to m_prev and must move to m_new before PV of this block is issued,
         //    i.e. before the arrival on p_full; this warpgroup rescales its 64 columns of O
         if (i > 0 && __any_sync(0xffffffffu, m_new != m_prev)) {
-          ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kPvDone + ((G - 1) % kStagesV)),
-                                                 ((G - 1) / kStagesV) & 1, wc, kSitePvDone));
+          ok = __all_sync(0xffffffffu, mbar_wait_flag(bars.at(Bars::kPvDone + ((G - 1) % kStagesV)),
+                                                 ((G - 1) / kStagesV) & 1, s_abort));
           if (!ok) break;
           tc_fence_after_sync();
           const float f = (m_new != m_prev) ? reference_factor(m_prev, m_new, sc.sl2) : 1.f;
@@ -793,7 +794,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         fin_slot[(slot * 128 + row) * 2] = l_sum;
         fin_slot[(slot * 128 + row) * 2 + 1] = m_ref;
         mbar_arrive(bars.at(Bars::kFin));
-        ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kFin), ti & 1, wc, kSiteFin));
+        ok = __all_sync(0xffffffffu, mbar_wait_flag(bars.at(Bars::kFin), ti & 1, s_abort));
         if (!ok) break;
         float lw[4], mw[4];
 #pragma unroll
@@ -814,7 +815,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
         const uint32_t Gl = gb + n - 1;
         ok = __all_sync(0xffffffffu,
-                        mbar_wait(bars.at(Bars::kPvDone + (Gl % kStagesV)), (Gl / kStagesV) & 1, wc, kSiteFinalO));
+                        mbar_wait_flag(bars.at(Bars::kPvDone + (Gl % kStagesV)), (Gl / kStagesV) & 1, s_abort));
         if (!ok) break;
         tc_fence_after_sync();
         scale = (l_tot > 0.f) ? sc.out_scale / l_tot : 0.f;
@@ -828,7 +829,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
       } else {
         if (it >= 1) {
           // the staging tile is free once the store warp's TMA has read the previous tile out of it
-          ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kStageFree), (it - 1) & 1, wc, kSiteStageFree));
+          ok = __all_sync(0xffffffffu, mbar_wait_flag(bars.at(Bars::kStageFree), (it - 1) & 1, s_abort));
           if (!ok) break;
         }
         if (kD == 128 || wg < kD / 32) {

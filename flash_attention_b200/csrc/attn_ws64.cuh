@@ -78,7 +78,8 @@ constexpr uint32_t kOffSFP = kOffSFV + kStagesV * kSfBytes;      // kPSlots x 51
 constexpr uint32_t kOffOut = kOffSFP + kPSlots * 512;            // 32 KB staging tile
 constexpr uint32_t kOffHand = kOffOut + 32 * 1024;               // kSBufs x 128 reference maxima
 constexpr uint32_t kOffFin = kOffHand + kSBufs * 128 * 4;        // 2 tiles x 4 WGs x 128 x (sum, ref)
-constexpr uint32_t kOffBar = kOffFin + 2 * 4 * 128 * 8;
+constexpr uint32_t kOffTiles = kOffFin + 2 * 4 * 128 * 8;       // kMaxTiles records
+constexpr uint32_t kOffBar = kOffTiles + kThreads * 32;
 
 struct Bars {
   uint32_t base;
@@ -93,7 +94,7 @@ struct Bars {
   __device__ __forceinline__ uint32_t at(uint32_t idx) const { return base + 8u * idx; }
 };
 constexpr uint32_t kOffMisc = kOffBar + 8 * Bars::kCount;
-constexpr uint32_t kSmemUsed = kOffMisc + 16;
+constexpr uint32_t kSmemUsed = kOffMisc + 16 + sizeof(WaitCtx);
 constexpr uint32_t kSmemRequest = kSmemUsed + 1024;
 static_assert(kSmemRequest <= 227 * 1024, "shared memory");
 
@@ -102,17 +103,68 @@ enum Site64 {
   kS64PFull, kS64PvDone, kS64Hand, kS64Fin, kS64FinFree, kS64FinalO, kS64OFree, kS64Ksf, kS64Vsf, kS64Epi
 };
 
+// The tiles of this CTA, decoded once at kernel start -- one thread per tile -- into a table in shared
+// memory that every role reads.  (Each of the seven roles used to decode every tile for itself: a few
+// hundred instructions that ran in all 24 warps at every tile change and, being seven copies, pushed
+// the rest of the kernel out of the instruction cache.)
+struct alignas(16) TileRec {
+  int m_blk, h, b;
+  int n;          // K/V blocks this tile visits; 0: none is visible; -1: the tile has no rows at all (packed batch)
+  int hk, sk;     // kv head; valid keys of the batch entry
+  int off;        // row r of the tile sees keys up to off + r (plus the right window limit)
+  int first;      // block the ascending visit starts at; negative: ~first, and the two blocks of the left edge last
+};
+static_assert(sizeof(TileRec) == 32, "two 16-byte loads");
+constexpr int kMaxTiles = kThreads;   // per CTA and launch (the host launches longer lists in pieces)
+
 // Visit order of a windowed tile: the i-th visited 128-key block.  Ascending from the first block
 // the window reaches, EXCEPT that the two blocks at the window's left edge -- where the lower rows
 // of the tile see a few keys or none, so that references taken there would be low -- are visited
 // last: a tile starts at a block every row sees whole.  (The right edge, the diagonal, is last in
-// ascending order anyway.)  rotate: the tile is cut on the left and has more than two blocks.
-__device__ __forceinline__ int window_visit_block(int i, int n, int nb_lo, bool rotate) {
-  if (!rotate) return nb_lo + i;
-  return i < n - 2 ? nb_lo + 2 + i : nb_lo + (i - (n - 2));
+// ascending order anyway.)
+__device__ __forceinline__ int window_visit_block(int i, const TileRec& t) {
+  if (t.first >= 0) return t.first + i;
+  const int lo = ~t.first;
+  return i < t.n - 2 ? lo + 2 + i : lo + (i - (t.n - 2));
 }
-__device__ __forceinline__ bool window_rotates(const KernelParams& p, const Tile& t) {
-  return p.win_left >= 0 && t.n_blocks > 2 && (t.m_blk * kBlockM + t.sk - t.sq - p.win_left) > 0;
+template <bool kGeneral>
+__device__ __forceinline__ TileRec make_tile_rec(const KernelParams& p, int tile_idx) {
+  const Tile t = decode_tile<kGeneral>(p, tile_idx);
+  TileRec r;
+  r.m_blk = t.m_blk;
+  r.h = t.h;
+  r.b = t.b;
+  r.n = t.n_blocks;
+  r.hk = t.hk;
+  r.sk = key_len<kGeneral>(p, t);
+  r.off = t.m_blk * kBlockM + r.sk - query_len<kGeneral>(p, t);
+  r.first = t.nb_top - t.n_blocks + 1;
+  if constexpr (kGeneral) {
+    if (p.win_left >= 0 && r.n > 2 && r.off - p.win_left > 0) r.first = ~r.first;
+    if (t.m_blk * kBlockM >= t.sq) r.n = -1;
+  } else {
+    r.first = 0;
+  }
+  return r;
+}
+// Last visible key of row `row` inside block nb (>= 127: no mask), the first one, and whether any row of
+// the tile needs a mask there (see causal_limit, lower_limit and block_needs_mask in attn_common.cuh).
+template <bool kWindow>
+__device__ __forceinline__ int upper_key(const KernelParams& p, const TileRec& t, int row, int nb) {
+  const int len = t.sk - 1 - nb * kBlockN;
+  if (!p.causal) return len;
+  const int c = t.off + row + (kWindow ? p.win_right : 0) - nb * kBlockN;
+  return c < len ? c : len;
+}
+__device__ __forceinline__ int lower_key(const KernelParams& p, const TileRec& t, int row, int nb) {
+  return p.win_left < 0 ? -(1 << 30) : t.off + row - p.win_left - nb * kBlockN;
+}
+template <bool kWindow>
+__device__ __forceinline__ bool needs_mask(const KernelParams& p, const TileRec& t, int nb) {
+  const int k0 = nb * kBlockN;
+  bool need = k0 + kBlockN > t.sk || (p.causal && k0 + kBlockN - 1 > t.off + (kWindow ? p.win_right : 0));
+  if constexpr (kWindow) need = need || (p.win_left >= 0 && k0 < t.off + kBlockM - 1 - p.win_left);
+  return need;
 }
 
 // byte offset of 16-byte chunk c (0, 1) of row r in a P tile (rows of 32 bytes, 32-byte swizzle)
@@ -146,7 +198,6 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   using ws::mask_scores_in_tmem;
   using ws::stage_accumulator_chunk;
   using ws::tile_of_round;
-  using ws::wait_probed;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
@@ -159,12 +210,13 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
-  const WaitCtx wc{s_abort, p.status, p.budget_ns, p.epoch};
-  const int num_tiles = p.num_m_blocks * p.Hq * p.B;
+  WaitCtx& wc = *reinterpret_cast<WaitCtx*>(gbase + kOffMisc + 16);
   const int ncta = gridDim.x, cta = blockIdx.x;
+  TileRec* s_tiles = reinterpret_cast<TileRec*>(gbase + kOffTiles);
 
   if (tid == 0) {
     *s_abort = 0u;
+    wc = WaitCtx{s_abort, p.status, p.budget_ns, p.epoch};
     for (int b = 0; b < 2; ++b) {
       mbar_init(bars.at(Bars::kQFull + b), 1);
       mbar_init(bars.at(Bars::kQEmpty + b), 1);
@@ -208,6 +260,11 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
   tc_fence_before_sync();
   pdl_wait();
+  // this CTA's tiles: p.tile_begin + tile_of_round(0), (1), ... below p.tile_end
+  {
+    const int tile = p.tile_begin + tile_of_round(tid, cta, ncta);
+    if (tile < p.tile_end) s_tiles[tid] = make_tile_rec<kWindow || kCache>(p, tile);
+  }
   __syncthreads();
   tc_fence_after_sync();
   pdl_trigger();
@@ -236,11 +293,13 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     return make_desc_sw32(tile + 4096 * j);
   };
 
+  // whole rounds, and the last partial one if it reaches this CTA
+  const int num_rounds = (p.tile_end - p.tile_begin) / ncta +
+                         (p.tile_begin + tile_of_round((p.tile_end - p.tile_begin) / ncta, cta, ncta) < p.tile_end ? 1 : 0);
 #define FA4_FOR_EACH_TILE                                                                        \
   uint32_t gb = 0, ti = 0;                                                                       \
   bool ok = true;                                                                                \
-  for (int it = 0, tile = tile_of_round(0, cta, ncta); ok && tile < num_tiles;                   \
-       ++it, tile = tile_of_round(it, cta, ncta))
+  for (int it = 0; ok && it < num_rounds; ++it)
 
   if (warp >= kEpilogueWarp0) {
     // =========================================== epilogue warpgroup =============================
@@ -258,21 +317,21 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     uint32_t epi_phase = 0;
 #define FA4_EPI_SYNC()                                                                              \
   mbar_arrive(bars.at(Bars::kEpi));                                                                 \
-  ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kEpi), epi_phase & 1, wc, kS64Epi));          \
+  ok = __all_sync(0xffffffffu, mbar_wait_flag(bars.at(Bars::kEpi), epi_phase & 1, s_abort));          \
   epi_phase += 1;                                                                                   \
   if (!ok) break;
     FA4_FOR_EACH_TILE {
-      const Tile t = decode_tile<kWindow || kCache>(p, tile);
-      const int n = t.n_blocks;
+      const TileRec t = s_tiles[it];
+      const int n = t.n;
       const int q_idx = t.m_blk * kBlockM + row;
       if constexpr (kWindow || kCache) {
         // a tile past the end of a short sequence of a packed batch has no rows at all
-        if (t.m_blk * kBlockM >= t.sq) continue;
+        if (n < 0) continue;
       }
       float scale = 0.f, m_fin = kNegInf, l_tot = 0.f;
       if (n > 0) {
         const uint32_t fb = ti & 1;
-        ok = __all_sync(0xffffffffu, mbar_wait_relaxed<kSlackNs>(bars.at(Bars::kFin + fb), (ti >> 1) & 1, wc, kS64Fin));
+        ok = __all_sync(0xffffffffu, mbar_wait_flag(bars.at(Bars::kFin + fb), (ti >> 1) & 1, s_abort));
         if (!ok) break;
         volatile float* fin_slot = s_fin + fb * (4 * 128 * 2);
         float lw[4], mw[4];
@@ -294,7 +353,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
         const uint32_t Jl = 2 * gb + 2 * n - 1;
         ok = __all_sync(0xffffffffu,
-                        mbar_wait(bars.at(Bars::kPvDone + (Jl % kPSlots)), (Jl / kPSlots) & 1, wc, kS64FinalO));
+                        mbar_wait_flag(bars.at(Bars::kPvDone + (Jl % kPSlots)), (Jl / kPSlots) & 1, s_abort));
         if (!ok) break;
         tc_fence_after_sync();
         scale = (l_tot > 0.f) ? sc.out_scale / l_tot : 0.f;
@@ -332,14 +391,15 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       }
       fence_proxy_async_smem();
       FA4_EPI_SYNC()
-      const int sq = query_len<kWindow || kCache>(p, t);
       const bool packed = (kWindow || kCache) && p.cu_seqlens_q != nullptr;
+      const int q0 = packed ? p.cu_seqlens_q[t.b] : 0;
+      const int sq = packed ? p.cu_seqlens_q[t.b + 1] - q0 : p.Sq;
       if (packed && (t.m_blk + 1) * kBlockM > sq) {
         // last, partial tile of a packed sequence: a tiled store would run into the rows of the
         // next sequence (the tensor map only clips at the end of the whole batch), so every
         // thread copies its own row from the staging tile, if it has one
         if (q_idx < sq) {
-          __nv_bfloat16* orow = p.out + (int64_t)(t.q0 + q_idx) * p.o_stride_s + (int64_t)t.h * p.o_stride_h;
+          __nv_bfloat16* orow = p.out + (int64_t)(q0 + q_idx) * p.o_stride_s + (int64_t)t.h * p.o_stride_h;
 #pragma unroll
           for (int c16 = 0; c16 < kDv / 8; ++c16) {
             const uint8_t* src = gbase + kOffOut + (c16 >> 3) * (16 * 1024) + row * 128 + (((c16 & 7) ^ (row & 7)) << 4);
@@ -349,7 +409,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       } else if (leader) {
 #pragma unroll
         for (int bx = 0; bx < kDv / 64; ++bx) {
-          tma_store_4d(&tm_o, base + kOffOut + bx * 16 * 1024, 64 * bx, t.h, t.q0 + t.m_blk * kBlockM,
+          tma_store_4d(&tm_o, base + kOffOut + bx * 16 * 1024, 64 * bx, t.h, q0 + t.m_blk * kBlockM,
                        packed ? 0 : t.b);
         }
         bulk_commit_group();
@@ -361,7 +421,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           if (p.sink != nullptr && m_fin == kNegInf) lse_v = p.sink[t.h];
         }
         if (packed) {
-          p.lse[(int64_t)t.h * p.total_q + t.q0 + q_idx] = lse_v;   // (Hq, total_q)
+          p.lse[(int64_t)t.h * p.total_q + q0 + q_idx] = lse_v;   // (Hq, total_q)
         } else {
           p.lse[((int64_t)t.b * p.Hq + t.h) * p.Sq + q_idx] = lse_v;
         }
@@ -377,8 +437,8 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       // ========================================= TMA producer ===================================
       uint32_t issued_k = 0, issued_v = 0, issued_q = 0;
       FA4_FOR_EACH_TILE {
-        const Tile t = decode_tile<kWindow || kCache, kWindow || kCache>(p, tile);
-        const int n = t.n_blocks;
+        const TileRec t = s_tiles[it];
+        const int n = t.n;
         if (n == 0) continue;
         if (status_poisoned(p.status, p.epoch)) {
           // another CTA of this launch failed: stop this one quickly.  Only this role polls the
@@ -396,8 +456,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         // a packed batch has no batch dimension: the sequence's first row is added to the row
         // coordinate instead (the scale tiles stay per sequence)
         const bool packed = (kWindow || kCache) && p.cu_seqlens_q != nullptr;
+        const int q0 = packed ? p.cu_seqlens_q[t.b] : 0, k0 = packed ? p.cu_seqlens_k[t.b] : 0;
+        const int v0 = packed && p.cu_seqlens_v != nullptr ? p.cu_seqlens_v[t.b] : k0;
         load_qk_tile(base + kOffQ + qb * kQkSlot, &tm_q, bars.at(Bars::kQFull + qb), t.h,
-                     t.q0 + t.m_blk * kBlockM, packed ? 0 : t.b);
+                     q0 + t.m_blk * kBlockM, packed ? 0 : t.b);
         bulk_load(base + kOffSFQ + qb * kQkSfSlot,
                   p.q_sf + t.b * p.qsf_stride_b + t.h * p.qsf_stride_h + (int64_t)t.m_blk * kQkSfBytes,
                   kQkSfBytes, bars.at(Bars::kQFull + qb));
@@ -420,7 +482,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           const int ik = step, iv = step - 2;
           if (ik < n) {
             const uint32_t G = gb + ik, st = G % kStagesK;
-            const int nb = kWindow ? window_visit_block(ik, n, t.nb_top - n + 1, window_rotates(p, t)) : ik;  // ascending
+            const int nb = kWindow ? window_visit_block(ik, t) : ik;  // ascending
             if (G >= kStagesK) {
               ok = mbar_wait_relaxed<kSlackNs>(bars.at(Bars::kKFree + st), ((G - kStagesK) / kStagesK) & 1, wc, kS64KFree);
               if (!ok) break;
@@ -429,7 +491,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
             int kb, nbl;
             locate(nb, kb, nbl);
             load_qk_tile(base + kOffK + st * kQkSlot, &tm_k, bars.at(Bars::kKFull + st), t.hk,
-                         t.k0 + nbl * kBlockN, packed ? 0 : kb);
+                         k0 + nbl * kBlockN, packed ? 0 : kb);
             bulk_load(base + kOffSFK + st * kQkSfSlot,
                       p.k_sf + kb * p.ksf_stride_b + t.hk * p.ksf_stride_h + (int64_t)nbl * kQkSfBytes,
                       kQkSfBytes, bars.at(Bars::kKFull + st));
@@ -437,7 +499,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           }
           if (iv >= 0 && iv < n) {
             const uint32_t G = gb + iv, st = G % kStagesV;
-            const int nb = kWindow ? window_visit_block(iv, n, t.nb_top - n + 1, window_rotates(p, t)) : iv;
+            const int nb = kWindow ? window_visit_block(iv, t) : iv;
             if (G >= kStagesV) {
               ok = mbar_wait_relaxed<kSlackNs>(bars.at(Bars::kVFree + st), ((G - kStagesV) / kStagesV) & 1, wc, kS64VFree);
               if (!ok) break;
@@ -446,7 +508,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
             int kb, nbl;
             locate(nb, kb, nbl);
             tma_load_4d(base + kOffV + st * kTileBytes, &tm_v, bars.at(Bars::kVFull + st),
-                        (t.v0 + nbl * kBlockN) / 2, 0, t.hk, packed ? 0 : kb);
+                        (v0 + nbl * kBlockN) / 2, 0, t.hk, packed ? 0 : kb);
             bulk_load(base + kOffSFV + st * kSfBytes,
                       p.v_sf + kb * p.vsf_stride_b + t.hk * p.vsf_stride_h + (int64_t)nbl * kSfBytes,
                       kSfBytes, bars.at(Bars::kVFull + st));
@@ -475,8 +537,8 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     } else if (warp == kIssuerWarp && lane == 0) {
       // ========================================= QK^T issuer ====================================
       FA4_FOR_EACH_TILE {
-        const Tile t = decode_tile<kWindow || kCache, kWindow || kCache>(p, tile);
-        const int n = t.n_blocks;
+        const TileRec t = s_tiles[it];
+        const int n = t.n;
         if (n == 0) continue;
         const uint32_t qb = ti & 1;
         ok = mbar_wait(bars.at(Bars::kQFull + qb), (ti >> 1) & 1, wc, kS64QFull);
@@ -527,8 +589,8 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     } else if (warp == kPvIssuerWarp && lane == 0) {
       // ========================================= P V issuer =====================================
       FA4_FOR_EACH_TILE {
-        const Tile t = decode_tile<kWindow || kCache, kWindow || kCache>(p, tile);
-        const int n = t.n_blocks;
+        const TileRec t = s_tiles[it];
+        const int n = t.n;
         if (n == 0) continue;
         for (int i = 0; ok && i < n; ++i) {
           const uint32_t G = gb + i, st = G % kStagesV;
@@ -572,8 +634,8 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       // A stage's tensor-memory slot is free when its shared-memory stage is: the producer
       // reloads the stage only after the products that used it have completed.
       FA4_FOR_EACH_TILE {
-        const Tile t = decode_tile<kWindow || kCache, kWindow || kCache>(p, tile);
-        const int n = t.n_blocks;
+        const TileRec t = s_tiles[it];
+        const int n = t.n;
         if (n == 0) continue;
         for (int step = 0; ok && step < n + 2; ++step) {
           const int ik = step, iv = step - 2;  // the producer's order
@@ -616,28 +678,28 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     const uint32_t s_addr = lane_addr + kTmS64 + 64 * wg;
 
     FA4_FOR_EACH_TILE {
-      const Tile t = decode_tile<kWindow || kCache>(p, tile);
-      const int n = t.n_blocks;
+      const TileRec t = s_tiles[it];
+      const int n = t.n;
       float m_ref = kNegInf, l_sum = 0.f;
 
       for (int j = (wg - 2 * (int)gb) & 3; j < 2 * n; j += 4) {
         const uint32_t J = 2 * gb + j, slot = J % kPSlots;  // J % 4 == wg
-        const int nb = kWindow ? window_visit_block(j >> 1, n, t.nb_top - n + 1, window_rotates(p, t)) : (j >> 1);
+        const int nb = kWindow ? window_visit_block(j >> 1, t) : (j >> 1);
         const int h64 = j & 1;
         const uint32_t bar_s = bars.at(Bars::kSFull + (wg & 2)), par_s = (J / kSBufs) & 1;
         const uint32_t bar_p = bars.at(Bars::kPvDone + slot), par_p = ((J - kPSlots) / kPSlots) & 1;
         const bool r_p = (J >= kPSlots) ? mbar_test(bar_p, par_p) : true;
 
         // 1. the scores of this sub-block: the whole 64-key row of this thread
-        ok = wait_probed(mbar_test(bar_s, par_s), bar_s, par_s, wc, kS64SFull);
+        ok = __all_sync(0xffffffffu, mbar_test(bar_s, par_s)) || __all_sync(0xffffffffu, mbar_wait_flag(bar_s, par_s, s_abort));
         if (!ok) break;
         tc_fence_after_sync();
-        if (block_needs_mask<kWindow || kCache, kWindow>(p, t, nb)) {
+        if (needs_mask<kWindow>(p, t, nb)) {
           if constexpr (kWindow) {
-            ws::mask_scores_in_tmem_range(s_addr, lower_limit(p, t, row, nb) - 64 * h64,
-                                          causal_limit<true>(p, t, row, nb) - 64 * h64);
+            ws::mask_scores_in_tmem_range(s_addr, lower_key(p, t, row, nb) - 64 * h64,
+                                          upper_key<true>(p, t, row, nb) - 64 * h64);
           } else {
-            mask_scores_in_tmem(s_addr, causal_limit<kWindow || kCache, kWindow>(p, t, row, nb) - 64 * h64);
+            mask_scores_in_tmem(s_addr, upper_key<false>(p, t, row, nb) - 64 * h64);
           }
         }
         float s[64];
@@ -653,7 +715,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         float m_prev = kNegInf;
         if (J > 0) {
           const uint32_t pw = (uint32_t)(wg + 3) & 3u;
-          ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kHand + 4 * pw + (warp & 3)), ((J - 1) / kSBufs) & 1, wc, kS64Hand));
+          ok = __all_sync(0xffffffffu, mbar_wait_flag(bars.at(Bars::kHand + 4 * pw + (warp & 3)), ((J - 1) / kSBufs) & 1, s_abort));
           if (!ok) break;
           if (j > 0) m_prev = s_hand[pw * 128 + row];
         }
@@ -702,7 +764,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         m_ref = m_new;
 
         // 3. exponentials and quantisation; P slot J % 8 is free once P V of sub-block J - 8 has run
-        ok = wait_probed(r_p, bar_p, par_p, wc, kS64PvDone);
+        ok = __all_sync(0xffffffffu, r_p) || __all_sync(0xffffffffu, mbar_wait_flag(bar_p, par_p, s_abort));
         if (!ok) break;
         uint8_t* p_tile = gbase + kOffP + slot * kPTileBytes;
         {
@@ -727,8 +789,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         const bool fix = (m_new != m_prev) && (m_prev != kNegInf);
         if (j > 0 && __any_sync(0xffffffffu, fix)) {
           const uint32_t Jp = J - 1;
-          ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kPvDone + (Jp % kPSlots)),
-                                                 (Jp / kPSlots) & 1, wc, kS64PvDone));
+          ok = __all_sync(0xffffffffu, mbar_wait_flag(bars.at(Bars::kPvDone + (Jp % kPSlots)), (Jp / kPSlots) & 1, s_abort));
           if (!ok) break;
           tc_fence_after_sync();
           const float f = fix ? reference_factor(m_prev, m_new, sc.sl2) : 1.f;
@@ -747,7 +808,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         const uint32_t fb = ti & 1;
         if (ti >= 2) {
           ok = __all_sync(0xffffffffu,
-                          mbar_wait(bars.at(Bars::kFinFree + fb), ((ti - 2) >> 1) & 1, wc, kS64FinFree));
+                          mbar_wait_flag(bars.at(Bars::kFinFree + fb), ((ti - 2) >> 1) & 1, s_abort));
           if (!ok) break;
         }
         volatile float* fin_slot = s_fin + fb * (4 * 128 * 2);

@@ -18,6 +18,8 @@ namespace fa4 {
 // ---------------------------------------------------------------------------------------------
 constexpr uint32_t kStatusWaitExpired = 1u;
 
+// (The attention kernels keep theirs in shared memory, written once by one thread: waits that block
+// pass its address to one out-of-line function, and no role holds these words in registers.)
 struct WaitCtx {
   volatile uint32_t* s_abort;  // shared-memory flag, set by the first role that gives up
   uint32_t* g_status;          // device status word (may be null)
@@ -102,7 +104,7 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
 #ifndef FA4_WAIT_HINT_NS
 #define FA4_WAIT_HINT_NS 64
 #endif
-__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity, uint32_t hint_ns = FA4_WAIT_HINT_NS) {
   uint32_t ok;
   asm volatile(
       "{\n"
@@ -111,56 +113,54 @@ __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity) {
       "selp.b32 %0, 1, 0, p;\n"
       "}\n"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"((uint32_t)FA4_WAIT_HINT_NS)
+      : "r"(bar), "r"(parity), "r"(hint_ns)
       : "memory");
   return ok != 0;
 }
-// Bounded wait.  Returns false when the CTA is aborting (this wait ran out, or another
-// role's did); the caller must then leave its loop and go to the common tear-down.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx& w,
-                                          uint32_t site) {
-  if (mbar_poll(bar, parity)) return true;
+// The part of a bounded wait that is reached when the first poll fails.  Out of line: inlined at some
+// thirty sites it was half of the code of the 64-key kernel, which on short tiles visits all of it
+// once per tile and then waits for instructions more than for anything else (a 127-key window:
+// 36 % of the instruction-cache requests missed, 5.5 of its 14 stalled warps per issue slot).
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, const WaitCtx* w, uint32_t site,
+                                            uint32_t hint_ns) {
   const uint64_t t0 = globaltimer_ns();
   for (;;) {
 #pragma unroll 1
     for (int i = 0; i < 32; ++i) {
-      if (mbar_poll(bar, parity)) return true;
+      if (mbar_poll(bar, parity, hint_ns)) return true;
     }
-    if (*w.s_abort) return false;
-    if (globaltimer_ns() - t0 > w.budget_ns) {
-      report_status(w, kStatusWaitExpired, site);
+    if (*w->s_abort) return false;
+    if (globaltimer_ns() - t0 > w->budget_ns) {
+      report_status(*w, kStatusWaitExpired, site);
       return false;
     }
   }
+}
+// Bounded wait.  Returns false when the CTA is aborting (this wait ran out, or another
+// role's did); the caller must then leave its loop and go to the common tear-down.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const WaitCtx& w, uint32_t site) {
+  return mbar_poll(bar, parity) || mbar_wait_slow(bar, parity, &w, site, FA4_WAIT_HINT_NS);
 }
 
 // The same bounded wait for roles with slack (producer, scale copier, epilogue): a longer suspend
 // hint per poll, so that a warp that waits most of the time takes fewer issue slots from the
 // softmax warps of its scheduler.
 template <uint32_t kHintNs>
-__device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, const WaitCtx& w,
-                                                  uint32_t site) {
-  const uint64_t t0 = globaltimer_ns();
+__device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity, const WaitCtx& w, uint32_t site) {
+  return mbar_poll(bar, parity, kHintNs) || mbar_wait_slow(bar, parity, &w, site, kHintNs);
+}
+
+// A wait of the softmax warps: no call (they hold a row of scores in registers, some of them still on
+// their way from tensor memory) and no clock of its own, only the CTA's abort flag.  It is bounded all
+// the same: whatever keeps a softmax warp waiting soon keeps the issuers and the producer waiting too,
+// their waits run out, and the first of them raises the flag.
+__device__ __forceinline__ bool mbar_wait_flag(uint32_t bar, uint32_t parity, const volatile uint32_t* s_abort) {
   for (;;) {
 #pragma unroll 1
     for (int i = 0; i < 32; ++i) {
-      uint32_t ok;
-      asm volatile(
-          "{\n"
-          ".reg .pred p;\n"
-          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
-          "selp.b32 %0, 1, 0, p;\n"
-          "}\n"
-          : "=r"(ok)
-          : "r"(bar), "r"(parity), "r"(kHintNs)
-          : "memory");
-      if (ok) return true;
+      if (mbar_poll(bar, parity)) return true;
     }
-    if (*w.s_abort) return false;
-    if (globaltimer_ns() - t0 > w.budget_ns) {
-      report_status(w, kStatusWaitExpired, site);
-      return false;
-    }
+    if (*s_abort) return false;
   }
 }
 
