@@ -439,7 +439,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       FA4_FOR_EACH_TILE {
         const TileRec t = s_tiles[it];
         const int n = t.n;
-        if (n == 0) continue;
+        if (n <= 0) continue;
         if (status_poisoned(p.status, p.epoch)) {
           // another CTA of this launch failed: stop this one quickly.  Only this role polls the
           // status word (a global load at every tile start); the others see the abort flag in
@@ -539,7 +539,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       FA4_FOR_EACH_TILE {
         const TileRec t = s_tiles[it];
         const int n = t.n;
-        if (n == 0) continue;
+        if (n <= 0) continue;
         const uint32_t qb = ti & 1;
         ok = mbar_wait(bars.at(Bars::kQFull + qb), (ti >> 1) & 1, wc, kS64QFull);
         if (!ok) break;
@@ -591,7 +591,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       FA4_FOR_EACH_TILE {
         const TileRec t = s_tiles[it];
         const int n = t.n;
-        if (n == 0) continue;
+        if (n <= 0) continue;
         for (int i = 0; ok && i < n; ++i) {
           const uint32_t G = gb + i, st = G % kStagesV;
           ok = mbar_wait(bars.at(Bars::kVsf + st), (G / kStagesV) & 1, wc, kS64Vsf);
@@ -636,7 +636,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       FA4_FOR_EACH_TILE {
         const TileRec t = s_tiles[it];
         const int n = t.n;
-        if (n == 0) continue;
+        if (n <= 0) continue;
         for (int step = 0; ok && step < n + 2; ++step) {
           const int ik = step, iv = step - 2;  // the producer's order
           if (ik < n) {
@@ -680,6 +680,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     FA4_FOR_EACH_TILE {
       const TileRec t = s_tiles[it];
       const int n = t.n;
+      if (n <= 0) continue;
       float m_ref = kNegInf, l_sum = 0.f;
 
       for (int j = (wg - 2 * (int)gb) & 3; j < 2 * n; j += 4) {
@@ -804,7 +805,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
 
       // ---- tile end: hand the partial row sum and its reference to the epilogue warpgroup and
       //      go on with the next tile
-      if (n > 0) {
+      {
         const uint32_t fb = ti & 1;
         if (ti >= 2) {
           ok = __all_sync(0xffffffffu,
@@ -820,7 +821,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         mbar_arrive(bars.at(Bars::kFin + fb));
       }
       gb += n;
-      ti += (n > 0) ? 1u : 0u;
+      ti += 1;
     }
   }
 #undef FA4_FOR_EACH_TILE
