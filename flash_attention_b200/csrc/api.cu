@@ -38,13 +38,13 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
 
 // Byte tensor of rank 4, innermost dimension contiguous; box = {box0, box1, box2, box3} bytes /
 // rows; 64-byte swizzle when the innermost box is 64 bytes.
-// bf16 output tensor (B, Sq, Hq, Dv) as {Dv, Hq, Sq, B}; box = 64 columns x 128 rows, 128-byte
-// swizzle (the staging layout of the warp-specialised kernel's epilogue).
-bool encode_out_4d(CUtensorMap* m, void* base, const uint64_t (&dims)[4], const uint64_t (&strides)[3]) {
+// bf16 output tensor (B, Sq, Hq, Dv) as {Dv, Hq, Sq, B}; box = 64 columns x `rows` rows, 128-byte
+// swizzle (the staging layout of the warp-specialised kernels' epilogues).
+bool encode_out_4d(CUtensorMap* m, void* base, const uint64_t (&dims)[4], const uint64_t (&strides)[3], uint32_t rows) {
   auto fn = get_encode();
   if (fn == nullptr) return false;
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const cuuint32_t box[4] = {64, 1, 128, 1};
+  const cuuint32_t box[4] = {64, 1, rows, 1};
   const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, base, dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                         CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -521,7 +521,8 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
                                packed ? 1u : (uint64_t)p->B};
       const uint64_t s_o[3] = {(uint64_t)p->o_stride_h * 2, (uint64_t)p->o_stride_s * 2,
                                (uint64_t)p->o_stride_b * 2};
-      if (!encode_out_4d(&tm_o, p->out, d_o, s_o)) return -FA4_E_TENSORMAP;
+      // the 64-key kernel stores per warp (32 rows), the 128-key kernel a whole tile at a time
+      if (!encode_out_4d(&tm_o, p->out, d_o, s_o, variant == FA4_VARIANT_WS64 ? 32u : 128u)) return -FA4_E_TENSORMAP;
     }
     auto launch = [&](auto kernel) -> int {
       if (int e = ensure_kernel(kernel, ws::kSmemRequest, ws::kRegsLaunch)) return e;

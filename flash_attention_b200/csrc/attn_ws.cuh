@@ -152,9 +152,12 @@ __device__ __forceinline__ bool wait_probed(bool probed, uint32_t bar, uint32_t 
 }
 
 // O[:, 32 * nchunks columns from taddr] *= f for this thread's row.  Rare (the reference maximum
-// moved by more than the lazy threshold), so it is kept out of line: its 32 registers would
-// otherwise be added to the pressure of the exponential loop.
-__device__ __noinline__ void rescale_accumulator(uint32_t taddr, float f, int nchunks) {
+// moved by more than the lazy threshold).  A rolled loop, but in line, like the masks below: no row of
+// scores is live at either place, and a call from the softmax loop costs the registers of its calling
+// convention there (64-key kernel, us: long context with outlier channels 12530 -> 12180, 127-key
+// window 134 -> 113, non-causal S = 4096 713 -> 703).
+__device__ __forceinline__ void rescale_accumulator(uint32_t taddr, float f, int nchunks) {
+#pragma unroll 1
   for (int c = 0; c < nchunks; ++c) {
     uint32_t o[32];
     tmem_ld32(taddr + 32 * c, o);
@@ -166,8 +169,9 @@ __device__ __noinline__ void rescale_accumulator(uint32_t taddr, float f, int nc
 }
 
 // Keys with in-chunk index > limit of this thread's 64 scores at taddr become -inf.  Only on
-// diagonal blocks; out of line like the rescale.
-__device__ __noinline__ void mask_scores_in_tmem(uint32_t taddr, int limit) {
+// diagonal blocks.
+__device__ __forceinline__ void mask_scores_in_tmem(uint32_t taddr, int limit) {
+#pragma unroll 1
   for (int c = 0; c < 2; ++c) {
     // tcgen05.ld / st are warp-collective: the skip must be decided by the whole warp
     if (__all_sync(0xffffffffu, limit >= 32 * c + 31)) continue;  // chunk fully visible
@@ -182,7 +186,8 @@ __device__ __noinline__ void mask_scores_in_tmem(uint32_t taddr, int limit) {
 }
 
 // The same with a lower limit as well (local attention): keys outside [lower, limit] become -inf.
-__device__ __noinline__ void mask_scores_in_tmem_range(uint32_t taddr, int lower, int limit) {
+__device__ __forceinline__ void mask_scores_in_tmem_range(uint32_t taddr, int lower, int limit) {
+#pragma unroll 1
   for (int c = 0; c < 2; ++c) {
     if (__all_sync(0xffffffffu, limit >= 32 * c + 31 && lower <= 32 * c)) continue;  // fully visible
     uint32_t v[32];

@@ -17,10 +17,10 @@
 //   warps 0-15  softmax: warpgroup w takes the sub-blocks with running index J % 4 == w; the
 //               running reference maximum of a row is handed from the warpgroup of sub-block
 //               J - 1 to that of J through shared memory
-//   warp 16     TMA producer (Q double buffered, K / V rings of 128-key tiles)
-//   warp 17     QK^T issuer: per K tile one N = 128 product into two neighbouring S buffers
+//   warp 16     TMA loads of Q (double buffered) and K (ring of 128-key tiles), K scales to tensor memory
+//   warp 17     Q K^T issuer: per K tile one N = 128 product into two neighbouring S buffers
 //   warp 18     P V issuer: per sub-block one K = 64 step into O
-//   warp 19     copies the K / V scale tiles into tensor memory as they land
+//   warp 19     TMA loads of V (its own ring), V scales to tensor memory
 //   warps 20-23 epilogue: combine the partial row sums, read O out, TMA store, LSE -- while the
 //               softmax warpgroups already work on the next tile
 //
@@ -41,7 +41,7 @@ constexpr int kStagesK = 4, kStagesV = 4;  // 128-key tiles
 constexpr int kSBufs = 4;                  // S buffers of 64 columns
 constexpr int kPSlots = 8;                 // P tiles of 64 keys (4 KB each)
 constexpr int kThreads = 768;
-constexpr int kProducerWarp = 16, kIssuerWarp = 17, kPvIssuerWarp = 18, kCopyWarp = 19, kEpilogueWarp0 = 20;
+constexpr int kLoadKWarp = 16, kIssuerWarp = 17, kPvIssuerWarp = 18, kLoadVWarp = 19, kEpilogueWarp0 = 20;
 // Registers are a per-scheduler resource: 16384 per SM sub-partition, warp w living on sub-partition
 // w % 4.  With 21-24 warps a sub-partition holds 6, so the launch gets 80 registers per thread and
 // the CTA's pool per sub-partition is 6 x 32 x 80 = 15360.  setmaxnreg.inc draws from that pool
@@ -56,7 +56,7 @@ static_assert((kThreads / 128) * 32 * kRegsLaunch <= 16384, "register file of a 
 
 // tensor memory: S[4] x 64 columns, O 128, scale factors
 // (O at column 256 and Q scales at 384 as in the 128-key kernel); K and V scales have one slot of
-// 8 columns per shared-memory stage, written by the copy warp as soon as the tile has landed
+// 8 columns per shared-memory stage, written by the loader as soon as the tile has landed
 // (sized for head dim 192: three 64-element steps, 12 scale columns per Q / K tile)
 constexpr uint32_t kTmS64 = 0, kTmSFQ64 = 384 /* 12 */, kTmSFK64 = 396 /* 4 x 12 */, kTmSFV64 = 444 /* 4 x 8 */,
                    kTmSFP64 = 476 /* 4 x 4 */;
@@ -65,6 +65,7 @@ static_assert(kTmSFP64 + 16 <= 512, "tensor memory columns");
 // bytes as three 32-byte-wide sub-tiles; three scale chunks)
 constexpr uint32_t kQkSlot = 128 * 96, kQkSfSlot = 3 * 512;
 constexpr uint32_t kSlackNs = 500;         // suspend hint of the waits of roles with slack
+constexpr uint32_t kCopySlackNs = 500;     // and of the loaders waiting for a tile whose scales they copy
 constexpr uint32_t kPTileBytes = 128 * 32;  // 128 rows x 64 e2m1 keys
 
 constexpr uint32_t kOffQ = 0;
@@ -88,8 +89,8 @@ struct Bars {
                             kSFull = kVFree + kStagesV, kSFree = kSFull + kSBufs,
                             kHand = kSFree + kSBufs, kPFull = kHand + 4 * kSBufs, kPvDone = kPFull + kPSlots,
                             kFin = kPvDone + kPSlots, kFinFree = kFin + 2, kOFree = kFinFree + 2,
-                            kEpi = kOFree + 1, kKsf = kEpi + 1, kVsf = kKsf + kStagesK,
-                            kDrain = kVsf + kStagesV, kCount = kDrain + 3;
+                            kKsf = kOFree + 1, kVsf = kKsf + kStagesK,
+                            kDrain = kVsf + kStagesV, kCount = kDrain + 4;
   __device__ explicit Bars(uint32_t b) : base(b) {}
   __device__ __forceinline__ uint32_t at(uint32_t idx) const { return base + 8u * idx; }
 };
@@ -100,7 +101,7 @@ static_assert(kSmemRequest <= 227 * 1024, "shared memory");
 
 enum Site64 {
   kS64QFull = 40, kS64QEmpty, kS64KFree, kS64VFree, kS64KFull, kS64VFull, kS64SFull, kS64SFree,
-  kS64PFull, kS64PvDone, kS64Hand, kS64Fin, kS64FinFree, kS64FinalO, kS64OFree, kS64Ksf, kS64Vsf, kS64Epi
+  kS64PFull, kS64PvDone, kS64Hand, kS64Fin, kS64FinFree, kS64FinalO, kS64OFree, kS64Ksf, kS64Vsf
 };
 
 // The tiles of this CTA, decoded once at kernel start -- one thread per tile -- into a table in shared
@@ -221,7 +222,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_init(bars.at(Bars::kQFull + b), 1);
       mbar_init(bars.at(Bars::kQEmpty + b), 1);
     }
-    for (int b = 0; b < 3; ++b) mbar_init(bars.at(Bars::kDrain + b), 1);
+    for (int b = 0; b < 4; ++b) mbar_init(bars.at(Bars::kDrain + b), 1);
     for (int s = 0; s < kStagesK; ++s) {
       mbar_init(bars.at(Bars::kKFull + s), 1);
       mbar_init(bars.at(Bars::kKFree + s), 1);
@@ -246,14 +247,13 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_init(bars.at(Bars::kFinFree + b), 128);  // the epilogue warpgroup
     }
     mbar_init(bars.at(Bars::kOFree), 128);
-    mbar_init(bars.at(Bars::kEpi), 128);            // the epilogue warpgroup's own rendezvous
     fence_barrier_init();
   }
-  if (warp == kProducerWarp && lane == 0) {
+  if (warp == kLoadKWarp && lane == 0) {
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
-    tma_prefetch_desc(&tm_v);
   }
+  if (warp == kLoadVWarp && lane == 0) tma_prefetch_desc(&tm_v);
   if (warp == kIssuerWarp) {
     tmem_alloc(base + kOffMisc, kTmemCols);
     tmem_relinquish();
@@ -306,20 +306,12 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     // Thread = row.  Per tile: combine the four partial row sums, wait for the last P V, move O
     // from tensor memory to the staging tile (bf16, normalised), send it with TMA, write the LSE.
     // The softmax warpgroups meanwhile work on the next tile; only the P V issuer waits for the
-    // accumulator to be read out.
+    // accumulator to be read out.  Every warp stages and sends its own 32 rows: no rendezvous of the
+    // four.
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsEpilogue));
     const int row = tid & 127;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
-    const bool leader = (tid == kEpilogueWarp0 * 32);
-    if (leader) tma_prefetch_desc(&tm_o);
-    // rendezvous of the 128 epilogue threads on an mbarrier: unlike bar.sync the wait is bounded, so
-    // a warp that gave up elsewhere cannot leave the others blocked
-    uint32_t epi_phase = 0;
-#define FA4_EPI_SYNC()                                                                              \
-  mbar_arrive(bars.at(Bars::kEpi));                                                                 \
-  ok = __all_sync(0xffffffffu, mbar_wait_flag(bars.at(Bars::kEpi), epi_phase & 1, s_abort));          \
-  epi_phase += 1;                                                                                   \
-  if (!ok) break;
+    if (warp == kEpilogueWarp0 && lane == 0) tma_prefetch_desc(&tm_o);
     FA4_FOR_EACH_TILE {
       const TileRec t = s_tiles[it];
       const int n = t.n;
@@ -328,6 +320,9 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         // a tile past the end of a short sequence of a packed batch has no rows at all
         if (n < 0) continue;
       }
+      // the staging rows are free once the previous store has read them
+      if (lane == 0) bulk_wait_group_read0();
+      __syncwarp();
       float scale = 0.f, m_fin = kNegInf, l_tot = 0.f;
       if (n > 0) {
         const uint32_t fb = ti & 1;
@@ -358,11 +353,6 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         tc_fence_after_sync();
         scale = (l_tot > 0.f) ? sc.out_scale / l_tot : 0.f;
       }
-      // the staging tile is free once the previous store has read it
-      if (it >= 1) {
-        if (leader) bulk_wait_group_read0();
-        FA4_EPI_SYNC()
-      }
 #pragma unroll 1
       for (int c = 0; c < kDv / 32; ++c) {
         uint8_t* box_row = gbase + kOffOut + (c >> 1) * (16 * 1024) + row * 128;
@@ -390,12 +380,13 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
       }
       fence_proxy_async_smem();
-      FA4_EPI_SYNC()
+      __syncwarp();
       const bool packed = (kWindow || kCache) && p.cu_seqlens_q != nullptr;
       const int q0 = packed ? p.cu_seqlens_q[t.b] : 0;
       const int sq = packed ? p.cu_seqlens_q[t.b + 1] - q0 : p.Sq;
-      if (packed && (t.m_blk + 1) * kBlockM > sq) {
-        // last, partial tile of a packed sequence: a tiled store would run into the rows of the
+      const int row0 = t.m_blk * kBlockM + (warp & 3) * 32;     // first row of this warp
+      if (packed && row0 + 32 > sq) {
+        // last, partial rows of a packed sequence: a tiled store would run into the rows of the
         // next sequence (the tensor map only clips at the end of the whole batch), so every
         // thread copies its own row from the staging tile, if it has one
         if (q_idx < sq) {
@@ -406,10 +397,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
             reinterpret_cast<uint4*>(orow)[c16] = *reinterpret_cast<const uint4*>(src);
           }
         }
-      } else if (leader) {
+      } else if (lane == 0 && row0 < sq) {
 #pragma unroll
         for (int bx = 0; bx < kDv / 64; ++bx) {
-          tma_store_4d(&tm_o, base + kOffOut + bx * 16 * 1024, 64 * bx, t.h, q0 + t.m_blk * kBlockM,
+          tma_store_4d(&tm_o, base + kOffOut + bx * 16 * 1024 + (warp & 3) * 4096, 64 * bx, t.h, q0 + row0,
                        packed ? 0 : t.b);
         }
         bulk_commit_group();
@@ -429,46 +420,80 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       gb += n;
       ti += (n > 0) ? 1u : 0u;
     }
-#undef FA4_EPI_SYNC
-    if (leader) bulk_wait_group0();
-  } else if (warp >= kProducerWarp) {
+    if (lane == 0) bulk_wait_group0();
+  } else if (warp >= kLoadKWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
-    if (warp == kProducerWarp && lane == 0) {
-      // ========================================= TMA producer ===================================
-      uint32_t issued_k = 0, issued_v = 0, issued_q = 0;
+    if ((warp == kLoadKWarp || warp == kLoadVWarp) && lane == 0) {
+      // ========================================= TMA loaders ====================================
+      // One warp streams Q and K, the other V, each as far ahead as its own ring allows: what Q K^T of
+      // the next tile needs never queues behind a V stage that P V has yet to free.
+      // Each also copies the scales of its tiles into tensor memory as soon as they have landed, one tile
+      // behind its loads, so that the two issuers spend their (slow, in-order) tcgen05 issue slots on
+      // products only (copies issued there: non-causal S = 4096 719 -> 755 us).  A stage's tensor-memory
+      // slot is free when its shared-memory stage is.
+      static_assert(kStagesK == kStagesV, "one ring arithmetic for both loaders");
+      const bool is_k = warp == kLoadKWarp;
+      const uint32_t full0 = is_k ? Bars::kKFull : Bars::kVFull, free0 = is_k ? Bars::kKFree : Bars::kVFree;
+      auto copy_scales = [&](uint32_t G) -> bool {
+        const uint32_t st = G % kStagesK;
+        if (!mbar_wait_relaxed<kCopySlackNs>(bars.at(full0 + st), (G / kStagesK) & 1, wc, is_k ? kS64KFull : kS64VFull))
+          return false;
+        tc_fence_after_sync();
+        if (is_k) {
+#pragma unroll
+          for (int ks = 0; ks < kSteps; ++ks)
+            tc_cp_sf(tmem + kTmSFK64 + 12 * st + 4 * ks, base + kOffSFK + st * kQkSfSlot + 512 * ks);
+        } else {
+          tc_cp_sf(tmem + kTmSFV64 + 8 * st, base + kOffSFV + st * kSfBytes);
+          tc_cp_sf(tmem + kTmSFV64 + 8 * st + 4, base + kOffSFV + st * kSfBytes + 512);
+        }
+        tc_commit(bars.at((is_k ? Bars::kKsf : Bars::kVsf) + st));
+        return true;
+      };
+      uint32_t issued = 0, issued_q = 0, copied = 0;
       FA4_FOR_EACH_TILE {
         const TileRec t = s_tiles[it];
         const int n = t.n;
         if (n <= 0) continue;
-        if (status_poisoned(p.status, p.epoch)) {
-          // another CTA of this launch failed: stop this one quickly.  Only this role polls the
-          // status word (a global load at every tile start); the others see the abort flag in
-          // their next wait, when the tiles stop coming
-          *s_abort = 1u;
-          break;
-        }
-        const uint32_t qb = ti & 1;
-        if (ti >= 2) {
-          ok = mbar_wait_relaxed<kSlackNs>(bars.at(Bars::kQEmpty + qb), ((ti - 2) >> 1) & 1, wc, kS64QEmpty);
-          if (!ok) break;
-        }
-        mbar_arrive_expect_tx(bars.at(Bars::kQFull + qb), kQkBytes + kQkSfBytes);
         // a packed batch has no batch dimension: the sequence's first row is added to the row
         // coordinate instead (the scale tiles stay per sequence)
         const bool packed = (kWindow || kCache) && p.cu_seqlens_q != nullptr;
-        const int q0 = packed ? p.cu_seqlens_q[t.b] : 0, k0 = packed ? p.cu_seqlens_k[t.b] : 0;
-        const int v0 = packed && p.cu_seqlens_v != nullptr ? p.cu_seqlens_v[t.b] : k0;
-        load_qk_tile(base + kOffQ + qb * kQkSlot, &tm_q, bars.at(Bars::kQFull + qb), t.h,
-                     q0 + t.m_blk * kBlockM, packed ? 0 : t.b);
-        bulk_load(base + kOffSFQ + qb * kQkSfSlot,
-                  p.q_sf + t.b * p.qsf_stride_b + t.h * p.qsf_stride_h + (int64_t)t.m_blk * kQkSfBytes,
-                  kQkSfBytes, bars.at(Bars::kQFull + qb));
-        issued_q = ti + 1;
-        // where logical K/V block nb of this batch entry lives: the entry itself, or (window
-        // instantiation, which also serves KV-cache views) a page of the pool and the block in it
-        auto locate = [&](int nb, int& kb, int& nbl) {
-          kb = t.b;
-          nbl = nb;
+        int k0 = 0;      // first key of the sequence inside the packed tensor
+        if (packed) k0 = !is_k && p.cu_seqlens_v != nullptr ? p.cu_seqlens_v[t.b] : p.cu_seqlens_k[t.b];
+        if (is_k) {
+          if (status_poisoned(p.status, p.epoch)) {
+            // another CTA of this launch failed: stop this one quickly.  Only this role polls the
+            // status word (a global load at every tile start); the others see the abort flag in
+            // their next wait, when the tiles stop coming
+            *s_abort = 1u;
+            break;
+          }
+          const uint32_t qb = ti & 1;
+          if (ti >= 2) {
+            ok = mbar_wait_relaxed<kSlackNs>(bars.at(Bars::kQEmpty + qb), ((ti - 2) >> 1) & 1, wc, kS64QEmpty);
+            if (!ok) break;
+          }
+          mbar_arrive_expect_tx(bars.at(Bars::kQFull + qb), kQkBytes + kQkSfBytes);
+          load_qk_tile(base + kOffQ + qb * kQkSlot, &tm_q, bars.at(Bars::kQFull + qb), t.h,
+                       (packed ? p.cu_seqlens_q[t.b] : 0) + t.m_blk * kBlockM, packed ? 0 : t.b);
+          bulk_load(base + kOffSFQ + qb * kQkSfSlot,
+                    p.q_sf + t.b * p.qsf_stride_b + t.h * p.qsf_stride_h + (int64_t)t.m_blk * kQkSfBytes,
+                    kQkSfBytes, bars.at(Bars::kQFull + qb));
+          issued_q = ti + 1;
+        }
+        for (int i = 0; i < n; ++i) {
+          const uint32_t G = gb + i, st = G % kStagesK;
+          const int nb = kWindow ? window_visit_block(i, t) : i;  // ascending
+          if (G >= kStagesK) {
+            ok = mbar_wait_relaxed<kSlackNs>(bars.at(free0 + st), ((G - kStagesK) / kStagesK) & 1, wc,
+                                             is_k ? kS64KFree : kS64VFree);
+            if (!ok) break;
+          }
+          const uint32_t full = bars.at(full0 + st);
+          mbar_arrive_expect_tx(full, is_k ? kQkBytes + kQkSfBytes : kVBytes + kSfBytes);
+          // where logical K/V block nb of this batch entry lives: the entry itself, or (KV-cache views) a
+          // page of the pool and the block in it
+          int kb = t.b, nbl = nb;
           if constexpr (kWindow || kCache) {
             if (p.page_table != nullptr) {
               const int key0 = nb * kBlockN, pg = key0 / p.page_size;
@@ -476,63 +501,39 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
               nbl = (key0 - pg * p.page_size) / kBlockN;
             }
           }
-        };
-        // K runs two blocks ahead of V
-        for (int step = 0; ok && step < n + 2; ++step) {
-          const int ik = step, iv = step - 2;
-          if (ik < n) {
-            const uint32_t G = gb + ik, st = G % kStagesK;
-            const int nb = kWindow ? window_visit_block(ik, t) : ik;  // ascending
-            if (G >= kStagesK) {
-              ok = mbar_wait_relaxed<kSlackNs>(bars.at(Bars::kKFree + st), ((G - kStagesK) / kStagesK) & 1, wc, kS64KFree);
-              if (!ok) break;
-            }
-            mbar_arrive_expect_tx(bars.at(Bars::kKFull + st), kQkBytes + kQkSfBytes);
-            int kb, nbl;
-            locate(nb, kb, nbl);
-            load_qk_tile(base + kOffK + st * kQkSlot, &tm_k, bars.at(Bars::kKFull + st), t.hk,
-                         k0 + nbl * kBlockN, packed ? 0 : kb);
+          if (is_k) {
+            load_qk_tile(base + kOffK + st * kQkSlot, &tm_k, full, t.hk, k0 + nbl * kBlockN, packed ? 0 : kb);
             bulk_load(base + kOffSFK + st * kQkSfSlot,
-                      p.k_sf + kb * p.ksf_stride_b + t.hk * p.ksf_stride_h + (int64_t)nbl * kQkSfBytes,
-                      kQkSfBytes, bars.at(Bars::kKFull + st));
-            issued_k = G + 1;
-          }
-          if (iv >= 0 && iv < n) {
-            const uint32_t G = gb + iv, st = G % kStagesV;
-            const int nb = kWindow ? window_visit_block(iv, t) : iv;
-            if (G >= kStagesV) {
-              ok = mbar_wait_relaxed<kSlackNs>(bars.at(Bars::kVFree + st), ((G - kStagesV) / kStagesV) & 1, wc, kS64VFree);
-              if (!ok) break;
-            }
-            mbar_arrive_expect_tx(bars.at(Bars::kVFull + st), kVBytes + kSfBytes);
-            int kb, nbl;
-            locate(nb, kb, nbl);
-            tma_load_4d(base + kOffV + st * kTileBytes, &tm_v, bars.at(Bars::kVFull + st),
-                        (v0 + nbl * kBlockN) / 2, 0, t.hk, packed ? 0 : kb);
+                      p.k_sf + kb * p.ksf_stride_b + t.hk * p.ksf_stride_h + (int64_t)nbl * kQkSfBytes, kQkSfBytes, full);
+          } else {
+            tma_load_4d(base + kOffV + st * kTileBytes, &tm_v, full, (k0 + nbl * kBlockN) / 2, 0, t.hk, packed ? 0 : kb);
             bulk_load(base + kOffSFV + st * kSfBytes,
-                      p.v_sf + kb * p.vsf_stride_b + t.hk * p.vsf_stride_h + (int64_t)nbl * kSfBytes,
-                      kSfBytes, bars.at(Bars::kVFull + st));
-            issued_v = G + 1;
+                      p.v_sf + kb * p.vsf_stride_b + t.hk * p.vsf_stride_h + (int64_t)nbl * kSfBytes, kSfBytes, full);
+          }
+          issued = G + 1;
+          if (G > copied) {
+            ok = copy_scales(copied);
+            if (!ok) break;
+            copied += 1;
           }
         }
+        if (!ok) break;
         gb += n;
         ti += 1;
       }
+      for (; ok && copied < issued; ++copied) ok = copy_scales(copied);
       if (!ok) {
         // bounded drain: let the copies already issued land before the CTA's memory is released
+        tc_commit(bars.at(Bars::kDrain + (is_k ? 2 : 3)));
         const uint64_t t0 = globaltimer_ns();
         const uint64_t lim = 50ull * 1000 * 1000;
-        for (uint32_t i = issued_k > kStagesK ? issued_k - kStagesK : 0; i < issued_k; ++i) {
-          while (!mbar_try_wait(bars.at(Bars::kKFull + (i % kStagesK)), (i / kStagesK) & 1) &&
-                 globaltimer_ns() - t0 < lim) {}
-        }
-        for (uint32_t i = issued_v > kStagesV ? issued_v - kStagesV : 0; i < issued_v; ++i) {
-          while (!mbar_try_wait(bars.at(Bars::kVFull + (i % kStagesV)), (i / kStagesV) & 1) &&
-                 globaltimer_ns() - t0 < lim) {}
+        for (uint32_t i = issued > kStagesK ? issued - kStagesK : 0; i < issued; ++i) {
+          while (!mbar_try_wait(bars.at(full0 + (i % kStagesK)), (i / kStagesK) & 1) && globaltimer_ns() - t0 < lim) {}
         }
         for (uint32_t i = issued_q > 2 ? issued_q - 2 : 0; i < issued_q; ++i) {
           while (!mbar_try_wait(bars.at(Bars::kQFull + (i & 1)), (i >> 1) & 1) && globaltimer_ns() - t0 < lim) {}
         }
+        while (!mbar_try_wait(bars.at(Bars::kDrain + (is_k ? 2 : 3)), 0) && globaltimer_ns() - t0 < lim) {}
       }
     } else if (warp == kIssuerWarp && lane == 0) {
       // ========================================= QK^T issuer ====================================
@@ -552,7 +553,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
         for (int i = 0; ok && i < n; ++i) {
           const uint32_t G = gb + i, st = G % kStagesK;
-          // the K tile has landed (the copy warp saw k_full) and its scales are in tensor memory
+          // the K tile has landed (its loader saw k_full) and its scales are in tensor memory
           ok = mbar_wait(bars.at(Bars::kKsf + st), (G / kStagesK) & 1, wc, kS64Ksf);
           if (!ok) break;
           tc_fence_after_sync();
@@ -626,47 +627,6 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         const uint64_t t0 = globaltimer_ns();
         tc_commit(bars.at(Bars::kDrain + 1));
         while (!mbar_try_wait(bars.at(Bars::kDrain + 1), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
-      }
-    } else if (warp == kCopyWarp && lane == 0) {
-      // ========================================= scale copier ===================================
-      // moves the K and V scale tiles of every stage into tensor memory as soon as they land, so
-      // that the two issuers spend their (slow, in-order) tcgen05 issue slots on products only.
-      // A stage's tensor-memory slot is free when its shared-memory stage is: the producer
-      // reloads the stage only after the products that used it have completed.
-      FA4_FOR_EACH_TILE {
-        const TileRec t = s_tiles[it];
-        const int n = t.n;
-        if (n <= 0) continue;
-        for (int step = 0; ok && step < n + 2; ++step) {
-          const int ik = step, iv = step - 2;  // the producer's order
-          if (ik < n) {
-            const uint32_t G = gb + ik, st = G % kStagesK;
-            ok = mbar_wait_relaxed<kSlackNs>(bars.at(Bars::kKFull + st), (G / kStagesK) & 1, wc, kS64KFull);
-            if (!ok) break;
-            tc_fence_after_sync();
-            const uint32_t ksf = base + kOffSFK + st * kQkSfSlot;
-#pragma unroll
-            for (int ks = 0; ks < kSteps; ++ks) tc_cp_sf(tmem + kTmSFK64 + 12 * st + 4 * ks, ksf + 512 * ks);
-            tc_commit(bars.at(Bars::kKsf + st));
-          }
-          if (iv >= 0 && iv < n) {
-            const uint32_t G = gb + iv, st = G % kStagesV;
-            ok = mbar_wait_relaxed<kSlackNs>(bars.at(Bars::kVFull + st), (G / kStagesV) & 1, wc, kS64VFull);
-            if (!ok) break;
-            tc_fence_after_sync();
-            const uint32_t vsf = base + kOffSFV + st * kSfBytes;
-            tc_cp_sf(tmem + kTmSFV64 + 8 * st, vsf);
-            tc_cp_sf(tmem + kTmSFV64 + 8 * st + 4, vsf + 512);
-            tc_commit(bars.at(Bars::kVsf + st));
-          }
-        }
-        gb += n;
-        ti += 1;
-      }
-      if (!ok) {
-        const uint64_t t0 = globaltimer_ns();
-        tc_commit(bars.at(Bars::kDrain + 2));
-        while (!mbar_try_wait(bars.at(Bars::kDrain + 2), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
       }
     }
   } else {
