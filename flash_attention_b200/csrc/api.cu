@@ -541,7 +541,15 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
         }
         return 0;
       };
-      if (general && local) {   // window (with or without sink / softcap / cache view)
+      // Windows of up to two blocks' worth of keys run the narrow form of the kernel.  us at B=2, S=4096,
+      // Hq=32, Hkv=8, causal, wide form / narrow form, D = 64 and 128: 128 keys 59/50, 65/59; 256 keys 74/61,
+      // 77/72; 384 keys 71/69, 73/77; 512 keys 82/82, 83/89.
+      const bool narrow = win_left >= 0 && win_right >= 0 && (int64_t)win_left + win_right <= 256;
+      if (general && local && narrow) {
+        rc = p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, true, true, true, true>)
+                         : (p->D == 64 ? launch64(attn_fwd_ws64_kernel<64, true, true, true, true>)
+                                       : launch64(attn_fwd_ws64_kernel<192, true, true, true, true>));
+      } else if (general && local) {   // window (with or without sink / softcap / cache view)
         rc = p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, true>)
                          : (p->D == 64 ? launch64(attn_fwd_ws64_kernel<64, true>)
                                        : launch64(attn_fwd_ws64_kernel<192, true>));

@@ -188,7 +188,13 @@ __device__ __forceinline__ uint32_t sw32_offset(uint32_t row, uint32_t chunk) {
 // the hot loop, sink and soft cap do not -- a call with only those keeps the plain geometry code,
 // which measured 16 % faster than carrying the window arithmetic along.)
 // kCache: per-entry key counts and page tables without the window arithmetic.
-template <int kD, bool kGeneral = false, bool kWindow = kGeneral, bool kCache = kWindow>
+// kNarrow (windows of a few blocks): most visited blocks are masked and a tile is over after a handful of
+// steps.  Masks go to the scores in registers instead of through tensor memory, and the Q K^T issuer
+// waits for the P slot of a step before it issues the step's scores, one wait instead of 512.  Both
+// shorten the chain of a short tile and cost a long one: the branch sits in the hot loop, and Q K^T no
+// longer runs ahead of P V.  us, wide form -> this one: 127-key window, D = 64 114 -> 93; 1023 keys, D = 128
+// 143 -> 161.
+template <int kD, bool kGeneral = false, bool kWindow = kGeneral, bool kCache = kWindow, bool kNarrow = false>
 __global__ void __launch_bounds__(ws64::kThreads, 1)
 attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
                      const __grid_constant__ CUtensorMap tm_k,
@@ -563,6 +569,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           // (keys 0-63 and 64-127 of the tile): half the tcgen05 instructions of two N = 64
           // products, and the in-order issue slots of this thread are scarce
           const uint32_t J0 = 2 * G, b0 = J0 % kSBufs;  // 0 or 2
+          if (kNarrow && J0 >= kPSlots) {
+            ok = mbar_wait(bars.at(Bars::kPvDone + ((J0 + 1) % kPSlots)), ((J0 + 1 - kPSlots) / kPSlots) & 1, wc, kS64PvDone);
+            if (!ok) break;
+          }
           if (J0 >= kSBufs) {
             ok = mbar_wait(bars.at(Bars::kSFree + b0), ((J0 - kSBufs) / kSBufs) & 1, wc, kS64SFree) &&
                  mbar_wait(bars.at(Bars::kSFree + b0 + 1), ((J0 - kSBufs) / kSBufs) & 1, wc, kS64SFree);
@@ -649,18 +659,20 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         const int h64 = j & 1;
         const uint32_t bar_s = bars.at(Bars::kSFull + (wg & 2)), par_s = (J / kSBufs) & 1;
         const uint32_t bar_p = bars.at(Bars::kPvDone + slot), par_p = ((J - kPSlots) / kPSlots) & 1;
-        const bool r_p = (J >= kPSlots) ? mbar_test(bar_p, par_p) : true;
+        const bool r_p = (kNarrow || J < kPSlots) ? true : mbar_test(bar_p, par_p);
 
         // 1. the scores of this sub-block: the whole 64-key row of this thread
         ok = __all_sync(0xffffffffu, mbar_test(bar_s, par_s)) || __all_sync(0xffffffffu, mbar_wait_flag(bar_s, par_s, s_abort));
         if (!ok) break;
         tc_fence_after_sync();
-        if (needs_mask<kWindow>(p, t, nb)) {
-          if constexpr (kWindow) {
-            ws::mask_scores_in_tmem_range(s_addr, lower_key(p, t, row, nb) - 64 * h64,
-                                          upper_key<true>(p, t, row, nb) - 64 * h64);
-          } else {
-            mask_scores_in_tmem(s_addr, upper_key<false>(p, t, row, nb) - 64 * h64);
+        if constexpr (!kNarrow) {
+          if (needs_mask<kWindow>(p, t, nb)) {
+            if constexpr (kWindow) {
+              ws::mask_scores_in_tmem_range(s_addr, lower_key(p, t, row, nb) - 64 * h64,
+                                            upper_key<true>(p, t, row, nb) - 64 * h64);
+            } else {
+              mask_scores_in_tmem(s_addr, upper_key<false>(p, t, row, nb) - 64 * h64);
+            }
           }
         }
         float s[64];
@@ -683,6 +695,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         tc_wait_ld();
         tc_fence_before_sync();
         mbar_arrive(bars.at(Bars::kSFree + wg));
+        if constexpr (kNarrow) {
+          if (needs_mask<true>(p, t, nb))
+            mask_scores64(s, lower_key(p, t, row, nb) - 64 * h64, upper_key<true>(p, t, row, nb) - 64 * h64);
+        }
         if constexpr (kGeneral) {
           if (sc.softcap_c1 != 0.f) {
 #pragma unroll
@@ -725,8 +741,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         m_ref = m_new;
 
         // 3. exponentials and quantisation; P slot J % 8 is free once P V of sub-block J - 8 has run
-        ok = __all_sync(0xffffffffu, r_p) || __all_sync(0xffffffffu, mbar_wait_flag(bar_p, par_p, s_abort));
-        if (!ok) break;
+        if constexpr (!kNarrow) {
+          ok = __all_sync(0xffffffffu, r_p) || __all_sync(0xffffffffu, mbar_wait_flag(bar_p, par_p, s_abort));
+          if (!ok) break;
+        }
         uint8_t* p_tile = gbase + kOffP + slot * kPTileBytes;
         {
           uint32_t pk[8];

@@ -315,10 +315,17 @@ __device__ __forceinline__ float quantize_row(const float (&s)[128], const float
   return acc;
 }
 
-// Causal / key-length mask of one row: keys with in-block index > limit become -inf.
-__device__ __forceinline__ void mask_row(float (&s)[128], int limit) {
+// Mask of 64 scores of a row in registers: keys with index > limit or < lower become -inf.  As bit words,
+// so that a score costs a predicate extraction shared by a few of them and a select.
+__device__ __forceinline__ void mask_scores64(float (&s)[64], int lower, int limit) {
 #pragma unroll
-  for (int c = 0; c < 128; ++c) s[c] = (c <= limit) ? s[c] : kNegInf;
+  for (int w = 0; w < 2; ++w) {
+    const int n = limit + 1 - 32 * w, m = lower - 32 * w;
+    uint32_t keep = n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u);
+    keep &= m <= 0 ? 0xffffffffu : (m >= 32 ? 0u : 0xffffffffu << m);
+#pragma unroll
+    for (int x = 0; x < 32; ++x) s[32 * w + x] = ((keep >> x) & 1u) ? s[32 * w + x] : kNegInf;
+  }
 }
 
 }  // namespace fa4

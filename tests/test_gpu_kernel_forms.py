@@ -1,0 +1,93 @@
+"""The branches of the dispatch and of the host path at the sizes where they can go wrong: the edge between
+the narrow and the wide window form, more tiles than CTAs with tiles that have no rows between them, tile
+lists longer than a CTA's table, and the quantiser's small, unaligned and strided inputs."""
+import numpy as np
+import pytest
+import torch
+
+import flash_attention_b200 as fa
+from oracle import nvfp4_oracle as orc
+from tests.helpers import assert_parity, make_qkv, oracles
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D", [64, 128, 192])
+@pytest.mark.parametrize("window", [(256, 0), (257, 0), (128, 128), (0, 0), (1, 300)])
+def test_window_forms_over_several_tiles_per_cta(cuda_device, window, D):
+    q, k, v = make_qkv(2, 430, 430, 24, 2, D, seed=3, device=cuda_device)
+    if D == 192:
+        v = v[..., :128].contiguous()
+    Q, K, V = fa.quantize_qkv(q, k, v)
+    out, lse = fa.flash_attn_func(Q, K, V, window_size=window, return_lse=True)
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    assert_parity(out, lse, *oracles(Q, K, V, False, window=window))
+
+
+@pytest.mark.parametrize("causal", [True, False])
+def test_packed_batch_with_empty_tiles_between_full_ones(cuda_device, causal):
+    lens = [700, 1, 130, 390, 5, 700, 64, 257, 129, 31]
+    cu = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32, device=cuda_device)
+    q, k, v = (t[0] for t in make_qkv(1, sum(lens), sum(lens), 8, 2, 128, seed=4, device=cuda_device))
+    Q, K, V, cu_v = fa.quantize_varlen_qkv(q, k, v, cu)
+    out, lse = fa.flash_attn_varlen_fp4_func(Q.data[0], K.data[0], V.data[0], Q.sf[0], K.sf[0], V.sf[0], Q.scale, K.scale,
+                                             V.scale, cu, cu, cu_seqlens_v=cu_v, max_seqlen_q=700, max_seqlen_k=700,
+                                             causal=causal, return_lse=True)
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    for i, n in enumerate(lens):
+        a, b, s0 = int(cu[i]), int(cu[i + 1]), int(cu_v[i])
+        s1 = s0 + (n + 31) // 32 * 32
+        o, l = fa.flash_attn_fp4_func(
+            Q.data[:, a:b], K.data[:, a:b], V.data[..., s0 // 2:s1 // 2].contiguous(), Q.sf[:, a:b].contiguous(),
+            K.sf[:, a:b].contiguous(), V.sf[..., s0 // 16:s1 // 16].contiguous(), Q.scale, K.scale, V.scale, causal=causal,
+            return_lse=True, variant=fa.VARIANT_WS64)
+        assert torch.equal(out[a:b], o[0]) and torch.equal(lse[:, a:b], l[0]), i
+
+
+def test_tile_list_longer_than_the_table_of_a_cta(cuda_device):
+    sms = torch.cuda.get_device_properties(cuda_device).multi_processor_count
+    Hq, Sq = 256, 16
+    B = 768 * sms // Hq + 20                      # a second launch with a partial round
+    g = torch.Generator(device=cuda_device).manual_seed(5)
+    q, k, v = (torch.randn(B, S, H, 64, generator=g, device=cuda_device, dtype=torch.bfloat16)
+               for S, H in ((Sq, Hq), (96, 8), (96, 8)))
+    Q, K, V = fa.quantize_qkv_fused(q, k, v)
+    out, _ = fa.flash_attn_func(Q, K, V, causal=True)
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    for b in (0, B // 2, B - 3, B - 1):
+        part = [fa.NVFP4Tensor(t.data[b:b + 1], t.sf[b:b + 1], t.scale, is_v=t.is_v) for t in (Q, K, V)]
+        assert torch.equal(out[b:b + 1], fa.flash_attn_func(*part, causal=True)[0]), b
+
+
+@pytest.mark.parametrize("B,S,H,D,offset", [(1, 1, 1, 64, 0), (1, 333, 4, 128, 0), (2, 129, 3, 192, 0),
+                                            (3, 700, 16, 128, 0), (1, 200, 4, 64, 8)])
+def test_quantiser_against_the_oracle(cuda_device, B, S, H, D, offset):
+    """Small tensors (one row per work item), large ones (four), and views whose 32-byte pieces are only
+    16-byte aligned; the scale is fetched from the device when it is read."""
+    g = torch.Generator().manual_seed(6)
+    base = torch.randn(B, S, H + 1, D + 8, generator=g).bfloat16().to(cuda_device)
+    x = base[:, :, :H, offset:offset + D]
+    Q, K, V = fa.quantize_qkv_fused(x, x, x)
+    want = orc.quantize_nvfp4(x.float().cpu().numpy())
+    for t in (Q, K):
+        assert t.scale == want.scale
+        assert np.array_equal(t.data.cpu().numpy(), want.data) and np.array_equal(t.sf.cpu().numpy(), want.sf)
+        lin = np.transpose(want.sf, (0, 2, 1, 3))
+        assert np.array_equal(t.sf_tiled.cpu().numpy(), orc.sf_linear_to_tiled(lin, 1))
+    padded = torch.nn.functional.pad(x.float().cpu(), (0, 0, 0, 0, 0, -S % 32)).permute(0, 2, 3, 1).numpy()
+    want_v = orc.quantize_nvfp4(padded)
+    assert np.array_equal(V.data.cpu().numpy(), want_v.data) and np.array_equal(V.sf.cpu().numpy(), want_v.sf)
+    assert np.array_equal(V.sf_tiled.cpu().numpy(), orc.sf_linear_to_tiled(want_v.sf, 2))
+
+
+def test_scales_on_the_device_give_the_bits_of_scales_on_the_host(cuda_device):
+    q, k, v = make_qkv(1, 200, 300, 4, 2, 128, seed=7, device=cuda_device)
+    for kw in ({"causal": True}, {"softcap": 5.0}, {"num_splits": 2}):
+        lazy = fa.flash_attn_func(*fa.quantize_qkv_fused(q, k, v), return_lse=True, **kw)
+        ops = fa.quantize_qkv_fused(q, k, v)
+        assert all(isinstance(t.scale, float) for t in ops)
+        known = fa.flash_attn_func(*ops, return_lse=True, **kw)
+        assert torch.equal(lazy[0], known[0]) and torch.equal(lazy[1], known[1]), kw
