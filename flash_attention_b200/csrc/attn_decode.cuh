@@ -24,9 +24,11 @@
 // combine_splits_kernel, like the split-KV path of attn_ws.cuh.  Grid = (splits, Hkv, B).
 //   warps 0-3  softmax / correction / epilogue (thread = key lane, after the transpose a row; in the
 //              correction and the epilogue a dv lane)
+//   warps 8-11 up to eight rows: a second softmax warpgroup, which takes the odd blocks
 //   warp 4     TMA producer of K (ring of three tiles, through the page table if there is one)
-//   warp 5     MMA issuer (owns tensor memory)
+//   warp 5     issuer of K . Q^T (owns tensor memory)
 //   warp 6     TMA producer of V (its own ring, independent of K's)
+//   warp 7     issuer of V^T . P^T
 // Every wait is bounded, like everywhere else.
 #pragma once
 #include "attn_common.cuh"
@@ -35,13 +37,16 @@
 namespace fa4 {
 namespace dec {
 
-constexpr int kThreads = 224;
 // Three of everything: 70 KB of shared memory and 128 tensor-memory columns per CTA (256 in the
 // 32-row form), so that THREE CTAs share an SM (two in the 32-row form).
 constexpr int kStages = 3;   // K and V tiles in flight
 constexpr int kSBufs = 3;    // S^T buffers (N columns each)
 constexpr int kPSlots = 3;   // P^T tiles (N rows x 64 bytes) and their scale chunks
 constexpr int kMaxRows = 32; // query rows per kv head: Sq * group
+// Softmax warpgroups: two up to eight rows, one above (registers: three CTAs of twelve warps per SM
+// leave 56 per thread).  With two, even blocks go to one and odd ones to the other.
+__host__ __device__ constexpr int softmax_wgs(int rows) { return rows <= 8 ? 2 : 1; }
+__host__ __device__ constexpr int threads_of(int rows) { return softmax_wgs(rows) == 2 ? 384 : 256; }
 
 // shared memory
 constexpr uint32_t kOffK = 0;
@@ -53,15 +58,16 @@ constexpr uint32_t kOffQ = kOffSFV + kStages * kSfBytes;   // rows x 64 bytes, 6
 constexpr uint32_t kOffSFQ = kOffQ + kQBytes;              // two 512-byte chunks
 constexpr uint32_t kOffP = kOffSFQ + 1024;                 // kPSlots x kQBytes
 constexpr uint32_t kOffSFP = kOffP + kPSlots * kQBytes;    // kPSlots x 2 chunks x 512
-constexpr uint32_t kOffRed = kOffSFP + kPSlots * 1024;     // 2 x 4 warps x 32 floats
-constexpr uint32_t kOffBar = kOffRed + 2 * 4 * kMaxRows * 4;
+constexpr uint32_t kOffRed = kOffSFP + kPSlots * 1024;     // 2 WGs x 2 x 4 warps x 32 floats
+constexpr uint32_t kOffHand = kOffRed + 2 * 2 * 4 * kMaxRows * 4;   // 2 WGs x 4 warps x 32 references
+constexpr uint32_t kOffBar = kOffHand + 2 * 4 * kMaxRows * 4;
 struct Bars {
   uint32_t base;
-  static constexpr uint32_t kKFull = 0, kVFull = kKFull + kStages, kKFree = kVFull + kStages,
-                            kVFree = kKFree + kStages, kSFull = kVFree + kStages,
+  static constexpr uint32_t kKFull = 0, kVFull = kKFull + kStages, kSFull = kVFull + kStages,
                             kSFree = kSFull + kSBufs, kPFull = kSFree + kSBufs,
                             kPvDone = kPFull + kPSlots, kQReady = kPvDone + kPSlots,
-                            kSync = kQReady + 1, kDrain = kSync + 1, kCount = kDrain + 1;
+                            kSync = kQReady + 1 /* 2 */, kHand = kSync + 2 /* 2 x 4 */, kFin = kHand + 8,
+                            kDrain = kFin + 1 /* 2 */, kCount = kDrain + 2;
   __device__ explicit Bars(uint32_t b) : base(b) {}
   __device__ __forceinline__ uint32_t at(uint32_t idx) const { return base + 8u * idx; }
 };
@@ -84,7 +90,7 @@ struct Tm {
   static_assert(kSFP + 16 <= kCols, "tensor-memory map of the decode kernel");
 };
 
-enum Site { kDKFull = 80, kDVFull, kDKFree, kDVFree, kDSFull, kDSFree, kDPFull, kDPvDone, kDQReady, kDSync };
+enum Site { kDKFull = 80, kDVFull, kDKFree, kDVFree, kDSFull, kDSFree, kDPFull, kDPvDone, kDQReady, kDSync, kDHand, kDFin };
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
   asm volatile(
@@ -205,7 +211,7 @@ struct DecodeParams {
 // lane-group transpose and the number of keys a thread owns afterwards.  N (the MMA's N, the
 // columns of an S^T buffer) is 16 up to sixteen rows and 32 above.
 template <int kR>
-__global__ void __launch_bounds__(dec::kThreads, kR <= 16 ? 3 : 2)
+__global__ void __launch_bounds__(dec::threads_of(kR), kR <= 16 ? 3 : 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const KernelParams p, const DecodeParams d) {
   using namespace dec;
@@ -215,7 +221,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   const Bars bars(base + kOffBar);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + kOffMisc);
   volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(gbase + kOffMisc + 4);
-  volatile float* s_red = reinterpret_cast<volatile float*>(gbase + kOffRed);  // [2][4][32]
+  volatile float* s_red = reinterpret_cast<volatile float*>(gbase + kOffRed);    // [2][2][4][32]
+  volatile float* s_hand = reinterpret_cast<volatile float*>(gbase + kOffHand);  // [2][4][32]
+  constexpr int kWgs = softmax_wgs(kR);
   constexpr int kN = kR <= 16 ? 16 : 32;
   using TM = Tm<kN>;
 
@@ -230,16 +238,16 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bars.at(Bars::kKFull + s), 1);
       mbar_init(bars.at(Bars::kVFull + s), 1);
-      mbar_init(bars.at(Bars::kKFree + s), 1);
-      mbar_init(bars.at(Bars::kVFree + s), 1);
       mbar_init(bars.at(Bars::kSFull + s), 1);
       mbar_init(bars.at(Bars::kSFree + s), 128);
       mbar_init(bars.at(Bars::kPFull + s), 128);
       mbar_init(bars.at(Bars::kPvDone + s), 1);
     }
     mbar_init(bars.at(Bars::kQReady), 128);
-    mbar_init(bars.at(Bars::kSync), 128);
-    mbar_init(bars.at(Bars::kDrain), 1);
+    for (int w = 0; w < 2; ++w) mbar_init(bars.at(Bars::kSync + w), 128);
+    for (int w = 0; w < 8; ++w) mbar_init(bars.at(Bars::kHand + w), 32);
+    mbar_init(bars.at(Bars::kFin), 128);
+    for (int w = 0; w < 2; ++w) mbar_init(bars.at(Bars::kDrain + w), 1);
     fence_barrier_init();
   }
   if (warp == 4 && lane == 0) tma_prefetch_desc(&tm_k);
@@ -302,7 +310,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     // the kernel ran at one block per memory latency.)
     if (lane == 0) {
       const bool is_k = warp == 4;
-      const uint32_t full0 = is_k ? Bars::kKFull : Bars::kVFull, free0 = is_k ? Bars::kKFree : Bars::kVFree;
+      // (a K stage is free once its scores are in tensor memory, a V stage once its product is in O: no
+      // commits of their own)
+      static_assert(kStages == kSBufs && kStages == kPSlots, "stages are recycled through s_full and pv_done");
+      const uint32_t full0 = is_k ? Bars::kKFull : Bars::kVFull, free0 = is_k ? Bars::kSFull : Bars::kPvDone;
       const uint32_t tile0 = base + (is_k ? kOffK : kOffV), sf0 = base + (is_k ? kOffSFK : kOffSFV);
       const uint8_t* sf_src = is_k ? p.k_sf + hk * p.ksf_stride_h : p.v_sf + hk * p.vsf_stride_h;
       const int64_t sf_stride_b = is_k ? p.ksf_stride_b : p.vsf_stride_b;
@@ -340,7 +351,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       }
     }
   } else if (warp == 5) {
-    // ============================================ MMA issuer ====================================
+    // ============================================ K . Q^T issuer ===============================
+    // (One thread that issued both products paced the kernel: the copies, products and commits of a
+    // block are fourteen tcgen05 instructions, about 100 clocks of issue each.)
     if (lane == 0 && n > 0) {
       ok = mbar_wait(bars.at(Bars::kQReady), 0, wc, kDQReady);
       uint64_t dq[2];
@@ -352,53 +365,25 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           dq[ks] = make_desc_sw64(base + kOffQ + 32 * ks);
         }
       }
-      for (int step = 0; ok && step < n + 2; ++step) {
-        if (step < n) {
-          // S^T = K . Q^T of block step
-          const uint32_t li = step, st = li % kStages, buf = li % kSBufs;
-          ok = mbar_wait(bars.at(Bars::kKFull + st), (li / kStages) & 1, wc, kDKFull);
+      for (int li = 0; ok && li < n; ++li) {
+        const uint32_t st = li % kStages, buf = li % kSBufs;
+        ok = mbar_wait(bars.at(Bars::kKFull + st), (li / kStages) & 1, wc, kDKFull);
+        if (!ok) break;
+        if (li >= kSBufs) {
+          ok = mbar_wait(bars.at(Bars::kSFree + buf), ((li - kSBufs) / kSBufs) & 1, wc, kDSFree);
           if (!ok) break;
-          if (li >= kSBufs) {
-            ok = mbar_wait(bars.at(Bars::kSFree + buf), ((li - kSBufs) / kSBufs) & 1, wc, kDSFree);
-            if (!ok) break;
-          }
-          tc_fence_after_sync();
-          const uint32_t sfk = tmem + TM::kSFK + 8 * (li & 1);
-          const uint32_t kt = base + kOffK + st * kTileBytes, ksf = base + kOffSFK + st * kSfBytes;
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks) tc_cp_sf(sfk + 4 * ks, ksf + 512 * ks);
-#pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            mma_nvf4(tmem + TM::kS + kN * buf, make_desc_sw64(kt + 32 * ks), dq[ks], idesc, sfk + 4 * ks,
-                     tmem + TM::kSFQ + 4 * ks, ks > 0 ? 1u : 0u);
-          }
-          tc_commit(bars.at(Bars::kSFull + buf));
-          tc_commit(bars.at(Bars::kKFree + st));
         }
-        if (step >= 2) {
-          // O^T += V^T . P^T of block step - 2
-          const uint32_t li = step - 2, st = li % kStages, slot = li % kPSlots;
-          ok = mbar_wait(bars.at(Bars::kVFull + st), (li / kStages) & 1, wc, kDVFull);
-          if (!ok) break;
-          ok = mbar_wait(bars.at(Bars::kPFull + slot), (li / kPSlots) & 1, wc, kDPFull);
-          if (!ok) break;
-          tc_fence_after_sync();
-          const uint32_t sfv = tmem + TM::kSFV + 8 * (li & 1), sfp = tmem + TM::kSFP + 8 * (li & 1);
-          const uint32_t vt = base + kOffV + st * kTileBytes, vsf = base + kOffSFV + st * kSfBytes;
-          const uint32_t pt = base + kOffP + slot * kQBytes, psf = base + kOffSFP + slot * 1024;
+        tc_fence_after_sync();
+        const uint32_t sfk = tmem + TM::kSFK + 8 * (li & 1);
+        const uint32_t kt = base + kOffK + st * kTileBytes, ksf = base + kOffSFK + st * kSfBytes;
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            tc_cp_sf(sfv + 4 * ks, vsf + 512 * ks);
-            tc_cp_sf(sfp + 4 * ks, psf + 512 * ks);
-          }
+        for (int ks = 0; ks < 2; ++ks) tc_cp_sf(sfk + 4 * ks, ksf + 512 * ks);
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            mma_nvf4(tmem + TM::kO, make_desc_sw64(vt + 32 * ks), make_desc_sw64(pt + 32 * ks), idesc,
-                     sfv + 4 * ks, sfp + 4 * ks, (li > 0 || ks > 0) ? 1u : 0u);
-          }
-          tc_commit(bars.at(Bars::kPvDone + slot));
-          tc_commit(bars.at(Bars::kVFree + st));
+        for (int ks = 0; ks < 2; ++ks) {
+          mma_nvf4(tmem + TM::kS + kN * buf, make_desc_sw64(kt + 32 * ks), dq[ks], idesc, sfk + 4 * ks,
+                   tmem + TM::kSFQ + 4 * ks, ks > 0 ? 1u : 0u);
         }
+        tc_commit(bars.at(Bars::kSFull + buf));   // scores ready; also: the K stage is free
       }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();
@@ -406,22 +391,60 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         while (!mbar_try_wait(bars.at(Bars::kDrain), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
       }
     }
-  } else {
-    // ============================================ softmax / epilogue warpgroup ==================
-    const uint32_t lane_addr = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+  } else if (warp == 7) {
+    // ============================================ V^T . P^T issuer =============================
+    if (lane == 0) {
+      for (int li = 0; ok && li < n; ++li) {
+        const uint32_t st = li % kStages, slot = li % kPSlots;
+        ok = mbar_wait(bars.at(Bars::kVFull + st), (li / kStages) & 1, wc, kDVFull);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t sfv = tmem + TM::kSFV + 8 * (li & 1), sfp = tmem + TM::kSFP + 8 * (li & 1);
+        const uint32_t vt = base + kOffV + st * kTileBytes, vsf = base + kOffSFV + st * kSfBytes;
+        const uint32_t pt = base + kOffP + slot * kQBytes, psf = base + kOffSFP + slot * 1024;
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) tc_cp_sf(sfv + 4 * ks, vsf + 512 * ks);
+        ok = mbar_wait(bars.at(Bars::kPFull + slot), (li / kPSlots) & 1, wc, kDPFull);
+        if (!ok) break;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) tc_cp_sf(sfp + 4 * ks, psf + 512 * ks);
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+          mma_nvf4(tmem + TM::kO, make_desc_sw64(vt + 32 * ks), make_desc_sw64(pt + 32 * ks), idesc,
+                   sfv + 4 * ks, sfp + 4 * ks, (li > 0 || ks > 0) ? 1u : 0u);
+        }
+        tc_commit(bars.at(Bars::kPvDone + slot));   // O stable; also: the P slot and the V stage are free
+      }
+      if (!ok) {
+        const uint64_t t0 = globaltimer_ns();
+        tc_commit(bars.at(Bars::kDrain + 1));
+        while (!mbar_try_wait(bars.at(Bars::kDrain + 1), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
+      }
+    }
+  } else if (warp < 4 || warp >= 8) {
+    // ============================================ softmax warpgroups, epilogue ==================
+    // Warpgroup wg takes the blocks li = wg, wg + kWgs, ...; the first one also prepares the operands
+    // and writes the result.  What a block hands to the next one is the reference maximum of its rows,
+    // from warp wq of one warpgroup to warp wq of the other (every warp knows all rows); everything
+    // else of a block -- about 1000 clocks of latencies -- then runs beside the neighbouring block's.
+    const int wg = warp >> 3, wq = warp & 3;
+    const uint32_t lane_addr = tmem + (static_cast<uint32_t>(wq * 32) << 16);
+    s_red += wg * (2 * 4 * kMaxRows);
     uint32_t sync_phase = 0;
     // rendezvous of the 128 threads on an mbarrier (bounded, unlike bar.sync)
 #define FA4_DEC_SYNC()                                                                          \
-  mbar_arrive(bars.at(Bars::kSync));                                                            \
-  ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kSync), sync_phase & 1, wc, kDSync));     \
+  mbar_arrive(bars.at(Bars::kSync + wg));                                                       \
+  ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kSync + wg), sync_phase & 1, wc, kDSync)); \
   sync_phase += 1;
 
     // ---- set-up: Q^T operand (rows x 64 bytes, rows past R zero), its scale chunks, zeroed
     //      P^T tiles and scale chunks (rows past R are never written again)
+    ok = true;
+    if (wg == 0) {
     for (uint32_t i = tid; i < (kOffRed - kOffQ) / 16; i += 128) {
       *reinterpret_cast<uint4*>(gbase + kOffQ + i * 16) = make_uint4(0u, 0u, 0u, 0u);  // Q, SFQ, P, SFP are contiguous
     }
-    ok = true;
     FA4_DEC_SYNC()
     if (ok) {
       const int r = tid >> 2, ch = tid & 3;
@@ -434,13 +457,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
     fence_proxy_async_smem();
     mbar_arrive(bars.at(Bars::kQReady));
+    }
 
     // After the transpose below a thread owns ONE query row (row = lane % kR) with kR neighbouring
     // keys of its warp's 32 (group = lane / kR), so everything per row -- mask limit, reference
     // maximum, block exponent, running sum -- is scalar per thread and runs once per block, where a
     // thread that kept "its key, all rows" ran it kR times.
     const int my_row = lane & (kR - 1), grp = lane / kR;
-    const int key_in_blk = warp * 32 + grp * kR;   // first of this thread's kR keys inside the block
+    const int key_in_blk = wq * 32 + grp * kR;   // first of this thread's kR keys inside the block
     float m_ref = kNegInf, l_sum = 0.f;
     // last visible key of the row (causal: bottom-right aligned on the entry's key count); rows
     // past R see nothing
@@ -450,7 +474,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       lim = (p.causal && c < sk - 1) ? c : sk - 1;
     }
 
-    for (int li = 0; ok && li < n; ++li) {
+    for (int li = wg; ok && li < n; li += kWgs) {
       const int nb = i0 + li;
       const uint32_t buf = li % kSBufs, slot = li % kPSlots;
       ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kSFull + buf), (li / kSBufs) & 1, wc, kDSFull));
@@ -487,21 +511,36 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       } else {
         wm = fmaxf(bm[0], bm[kB - 1]);
       }
-      volatile float* red = s_red + (li & 1) * (4 * kMaxRows);
-      if (lane < kR) red[warp * kMaxRows + lane] = wm;
+      volatile float* red = s_red + ((li / kWgs) & 1) * (4 * kMaxRows);
+      if (lane < kR) red[wq * kMaxRows + lane] = wm;
       FA4_DEC_SYNC()
       if (!ok) break;
 
       // reference maximum of the row (CTA-uniform per row: every warp computes the same value)
       const float m_loc = fmaxf(fmaxf(red[my_row], red[kMaxRows + my_row]),
                                 fmaxf(red[2 * kMaxRows + my_row], red[3 * kMaxRows + my_row]));
-      const float m_new = next_reference(m_ref, m_loc, sc.sl2);
+      float m_prev = m_ref;
+      if (kWgs == 2 && li > 0) {
+        // the reference after block li - 1 (the unbroken chain also orders the reuse of the slots: block
+        // li + 1 overwrites this one's source only after it has read what this block hands on)
+        ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kHand + 4 * (wg ^ 1) + wq), ((li - 1) >> 1) & 1, wc, kDHand));
+        if (!ok) break;
+        m_prev = s_hand[((wg ^ 1) * 4 + wq) * kMaxRows + my_row];
+      }
+      const float m_new = next_reference(m_prev, m_loc, sc.sl2);
+      if (kWgs == 2) {
+        if (lane < kR) s_hand[(wg * 4 + wq) * kMaxRows + my_row] = m_new;
+        mbar_arrive(bars.at(Bars::kHand + 4 * wg + wq));
+      }
       float fac = 1.f;
       bool moved_row = false;
+      if (m_new != m_prev) {
+        fac = reference_factor(m_prev, m_new, sc.sl2);
+        moved_row = m_prev != kNegInf;
+      }
+      // this warpgroup's share of the row sum follows the reference (kWgs = 1: by the same factor)
       if (m_new != m_ref) {
-        fac = reference_factor(m_ref, m_new, sc.sl2);
-        moved_row = m_ref != kNegInf;
-        l_sum *= fac;
+        l_sum *= kWgs == 1 ? fac : reference_factor(m_ref, m_new, sc.sl2);
         m_ref = m_new;
       }
       const bool moved = __any_sync(0xffffffffu, moved_row);   // every warp holds all rows
@@ -585,19 +624,28 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
     // ---- epilogue: row sums over the 128 key lanes, then thread = dv lane of O^T --------------
     if (ok) {
-      volatile float* red = s_red + (n & 1) * (4 * kMaxRows);
       float v = l_sum;   // this thread's share of its row; the lanes of one row are kR apart
 #pragma unroll
       for (int o = kR; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane < kR) red[warp * kMaxRows + lane] = v;
-      FA4_DEC_SYNC()
+      // (the buffer of the exchange after the last one)
+      volatile float* red = s_red + (((n + kWgs - 1 - wg) / kWgs) & 1) * (4 * kMaxRows);
+      if (lane < kR) red[wq * kMaxRows + lane] = v;
+      if (kWgs == 2 && wg == 1) {
+        // the second warpgroup leaves its sums and their reference to the first and is done
+        if (wq == 0 && lane < kR) s_hand[4 * kMaxRows + kMaxRows + lane] = m_ref;
+        mbar_arrive(bars.at(Bars::kFin));
+      } else {
+        FA4_DEC_SYNC()
+      }
     }
-    if (ok) {
-      volatile float* red = s_red + (n & 1) * (4 * kMaxRows);
+    if (ok && wg == 0) {
+      volatile float* red = s_red + (((n + kWgs - 1) / kWgs) & 1) * (4 * kMaxRows);
+      volatile float* red_b = s_red + 2 * 4 * kMaxRows + ((n / 2) & 1) * (4 * kMaxRows);
       float o[kR];
 #pragma unroll
       for (int r = 0; r < kR; ++r) o[r] = 0.f;
-      if (n > 0) {
+      if (kWgs == 2) ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kFin), 0, wc, kDFin));
+      if (ok && n > 0) {
         ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kPvDone + ((n - 1) % kPSlots)),
                                                ((n - 1) / kPSlots) & 1, wc, kDPvDone));
         if (ok) {
@@ -610,14 +658,21 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
           if (r < R) {
-            // fixed order over the four warps: the sum of a row does not depend on timing
-            const float l_tot = ((red[r] + red[kMaxRows + r]) + red[2 * kMaxRows + r]) + red[3 * kMaxRows + r];
+            // fixed order over the warps: the sum of a row does not depend on timing
+            float l_tot = ((red[r] + red[kMaxRows + r]) + red[2 * kMaxRows + r]) + red[3 * kMaxRows + r];
+            float m_fin = __shfl_sync(0xffffffffu, m_ref, r);      // lane r of every warp owns row r
+            if (kWgs == 2) {
+              const float m_a = m_fin, m_b = s_hand[5 * kMaxRows + r];
+              m_fin = fmaxf(m_a, m_b);
+              const float l_b = ((red_b[r] + red_b[kMaxRows + r]) + red_b[2 * kMaxRows + r]) + red_b[3 * kMaxRows + r];
+              l_tot = l_tot * reference_factor(m_a, m_fin, sc.sl2) + l_b * reference_factor(m_b, m_fin, sc.sl2);
+            }
             const int s = r / p.group, h = hk * p.group + r % p.group;
             const float scale = (l_tot > 0.f && n > 0) ? sc.out_scale / l_tot : 0.f;
             d.o_partial[((((int64_t)split * p.B + b) * p.Sq + s) * p.Hq + h) * 128 + tid] = o[r] * scale;
-            if (tid == r) {   // thread r (warp 0, lane r) owns row r: its m_ref is the row's
+            if (tid == r) {
               d.lse_partial[(((int64_t)split * p.B + b) * p.Hq + h) * p.Sq + s] =
-                  finish_lse(m_ref, l_tot, sc.sl2);
+                  finish_lse(m_fin, l_tot, sc.sl2);
             }
           }
         }
