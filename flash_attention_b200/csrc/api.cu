@@ -114,19 +114,26 @@ int ensure_kernel(Kernel kernel, uint32_t bytes, int expected_regs) {
 // Every kernel asks for the largest shared-memory carve-out, also those that use none: an SM changes
 // its carve-out only while it is empty, which would take the overlap away again.
 template <class... KArgs, class... Args>
-int launch_pdl(void (*kernel)(KArgs...), dim3 grid, unsigned threads, uint32_t smem, cudaStream_t stream, Args&&... args) {
+int launch_pdl_cluster(unsigned cluster, void (*kernel)(KArgs...), dim3 grid, unsigned threads, uint32_t smem,
+                       cudaStream_t stream, Args&&... args) {
   if (int e = prepare_kernel(reinterpret_cast<const void*>(kernel), smem, 0)) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim = {cluster, 1, 1};
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return (int)cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <class Kernel, class... Args>
+int launch_pdl(Kernel kernel, dim3 grid, unsigned threads, uint32_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_pdl_cluster(1, kernel, grid, threads, smem, stream, std::forward<Args>(args)...);
 }
 
 }  // namespace
@@ -146,6 +153,15 @@ extern "C" int fa4_nvfp4_query(int32_t what) {
 }
 
 namespace {
+// Whether the decode kernel merges the splits of an entry itself, as one cluster: up to eight (the
+// portable cluster size), while all CTAs are resident at once.  Beyond that the clusters start unevenly
+// (B=64, Sk=4096, two splits, 1024 CTAs: 64 us with the combine kernel, 68 with clusters; one token at
+// Sk=777, 24 CTAs: 8.8 and 7.7).  A single split needs neither.
+bool decode_in_cluster(const fa4_nvfp4_params* p, int num_splits) {
+  const int64_t ctas = (int64_t)num_splits * p->Hkv * p->B;
+  const int64_t resident = 148 * (p->Sq * (p->Hq / p->Hkv) <= 16 ? 3 : 2);
+  return num_splits == 1 || (num_splits <= dec::kMaxCluster && ctas <= resident);
+}
 int64_t splitkv_bytes(const fa4_nvfp4_params* p, int num_splits) {
   // partial O (num_splits, B, Sq, Hq, Dv) fp32, then partial LSE (num_splits, B, Hq, Sq) fp32
   return (int64_t)num_splits * p->B * p->Sq * p->Hq * ((int64_t)p->Dv + 1) * 4;
@@ -292,6 +308,7 @@ extern "C" int64_t fa4_nvfp4_splitkv_workspace_bytes(const fa4_nvfp4_params* p, 
   if (p == nullptr || p->struct_size != sizeof(fa4_nvfp4_params)) return -FA4_E_STRUCT;
   if (num_splits < 1 || num_splits > 128 || p->B <= 0 || p->Sq <= 0 || p->Hq <= 0 || p->Dv <= 0)
     return -FA4_E_SHAPE;
+  if (p->variant == FA4_VARIANT_DECODE && p->Hkv > 0 && p->Hq >= p->Hkv && decode_in_cluster(p, num_splits)) return 0;
   return num_splits == 1 ? 0 : splitkv_bytes(p, num_splits);
 }
 
@@ -348,19 +365,20 @@ int validate_fwd(const fa4_nvfp4_params* p, int num_splits, const void* workspac
     return -FA4_E_VARIANT;
   const bool decode = variant == FA4_VARIANT_DECODE;
   if (decode) {
-    // a handful of query rows per kv head, head dim 128, causal or unmasked; always through the
-    // partial-output workspace and the combine kernel
+    // a handful of query rows per kv head, head dim 128, causal or unmasked
     if (p->D != 128 || p->Dv != 128 || (int64_t)p->Sq * (p->Hq / p->Hkv) > dec::kMaxRows) return -FA4_E_SHAPE;
     if (win_left >= 0 || win_right > 0 || sink != nullptr || softcap > 0.f) return -FA4_E_SHAPE;
-    if (workspace == nullptr || !aligned16(workspace)) return -FA4_E_NULL;
-    if (workspace_bytes < (uint64_t)splitkv_bytes(p, num_splits)) return -FA4_E_TOO_LARGE;
+    if (!decode_in_cluster(p, num_splits)) {
+      if (workspace == nullptr || !aligned16(workspace)) return -FA4_E_NULL;
+      if (workspace_bytes < (uint64_t)splitkv_bytes(p, num_splits)) return -FA4_E_TOO_LARGE;
+    }
   }
   if (variant == FA4_VARIANT_WS64 && !takes64) return -FA4_E_SHAPE;
   if (d192 && variant != FA4_VARIANT_WS64) return -FA4_E_SHAPE;
   // window limits: `causal` is the right limit 0; an explicit right limit overrides it
   if (p->causal && win_right < 0) win_right = 0;
   const bool local = win_left >= 0 || win_right > 0;
-  if (num_splits > 1) {
+  if (num_splits > 1 && !decode) {
     if (workspace == nullptr) return -FA4_E_NULL;
     if (!aligned16(workspace)) return -FA4_E_ALIGN;
     if (workspace_bytes < (uint64_t)splitkv_bytes(p, num_splits)) return -FA4_E_TOO_LARGE;
@@ -482,7 +500,7 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
   kp.num_splits = num_splits;
   kp.Dv = p->Dv;
   kp.o_partial = static_cast<float*>(workspace);
-  kp.lse_partial = (num_splits > 1 || decode)
+  kp.lse_partial = workspace != nullptr
                        ? kp.o_partial + (int64_t)num_splits * p->B * p->Sq * p->Hq * p->Dv
                        : nullptr;
 
@@ -498,15 +516,20 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     dp.num_splits = num_splits;
     dp.o_partial = kp.o_partial;
     dp.lse_partial = kp.lse_partial;
+    const bool merge = decode_in_cluster(p, num_splits);
     auto launch_dec = [&](auto kernel, int rows, uint32_t smem) -> int {
-      return launch_pdl(kernel, dim3((unsigned)num_splits, (unsigned)p->Hkv, (unsigned)p->B), dec::threads_of(rows), smem, stream,
-                        tm_k, tm_v, kp, dp);
+      return launch_pdl_cluster(merge ? (unsigned)num_splits : 1u, kernel,
+                                dim3((unsigned)num_splits, (unsigned)p->Hkv, (unsigned)p->B), dec::threads_of(rows), smem,
+                                stream, tm_k, tm_v, kp, dp);
     };
-    const int rc = dec_rows <= 4    ? launch_dec(attn_decode_kernel<4>, 4, dec::kSmemRequest)
-                   : dec_rows <= 8  ? launch_dec(attn_decode_kernel<8>, 8, dec::kSmemRequest)
-                   : dec_rows <= 16 ? launch_dec(attn_decode_kernel<16>, 16, dec::kSmemRequest)
-                                    : launch_dec(attn_decode_kernel<32>, 32, dec::kSmemRequestWide);
-    if (rc != 0) return rc;
+#define FA4_DEC(rows, smem) \
+  (merge ? launch_dec(attn_decode_kernel<rows, true>, rows, smem) : launch_dec(attn_decode_kernel<rows, false>, rows, smem))
+    const int rc = dec_rows <= 4    ? FA4_DEC(4, dec::kSmemRequest)
+                   : dec_rows <= 8  ? FA4_DEC(8, dec::kSmemRequest)
+                   : dec_rows <= 16 ? FA4_DEC(16, dec::kSmemRequest)
+                                    : FA4_DEC(32, dec::kSmemRequestWide);
+#undef FA4_DEC
+    if (rc != 0 || merge) return rc;
   } else {
     // persistent: one CTA per SM walks the tile list
     int dev = 0, sms = 0;
@@ -720,7 +743,6 @@ extern "C" int fa4_nvfp4_quantize_jobs_bf16(const fa4_nvfp4_quant_job* jobs, int
     const fa4_nvfp4_quant_job& a = jobs[i];
     if (int e = describe_tensor(&q.job[i], a.x, a.B, a.S, a.H, a.D, a.stride_b, a.stride_s, a.stride_h)) return e;
     if (int e = describe_outputs(&q.job[i], a.is_v != 0, a.S_out, a.packed, a.sf_linear, a.sf_tiled, a.scale_out)) return e;
-    q.job[i].scale_host = a.scale_host;
   }
   const cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   if (int e = launch_amax(q, stream)) return e;

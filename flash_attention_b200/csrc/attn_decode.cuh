@@ -20,8 +20,9 @@
 // row and 16 keys, lazy reference).
 //
 // One CTA = one (split, kv head, batch entry): a contiguous share of the entry's 128-key blocks,
-// visited in ascending order; it writes a normalised fp32 partial O and a partial LSE for
-// combine_splits_kernel, like the split-KV path of attn_ws.cuh.  Grid = (splits, Hkv, B).
+// visited in ascending order; its normalised fp32 partial O and partial LSE are merged inside the
+// cluster of an entry's splits (up to eight), or by combine_splits_kernel as on the split-KV path of
+// attn_ws.cuh.  Grid = (splits, Hkv, B).
 //   warps 0-3  softmax / correction / epilogue (thread = key lane, after the transpose a row; in the
 //              correction and the epilogue a dv lane)
 //   warps 8-11 up to eight rows: a second softmax warpgroup, which takes the odd blocks
@@ -42,6 +43,7 @@ namespace dec {
 constexpr int kStages = 3;   // K and V tiles in flight
 constexpr int kSBufs = 3;    // S^T buffers (N columns each)
 constexpr int kPSlots = 3;   // P^T tiles (N rows x 64 bytes) and their scale chunks
+constexpr int kMaxCluster = 8;  // splits that are merged inside a cluster (portable cluster size)
 constexpr int kMaxRows = 32; // query rows per kv head: Sq * group
 // Softmax warpgroups: two up to eight rows, one above (registers: three CTAs of twelve warps per SM
 // leave 56 per thread).  With two, even blocks go to one and odd ones to the other.
@@ -210,7 +212,9 @@ struct DecodeParams {
 // kR: query rows the softmax code is built for (4, 8, 16 or 32 >= Sq * group): the size of the
 // lane-group transpose and the number of keys a thread owns afterwards.  N (the MMA's N, the
 // columns of an S^T buffer) is 16 up to sixteen rows and 32 above.
-template <int kR>
+// kMerge: the splits of a (kv head, batch entry) are one cluster, which merges their partials through
+// distributed shared memory and writes the result; otherwise they go to o_partial / lse_partial.
+template <int kR, bool kMerge>
 __global__ void __launch_bounds__(dec::threads_of(kR), kR <= 16 ? 3 : 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const KernelParams p, const DecodeParams d) {
@@ -669,10 +673,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             }
             const int s = r / p.group, h = hk * p.group + r % p.group;
             const float scale = (l_tot > 0.f && n > 0) ? sc.out_scale / l_tot : 0.f;
-            d.o_partial[((((int64_t)split * p.B + b) * p.Sq + s) * p.Hq + h) * 128 + tid] = o[r] * scale;
-            if (tid == r) {
-              d.lse_partial[(((int64_t)split * p.B + b) * p.Hq + h) * p.Sq + s] =
-                  finish_lse(m_fin, l_tot, sc.sl2);
+            const float lse = finish_lse(m_fin, l_tot, sc.sl2);
+            if constexpr (kMerge) {
+              // (the K ring is free: every product has completed)
+              reinterpret_cast<float*>(gbase + kOffK)[r * 128 + tid] = o[r] * scale;
+              if (tid == r) reinterpret_cast<float*>(gbase + kOffV)[r] = lse;
+            } else {
+              d.o_partial[((((int64_t)split * p.B + b) * p.Sq + s) * p.Hq + h) * 128 + tid] = o[r] * scale;
+              if (tid == r) d.lse_partial[(((int64_t)split * p.B + b) * p.Hq + h) * p.Sq + s] = lse;
             }
           }
         }
@@ -681,6 +689,42 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 #undef FA4_DEC_SYNC
   }
 
+  if constexpr (kMerge) {
+    // Merge (the arithmetic of combine_splits_kernel): row r by CTA r % splits, thread = dv.  A launch of
+    // its own for it costs 2-3 us behind a kernel of 6.  Every thread of every CTA comes here, also
+    // after a wait that ran out (then nothing is written).
+    cluster_sync();
+    if (warp < 4) {
+      const uint32_t ns = d.num_splits;
+      uint32_t gave_up = 0;
+      for (uint32_t i = 0; i < ns; ++i) gave_up |= ld_cluster_u32(base + kOffMisc + 4, i);
+      for (int r = split; r < R && gave_up == 0; r += ns) {
+        float l[kMaxCluster], v[kMaxCluster], m = kNegInf;
+#pragma unroll
+        for (uint32_t i = 0; i < kMaxCluster; ++i) {
+          l[i] = i < ns ? __uint_as_float(ld_cluster_u32(base + kOffV + 4 * r, i)) : kNegInf;
+          v[i] = i < ns ? __uint_as_float(ld_cluster_u32(base + kOffK + 4 * (r * 128 + tid), i)) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < kMaxCluster; ++i) m = fmaxf(m, l[i]);
+        float acc = 0.f, sum = 0.f;
+        if (m != kNegInf) {
+#pragma unroll
+          for (int i = 0; i < kMaxCluster; ++i) {
+            const float w = __expf(l[i] - m);
+            sum += w;
+            acc = fmaf(w, v[i], acc);
+          }
+          acc *= 1.f / sum;
+        }
+        const int s = r / p.group, h = hk * p.group + r % p.group;
+        p.out[b * p.o_stride_b + s * p.o_stride_s + h * p.o_stride_h + tid] = __float2bfloat16_rn(acc);
+        if (tid == 0 && p.lse != nullptr)
+          p.lse[((int64_t)b * p.Hq + h) * p.Sq + s] = m == kNegInf ? kNegInf : m + __logf(sum);
+      }
+    }
+    cluster_sync();      // no CTA leaves while another may read its shared memory
+  }
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 5) tmem_dealloc(tmem, TM::kCols);

@@ -15,7 +15,8 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
-#include <ATen/cuda/CachingHostAllocator.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Device.h>
@@ -102,25 +103,27 @@ bool truth_of(PyObject* o) {
   return v != 0;
 }
 // ---- per-tensor scales that are still on their way ------------------------------------------------
-// What quantize_qkv hands out for a scale: the quantiser writes it to the device and to pinned host
-// memory.  An attention call on the quantiser's stream reads the device copy, so quantising and
-// attending never wait on the host; float(scale) waits for the stream once, for all three tensors.
+// What quantize_qkv hands out for a scale: the quantiser leaves it on the device, and an attention call
+// on the quantiser's stream reads it there, so quantising and attending never wait on the host.
+// float(scale) copies all three back and waits for the stream, once.
 struct ScaleState {
-  at::Tensor device, pinned;        // three floats each
+  c10::DataPtr device;              // three floats
   cudaStream_t stream;
   bool known = false;
   float value[3];
+  const float* ptr(int i) const { return static_cast<const float*>(device.get()) + i; }
   void fetch() {
     if (known) return;
     cudaError_t e;
+    float v[3];
+    c10::cuda::CUDAGuard guard(device.device().index());
     Py_BEGIN_ALLOW_THREADS
-    e = cudaStreamSynchronize(stream);
+    e = cudaMemcpyAsync(v, device.get(), sizeof v, cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     Py_END_ALLOW_THREADS
     C10_CUDA_CHECK(e);
-    if (known) return;              // another thread was faster
-    std::copy_n(pinned.data_ptr<float>(), 3, value);
+    std::copy_n(v, 3, value);
     known = true;
-    pinned.reset();
   }
 };
 struct LazyScale {
@@ -155,8 +158,8 @@ bool device_scales(PyObject* const* o, const at::Device& device, cudaStream_t st
     if (!is_lazy(o[i])) return false;
     const LazyScale* s = reinterpret_cast<const LazyScale*>(o[i]);
     const ScaleState& st = **s->state;
-    if (st.known || st.stream != stream || st.device.device() != device) return false;
-    ptr[i] = st.device.data_ptr<float>() + s->which;
+    if (st.stream != stream || st.device.device() != device) return false;
+    ptr[i] = st.ptr(s->which);
   }
   return true;
 }
@@ -271,6 +274,14 @@ at::Tensor sink_of(PyObject* o, int64_t Hq, const at::Device& device) {
   return t.to(device, at::kFloat).contiguous();
 }
 
+// ---- allocation ---------------------------------------------------------------------------------------
+// (at::empty goes through the dispatcher, 2-4 us a call on the hosts of these GPUs; these do not)
+at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dtype, const at::Device& device) {
+  return at::detail::empty_cuda(sizes, dtype, device, std::nullopt);
+}
+// Scratch of the current stream, given back to it when the launches that use it have been issued.
+c10::DataPtr scratch_bytes(int64_t bytes) { return c10::cuda::CUDACachingAllocator::get()->allocate((size_t)bytes); }
+
 // ---- linear scales -> the tiled layout, the three tensors of a call in one launch ------------------
 // One job: (outer, inner) matrices of rows x cols bytes.
 fa4_nvfp4_sf_job sf_job(const at::Tensor& sf, int64_t outer, int64_t inner, int64_t rows, int64_t cols,
@@ -287,7 +298,7 @@ fa4_nvfp4_sf_job sf_job(const at::Tensor& sf, int rows_dim, int head_dim, int64_
                 sf.stride(rows_dim), mult);
 }
 // Allocates the tiles of all jobs as one buffer and launches; the tiles of job i are at jobs[i].dst.
-at::Tensor tile_scales(fa4_nvfp4_sf_job (&jobs)[3], const at::Tensor& like, void* stream) {
+c10::DataPtr tile_scales(fa4_nvfp4_sf_job (&jobs)[3], void* stream) {
   int64_t bytes[3], total = 0;
   for (int i = 0; i < 3; ++i) {
     const fa4_nvfp4_sf_job& j = jobs[i];
@@ -295,8 +306,8 @@ at::Tensor tile_scales(fa4_nvfp4_sf_job (&jobs)[3], const at::Tensor& like, void
     bytes[i] = (int64_t)j.n_outer * j.n_inner * cdiv(j.rows, 128) * ct * 512;
     total += bytes[i];
   }
-  at::Tensor out = at::empty({total}, like.options());
-  uint8_t* at_byte = out.data_ptr<uint8_t>();
+  c10::DataPtr out = scratch_bytes(total);
+  uint8_t* at_byte = static_cast<uint8_t*>(out.get());
   for (int i = 0; i < 3; at_byte += bytes[i++]) jobs[i].dst = at_byte;
   check_rc(fa4_nvfp4_sf_tile_jobs(jobs, 3, stream), "fa4_nvfp4_sf_tile_jobs");
   return out;
@@ -369,7 +380,7 @@ PyObject* fwd(PyObject* const* a) {
   if (device.index() != c10::cuda::current_device()) guard.set_device(device);
   void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
 
-  at::Tensor tiles;                       // scratch for tiled copies of linear scales
+  c10::DataPtr tiles;                     // scratch for tiled copies of linear scales
   const void* sf_ptr[3];
   const char* layout = PyUnicode_Check(a[14]) ? PyUnicode_AsUTF8(a[14]) : nullptr;
   if (layout != nullptr && !strcmp(layout, "linear")) {
@@ -380,7 +391,7 @@ PyObject* fwd(PyObject* const* a) {
     k_sf = inner_contiguous(std::move(k_sf));
     v_sf = inner_contiguous(std::move(v_sf));
     fa4_nvfp4_sf_job jobs[3] = {sf_job(q_sf, 1, 2, 1), sf_job(k_sf, 1, 2, 1), sf_job(v_sf, 2, 1, 2)};
-    tiles = tile_scales(jobs, q, stream);
+    tiles = tile_scales(jobs, stream);
     for (int i = 0; i < 3; ++i) sf_ptr[i] = jobs[i].dst;
   } else if (layout != nullptr && !strcmp(layout, "tiled")) {
     validate(q_sf, "q_sf", {B, Hq, cdiv(Sq, 128), D / 64, 512}, at::kByte, device);
@@ -398,7 +409,7 @@ PyObject* fwd(PyObject* const* a) {
 
   at::Tensor out, lse;
   if (is_none(out_o)) {
-    out = at::empty({B, Sq, Hq, Dv}, q.options().dtype(at::kBFloat16));
+    out = new_tensor({B, Sq, Hq, Dv}, at::kBFloat16, device);
   } else {
     out = tensor_of(out_o, "out");
     validate(out, "out", {B, Sq, Hq, Dv}, at::kBFloat16, device);
@@ -409,7 +420,7 @@ PyObject* fwd(PyObject* const* a) {
     validate(lse, "lse", {B, Hq, Sq}, at::kFloat, device);
     FA4_ASSERT(lse.is_contiguous(), "lse must be contiguous");
   } else if (truth_of(a[11])) {
-    lse = at::empty({B, Hq, Sq}, q.options().dtype(at::kFloat));
+    lse = new_tensor({B, Hq, Sq}, at::kFloat, device);
   }
 
   fa4_nvfp4_params p = {};
@@ -477,12 +488,12 @@ PyObject* fwd(PyObject* const* a) {
       x.pages_per_seq = (int32_t)pages_per_seq;
       x.num_pages = (int32_t)B_kv;
     }
-    at::Tensor workspace;   // stream-ordered scratch
-    if (num_splits > 1 || decode) {
-      const int64_t bytes = fa4_nvfp4_splitkv_workspace_bytes(&p, (int32_t)std::max(2l, num_splits));
-      if (bytes < 0) check_rc((int)bytes, "fa4_nvfp4_splitkv_workspace_bytes");
-      workspace = at::empty({bytes}, q.options());
-      x.workspace = workspace.data_ptr();
+    c10::DataPtr workspace;
+    const int64_t bytes = fa4_nvfp4_splitkv_workspace_bytes(&p, (int32_t)num_splits);
+    if (bytes < 0) check_rc((int)bytes, "fa4_nvfp4_splitkv_workspace_bytes");
+    if (bytes > 0) {
+      workspace = scratch_bytes(bytes);
+      x.workspace = workspace.get();
       x.workspace_bytes = (uint64_t)bytes;
     }
     if (lazy)
@@ -561,9 +572,9 @@ PyObject* varlen_fwd(PyObject* const* a) {
   jobs[1].cu_seqlens = cu_k.data_ptr<int32_t>();
   jobs[2].cu_seqlens = (cu_v.defined() ? cu_v : cu_k).data_ptr<int32_t>();
   jobs[0].packed_rows = jobs[1].packed_rows = 1;
-  const at::Tensor tiles = tile_scales(jobs, q, stream);
-  at::Tensor out = at::empty({total_q, Hq, Dv}, q.options().dtype(at::kBFloat16)), lse;
-  if (truth_of(a[21])) lse = at::empty({Hq, total_q}, q.options().dtype(at::kFloat));
+  const c10::DataPtr tiles = tile_scales(jobs, stream);
+  at::Tensor out = new_tensor({total_q, Hq, Dv}, at::kBFloat16, device), lse;
+  if (truth_of(a[21])) lse = new_tensor({Hq, total_q}, at::kFloat, device);
 
   fa4_nvfp4_params p = {};
   p.struct_size = sizeof p;
@@ -611,7 +622,8 @@ PyObject* quantize_qkv(PyObject* const* a) {
   const bool linear = truth_of(a[3]);
   const at::Device device = tensor_of(a[0], "q").device();
   fa4_nvfp4_quant_job jobs[3] = {};
-  at::Tensor packed[3], lin[3], tiled[3], scratch, scales, pinned;
+  at::Tensor packed[3], lin[3], tiled[3];
+  c10::DataPtr scratch, scales;
   c10::cuda::OptionalCUDAGuard guard;
   for (int i = 0; i < 3; ++i) {
     const at::Tensor& x = tensor_of(a[i], names[i]);
@@ -620,22 +632,20 @@ PyObject* quantize_qkv(PyObject* const* a) {
                "quantize_qkv_fused takes CUDA bf16 (B, S, H, D) tensors, last dim contiguous");
     if (i == 0) {
       if (device.index() != c10::cuda::current_device()) guard.set_device(device);
-      scales = at::empty({3}, x.options().dtype(at::kFloat));
-      scratch = at::empty({FA4_QUANT_SCRATCH_FLOATS}, scales.options());
-      pinned = at::empty({3}, at::TensorOptions().dtype(at::kFloat).pinned_memory(true));
+      scales = scratch_bytes(3 * sizeof(float));
+      scratch = scratch_bytes(FA4_QUANT_SCRATCH_FLOATS * sizeof(float));
     }
-    const auto bytes = x.options().dtype(at::kByte);
     const int64_t B = x.size(0), S = x.size(1), H = x.size(2), D = x.size(3);
     // V is blocked along its key axis, stored padded with zeros to whole 32-key groups
     const int64_t s_out = i == 2 ? cdiv(S, 32) * 32 : S;
     if (i == 2) {
-      packed[i] = at::empty({B, H, D, s_out / 2}, bytes);
-      if (linear) lin[i] = at::empty({B, H, D, s_out / 16}, bytes);
-      tiled[i] = at::empty({B, H, cdiv(D, 128), 2 * cdiv(s_out, 128), 512}, bytes);
+      packed[i] = new_tensor({B, H, D, s_out / 2}, at::kByte, device);
+      if (linear) lin[i] = new_tensor({B, H, D, s_out / 16}, at::kByte, device);
+      tiled[i] = new_tensor({B, H, cdiv(D, 128), 2 * cdiv(s_out, 128), 512}, at::kByte, device);
     } else {
-      packed[i] = at::empty({B, S, H, D / 2}, bytes);
-      if (linear) lin[i] = at::empty({B, S, H, D / 16}, bytes);
-      tiled[i] = at::empty({B, H, cdiv(S, 128), D / 64, 512}, bytes);
+      packed[i] = new_tensor({B, S, H, D / 2}, at::kByte, device);
+      if (linear) lin[i] = new_tensor({B, S, H, D / 16}, at::kByte, device);
+      tiled[i] = new_tensor({B, H, cdiv(S, 128), D / 64, 512}, at::kByte, device);
     }
     fa4_nvfp4_quant_job& j = jobs[2 - i];   // V first: its tiles take longest
     j.x = x.data_ptr();
@@ -646,16 +656,12 @@ PyObject* quantize_qkv(PyObject* const* a) {
     j.packed = packed[i].data_ptr();
     j.sf_linear = linear ? lin[i].data_ptr() : nullptr;
     j.sf_tiled = tiled[i].data_ptr();
-    j.scale_out = scales.data_ptr<float>() + i;
-    j.scale_host = pinned.data_ptr<float>() + i;
+    j.scale_out = static_cast<float*>(scales.get()) + i;
   }
   const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(device.index());
-  check_rc(fa4_nvfp4_quantize_jobs_bf16(jobs, 3, scratch.data_ptr<float>(), stream.stream()), "fa4_nvfp4_quantize_jobs_bf16");
-  // the pinned words go back to their pool no earlier than the launch has written them
-  at::getHostAllocator(at::kCUDA)->record_event(pinned.data_ptr(), pinned.storage().data_ptr().get_context(), stream.unwrap());
+  check_rc(fa4_nvfp4_quantize_jobs_bf16(jobs, 3, static_cast<float*>(scratch.get()), stream.stream()), "fa4_nvfp4_quantize_jobs_bf16");
   auto state = std::make_shared<ScaleState>();
-  state->device = scales;
-  state->pinned = pinned;
+  state->device = std::move(scales);
   state->stream = stream.stream();
   PyObject* res = PyTuple_New(3);
   for (int i = 0; i < 3; ++i) {

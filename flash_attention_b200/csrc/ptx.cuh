@@ -197,6 +197,28 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------------------------
+// thread-block clusters
+// ---------------------------------------------------------------------------------------------
+// Rendezvous of all threads of a cluster; what was written to shared memory before is visible after.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// The word at shared-memory address `addr` of CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr, uint32_t rank) {
+  uint32_t v;
+  asm volatile(
+      "{\n"
+      ".reg .b32 a;\n"
+      "mapa.shared::cluster.u32 a, %1, %2;\n"
+      "ld.shared::cluster.u32 %0, [a];\n"
+      "}\n"
+      : "=r"(v)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
+}
+
+// ---------------------------------------------------------------------------------------------
 // proxy / tcgen05 fences
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {

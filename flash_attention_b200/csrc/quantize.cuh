@@ -192,7 +192,7 @@ struct QuantJob {
   FastDiv div_nb, div_rt, div_h;
   int nb, rt;                   // Q / K: blocks of a row of all heads; 128-row (V: 128-key) tiles
   uint8_t *packed, *lin, *tiled;
-  float *scale_out, *scale_host;   // either may be null
+  float* scale_out;
 };
 struct QuantJobs {
   QuantJob job[3];
@@ -496,10 +496,7 @@ quantize_kernel(const __grid_constant__ QuantJobs jobs) {
     m = j.parts[0];
   }
   const TensorScale ts = make_tensor_scale(m);
-  if (first == 0 && threadIdx.x == 0) {
-    if (j.scale_out != nullptr) *j.scale_out = ts.g;
-    if (j.scale_host != nullptr) *j.scale_host = ts.g;
-  }
+  if (j.scale_out != nullptr && first == 0 && threadIdx.x == 0) *j.scale_out = ts.g;
   if (j.is_v) {
 #pragma unroll 1
     for (;;) {

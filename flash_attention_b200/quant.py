@@ -168,5 +168,8 @@ def quantize_qkv_fused(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, linear
     ``linear_sf=False`` skips the linear copies (then ``NVFP4Tensor.dequantize`` is unavailable).
     No host synchronisation: the per-tensor scales are fetched when ``scale`` is first read.
     """
-    return tuple(NVFP4Tensor(packed, lin, sc, False, is_v, tiled) if linear_sf else NVFP4Tensor(packed, tiled, sc, True, is_v)
-                 for (packed, lin, tiled, sc), is_v in zip(_lib.host().quantize_qkv(q, k, v, linear_sf), (False, False, True)))
+    (qd, ql, qt, qg), (kd, kl, kt, kg), (vd, vl, vt, vg) = _lib.host().quantize_qkv(q, k, v, linear_sf)
+    if linear_sf:
+        return (NVFP4Tensor(qd, ql, qg, False, False, qt), NVFP4Tensor(kd, kl, kg, False, False, kt),
+                NVFP4Tensor(vd, vl, vg, False, True, vt))
+    return NVFP4Tensor(qd, qt, qg, True), NVFP4Tensor(kd, kt, kg, True), NVFP4Tensor(vd, vt, vg, True, True)

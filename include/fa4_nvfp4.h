@@ -143,7 +143,8 @@ int fa4_nvfp4_fwd(const fa4_nvfp4_params* p, void* cuda_stream);
  * Sq (decode) this is what fills the GPU: without it there are only B * Hq * ceil(Sq/128) work
  * items.  `workspace`: caller-owned device memory, 16-byte aligned, at least
  * fa4_nvfp4_splitkv_workspace_bytes(p, num_splits) bytes (= num_splits * B * Sq * Hq * (Dv + 1)
- * floats; 0 for num_splits = 1, in which case this is fa4_nvfp4_fwd).  Split calls run the
+ * floats; 0 for num_splits = 1, in which case this is fa4_nvfp4_fwd, and 0 for FA4_VARIANT_DECODE
+ * when the kernel merges the splits itself).  Split calls run the
  * 128-key kernel (FA4_VARIANT_WS) or the decode kernel; D = 128 and 64.
  */
 int64_t fa4_nvfp4_splitkv_workspace_bytes(const fa4_nvfp4_params* p, int32_t num_splits);
@@ -360,8 +361,7 @@ typedef struct fa4_nvfp4_quant_job {
   void* packed;
   void* sf_linear;   /* or NULL */
   void* sf_tiled;    /* or NULL */
-  float* scale_out;  /* device, or NULL */
-  float* scale_host; /* the same in device-accessible (pinned) host memory, or NULL */
+  float* scale_out;  /* or NULL */
 } fa4_nvfp4_quant_job;
 int fa4_nvfp4_quantize_jobs_bf16(const fa4_nvfp4_quant_job* jobs, int32_t n, float* scratch, void* cuda_stream);
 
