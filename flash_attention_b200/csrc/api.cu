@@ -136,6 +136,34 @@ int launch_pdl(Kernel kernel, dim3 grid, unsigned threads, uint32_t smem, cudaSt
   return launch_pdl_cluster(1, kernel, grid, threads, smem, stream, std::forward<Args>(args)...);
 }
 
+// How many clusters of `cluster` CTAs can be resident at once (asked once per kernel, size and device;
+// 0 if the runtime cannot say).
+int clusters_at_once(const void* kernel, int cluster, unsigned threads, uint32_t smem) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, std::pair<int, int>>, int> seen;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_pair(kernel, std::make_pair(cluster, dev));
+  const auto it = seen.find(key);
+  if (it != seen.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cluster);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim = {(unsigned)cluster, 1, 1};
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    n = 0;
+  }
+  return seen[key] = n;
+}
+
 }  // namespace
 
 extern "C" int fa4_nvfp4_query(int32_t what) {
@@ -506,6 +534,8 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
 
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   const unsigned tiles = (unsigned)(kp.num_m_blocks * p->Hq * p->B * num_splits);
+  kp.merge_splits = 0;
+  bool merged = false;
   if (decode) {
     DecodeParams dp;
     dp.q = static_cast<const uint8_t*>(p->q);
@@ -549,7 +579,12 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     }
     auto launch = [&](auto kernel) -> int {
       if (int e = ensure_kernel(kernel, ws::kSmemRequest, ws::kRegsLaunch)) return e;
-      return launch_pdl(kernel, dim3(grid), ws::kThreads, ws::kSmemRequest, stream, tm_q, tm_k, tm_v, tm_o, kp);
+      // one work item per CTA and all clusters resident at once: the cluster of a tile merges its splits
+      kp.merge_splits = num_splits > 1 && num_splits <= ws::kMaxCluster && tiles <= (unsigned)sms &&
+                        clusters_at_once(reinterpret_cast<const void*>(kernel), num_splits, ws::kThreads,
+                                         ws::kSmemRequest) * num_splits >= (int)tiles;
+      merged = kp.merge_splits != 0;
+      return launch_pdl_cluster(merged ? (unsigned)num_splits : 1u, kernel, dim3(grid), ws::kThreads, ws::kSmemRequest, stream, tm_q, tm_k, tm_v, tm_o, kp);
     };
     int rc;
     if (variant == FA4_VARIANT_WS64) {
@@ -590,14 +625,18 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
       }
     } else if (p->D == 128) {
       rc = !general ? launch(attn_fwd_ws_kernel<128, false>)
-                    : (local ? launch(attn_fwd_ws_kernel<128, true>) : launch(attn_fwd_ws_kernel<128, true, false>));
+                    : (local ? launch(attn_fwd_ws_kernel<128, true>)
+                             : (softcap > 0.f ? launch(attn_fwd_ws_kernel<128, true, false>)
+                                              : launch(attn_fwd_ws_kernel<128, true, false, false>)));
     } else {
       rc = !general ? launch(attn_fwd_ws_kernel<64, false>)
-                    : (local ? launch(attn_fwd_ws_kernel<64, true>) : launch(attn_fwd_ws_kernel<64, true, false>));
+                    : (local ? launch(attn_fwd_ws_kernel<64, true>)
+                             : (softcap > 0.f ? launch(attn_fwd_ws_kernel<64, true, false>)
+                                              : launch(attn_fwd_ws_kernel<64, true, false, false>)));
     }
     if (rc != 0) return rc;
   }
-  if (num_splits > 1 || decode) {
+  if ((num_splits > 1 || decode) && !merged) {
     const int64_t items = (int64_t)p->B * p->Sq * p->Hq * (p->Dv / 4);
     int64_t blocks = (items + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;

@@ -59,6 +59,9 @@ struct KernelParams {
   // combine_splits_kernel merges them (flash_attn/cute/interface.py:494-510,804-812 and
   // flash_fwd_combine.py in the reference)
   int num_splits;
+  // 1: the splits of a tile are one cluster (one work item per CTA), which merges its partials through
+  // distributed shared memory and writes the result; the workspace is not used
+  int merge_splits;
   float* o_partial;    // (num_splits, B, Sq, Hq, Dv) fp32
   float* lse_partial;  // (num_splits, B, Hq, Sq) fp32
   int Dv;

@@ -243,15 +243,16 @@ __device__ __noinline__ void stage_accumulator_chunk(uint32_t taddr, uint8_t* st
   }
 }
 
-// Split-KV flavour of the same step: the 32 columns go out as fp32 (normalised by this split's
-// row sum) into the partial-output workspace.
-__device__ __noinline__ void store_accumulator_partial(uint32_t taddr, float* dst, float scale,
-                                                       uint32_t o_free_bar) {
+// Split-KV flavour of the same step: 32 columns go out as fp32 (normalised by this split's row sum), to
+// 16-byte chunks chunk0 .. chunk0 + 7 of the row at `dst` (each at its index XOR swz), in the
+// partial-output workspace or in shared memory.
+__device__ __noinline__ void store_accumulator_partial(uint32_t taddr, float* dst, uint32_t chunk0, uint32_t swz,
+                                                       float scale, uint32_t o_free_bar) {
   float4* d4 = reinterpret_cast<float4*>(dst);
   if (o_free_bar == 0u) {
     if (dst != nullptr) {
 #pragma unroll
-      for (int v = 0; v < 8; ++v) d4[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int v = 0; v < 8; ++v) d4[(chunk0 + v) ^ swz] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     return;
   }
@@ -263,10 +264,13 @@ __device__ __noinline__ void store_accumulator_partial(uint32_t taddr, float* ds
   if (dst == nullptr) return;
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
-    d4[v] = make_float4(__uint_as_float(o[4 * v]) * scale, __uint_as_float(o[4 * v + 1]) * scale,
-                        __uint_as_float(o[4 * v + 2]) * scale, __uint_as_float(o[4 * v + 3]) * scale);
+    d4[(chunk0 + v) ^ swz] =
+        make_float4(__uint_as_float(o[4 * v]) * scale, __uint_as_float(o[4 * v + 1]) * scale,
+                    __uint_as_float(o[4 * v + 2]) * scale, __uint_as_float(o[4 * v + 3]) * scale);
   }
 }
+
+constexpr int kMaxCluster = 8;   // splits of a tile that are merged inside a cluster (portable size)
 
 // Tile visited by CTA `cta` in round `it`: rounds alternate direction so that, with tiles sorted
 // by decreasing work, every CTA gets about the same total.
@@ -294,7 +298,9 @@ __device__ __forceinline__ uint64_t make_desc_qk(uint32_t tile_addr, int j) {
 // right window limits of local attention.
 // kWindow: the window half of kGeneral (mask arithmetic of the hot loops); general calls without a
 // window leave it out, which measured a third faster.
-template <int kD, bool kGeneral, bool kWindow = kGeneral>
+// kCap: the soft cap (its 64 hyperbolic tangents sit in the hot loop; chunk calls without it run 3 % faster
+// when they are not there).
+template <int kD, bool kGeneral, bool kWindow = kGeneral, bool kCap = kGeneral>
 __global__ void __launch_bounds__(ws::kThreads, 1)
 attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_k,
@@ -652,7 +658,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
         tc_fence_before_sync();
         mbar_arrive(bars.at(Bars::kSFree + b));
-        if constexpr (kGeneral) {
+        if constexpr (kCap) {
           // tanh is monotone: capping the eight block maxima is capping every score under them
           if (sc.softcap_c1 != 0.f) {
 #pragma unroll
@@ -747,7 +753,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         tc_wait_ld();
         tc_fence_before_sync();
         mbar_arrive(bars.at(Bars::kSFree + b));
-        if constexpr (kGeneral) {
+        if constexpr (kCap) {
           if (sc.softcap_c1 != 0.f) {
 #pragma unroll
             for (int x = 0; x < 64; ++x) s[x] = soft_cap(s[x], sc.softcap_c1);
@@ -827,10 +833,12 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
       }
       // warpgroup k stores output columns [32 k, 32 k + 32); with kD = 64 two of them only arrive
       if (kGeneral && p.num_splits > 1 && (kD == 128 || wg < kD / 32)) {
-        float* prow = p.o_partial +
-                      ((((int64_t)t.split * p.B + t.b) * p.Sq + q_idx) * p.Hq + t.h) * kD + 32 * wg;
-        store_accumulator_partial(lane_addr + kTmO + 32 * wg, q_idx < p.Sq ? prow : nullptr, scale,
-                                  n > 0 ? bars.at(Bars::kOFree) : 0u);
+        // (merged in the cluster: into the K and V rings, which are free -- every product has completed)
+        float* prow = p.merge_splits
+                          ? reinterpret_cast<float*>(gbase + kOffK) + row * kD
+                          : p.o_partial + ((((int64_t)t.split * p.B + t.b) * p.Sq + q_idx) * p.Hq + t.h) * kD;
+        store_accumulator_partial(lane_addr + kTmO + 32 * wg, q_idx < p.Sq ? prow : nullptr, 8 * wg,
+                                  p.merge_splits ? row & (kD / 4 - 1) : 0, scale, n > 0 ? bars.at(Bars::kOFree) : 0u);
       } else {
         if (it >= 1) {
           // the staging tile is free once the store warp's TMA has read the previous tile out of it
@@ -852,7 +860,9 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
           // a row without visible keys still has its sink: LSE = sink, output zero
           if (p.sink != nullptr && t.split == 0 && m_fin == kNegInf) lse_v = p.sink[t.h];
         }
-        if (kGeneral && p.num_splits > 1) {
+        if (kGeneral && p.merge_splits) {
+          reinterpret_cast<float*>(gbase + kOffOut)[row] = lse_v;
+        } else if (kGeneral && p.num_splits > 1) {
           p.lse_partial[(((int64_t)t.split * p.B + t.b) * p.Hq + t.h) * p.Sq + q_idx] = lse_v;
         } else if (p.lse != nullptr) {
           p.lse[((int64_t)t.b * p.Hq + t.h) * p.Sq + q_idx] = lse_v;
@@ -861,9 +871,66 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
       gb += n;
       ti += (n > 0) ? 1u : 0u;
     }
+    if constexpr (kGeneral) {
+      if (p.merge_splits) {
+        // The arithmetic of combine_splits_kernel, row r of the tile by CTA r % splits of the cluster, a warp
+        // per row.  Through the workspace the uncoalesced partial rows and the second launch cost 3 us more of
+        // 46 (B = 1, Sq = 128, Sk = 16384, Hq = 32).  Every thread comes here, also after a wait that ran
+        // out (then nothing is written).
+        static_assert(128 * kD * 4 <= (kStagesK + kStagesV) * kTileBytes, "partial O in the K and V rings");
+        cluster_sync();
+        {
+          const Tile t = decode_tile<true>(p, cta);     // one work item per CTA; its split is its rank
+          const uint32_t ns = p.num_splits;
+          uint32_t gave_up = 0;
+          for (uint32_t i = 0; i < ns; ++i) gave_up |= ld_cluster_u32(base + kOffMisc + 4, i);
+          for (uint32_t r = warp * ns + t.split; r < 128 && gave_up == 0; r += kStatsWarp0 * ns) {
+            const int q_idx = t.m_blk * kBlockM + r;
+            if (q_idx >= p.Sq) break;
+            const uint32_t o_addr = base + kOffK + r * (kD * 4) + ((lane ^ (r & (kD / 4 - 1))) << 4);
+            float l[kMaxCluster], m = kNegInf;
+            float4 v[kMaxCluster];
+#pragma unroll
+            for (uint32_t i = 0; i < kMaxCluster; ++i) {
+              l[i] = i < ns ? __uint_as_float(ld_cluster_u32(base + kOffOut + 4 * r, i)) : kNegInf;
+              v[i] = i < ns && lane < kD / 4 ? ld_cluster_f4(o_addr, i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < kMaxCluster; ++i) m = fmaxf(m, l[i]);
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            float sum = 0.f;
+            if (m != kNegInf) {
+#pragma unroll
+              for (int i = 0; i < kMaxCluster; ++i) {
+                const float w = __expf(l[i] - m);
+                sum += w;
+                acc.x = fmaf(w, v[i].x, acc.x);
+                acc.y = fmaf(w, v[i].y, acc.y);
+                acc.z = fmaf(w, v[i].z, acc.z);
+                acc.w = fmaf(w, v[i].w, acc.w);
+              }
+              const float inv = 1.f / sum;
+              acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
+            }
+            if (lane < kD / 4) {
+              __nv_bfloat16* dst = p.out + t.b * p.o_stride_b + q_idx * p.o_stride_s + t.h * p.o_stride_h + 4 * lane;
+              *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+            }
+            if (lane == 0 && p.lse != nullptr)
+              p.lse[((int64_t)t.b * p.Hq + t.h) * p.Sq + q_idx] = m == kNegInf ? kNegInf : m + __logf(sum);
+          }
+        }
+      }
+    }
   }
 #undef FA4_FOR_EACH_TILE
 
+  if constexpr (kGeneral) {
+    if (p.merge_splits) {
+      if (warp >= kStatsWarp0) cluster_sync();   // (the softmax warps have passed this one)
+      cluster_sync();      // no CTA leaves while another may read its shared memory
+    }
+  }
   tc_fence_before_sync();
   __syncthreads();
   if (warp == kIssuerWarp) tmem_dealloc(tmem, kTmemCols);

@@ -203,6 +203,20 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
+// Four floats at shared-memory address `addr` of CTA `rank` of the cluster.
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n"
+      ".reg .b32 a;\n"
+      "mapa.shared::cluster.u32 a, %4, %5;\n"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n"
+      "}\n"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
+}
 // The word at shared-memory address `addr` of CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr, uint32_t rank) {
   uint32_t v;
