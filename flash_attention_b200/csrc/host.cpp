@@ -15,6 +15,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CachingHostAllocator.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -676,6 +677,133 @@ PyObject* quantize_qkv(PyObject* const* a) {
   return res;
 }
 
+// ---- HostPipeline.run: the pieces of a call on operands in host memory -----------------------------
+// q k v q_sf k_sf v_sf (host) | the same on the device | out lse (device) | out_host lse_host | q_scale k_scale
+// v_scale softmax_scale causal | ranges [(s0, s1), ...] | streams in, compute, out (cudaStream_t as integers)
+//
+// Issued from Python a piece cost 140 us of host time against 155 us of its copy-out, so the loads went out
+// late; here it is about 45.  Tried and not kept: K and V by range as well, more and smaller pieces
+// (each copy beside a copy-out costs 30-40 us whatever its size), and loads by a kernel that reads the
+// pinned memory (no faster beside a copy-out, and it slows the kernels it runs next to).
+struct Event {
+  cudaEvent_t e = nullptr;
+  Event() { C10_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+  ~Event() { cudaEventDestroy(e); }
+  // what `then` is given next runs after what `first` holds now
+  void order(cudaStream_t first, cudaStream_t then) {
+    C10_CUDA_CHECK(cudaEventRecord(e, first));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(then, e, 0));
+  }
+};
+
+PyObject* host_pieces(PyObject* const* a) {
+  at::Tensor host[6], dev[6];
+  static const char* names[6] = {"q", "k", "v", "q_sf", "k_sf", "v_sf"};
+  for (int i = 0; i < 6; ++i) {
+    host[i] = tensor_of(a[i], names[i]);
+    dev[i] = tensor_of(a[6 + i], names[i]);
+  }
+  const at::Tensor out = tensor_of(a[12], "out"), lse = tensor_of(a[13], "lse"), out_host = tensor_of(a[14], "out_host");
+  at::Tensor lse_host;
+  if (!is_none(a[15])) lse_host = tensor_of(a[15], "lse_host");
+  const bool causal = truth_of(a[20]);
+  const auto device = dev[0].device();
+  cudaStream_t raw[3];
+  for (int i = 0; i < 3; ++i) {
+    raw[i] = static_cast<cudaStream_t>(PyLong_AsVoidPtr(a[22 + i]));
+    if (raw[i] == nullptr && PyErr_Occurred()) throw PyErrorSet();
+  }
+  const c10::cuda::CUDAStream s_in = c10::cuda::getStreamFromExternal(raw[0], device.index()),
+                              s_compute = c10::cuda::getStreamFromExternal(raw[1], device.index()),
+                              s_out = c10::cuda::getStreamFromExternal(raw[2], device.index());
+  const int64_t B = dev[0].size(0), Sq = dev[0].size(1), Hq = dev[0].size(2), Sk = dev[1].size(1), skp = 2 * dev[2].size(3);
+  PyObject* ranges = a[21];
+  c10::cuda::CUDAGuard device_guard(device);
+  Event in_done, compute_done;
+  PyObject* linear = PyUnicode_FromString("linear");
+  PyObject *zero = PyLong_FromLong(0), *one = PyLong_FromLong(1);
+  struct Refs {
+    PyObject* o[3];
+    ~Refs() { for (PyObject* x : o) Py_XDECREF(x); }
+  } refs{{linear, zero, one}};
+  // rows [r0, r1) of batch entry b (contiguous byte tensors, both sides)
+  auto load = [&](int i, int64_t b, int64_t r0, int64_t r1) {
+    const int64_t row = dev[i].stride(1), at_byte = b * dev[i].stride(0) + r0 * row;
+    C10_CUDA_CHECK(cudaMemcpyAsync(dev[i].data_ptr<uint8_t>() + at_byte,
+                                   static_cast<const uint8_t*>(host[i].data_ptr()) + at_byte, (r1 - r0) * row,
+                                   cudaMemcpyHostToDevice, raw[0]));
+  };
+  auto store = [&](const at::Tensor& to, const at::Tensor& from, int64_t b, int64_t r0, int64_t r1) {
+    if (to.is_contiguous() && to.scalar_type() == from.scalar_type() && to.sizes() == from.sizes()) {
+      const int64_t size = from.element_size(), row = from.stride(1) * size, at_byte = b * from.stride(0) * size + r0 * row;
+      C10_CUDA_CHECK(cudaMemcpyAsync(static_cast<uint8_t*>(to.data_ptr()) + at_byte,
+                                     static_cast<const uint8_t*>(from.data_ptr()) + at_byte, (r1 - r0) * row,
+                                     cudaMemcpyDeviceToHost, raw[2]));
+    } else {
+      c10::cuda::CUDAStreamGuard g(s_out);
+      to.select(0, b).narrow(0, r0, r1 - r0).copy_(from.select(0, b).narrow(0, r0, r1 - r0), /*non_blocking=*/true);
+    }
+  };
+  for (int64_t b = 0; b < B; ++b) {
+    // Few, large loads: while a copy-out runs, PCIe lets about 16 GB/s in, and each copy waits its turn.
+    // The query rows of the first entry come by range, so that its first piece starts early.
+    for (int i : {3, 4, 5, 1, 2}) load(i, b, 0, dev[i].size(1));
+    if (b > 0) load(0, b, 0, Sq);
+    for (Py_ssize_t n = 0; n < PyList_GET_SIZE(ranges); ++n) {
+      PyObject* r = PyList_GET_ITEM(ranges, n);
+      const int64_t s0 = integer_of(PyTuple_GET_ITEM(r, 0)), s1 = integer_of(PyTuple_GET_ITEM(r, 1));
+      const int64_t sk = causal ? s1 : Sk;     // s1 is a multiple of 128, or Sq == Sk for the last range
+      if (b == 0) load(0, b, s0, s1);
+      in_done.order(raw[0], raw[1]);
+      {
+        // one range of query rows against its keys, through the same entry as any other call.  The LSE of
+        // a partial range is a strided slice of (Hq, Sq): written compactly, then moved into place
+        c10::cuda::CUDAStreamGuard g(s_compute);
+        const bool whole = s1 - s0 == Sq;
+        const int64_t kp = cdiv(sk, 32) * 32;
+        const at::Tensor t[8] = {dev[0].narrow(0, b, 1).narrow(1, s0, s1 - s0), dev[1].narrow(0, b, 1).narrow(1, 0, sk),
+                                 dev[2].narrow(0, b, 1).narrow(3, 0, kp / 2),   dev[3].narrow(0, b, 1).narrow(1, s0, s1 - s0),
+                                 dev[4].narrow(0, b, 1).narrow(1, 0, sk),       dev[5].narrow(0, b, 1).narrow(3, 0, kp / 16),
+                                 out.narrow(0, b, 1).narrow(1, s0, s1 - s0),    lse.narrow(0, b, 1)};
+        PyObject* w[8];
+        for (int i = 0; i < 8; ++i) w[i] = THPVariable_Wrap(t[i]);
+        PyObject* args[23] = {w[0], w[1], w[2], w[3], w[4], w[5], a[16], a[17], a[18], a[19], a[20], Py_True, w[6],
+                              whole ? w[7] : Py_None, linear, zero, one, Py_None, Py_None, Py_None, zero, Py_None, Py_None};
+        PyObject* res = nullptr;
+        try {
+          res = fwd(args);
+        } catch (...) {
+          for (PyObject* x : w) Py_DECREF(x);
+          throw;
+        }
+        if (!whole) {
+          const at::Tensor& piece = THPVariable_Unpack(PyTuple_GET_ITEM(res, 1));
+          float* dst = lse.data_ptr<float>() + b * Hq * Sq + s0;
+          const cudaError_t e = cudaMemcpy2DAsync(dst, Sq * 4, piece.data_ptr<float>(), (s1 - s0) * 4, (s1 - s0) * 4, Hq,
+                                                  cudaMemcpyDeviceToDevice, raw[1]);
+          Py_DECREF(res);
+          res = nullptr;
+          for (PyObject*& x : w) Py_CLEAR(x);
+          C10_CUDA_CHECK(e);
+        }
+        Py_XDECREF(res);
+        for (PyObject* x : w) Py_XDECREF(x);
+      }
+      compute_done.order(raw[1], raw[2]);
+      store(out_host, out, b, s0, s1);
+    }
+    if (lse_host.defined()) store(lse_host, lse, b, 0, Hq);
+  }
+  // pinned blocks go back to their pool no earlier than these copies have run
+  auto keep = [](const at::Tensor& t, const c10::cuda::CUDAStream& s) {
+    if (t.is_pinned()) at::getHostAllocator(at::kCUDA)->record_event(t.data_ptr(), t.storage().data_ptr().get_context(), s.unwrap());
+  };
+  for (const at::Tensor& t : host) keep(t, s_in);
+  keep(out_host, s_out);
+  if (lse_host.defined()) keep(lse_host, s_out);
+  Py_RETURN_NONE;
+}
+
 // ---- the module -----------------------------------------------------------------------------------
 PyObject* choose_decode_splits(PyObject* const* a) {
   return PyLong_FromLongLong(decode_splits(integer_of(a[0]), integer_of(a[1]), integer_of(a[2]), integer_of(a[3])));
@@ -717,6 +845,7 @@ PyMethodDef methods[] = {method<fwd, 23>("fwd"),
                          method<choose_decode_splits, 4>("choose_decode_splits"),
                          method<choose_num_splits, 5>("choose_num_splits"),
                          method<quantize_qkv, 4>("quantize_qkv"),
+                         method<host_pieces, 25>("host_pieces"),
                          method<window_of, 3>("resolve_window"),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "Native host path of flash_attention_b200.", -1, methods,

@@ -18,7 +18,8 @@ from typing import Optional, Tuple
 
 import torch
 
-from .interface import flash_attn_fp4_func, check_status
+from . import _lib
+from .interface import check_status
 
 
 class HostPipeline:
@@ -82,49 +83,15 @@ class HostPipeline:
             self.s_in.wait_event(self.inputs_free)
         if self.outputs_free is not None:
             self.s_compute.wait_event(self.outputs_free)
-        last_compute = None
-        for b in range(B):
-            with torch.cuda.stream(self.s_in):
-                for dst, src in ((self.k, k), (self.v, v), (self.k_sf, k_sf), (self.v_sf, v_sf)):
-                    dst[b].copy_(src[b], non_blocking=True)
-            for (s0, s1) in self.ranges:
-                with torch.cuda.stream(self.s_in):
-                    self.q[b, s0:s1].copy_(q[b, s0:s1], non_blocking=True)
-                    self.q_sf[b, s0:s1].copy_(q_sf[b, s0:s1], non_blocking=True)
-                    ev_in = torch.cuda.Event()
-                    ev_in.record(self.s_in)
-                sk = s1 if causal else Sk        # s1 is a multiple of 128, or Sq == Sk for the last range
-                with torch.cuda.stream(self.s_compute):
-                    self.s_compute.wait_event(ev_in)
-                    self._piece(b, s0, s1, sk, q_scale, k_scale, v_scale, causal, softmax_scale)
-                    ev_c = torch.cuda.Event()
-                    ev_c.record(self.s_compute)
-                    last_compute = ev_c
-                with torch.cuda.stream(self.s_out):
-                    self.s_out.wait_event(ev_c)
-                    out_host[b, s0:s1].copy_(self.out[b, s0:s1], non_blocking=True)
-            if lse_host is not None:
-                with torch.cuda.stream(self.s_out):
-                    lse_host[b].copy_(self.lse[b], non_blocking=True)
-        self.inputs_free = last_compute
+        _lib.host().host_pieces(q, k, v, q_sf, k_sf, v_sf, self.q, self.k, self.v, self.q_sf, self.k_sf, self.v_sf,
+                                self.out, self.lse, out_host, lse_host, q_scale, k_scale, v_scale, softmax_scale, causal,
+                                self.ranges, self.s_in.cuda_stream, self.s_compute.cuda_stream, self.s_out.cuda_stream)
+        self.inputs_free = torch.cuda.Event()
+        self.inputs_free.record(self.s_compute)
         self.outputs_free = torch.cuda.Event()
         self.outputs_free.record(self.s_out)
         self.done = self.outputs_free
         return self.done
-
-    def _piece(self, b, s0, s1, sk, q_scale, k_scale, v_scale, causal, softmax_scale):
-        """One range of query rows of batch entry b against its first ``sk`` keys.  The LSE rows of
-        a partial range are a strided slice of (Hq, Sq): the kernel writes a small contiguous
-        buffer that is copied into place on the same stream."""
-        Sq = self.shape[1]
-        whole = (s1 - s0 == Sq)
-        _, lse_piece = flash_attn_fp4_func(
-            self.q[b:b + 1, s0:s1], self.k[b:b + 1, :sk], self.v[b:b + 1, :, :, :(sk + 31) // 32 * 16],
-            self.q_sf[b:b + 1, s0:s1], self.k_sf[b:b + 1, :sk], self.v_sf[b:b + 1, :, :, :(sk + 31) // 32 * 2],
-            q_scale, k_scale, v_scale, softmax_scale=softmax_scale, causal=causal, return_lse=True,
-            out=self.out[b:b + 1, s0:s1], lse=self.lse[b:b + 1] if whole else None, sf_layout="linear")
-        if not whole:
-            self.lse[b:b + 1, :, s0:s1].copy_(lse_piece)
 
     def wait(self):
         if self.done is not None:

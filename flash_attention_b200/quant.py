@@ -138,6 +138,14 @@ def _set_scale(t: NVFP4Tensor, value) -> None:
 NVFP4Tensor.scale = property(_get_scale, _set_scale)
 
 
+def _getstate(t: NVFP4Tensor) -> dict:
+    t.scale                                  # a copy or a pickle carries the number
+    return t.__dict__
+
+
+NVFP4Tensor.__getstate__ = _getstate
+
+
 def _pad_keys(v: torch.Tensor) -> torch.Tensor:
     """V (B, Sk, H, D) with its key axis padded with zeros to a multiple of 32: V is quantised and
     stored key-contiguous in blocks of 16 keys, and a row of the packed tensor must be a multiple
