@@ -552,12 +552,18 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
                                 dim3((unsigned)num_splits, (unsigned)p->Hkv, (unsigned)p->B), dec::threads_of(rows), smem,
                                 stream, tm_k, tm_v, kp, dp);
     };
-#define FA4_DEC(rows, smem) \
-  (merge ? launch_dec(attn_decode_kernel<rows, true>, rows, smem) : launch_dec(attn_decode_kernel<rows, false>, rows, smem))
-    const int rc = dec_rows <= 4    ? FA4_DEC(4, dec::kSmemRequest)
-                   : dec_rows <= 8  ? FA4_DEC(8, dec::kSmemRequest)
-                   : dec_rows <= 16 ? FA4_DEC(16, dec::kSmemRequest)
-                                    : FA4_DEC(32, dec::kSmemRequestWide);
+    // The deep form where several entries have lengths of their own and no third CTA per SM waits: the long entries
+    // then run on with few CTAs beside them, bound by the latency of their loads (paged batch of 16,
+    // longest 8192: 23.9 -> 21.6 us).  Even lengths keep HBM busy with three tiles, and the room beside two
+    // shallow CTAs lets the next call's start early (B=4, Sk=32768: 32.9 us shallow, 34.7 deep).
+    const bool deep = cache.seqused_k != nullptr && p->B >= 4 && (int64_t)num_splits * p->Hkv * p->B <= 2 * 148;
+#define FA4_DEC(rows, depth)                                                                             \
+  (merge ? launch_dec(attn_decode_kernel<rows, true, depth>, rows, dec::Smem<depth>::kRequest)          \
+         : launch_dec(attn_decode_kernel<rows, false, depth>, rows, dec::Smem<depth>::kRequest))
+    const int rc = dec_rows <= 4    ? (deep ? FA4_DEC(4, 5) : FA4_DEC(4, 3))
+                   : dec_rows <= 8  ? (deep ? FA4_DEC(8, 5) : FA4_DEC(8, 3))
+                   : dec_rows <= 16 ? (deep ? FA4_DEC(16, 5) : FA4_DEC(16, 3))
+                                    : FA4_DEC(32, 5);
 #undef FA4_DEC
     if (rc != 0 || merge) return rc;
   } else {

@@ -38,11 +38,10 @@
 namespace fa4 {
 namespace dec {
 
-// Three of everything: 70 KB of shared memory and 128 tensor-memory columns per CTA (256 in the
-// 32-row form), so that THREE CTAs share an SM (two in the 32-row form).
-constexpr int kStages = 3;   // K and V tiles in flight
-constexpr int kSBufs = 3;    // S^T buffers (N columns each)
-constexpr int kPSlots = 3;   // P^T tiles (N rows x 64 bytes) and their scale chunks
+// K and V tiles, S^T buffers (N columns each) and P^T tiles (N rows x 64 bytes) with their scale chunks:
+// kDepth of each.  Three let THREE CTAs share an SM (70 KB of shared memory, 128 tensor-memory columns),
+// five let two (115 KB, 256 columns).  A CTA's loads are bound by their latency, kDepth x 18 KB per round
+// trip, so five are better whenever no third CTA is there to run.
 constexpr int kMaxCluster = 8;  // splits that are merged inside a cluster (portable cluster size)
 constexpr int kMaxRows = 32; // query rows per kv head: Sq * group
 // Softmax warpgroups: two up to eight rows, one above (registers: three CTAs of twelve warps per SM
@@ -50,44 +49,41 @@ constexpr int kMaxRows = 32; // query rows per kv head: Sq * group
 __host__ __device__ constexpr int softmax_wgs(int rows) { return rows <= 8 ? 2 : 1; }
 __host__ __device__ constexpr int threads_of(int rows) { return softmax_wgs(rows) == 2 ? 384 : 256; }
 
-// shared memory
-constexpr uint32_t kOffK = 0;
-constexpr uint32_t kOffV = kOffK + kStages * kTileBytes;
-constexpr uint32_t kOffSFK = kOffV + kStages * kTileBytes;
-constexpr uint32_t kOffSFV = kOffSFK + kStages * kSfBytes;
 constexpr uint32_t kQBytes = kMaxRows * 64;                // Q^T / P^T operand: up to 32 rows x 64 bytes
-constexpr uint32_t kOffQ = kOffSFV + kStages * kSfBytes;   // rows x 64 bytes, 64-byte swizzle
-constexpr uint32_t kOffSFQ = kOffQ + kQBytes;              // two 512-byte chunks
-constexpr uint32_t kOffP = kOffSFQ + 1024;                 // kPSlots x kQBytes
-constexpr uint32_t kOffSFP = kOffP + kPSlots * kQBytes;    // kPSlots x 2 chunks x 512
-constexpr uint32_t kOffRed = kOffSFP + kPSlots * 1024;     // 2 WGs x 2 x 4 warps x 32 floats
-constexpr uint32_t kOffHand = kOffRed + 2 * 2 * 4 * kMaxRows * 4;   // 2 WGs x 4 warps x 32 references
-constexpr uint32_t kOffBar = kOffHand + 2 * 4 * kMaxRows * 4;
-struct Bars {
-  uint32_t base;
-  static constexpr uint32_t kKFull = 0, kVFull = kKFull + kStages, kSFull = kVFull + kStages,
-                            kSFree = kSFull + kSBufs, kPFull = kSFree + kSBufs,
-                            kPvDone = kPFull + kPSlots, kQReady = kPvDone + kPSlots,
+// shared memory
+template <int kDepth>
+struct Smem {
+  static constexpr uint32_t kOffK = 0;
+  static constexpr uint32_t kOffV = kOffK + kDepth * kTileBytes;
+  static constexpr uint32_t kOffSFK = kOffV + kDepth * kTileBytes;
+  static constexpr uint32_t kOffSFV = kOffSFK + kDepth * kSfBytes;
+  static constexpr uint32_t kOffQ = kOffSFV + kDepth * kSfBytes;    // rows x 64 bytes, 64-byte swizzle
+  static constexpr uint32_t kOffSFQ = kOffQ + kQBytes;              // two 512-byte chunks
+  static constexpr uint32_t kOffP = kOffSFQ + 1024;                 // kDepth x kQBytes
+  static constexpr uint32_t kOffSFP = kOffP + kDepth * kQBytes;     // kDepth x 2 chunks x 512
+  static constexpr uint32_t kOffRed = kOffSFP + kDepth * 1024;      // 2 WGs x 2 x 4 warps x 32 floats
+  static constexpr uint32_t kOffHand = kOffRed + 2 * 2 * 4 * kMaxRows * 4;   // 2 WGs x 4 warps x 32 references
+  static constexpr uint32_t kOffBar = kOffHand + 2 * 4 * kMaxRows * 4;
+  // barriers
+  static constexpr uint32_t kKFull = 0, kVFull = kKFull + kDepth, kSFull = kVFull + kDepth, kSFree = kSFull + kDepth,
+                            kPFull = kSFree + kDepth, kPvDone = kPFull + kDepth, kQReady = kPvDone + kDepth,
                             kSync = kQReady + 1 /* 2 */, kHand = kSync + 2 /* 2 x 4 */, kFin = kHand + 8,
                             kDrain = kFin + 1 /* 2 */, kCount = kDrain + 2;
-  __device__ explicit Bars(uint32_t b) : base(b) {}
-  __device__ __forceinline__ uint32_t at(uint32_t idx) const { return base + 8u * idx; }
+  static constexpr uint32_t kOffMisc = kOffBar + 8 * kCount;
+  static constexpr uint32_t kRequest = kOffMisc + 16 + sizeof(WaitCtx) + 1024;
 };
-constexpr uint32_t kOffMisc = kOffBar + 8 * Bars::kCount;
-constexpr uint32_t kSmemRequest = kOffMisc + 16 + sizeof(WaitCtx) + 1024;
-// The 32-row form allocates 256 tensor-memory columns: its request is padded so that only two CTAs
-// fit an SM (a third would sit inside tcgen05.alloc until one of them ends).
-constexpr uint32_t kSmemRequestWide = 100 * 1024;
-static_assert(kSmemRequest <= kSmemRequestWide && 3 * kSmemRequest <= 227 * 1024, "decode kernel shared memory");
+// (1 KB per CTA is the system's)
+static_assert(3 * (Smem<3>::kRequest + 1024) <= 228 * 1024 && 2 * (Smem<5>::kRequest + 1024) <= 228 * 1024,
+              "decode kernel shared memory");
+static_assert(Smem<5>::kOffMisc % 8 == 0 && Smem<3>::kOffMisc % 8 == 0, "the wait context is 8-byte aligned");
 
-// tensor memory of the form with N columns per operand (N = 16: 128 columns allocated, N = 32:
-// 256): S^T buffers, O^T, scale factors.  The K / V / P scale slots alternate between two copies:
-// the copy and the product that reads it are issued by one thread to the in-order tensor pipe, the
-// second copy keeps a copy from racing the product before.
-template <int kN>
+// tensor memory of the form with N columns per operand: S^T buffers, O^T, scale factors.  The K / V / P
+// scale slots alternate between two copies: the copy and the product that reads it are issued by one
+// thread to the in-order tensor pipe, the second copy keeps a copy from racing the product before.
+template <int kN, int kDepth>
 struct Tm {
-  static constexpr uint32_t kCols = kN == 16 ? 128 : 256;
-  static constexpr uint32_t kS = 0 /* 3 x N */, kO = 3 * kN, kSFQ = 4 * kN, kSFK = kSFQ + 8 /* 2 x 8 */,
+  static constexpr uint32_t kCols = kDepth == 3 ? 128 : 256;
+  static constexpr uint32_t kS = 0 /* kDepth x N */, kO = kDepth * kN, kSFQ = kO + kN, kSFK = kSFQ + 8 /* 2 x 8 */,
                             kSFV = kSFK + 16 /* 2 x 8 */, kSFP = kSFV + 16 /* 2 x 8 */;
   static_assert(kSFP + 16 <= kCols, "tensor-memory map of the decode kernel");
 };
@@ -214,50 +210,51 @@ struct DecodeParams {
 // columns of an S^T buffer) is 16 up to sixteen rows and 32 above.
 // kMerge: the splits of a (kv head, batch entry) are one cluster, which merges their partials through
 // distributed shared memory and writes the result; otherwise they go to o_partial / lse_partial.
-template <int kR, bool kMerge>
-__global__ void __launch_bounds__(dec::threads_of(kR), kR <= 16 ? 3 : 2)
+template <int kR, bool kMerge, int kDepth>
+__global__ void __launch_bounds__(dec::threads_of(kR), kDepth == 3 ? 3 : 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const KernelParams p, const DecodeParams d) {
   using namespace dec;
+  using L = Smem<kDepth>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
-  const Bars bars(base + kOffBar);
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + kOffMisc);
-  volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(gbase + kOffMisc + 4);
-  volatile float* s_red = reinterpret_cast<volatile float*>(gbase + kOffRed);    // [2][2][4][32]
-  volatile float* s_hand = reinterpret_cast<volatile float*>(gbase + kOffHand);  // [2][4][32]
+  auto bar = [&](uint32_t idx) -> uint32_t { return base + L::kOffBar + 8u * idx; };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + L::kOffMisc);
+  volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(gbase + L::kOffMisc + 4);
+  volatile float* s_red = reinterpret_cast<volatile float*>(gbase + L::kOffRed);    // [2][2][4][32]
+  volatile float* s_hand = reinterpret_cast<volatile float*>(gbase + L::kOffHand);  // [2][4][32]
   constexpr int kWgs = softmax_wgs(kR);
   constexpr int kN = kR <= 16 ? 16 : 32;
-  using TM = Tm<kN>;
+  using TM = Tm<kN, kDepth>;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-  WaitCtx& wc = *reinterpret_cast<WaitCtx*>(gbase + kOffMisc + 16);
+  WaitCtx& wc = *reinterpret_cast<WaitCtx*>(gbase + L::kOffMisc + 16);
   const int R = p.Sq * p.group;  // live query rows (<= kR)
 
   if (tid == 0) {
     *s_abort = 0u;
     wc = WaitCtx{s_abort, p.status, p.budget_ns, p.epoch};
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(bars.at(Bars::kKFull + s), 1);
-      mbar_init(bars.at(Bars::kVFull + s), 1);
-      mbar_init(bars.at(Bars::kSFull + s), 1);
-      mbar_init(bars.at(Bars::kSFree + s), 128);
-      mbar_init(bars.at(Bars::kPFull + s), 128);
-      mbar_init(bars.at(Bars::kPvDone + s), 1);
+    for (int s = 0; s < kDepth; ++s) {
+      mbar_init(bar(L::kKFull + s), 1);
+      mbar_init(bar(L::kVFull + s), 1);
+      mbar_init(bar(L::kSFull + s), 1);
+      mbar_init(bar(L::kSFree + s), 128);
+      mbar_init(bar(L::kPFull + s), 128);
+      mbar_init(bar(L::kPvDone + s), 1);
     }
-    mbar_init(bars.at(Bars::kQReady), 128);
-    for (int w = 0; w < 2; ++w) mbar_init(bars.at(Bars::kSync + w), 128);
-    for (int w = 0; w < 8; ++w) mbar_init(bars.at(Bars::kHand + w), 32);
-    mbar_init(bars.at(Bars::kFin), 128);
-    for (int w = 0; w < 2; ++w) mbar_init(bars.at(Bars::kDrain + w), 1);
+    mbar_init(bar(L::kQReady), 128);
+    for (int w = 0; w < 2; ++w) mbar_init(bar(L::kSync + w), 128);
+    for (int w = 0; w < 8; ++w) mbar_init(bar(L::kHand + w), 32);
+    mbar_init(bar(L::kFin), 128);
+    for (int w = 0; w < 2; ++w) mbar_init(bar(L::kDrain + w), 1);
     fence_barrier_init();
   }
   if (warp == 4 && lane == 0) tma_prefetch_desc(&tm_k);
   if (warp == 6 && lane == 0) tma_prefetch_desc(&tm_v);
   if (warp == 5) {
-    tmem_alloc(base + kOffMisc, TM::kCols);
+    tmem_alloc(base + L::kOffMisc, TM::kCols);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -316,40 +313,39 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       const bool is_k = warp == 4;
       // (a K stage is free once its scores are in tensor memory, a V stage once its product is in O: no
       // commits of their own)
-      static_assert(kStages == kSBufs && kStages == kPSlots, "stages are recycled through s_full and pv_done");
-      const uint32_t full0 = is_k ? Bars::kKFull : Bars::kVFull, free0 = is_k ? Bars::kSFull : Bars::kPvDone;
-      const uint32_t tile0 = base + (is_k ? kOffK : kOffV), sf0 = base + (is_k ? kOffSFK : kOffSFV);
+            const uint32_t full0 = is_k ? L::kKFull : L::kVFull, free0 = is_k ? L::kSFull : L::kPvDone;
+      const uint32_t tile0 = base + (is_k ? L::kOffK : L::kOffV), sf0 = base + (is_k ? L::kOffSFK : L::kOffSFV);
       const uint8_t* sf_src = is_k ? p.k_sf + hk * p.ksf_stride_h : p.v_sf + hk * p.vsf_stride_h;
       const int64_t sf_stride_b = is_k ? p.ksf_stride_b : p.vsf_stride_b;
       uint32_t issued = 0;
       for (int li = 0; ok && li < n; ++li) {
         const int nb = i0 + li;
-        const uint32_t st = li % kStages;
+        const uint32_t st = li % kDepth;
         int kb = b, nbl = nb;   // batch coordinate and block inside it (a page of the pool)
         if (p.page_table != nullptr) {
           const int key0 = nb * kBlockN, pg = key0 / p.page_size;
           kb = p.page_table[(int64_t)b * p.pages_per_seq + pg];
           nbl = (key0 - pg * p.page_size) / kBlockN;
         }
-        if (li >= kStages) {
-          ok = mbar_wait(bars.at(free0 + st), ((li - kStages) / kStages) & 1, wc, is_k ? kDKFree : kDVFree);
+        if (li >= kDepth) {
+          ok = mbar_wait(bar(free0 + st), ((li - kDepth) / kDepth) & 1, wc, is_k ? kDKFree : kDVFree);
           if (!ok) break;
         }
-        mbar_arrive_expect_tx(bars.at(full0 + st), kTileBytes + kSfBytes);
+        mbar_arrive_expect_tx(bar(full0 + st), kTileBytes + kSfBytes);
         if (is_k) {
-          tma_load_4d(tile0 + st * kTileBytes, &tm_k, bars.at(full0 + st), 0, hk, nbl * kBlockN, kb);
+          tma_load_4d(tile0 + st * kTileBytes, &tm_k, bar(full0 + st), 0, hk, nbl * kBlockN, kb);
         } else {
-          tma_load_4d(tile0 + st * kTileBytes, &tm_v, bars.at(full0 + st), nbl * (kBlockN / 2), 0, hk, kb);
+          tma_load_4d(tile0 + st * kTileBytes, &tm_v, bar(full0 + st), nbl * (kBlockN / 2), 0, hk, kb);
         }
         bulk_load(sf0 + st * kSfBytes, sf_src + kb * sf_stride_b + (int64_t)nbl * kSfBytes, kSfBytes,
-                  bars.at(full0 + st));
+                  bar(full0 + st));
         issued = li + 1;
       }
       if (!ok) {
         // bounded drain: let the copies already issued land before the CTA's memory is released
         const uint64_t t0 = globaltimer_ns();
-        for (uint32_t i = issued > kStages ? issued - kStages : 0; i < issued; ++i) {
-          while (!mbar_try_wait(bars.at(full0 + (i % kStages)), (i / kStages) & 1) &&
+        for (uint32_t i = issued > kDepth ? issued - kDepth : 0; i < issued; ++i) {
+          while (!mbar_try_wait(bar(full0 + (i % kDepth)), (i / kDepth) & 1) &&
                  globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
         }
       }
@@ -359,27 +355,27 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     // (One thread that issued both products paced the kernel: the copies, products and commits of a
     // block are fourteen tcgen05 instructions, about 100 clocks of issue each.)
     if (lane == 0 && n > 0) {
-      ok = mbar_wait(bars.at(Bars::kQReady), 0, wc, kDQReady);
+      ok = mbar_wait(bar(L::kQReady), 0, wc, kDQReady);
       uint64_t dq[2];
       if (ok) {
         tc_fence_after_sync();
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
-          tc_cp_sf(tmem + TM::kSFQ + 4 * ks, base + kOffSFQ + 512 * ks);
-          dq[ks] = make_desc_sw64(base + kOffQ + 32 * ks);
+          tc_cp_sf(tmem + TM::kSFQ + 4 * ks, base + L::kOffSFQ + 512 * ks);
+          dq[ks] = make_desc_sw64(base + L::kOffQ + 32 * ks);
         }
       }
       for (int li = 0; ok && li < n; ++li) {
-        const uint32_t st = li % kStages, buf = li % kSBufs;
-        ok = mbar_wait(bars.at(Bars::kKFull + st), (li / kStages) & 1, wc, kDKFull);
+        const uint32_t st = li % kDepth, buf = li % kDepth;
+        ok = mbar_wait(bar(L::kKFull + st), (li / kDepth) & 1, wc, kDKFull);
         if (!ok) break;
-        if (li >= kSBufs) {
-          ok = mbar_wait(bars.at(Bars::kSFree + buf), ((li - kSBufs) / kSBufs) & 1, wc, kDSFree);
+        if (li >= kDepth) {
+          ok = mbar_wait(bar(L::kSFree + buf), ((li - kDepth) / kDepth) & 1, wc, kDSFree);
           if (!ok) break;
         }
         tc_fence_after_sync();
         const uint32_t sfk = tmem + TM::kSFK + 8 * (li & 1);
-        const uint32_t kt = base + kOffK + st * kTileBytes, ksf = base + kOffSFK + st * kSfBytes;
+        const uint32_t kt = base + L::kOffK + st * kTileBytes, ksf = base + L::kOffSFK + st * kSfBytes;
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) tc_cp_sf(sfk + 4 * ks, ksf + 512 * ks);
 #pragma unroll
@@ -387,28 +383,28 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           mma_nvf4(tmem + TM::kS + kN * buf, make_desc_sw64(kt + 32 * ks), dq[ks], idesc, sfk + 4 * ks,
                    tmem + TM::kSFQ + 4 * ks, ks > 0 ? 1u : 0u);
         }
-        tc_commit(bars.at(Bars::kSFull + buf));   // scores ready; also: the K stage is free
+        tc_commit(bar(L::kSFull + buf));   // scores ready; also: the K stage is free
       }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();
-        tc_commit(bars.at(Bars::kDrain));
-        while (!mbar_try_wait(bars.at(Bars::kDrain), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
+        tc_commit(bar(L::kDrain));
+        while (!mbar_try_wait(bar(L::kDrain), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
       }
     }
   } else if (warp == 7) {
     // ============================================ V^T . P^T issuer =============================
     if (lane == 0) {
       for (int li = 0; ok && li < n; ++li) {
-        const uint32_t st = li % kStages, slot = li % kPSlots;
-        ok = mbar_wait(bars.at(Bars::kVFull + st), (li / kStages) & 1, wc, kDVFull);
+        const uint32_t st = li % kDepth, slot = li % kDepth;
+        ok = mbar_wait(bar(L::kVFull + st), (li / kDepth) & 1, wc, kDVFull);
         if (!ok) break;
         tc_fence_after_sync();
         const uint32_t sfv = tmem + TM::kSFV + 8 * (li & 1), sfp = tmem + TM::kSFP + 8 * (li & 1);
-        const uint32_t vt = base + kOffV + st * kTileBytes, vsf = base + kOffSFV + st * kSfBytes;
-        const uint32_t pt = base + kOffP + slot * kQBytes, psf = base + kOffSFP + slot * 1024;
+        const uint32_t vt = base + L::kOffV + st * kTileBytes, vsf = base + L::kOffSFV + st * kSfBytes;
+        const uint32_t pt = base + L::kOffP + slot * kQBytes, psf = base + L::kOffSFP + slot * 1024;
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) tc_cp_sf(sfv + 4 * ks, vsf + 512 * ks);
-        ok = mbar_wait(bars.at(Bars::kPFull + slot), (li / kPSlots) & 1, wc, kDPFull);
+        ok = mbar_wait(bar(L::kPFull + slot), (li / kDepth) & 1, wc, kDPFull);
         if (!ok) break;
         tc_fence_after_sync();
 #pragma unroll
@@ -418,12 +414,12 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           mma_nvf4(tmem + TM::kO, make_desc_sw64(vt + 32 * ks), make_desc_sw64(pt + 32 * ks), idesc,
                    sfv + 4 * ks, sfp + 4 * ks, (li > 0 || ks > 0) ? 1u : 0u);
         }
-        tc_commit(bars.at(Bars::kPvDone + slot));   // O stable; also: the P slot and the V stage are free
+        tc_commit(bar(L::kPvDone + slot));   // O stable; also: the P slot and the V stage are free
       }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();
-        tc_commit(bars.at(Bars::kDrain + 1));
-        while (!mbar_try_wait(bars.at(Bars::kDrain + 1), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
+        tc_commit(bar(L::kDrain + 1));
+        while (!mbar_try_wait(bar(L::kDrain + 1), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
       }
     }
   } else if (warp < 4 || warp >= 8) {
@@ -438,29 +434,29 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     uint32_t sync_phase = 0;
     // rendezvous of the 128 threads on an mbarrier (bounded, unlike bar.sync)
 #define FA4_DEC_SYNC()                                                                          \
-  mbar_arrive(bars.at(Bars::kSync + wg));                                                       \
-  ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kSync + wg), sync_phase & 1, wc, kDSync)); \
+  mbar_arrive(bar(L::kSync + wg));                                                       \
+  ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kSync + wg), sync_phase & 1, wc, kDSync)); \
   sync_phase += 1;
 
     // ---- set-up: Q^T operand (rows x 64 bytes, rows past R zero), its scale chunks, zeroed
     //      P^T tiles and scale chunks (rows past R are never written again)
     ok = true;
     if (wg == 0) {
-    for (uint32_t i = tid; i < (kOffRed - kOffQ) / 16; i += 128) {
-      *reinterpret_cast<uint4*>(gbase + kOffQ + i * 16) = make_uint4(0u, 0u, 0u, 0u);  // Q, SFQ, P, SFP are contiguous
+    for (uint32_t i = tid; i < (L::kOffRed - L::kOffQ) / 16; i += 128) {
+      *reinterpret_cast<uint4*>(gbase + L::kOffQ + i * 16) = make_uint4(0u, 0u, 0u, 0u);  // Q, SFQ, P, SFP are contiguous
     }
     FA4_DEC_SYNC()
     if (ok) {
       const int r = tid >> 2, ch = tid & 3;
-      if (r < R) *reinterpret_cast<uint4*>(gbase + kOffQ + sw64_offset(r, ch)) = q_pref;
+      if (r < R) *reinterpret_cast<uint4*>(gbase + L::kOffQ + sw64_offset(r, ch)) = q_pref;
     }
     if (ok && tid < 64) {
       // scale bytes of row r: two words (one per 64-element step) of the tiled layout
       const int r = tid >> 1, ks = tid & 1;
-      if (r < R) *reinterpret_cast<uint32_t*>(gbase + kOffSFQ + 512 * ks + r * 16) = qsf_pref;
+      if (r < R) *reinterpret_cast<uint32_t*>(gbase + L::kOffSFQ + 512 * ks + r * 16) = qsf_pref;
     }
     fence_proxy_async_smem();
-    mbar_arrive(bars.at(Bars::kQReady));
+    mbar_arrive(bar(L::kQReady));
     }
 
     // After the transpose below a thread owns ONE query row (row = lane % kR) with kR neighbouring
@@ -480,15 +476,15 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
     for (int li = wg; ok && li < n; li += kWgs) {
       const int nb = i0 + li;
-      const uint32_t buf = li % kSBufs, slot = li % kPSlots;
-      ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kSFull + buf), (li / kSBufs) & 1, wc, kDSFull));
+      const uint32_t buf = li % kDepth, slot = li % kDepth;
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kSFull + buf), (li / kDepth) & 1, wc, kDSFull));
       if (!ok) break;
       tc_fence_after_sync();
       float x[kR];
       tmem_ld_cols<kR>(lane_addr + TM::kS + kN * buf, reinterpret_cast<uint32_t*>(x));
       tc_wait_ld();
       tc_fence_before_sync();
-      mbar_arrive(bars.at(Bars::kSFree + buf));
+      mbar_arrive(bar(L::kSFree + buf));
 
       // (key = lane, all rows) -> (row = lane % kR, kR keys): x[j] = score of key key_in_blk + j
       lane_group_transpose<kR>(x, lane);
@@ -527,14 +523,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       if (kWgs == 2 && li > 0) {
         // the reference after block li - 1 (the unbroken chain also orders the reuse of the slots: block
         // li + 1 overwrites this one's source only after it has read what this block hands on)
-        ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kHand + 4 * (wg ^ 1) + wq), ((li - 1) >> 1) & 1, wc, kDHand));
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kHand + 4 * (wg ^ 1) + wq), ((li - 1) >> 1) & 1, wc, kDHand));
         if (!ok) break;
         m_prev = s_hand[((wg ^ 1) * 4 + wq) * kMaxRows + my_row];
       }
       const float m_new = next_reference(m_prev, m_loc, sc.sl2);
       if (kWgs == 2) {
         if (lane < kR) s_hand[(wg * 4 + wq) * kMaxRows + my_row] = m_new;
-        mbar_arrive(bars.at(Bars::kHand + 4 * wg + wq));
+        mbar_arrive(bar(L::kHand + 4 * wg + wq));
       }
       float fac = 1.f;
       bool moved_row = false;
@@ -549,9 +545,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       }
       const bool moved = __any_sync(0xffffffffu, moved_row);   // every warp holds all rows
 
-      // P slot free once P V of block li - kPSlots has run
-      if (li >= kPSlots) {
-        ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kPvDone + slot), ((li - kPSlots) / kPSlots) & 1, wc,
+      // P slot free once P V of block li - kDepth has run
+      if (li >= kDepth) {
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kPvDone + slot), ((li - kDepth) / kDepth) & 1, wc,
                                                kDPvDone));
         if (!ok) break;
       }
@@ -573,9 +569,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         if (my_row < R) {   // rows past R stay zero (written once at set-up)
           // kR keys = kR / 2 bytes of the row's 64, inside one 16-byte chunk of the swizzled tile
           const uint32_t col = static_cast<uint32_t>(key_in_blk) >> 1;
-          uint8_t* dst = gbase + kOffP + slot * kQBytes + sw64_offset(my_row, col >> 4) + (col & 15);
+          uint8_t* dst = gbase + L::kOffP + slot * kQBytes + sw64_offset(my_row, col >> 4) + (col & 15);
           // scale byte of 16-key block blk = key_in_blk / 16: chunk blk / 4, the row's word, byte blk % 4
-          uint8_t* sf_dst = gbase + kOffSFP + slot * 1024 + 512 * (key_in_blk >> 6) + my_row * 16 +
+          uint8_t* sf_dst = gbase + L::kOffSFP + slot * 1024 + 512 * (key_in_blk >> 6) + my_row * 16 +
                             ((key_in_blk >> 4) & 3);
           if constexpr (kR == 4) {
             *reinterpret_cast<uint16_t*>(dst) =
@@ -609,8 +605,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       // correction (rare): O^T holds the earlier blocks relative to the old references; here a
       // thread is a dv lane with all rows in its columns, the factor of row r sits in lane r
       if (li > 0 && moved) {
-        ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kPvDone + ((li - 1) % kPSlots)),
-                                               ((li - 1) / kPSlots) & 1, wc, kDPvDone));
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kPvDone + ((li - 1) % kDepth)),
+                                               ((li - 1) / kDepth) & 1, wc, kDPvDone));
         if (!ok) break;
         tc_fence_after_sync();
         float o[kR];
@@ -623,7 +619,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       }
       fence_proxy_async_smem();
       tc_fence_before_sync();
-      mbar_arrive(bars.at(Bars::kPFull + slot));
+      mbar_arrive(bar(L::kPFull + slot));
     }
 
     // ---- epilogue: row sums over the 128 key lanes, then thread = dv lane of O^T --------------
@@ -637,7 +633,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       if (kWgs == 2 && wg == 1) {
         // the second warpgroup leaves its sums and their reference to the first and is done
         if (wq == 0 && lane < kR) s_hand[4 * kMaxRows + kMaxRows + lane] = m_ref;
-        mbar_arrive(bars.at(Bars::kFin));
+        mbar_arrive(bar(L::kFin));
       } else {
         FA4_DEC_SYNC()
       }
@@ -648,10 +644,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       float o[kR];
 #pragma unroll
       for (int r = 0; r < kR; ++r) o[r] = 0.f;
-      if (kWgs == 2) ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kFin), 0, wc, kDFin));
+      if (kWgs == 2) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kFin), 0, wc, kDFin));
       if (ok && n > 0) {
-        ok = __all_sync(0xffffffffu, mbar_wait(bars.at(Bars::kPvDone + ((n - 1) % kPSlots)),
-                                               ((n - 1) / kPSlots) & 1, wc, kDPvDone));
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kPvDone + ((n - 1) % kDepth)),
+                                               ((n - 1) / kDepth) & 1, wc, kDPvDone));
         if (ok) {
           tc_fence_after_sync();
           tmem_ld_cols<kR>(lane_addr + TM::kO, reinterpret_cast<uint32_t*>(o));
@@ -676,8 +672,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             const float lse = finish_lse(m_fin, l_tot, sc.sl2);
             if constexpr (kMerge) {
               // (the K ring is free: every product has completed)
-              reinterpret_cast<float*>(gbase + kOffK)[r * 128 + tid] = o[r] * scale;
-              if (tid == r) reinterpret_cast<float*>(gbase + kOffV)[r] = lse;
+              reinterpret_cast<float*>(gbase + L::kOffK)[r * 128 + tid] = o[r] * scale;
+              if (tid == r) reinterpret_cast<float*>(gbase + L::kOffV)[r] = lse;
             } else {
               d.o_partial[((((int64_t)split * p.B + b) * p.Sq + s) * p.Hq + h) * 128 + tid] = o[r] * scale;
               if (tid == r) d.lse_partial[(((int64_t)split * p.B + b) * p.Hq + h) * p.Sq + s] = lse;
@@ -697,13 +693,13 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     if (warp < 4) {
       const uint32_t ns = d.num_splits;
       uint32_t gave_up = 0;
-      for (uint32_t i = 0; i < ns; ++i) gave_up |= ld_cluster_u32(base + kOffMisc + 4, i);
+      for (uint32_t i = 0; i < ns; ++i) gave_up |= ld_cluster_u32(base + L::kOffMisc + 4, i);
       for (int r = split; r < R && gave_up == 0; r += ns) {
         float l[kMaxCluster], v[kMaxCluster], m = kNegInf;
 #pragma unroll
         for (uint32_t i = 0; i < kMaxCluster; ++i) {
-          l[i] = i < ns ? __uint_as_float(ld_cluster_u32(base + kOffV + 4 * r, i)) : kNegInf;
-          v[i] = i < ns ? __uint_as_float(ld_cluster_u32(base + kOffK + 4 * (r * 128 + tid), i)) : 0.f;
+          l[i] = i < ns ? __uint_as_float(ld_cluster_u32(base + L::kOffV + 4 * r, i)) : kNegInf;
+          v[i] = i < ns ? __uint_as_float(ld_cluster_u32(base + L::kOffK + 4 * (r * 128 + tid), i)) : 0.f;
         }
 #pragma unroll
         for (int i = 0; i < kMaxCluster; ++i) m = fmaxf(m, l[i]);
