@@ -533,7 +533,7 @@ def run_gpu_arm(args, wl, rank, local_rank, world):
             "e2e": {"value": fl_job / (e2e_ms * 1e-3) / 1e12, "unit": "TFLOP/s",
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms,
                     "h2d_gbs_per_rank": h2d / (e2e_ms * 1e-3) / 1e9, "d2h_gbs_per_rank": d2h / (e2e_ms * 1e-3) / 1e9,
-                    "launches_per_step": Bs * len(pipe.ranges) * 5,
+                    "launches_per_step": Bs * len(pipe.ranges) * 2,
                     "pieces_per_step": Bs * len(pipe.ranges),
                     "note": "HostPipeline on this rank's shard: pinned host buffers, copy-in / compute / copy-out of "
                             "query-row ranges on three streams, successive steps overlap; bytes are per rank"},
@@ -549,7 +549,7 @@ def run_gpu_arm(args, wl, rank, local_rank, world):
                                  "gbs": quant_bytes / (quant_ms * 1e-3) / 1e9,
                                  "frac_of_hbm_peak": quant_bytes / (quant_ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
                                  "note": "fused bf16 -> NVFP4 quantiser of q, k, v of the whole problem on rank 0 "
-                                         "(6 launches + one scale read-back), outside the timed region"}
+                                         "(2 launches), outside the timed region"}
         if sustained:
             sus_tf = fl_job / (sus_ms * 1e-3) / 1e12 / world
             sus_peak = 4.0 * peaks.get("bf16_tflops_sustained", peaks["bf16_tflops"])
@@ -863,11 +863,11 @@ def run_decode(args):
                       "data": "synthetic",
                       "config": {"workload": "decode: Sq = 1, Hq = 32, Hkv = 8, D = 128, causal, (B, Sk) in "
                                              "{(4, 32768), (1, 131072), (8, 8192), (64, 4096)}; headline row "
-                                             "B = 4, Sk = 32768; one call = decode kernel + combine kernel",
+                                             "B = 4, Sk = 32768; one call = decode kernel (+ combine kernel beyond eight splits)",
                                  "l2": "L2 flushed between timed calls (256 MiB write)"},
                       "roofline": {"bound": "hbm", "achieved": head["decode"]["kv_gbs"], "peak": peaks["hbm_gbs"],
                                    "unit": "GB/s", "frac": head["decode"]["frac_of_hbm_peak"], "traffic": None},
-                      "gpu_launches": 2 * steps * 2 * len(rows), "decode": rows}), flush=True)
+                      "gpu_launches": steps * 2 * len(rows), "decode": rows}), flush=True)
 
 
 def main():
