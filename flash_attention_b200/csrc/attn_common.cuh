@@ -42,6 +42,7 @@ struct KernelParams {
   FastDiv div_tiles_per_m;   // Hq * B
   FastDiv div_hq, div_group, div_splits;
   int num_m_blocks, num_n_blocks;
+  int compact_tiles;         // packed batch whose slots are mostly empty: deal the existing tiles (64-key kernel)
   int tile_begin, tile_end;  // the part of the tile list this launch works on (64-key kernel)
   int causal;
   float sl2;        // softmax_scale * q_scale * k_scale * log2(e)

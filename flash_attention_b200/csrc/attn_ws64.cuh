@@ -152,6 +152,77 @@ __device__ __forceinline__ TileRec make_tile_rec(const KernelParams& p, int tile
   }
   return r;
 }
+// Packed batches: the list of the tiles that exist.  In a grid sized by the longest sequence most slots of
+// a batch of unequal lengths are empty, and dealing slots to the CTAs leaves them with unequal work (24
+// sequences of 32 to 2048 tokens: 23 % above the mean; dealt like this 1 %).  Sequences are ranked by their
+// number of tiles; causal: last row blocks first, over the sequences that have them; otherwise the
+// tiles of the longest sequence first.  All threads call it; `tile`: in: an index into this list; out: the
+// index make_tile_rec takes for that tile (or -1).  Returns (end of the list, that index).  `mem`: 4
+// kThreads words.  Out of line, so that the rest of the kernel's registers do not depend on it.
+__device__ __noinline__ int2 live_tiles(const int32_t* cu_seqlens_q, int n, int num_m_blocks, int Hq, FastDiv div_hq,
+                                        int causal, int tile, int tile_end, int* mem) {
+  // tiles by sequence; then in ranked order: tiles, tiles of those ranked before, sequence
+  int *count = mem, *sorted = mem + kThreads, *ahead = sorted + kThreads, *order = ahead + kThreads;
+  const int tid = threadIdx.x, n4 = (n + 3) & ~3;
+  int mine = 0;
+  if (tid < n) {
+    mine = (cu_seqlens_q[tid + 1] - cu_seqlens_q[tid] + kBlockM - 1) / kBlockM;
+    mine = mine < 0 ? 0 : (mine < num_m_blocks ? mine : num_m_blocks);
+  }
+  if (tid < n4) count[tid] = mine;
+  __syncthreads();
+  int rank = 0, before = 0, total = 0;
+#pragma unroll 2
+  for (int j = 0; j < n4; j += 4) {
+    const int4 c = *reinterpret_cast<const int4*>(count + j);
+    const int v[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const bool first = v[k] > mine || (v[k] == mine && j + k < tid);
+      rank += first ? 1 : 0;
+      before += first ? v[k] : 0;
+      total += v[k];
+    }
+  }
+  if (tid < n) {
+    sorted[rank] = mine;
+    ahead[rank] = before;
+    order[rank] = tid;
+  }
+  __syncthreads();
+  if ((int64_t)total * Hq < tile_end) tile_end = total * Hq;
+  if (tile >= tile_end) return make_int2(tile_end, -1);
+  const int u = fast_div(tile, div_hq), h = tile - u * Hq;
+  int m, r;
+  if (causal) {
+    // tiles in the row blocks above m: of the sequences with more than m + 1 tiles (the first c by rank),
+    // all but m + 1 each
+    auto above = [&](int m_blk) -> int {
+      int c = 0, hi = n;
+      while (c < hi) {
+        const int mid = (c + hi) >> 1;
+        if (sorted[mid] > m_blk + 1) c = mid + 1; else hi = mid;
+      }
+      return c == 0 ? 0 : ahead[c - 1] + sorted[c - 1] - c * (m_blk + 1);
+    };
+    int lo = 0, hi = num_m_blocks - 1;      // the smallest m with at most u tiles above it
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (above(mid) <= u) hi = mid; else lo = mid + 1;
+    }
+    m = lo;
+    r = u - above(m);
+  } else {
+    int lo = 0, hi = n - 1;                   // the last rank that starts at or before u
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (ahead[mid] <= u) lo = mid; else hi = mid - 1;
+    }
+    r = lo;
+    m = u - ahead[r];
+  }
+  return make_int2(tile_end, ((causal ? num_m_blocks - 1 - m : m) * n + order[r]) * Hq + h);
+}
 // Last visible key of row `row` inside block nb (>= 127: no mask), the first one, and whether any row of
 // the tile needs a mask there (see causal_limit, lower_limit and block_needs_mask in attn_common.cuh).
 template <bool kWindow>
@@ -270,10 +341,21 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   }
   tc_fence_before_sync();
   pdl_wait();
-  // this CTA's tiles: p.tile_begin + tile_of_round(0), (1), ... below p.tile_end
+  // this CTA's tiles: p.tile_begin + tile_of_round(0), (1), ... below tile_end
+  int tile_end = p.tile_end;
   {
-    const int tile = p.tile_begin + tile_of_round(tid, cta, ncta);
-    if (tile < p.tile_end) s_tiles[tid] = make_tile_rec<kWindow || kCache>(p, tile);
+    int tile = p.tile_begin + tile_of_round(tid, cta, ncta), list_end = tile_end;
+    if constexpr (kWindow || kCache) {
+      // (the P tiles' memory is free until the first scores)
+      if (p.compact_tiles) {
+        const int2 live = live_tiles(p.cu_seqlens_q, p.B, p.num_m_blocks, p.Hq, p.div_hq, p.causal, tile, tile_end,
+                                     reinterpret_cast<int*>(gbase + kOffP));
+        tile_end = live.x;
+        tile = live.y >= 0 ? live.y : 0x7fffffff;
+        list_end = 0x7fffffff;
+      }
+    }
+    if (tile < list_end) s_tiles[tid] = make_tile_rec<kWindow || kCache>(p, tile);
   }
   __syncthreads();
   tc_fence_after_sync();
@@ -304,8 +386,8 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   };
 
   // whole rounds, and the last partial one if it reaches this CTA
-  const int num_rounds = (p.tile_end - p.tile_begin) / ncta +
-                         (p.tile_begin + tile_of_round((p.tile_end - p.tile_begin) / ncta, cta, ncta) < p.tile_end ? 1 : 0);
+  const int num_rounds = (tile_end - p.tile_begin) / ncta +
+                         (p.tile_begin + tile_of_round((tile_end - p.tile_begin) / ncta, cta, ncta) < tile_end ? 1 : 0);
 #define FA4_FOR_EACH_TILE                                                                        \
   uint32_t gb = 0, ti = 0;                                                                       \
   bool ok = true;                                                                                \

@@ -26,17 +26,22 @@ def test_window_forms_over_several_tiles_per_cta(cuda_device, window, D):
 
 
 @pytest.mark.parametrize("causal", [True, False])
-def test_packed_batch_with_empty_tiles_between_full_ones(cuda_device, causal):
-    lens = [700, 1, 130, 390, 5, 700, 64, 257, 129, 31]
+@pytest.mark.parametrize("lens", [[700, 1, 130, 390, 5, 700, 64, 257, 129, 31],      # a slot per row block of the longest
+                                  [1025, 1, 130, 1300, 5, 128, 64, 257, 129, 31, 0, 897],   # only the tiles that exist
+                                  [2000] + [17] * 200], ids=["slots", "existing", "many"])
+def test_packed_batch_of_unequal_lengths(cuda_device, lens, causal):
     cu = torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32, device=cuda_device)
     q, k, v = (t[0] for t in make_qkv(1, sum(lens), sum(lens), 8, 2, 128, seed=4, device=cuda_device))
     Q, K, V, cu_v = fa.quantize_varlen_qkv(q, k, v, cu)
     out, lse = fa.flash_attn_varlen_fp4_func(Q.data[0], K.data[0], V.data[0], Q.sf[0], K.sf[0], V.sf[0], Q.scale, K.scale,
-                                             V.scale, cu, cu, cu_seqlens_v=cu_v, max_seqlen_q=700, max_seqlen_k=700,
+                                             V.scale, cu, cu, cu_seqlens_v=cu_v, max_seqlen_q=max(lens),
+                                             max_seqlen_k=max(lens),
                                              causal=causal, return_lse=True)
     torch.cuda.synchronize()
     fa.check_status(cuda_device)
-    for i, n in enumerate(lens):
+    for i, n in list(enumerate(lens))[:14]:
+        if n == 0:
+            continue
         a, b, s0 = int(cu[i]), int(cu[i + 1]), int(cu_v[i])
         s1 = s0 + (n + 31) // 32 * 32
         o, l = fa.flash_attn_fp4_func(
