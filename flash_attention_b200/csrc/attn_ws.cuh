@@ -570,6 +570,13 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         gb += n;
         ti += 1;
       }
+      if (ok && gb > 0) {
+        // The softmax warps' wait for a tile's last product has no clock (mbar_wait_flag).  Behind every other
+        // tile this thread waits for O; behind the last one it stays until its own product has run (with
+        // a TMA store the store warp waits too, with split outputs nobody else does).
+        const uint32_t Gl = gb - 1;
+        ok = mbar_wait(bars.at(Bars::kPvDone + (Gl % kStagesV)), (Gl / kStagesV) & 1, wc, kSiteFinalO);
+      }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();
         tc_commit(bars.at(Bars::kDrain + 1));

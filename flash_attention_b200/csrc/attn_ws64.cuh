@@ -719,6 +719,12 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         gb += n;
         ti += 1;
       }
+      if (ok && gb > 0) {
+        // The epilogue's wait for a tile's last product has no clock (mbar_wait_flag).  Behind every other tile
+        // this thread waits for O; behind the last one it stays until its own product has run.
+        const uint32_t Jl = 2 * gb - 1;
+        ok = mbar_wait(bars.at(Bars::kPvDone + (Jl % kPSlots)), (Jl / kPSlots) & 1, wc, kS64FinalO);
+      }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();
         tc_commit(bars.at(Bars::kDrain + 1));
