@@ -631,8 +631,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       volatile float* red = s_red + (((n + kWgs - 1 - wg) / kWgs) & 1) * (4 * kMaxRows);
       if (lane < kR) red[wq * kMaxRows + lane] = v;
       if (kWgs == 2 && wg == 1) {
-        // the second warpgroup leaves its sums and their reference to the first and is done
-        if (wq == 0 && lane < kR) s_hand[4 * kMaxRows + kMaxRows + lane] = m_ref;
+        // the second warpgroup leaves its sums and their reference to the first and is done (the reference in this
+        // warp's own slot: what its last block handed on there, or -inf if it had none.  Another warp's slot
+        // may not have been read yet: a warp of the first warpgroup can be a block behind this one)
+        if (wq == 0 && lane < kR) s_hand[(wg * 4 + wq) * kMaxRows + lane] = m_ref;
         mbar_arrive(bar(L::kFin));
       } else {
         FA4_DEC_SYNC()
@@ -662,7 +664,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             float l_tot = ((red[r] + red[kMaxRows + r]) + red[2 * kMaxRows + r]) + red[3 * kMaxRows + r];
             float m_fin = __shfl_sync(0xffffffffu, m_ref, r);      // lane r of every warp owns row r
             if (kWgs == 2) {
-              const float m_a = m_fin, m_b = s_hand[5 * kMaxRows + r];
+              const float m_a = m_fin, m_b = s_hand[4 * kMaxRows + r];
               m_fin = fmaxf(m_a, m_b);
               const float l_b = ((red_b[r] + red_b[kMaxRows + r]) + red_b[2 * kMaxRows + r]) + red_b[3 * kMaxRows + r];
               l_tot = l_tot * reference_factor(m_a, m_fin, sc.sl2) + l_b * reference_factor(m_b, m_fin, sc.sl2);

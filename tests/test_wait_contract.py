@@ -30,3 +30,19 @@ def test_the_last_product_of_a_cta_is_awaited_with_a_clock(name, banner):
 @pytest.mark.parametrize("name", ["attn_decode.cuh", "aux_kernels.cuh", "quantize.cuh"])
 def test_the_other_kernels_wait_with_a_clock_only(name):
     assert "mbar_wait_flag" not in open(os.path.join(CSRC, name)).read()
+
+
+def test_a_decode_warp_writes_only_its_own_hand_over_slot():
+    """Slot (wg, wq) is read by warp wq of the other warpgroup, and only its own hand-over barrier orders that
+    reader before the next write: a write by any other warp could come before the read."""
+    text = re.sub(r"//.*", "", open(os.path.join(CSRC, "attn_decode.cuh")).read())
+    writes = re.findall(r"if \(([^\n]*?)\) s_hand\[([^\n]+?)\] = ", text)
+    assert len(writes) == text.count("s_hand[") - len(re.findall(r"= s_hand\[", text)) == 2
+    k_max_rows, k_r = 32, 8
+    for cond, index in writes:
+        for wg in (0, 1):
+            for wq in range(4):
+                for lane in range(k_r):
+                    env = {"wg": wg, "wq": wq, "lane": lane, "my_row": lane, "kR": k_r, "kMaxRows": k_max_rows}
+                    if eval(cond.replace("&&", "and"), env):
+                        assert eval(index, env) == (wg * 4 + wq) * k_max_rows + lane, (cond, index, wg, wq)
