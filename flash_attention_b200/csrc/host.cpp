@@ -7,7 +7,10 @@
 // one-token call with linear scales), so the GPU waited for the host.  Here they take 5-8 us.
 //
 // The functions take their arguments positionally (METH_FASTCALL); interface.py and varlen.py own
-// the signatures, defaults and documentation.  Error types and messages are those of the
+// the signatures, defaults and documentation.  Each reads its Python arguments into plain values first and
+// then works without the interpreter lock: allocations, launches, reads of a value that is still on the
+// device and copies of pageable memory may all wait for the GPU, and other Python threads run meanwhile.
+// Error types and messages are those of the
 // reference's host code (flash_attn/cute/interface.py:231-236, 384-398): AssertionError for
 // malformed tensors, NotImplementedError for what is not built, ValueError for bad numbers.
 #define PY_SSIZE_T_CLEAN
@@ -25,18 +28,31 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <memory>
+#include <mutex>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "../../include/fa4_nvfp4.h"
 
 namespace {
 
-// A Python exception that has been set (PyErr_SetString) travels to the boundary as this.
+// What travels to the boundary: a Python exception that has been set; one to be set there (thrown with or
+// without the interpreter lock); a return code of the C ABI.
 struct PyErrorSet {};
+struct Failure {
+  PyObject* type;       // a built-in exception type
+  std::string message;
+};
+struct CallFailed {
+  int rc;
+  const char* what;
+};
 
 [[noreturn]] __attribute__((format(printf, 2, 3))) void fail(PyObject* type, const char* fmt, ...) {
   char msg[512];
@@ -44,9 +60,23 @@ struct PyErrorSet {};
   va_start(ap, fmt);
   vsnprintf(msg, sizeof msg, fmt, ap);
   va_end(ap);
-  PyErr_SetString(type, msg);
-  throw PyErrorSet();
+  throw Failure{type, msg};
 }
+void check_rc(int rc, const char* what) {
+  if (rc != 0) throw CallFailed{rc, what};
+}
+
+// The calling thread without the interpreter lock.  No Python object is touched while one is alive.
+class NoGil {
+ public:
+  NoGil() : state_(PyEval_SaveThread()) {}
+  ~NoGil() { PyEval_RestoreThread(state_); }
+  NoGil(const NoGil&) = delete;
+  NoGil& operator=(const NoGil&) = delete;
+
+ private:
+  PyThreadState* state_;
+};
 #define FA4_ASSERT(cond, ...) \
   do { if (!(cond)) fail(PyExc_AssertionError, __VA_ARGS__); } while (0)
 
@@ -61,6 +91,7 @@ const at::Tensor& tensor_of(PyObject* o, const char* name) {
   return THPVariable_Unpack(o);
 }
 bool is_none(PyObject* o) { return o == nullptr || o == Py_None; }
+at::Tensor optional_tensor(PyObject* o, const char* name) { return is_none(o) ? at::Tensor() : tensor_of(o, name); }
 
 // packed bytes arrive as uint8, float8_e4m3fn or float4_e2m1fn_x2
 at::Tensor as_u8(PyObject* o, const char* name) {
@@ -110,19 +141,18 @@ bool truth_of(PyObject* o) {
 struct ScaleState {
   c10::DataPtr device;              // three floats
   cudaStream_t stream;
-  bool known = false;
+  std::atomic<bool> known{false};
+  std::mutex fetching;
   float value[3];
   const float* ptr(int i) const { return static_cast<const float*>(device.get()) + i; }
-  void fetch() {
+  void fetch() {                    // without the interpreter lock
     if (known) return;
-    cudaError_t e;
-    float v[3];
+    std::lock_guard<std::mutex> lock(fetching);
+    if (known) return;
     c10::cuda::CUDAGuard guard(device.device().index());
-    Py_BEGIN_ALLOW_THREADS
-    e = cudaMemcpyAsync(v, device.get(), sizeof v, cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    Py_END_ALLOW_THREADS
-    C10_CUDA_CHECK(e);
+    float v[3];
+    C10_CUDA_CHECK(cudaMemcpyAsync(v, device.get(), sizeof v, cudaMemcpyDeviceToHost, stream));
+    C10_CUDA_CHECK(cudaStreamSynchronize(stream));
     std::copy_n(v, 3, value);
     known = true;
   }
@@ -134,9 +164,12 @@ struct LazyScale {
 };
 PyObject* lazy_float(PyObject* self) {
   HANDLE_TH_ERRORS
-  LazyScale* s = reinterpret_cast<LazyScale*>(self);
-  (*s->state)->fetch();
-  return PyFloat_FromDouble((*s->state)->value[s->which]);
+  const std::shared_ptr<ScaleState> state = *reinterpret_cast<LazyScale*>(self)->state;
+  if (!state->known) {
+    NoGil nogil;
+    state->fetch();
+  }
+  return PyFloat_FromDouble(state->value[reinterpret_cast<LazyScale*>(self)->which]);
   END_HANDLE_TH_ERRORS
 }
 void lazy_dealloc(PyObject* self) {
@@ -153,27 +186,42 @@ PyObject* new_lazy(const std::shared_ptr<ScaleState>& st, int which) {
   reinterpret_cast<LazyScale*>(o)->which = which;
   return o;
 }
+// A per-tensor scale as it was passed: a number, a one-element tensor, or one on its way.
+struct Scale {
+  double number = 0.0;
+  at::Tensor tensor;
+  std::shared_ptr<ScaleState> lazy;
+  int which = 0;
+  // its value (waits for one that lives on the device)
+  float value(const char* name) const {
+    if (lazy) {
+      lazy->fetch();
+      return lazy->value[which];
+    }
+    if (!tensor.defined()) return static_cast<float>(number);
+    FA4_ASSERT(tensor.numel() == 1, "%s must be a python float or a 1-element tensor", name);
+    return static_cast<float>(tensor.item<double>());
+  }
+};
+Scale scale_of(PyObject* o) {
+  Scale s;
+  if (is_lazy(o)) {
+    s.lazy = *reinterpret_cast<LazyScale*>(o)->state;
+    s.which = reinterpret_cast<LazyScale*>(o)->which;
+  } else if (THPVariable_Check(o)) {
+    s.tensor = THPVariable_Unpack(o);
+  } else {
+    s.number = number_of(o);
+  }
+  return s;
+}
 // The device copies of three scales for a call on `stream`; false: take their values instead.
-bool device_scales(PyObject* const* o, const at::Device& device, cudaStream_t stream, const float** ptr) {
+bool device_scales(const Scale (&s)[3], const at::Device& device, cudaStream_t stream, const float** ptr) {
   for (int i = 0; i < 3; ++i) {
-    if (!is_lazy(o[i])) return false;
-    const LazyScale* s = reinterpret_cast<const LazyScale*>(o[i]);
-    const ScaleState& st = **s->state;
-    if (st.stream != stream || st.device.device() != device) return false;
-    ptr[i] = st.ptr(s->which);
+    if (!s[i].lazy || s[i].lazy->stream != stream || s[i].lazy->device.device() != device) return false;
+    ptr[i] = s[i].lazy->ptr(s[i].which);
   }
   return true;
-}
-
-// a per-tensor scale: a number, or a one-element tensor whose value is read (synchronises if it
-// lives on the device)
-float scalar_of(PyObject* o, const char* name) {
-  if (THPVariable_Check(o)) {
-    const at::Tensor& t = THPVariable_Unpack(o);
-    FA4_ASSERT(t.numel() == 1, "%s must be a python float or a 1-element tensor", name);
-    return static_cast<float>(t.item<double>());
-  }
-  return static_cast<float>(number_of(o));
 }
 
 // The status word of a device (see DeviceStatus in interface.py, which owns it): address kept here.
@@ -197,17 +245,6 @@ uint32_t* status_word(const at::Device& device) {
     ptr[idx] = static_cast<uint32_t*>(THPVariable_Unpack(w).data_ptr());
   }
   return ptr[idx];
-}
-
-// Turns a return code of the C ABI into the exception _lib.check raises for it.
-void check_rc(int rc, const char* what) {
-  if (rc == 0) return;
-  PyObject* mod = PyImport_ImportModule("flash_attention_b200._lib");
-  if (mod == nullptr) throw PyErrorSet();
-  PyObject* r = PyObject_CallMethod(mod, "check", "is", rc, what);
-  Py_DECREF(mod);
-  Py_XDECREF(r);
-  throw PyErrorSet();
 }
 
 // ---- rules on sizes (interface.py documents them) ------------------------------------------------
@@ -267,9 +304,8 @@ bool head_dims_built(int64_t D, int64_t Dv) {
 }
 
 // The learnable sink as Hq contiguous fp32 values on the device.
-at::Tensor sink_of(PyObject* o, int64_t Hq, const at::Device& device) {
-  if (is_none(o)) return {};
-  const at::Tensor& t = tensor_of(o, "learnable_sink");
+at::Tensor sink_of(const at::Tensor& t, int64_t Hq, const at::Device& device) {
+  if (!t.defined()) return {};
   FA4_ASSERT(t.dim() == 1 && t.size(0) == Hq, "learnable_sink must have one entry per query head");
   if (t.device() == device && t.scalar_type() == at::kFloat && t.is_contiguous()) return t;
   return t.to(device, at::kFloat).contiguous();
@@ -330,10 +366,20 @@ PyObject* pair_of(PyObject* out_o, const at::Tensor& out, PyObject* lse_o, const
 // ---- flash_attn_fp4_func ------------------------------------------------------------------------
 // q k v q_sf k_sf v_sf q_scale k_scale v_scale softmax_scale causal return_lse out lse sf_layout
 // variant num_splits window_left window_right learnable_sink softcap seqused_k page_table
-PyObject* fwd(PyObject* const* a) {
-  at::Tensor q = as_u8(a[0], "q"), k = as_u8(a[1], "k"), v = as_u8(a[2], "v");
-  at::Tensor q_sf = as_u8(a[3], "q_sf"), k_sf = as_u8(a[4], "k_sf"), v_sf = as_u8(a[5], "v_sf");
-  PyObject *out_o = a[12], *lse_o = a[13], *used_o = a[21], *table_o = a[22];
+struct Call {
+  at::Tensor q, k, v, q_sf, k_sf, v_sf, out, lse, sink, used, table;
+  Scale scale[3];
+  bool default_softmax_scale = true, want_lse = true, tiled = false;
+  double softmax_scale = 0.0, softcap = 0.0;
+  int variant = FA4_VARIANT_AUTO;
+  long num_splits = 1;
+  Window win;
+  uint32_t* status = nullptr;
+};
+
+// Checks, allocates (out and lse where they are not given) and launches; no Python.
+void run(Call& c) {
+  at::Tensor &q = c.q, &k = c.k, &v = c.v, &q_sf = c.q_sf, &k_sf = c.k_sf, &v_sf = c.v_sf, &out = c.out, &lse = c.lse;
   FA4_ASSERT(q.dim() == 4 && k.dim() == 4 && v.dim() == 4, "q, k, v must be 4-D");
   FA4_ASSERT(q.is_cuda() && k.is_cuda() && v.is_cuda(), "inputs must be on CUDA");
   q = inner_contiguous(std::move(q));
@@ -342,12 +388,12 @@ PyObject* fwd(PyObject* const* a) {
   const int64_t B = q.size(0), Sq = q.size(1), Hq = q.size(2), D = 2 * q.size(3);
   const int64_t B_kv = k.size(0), Sk_kv = k.size(1), Hkv = k.size(2), Dv = v.size(2);
   const at::Device device = q.device();
-  const bool paged = !is_none(table_o);
+  const bool paged = c.table.defined();
   int64_t Sk = Sk_kv, pages_per_seq = 0;
   at::Tensor table, used;
   if (paged) {
     // k / v are a pool of B_kv pages of Sk_kv (= page_size) keys; Sk is the logical key length
-    const at::Tensor& t = tensor_of(table_o, "page_table");
+    const at::Tensor& t = c.table;
     FA4_ASSERT(t.dim() == 2 && t.size(0) == B && t.scalar_type() == at::kInt && t.is_cuda(),
                "page_table must be a (B, pages_per_seq) int32 CUDA tensor");
     FA4_ASSERT(v.size(0) == B_kv, "k and v pools differ in their number of pages");
@@ -359,8 +405,8 @@ PyObject* fwd(PyObject* const* a) {
   } else {
     FA4_ASSERT(B_kv == B && v.size(0) == B, "batch size mismatch");
   }
-  if (!is_none(used_o)) {
-    const at::Tensor& t = tensor_of(used_o, "seqused_k");
+  if (c.used.defined()) {
+    const at::Tensor& t = c.used;
     FA4_ASSERT(t.dim() == 1 && t.size(0) == B && t.scalar_type() == at::kInt && t.is_cuda(),
                "seqused_k must be a (B,) int32 CUDA tensor");
     used = t.contiguous();
@@ -375,7 +421,7 @@ PyObject* fwd(PyObject* const* a) {
     fail(PyExc_NotImplementedError,
          "head dims (D=%lld, Dv=%lld) not built; supported: (128, 128), (64, 64) and (192, 128)", (long long)D,
          (long long)Dv);
-  const double softmax_scale = is_none(a[9]) ? 1.0 / std::sqrt((double)D) : number_of(a[9]);
+  const double softmax_scale = c.default_softmax_scale ? 1.0 / std::sqrt((double)D) : c.softmax_scale;
 
   c10::cuda::OptionalCUDAGuard guard;
   if (device.index() != c10::cuda::current_device()) guard.set_device(device);
@@ -383,8 +429,7 @@ PyObject* fwd(PyObject* const* a) {
 
   c10::DataPtr tiles;                     // scratch for tiled copies of linear scales
   const void* sf_ptr[3];
-  const char* layout = PyUnicode_Check(a[14]) ? PyUnicode_AsUTF8(a[14]) : nullptr;
-  if (layout != nullptr && !strcmp(layout, "linear")) {
+  if (!c.tiled) {
     validate(q_sf, "q_sf", {B, Sq, Hq, D / 16}, at::kByte, device);
     validate(k_sf, "k_sf", {B_kv, Sk_kv, Hkv, D / 16}, at::kByte, device);
     validate(v_sf, "v_sf", {B_kv, Hkv, Dv, Sk_pad / 16}, at::kByte, device);
@@ -394,7 +439,7 @@ PyObject* fwd(PyObject* const* a) {
     fa4_nvfp4_sf_job jobs[3] = {sf_job(q_sf, 1, 2, 1), sf_job(k_sf, 1, 2, 1), sf_job(v_sf, 2, 1, 2)};
     tiles = tile_scales(jobs, stream);
     for (int i = 0; i < 3; ++i) sf_ptr[i] = jobs[i].dst;
-  } else if (layout != nullptr && !strcmp(layout, "tiled")) {
+  } else {
     validate(q_sf, "q_sf", {B, Hq, cdiv(Sq, 128), D / 64, 512}, at::kByte, device);
     validate(k_sf, "k_sf", {B_kv, Hkv, cdiv(Sk_kv, 128), D / 64, 512}, at::kByte, device);
     validate(v_sf, "v_sf", {B_kv, Hkv, cdiv(Dv, 128), 2 * cdiv(Sk_kv, 128), 512}, at::kByte, device);
@@ -403,30 +448,24 @@ PyObject* fwd(PyObject* const* a) {
     sf_ptr[0] = q_sf.data_ptr();
     sf_ptr[1] = k_sf.data_ptr();
     sf_ptr[2] = v_sf.data_ptr();
-  } else {
-    PyErr_Format(PyExc_ValueError, "sf_layout must be 'linear' or 'tiled', got %R", a[14]);
-    throw PyErrorSet();
   }
 
-  at::Tensor out, lse;
-  if (is_none(out_o)) {
+  if (!out.defined()) {
     out = new_tensor({B, Sq, Hq, Dv}, at::kBFloat16, device);
   } else {
-    out = tensor_of(out_o, "out");
     validate(out, "out", {B, Sq, Hq, Dv}, at::kBFloat16, device);
     FA4_ASSERT(out.stride(-1) == 1, "out's last dimension must be contiguous");
   }
-  if (!is_none(lse_o)) {
-    lse = tensor_of(lse_o, "lse");
+  if (lse.defined()) {
     validate(lse, "lse", {B, Hq, Sq}, at::kFloat, device);
     FA4_ASSERT(lse.is_contiguous(), "lse must be contiguous");
-  } else if (truth_of(a[11])) {
+  } else if (c.want_lse) {
     lse = new_tensor({B, Hq, Sq}, at::kFloat, device);
   }
 
   fa4_nvfp4_params p = {};
   p.struct_size = sizeof p;
-  p.variant = (int32_t)integer_of(a[15]);
+  p.variant = c.variant;
   p.q = q.data_ptr();
   p.k = k.data_ptr();
   p.v = v.data_ptr();
@@ -435,7 +474,7 @@ PyObject* fwd(PyObject* const* a) {
   p.v_sf = sf_ptr[2];
   p.out = out.data_ptr();
   p.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
-  p.status = status_word(device);
+  p.status = c.status;
   p.q_stride_b = q.stride(0); p.q_stride_s = q.stride(1); p.q_stride_h = q.stride(2);
   p.k_stride_b = k.stride(0); p.k_stride_s = k.stride(1); p.k_stride_h = k.stride(2);
   p.v_stride_b = v.stride(0); p.v_stride_h = v.stride(1); p.v_stride_d = v.stride(2);
@@ -443,22 +482,22 @@ PyObject* fwd(PyObject* const* a) {
   p.B = (int32_t)B; p.Sq = (int32_t)Sq; p.Sk = (int32_t)Sk; p.Hq = (int32_t)Hq; p.Hkv = (int32_t)Hkv;
   p.D = (int32_t)D; p.Dv = (int32_t)Dv;
   const float* scales[3];
-  const bool lazy = device_scales(a + 6, device, static_cast<cudaStream_t>(stream), scales);
+  const bool lazy = device_scales(c.scale, device, static_cast<cudaStream_t>(stream), scales);
   if (!lazy) {
-    p.q_scale = scalar_of(a[6], "q_scale");
-    p.k_scale = scalar_of(a[7], "k_scale");
-    p.v_scale = scalar_of(a[8], "v_scale");
+    p.q_scale = c.scale[0].value("q_scale");
+    p.k_scale = c.scale[1].value("k_scale");
+    p.v_scale = c.scale[2].value("v_scale");
   }
   p.softmax_scale = (float)softmax_scale;
 
-  long num_splits = integer_of(a[16]);
+  long num_splits = c.num_splits;
   if (num_splits < 0 || num_splits > 128) fail(PyExc_ValueError, "num_splits must be in 0..128");
   const bool auto_splits = num_splits == 0;
-  const Window win = resolve_window(truth_of(a[10]), a[17], a[18]);
+  const Window win = c.win;
   p.causal = win.causal ? 1 : 0;
-  const double softcap = is_none(a[20]) ? 0.0 : number_of(a[20]);
+  const double softcap = c.softcap;
   if (!(softcap >= 0.0) || !std::isfinite(softcap)) fail(PyExc_ValueError, "softcap must be a finite number >= 0");
-  const at::Tensor sink = sink_of(a[19], Hq, device);
+  const at::Tensor sink = sink_of(c.sink, Hq, device);
   // A handful of query rows per kv head (decode, append): the transposed kernel, which always
   // splits the keys over CTAs and merges with the combine kernel.
   const bool decode_ok = D == 128 && Dv == 128 && Sq * (Hq / Hkv) <= 32 && win.left < 0 && win.right <= 0 &&
@@ -502,13 +541,42 @@ PyObject* fwd(PyObject* const* a) {
     else
       check_rc(fa4_nvfp4_fwd_ex(&p, &x, stream), "fa4_nvfp4_fwd_ex");
   }
-  return pair_of(out_o, out, lse_o, lse);
+}
+
+PyObject* fwd(PyObject* const* a) {
+  Call c;
+  c.q = as_u8(a[0], "q"), c.k = as_u8(a[1], "k"), c.v = as_u8(a[2], "v");
+  c.q_sf = as_u8(a[3], "q_sf"), c.k_sf = as_u8(a[4], "k_sf"), c.v_sf = as_u8(a[5], "v_sf");
+  for (int i = 0; i < 3; ++i) c.scale[i] = scale_of(a[6 + i]);
+  c.default_softmax_scale = is_none(a[9]);
+  if (!c.default_softmax_scale) c.softmax_scale = number_of(a[9]);
+  c.want_lse = truth_of(a[11]);
+  c.out = optional_tensor(a[12], "out");
+  c.lse = optional_tensor(a[13], "lse");
+  const char* layout = PyUnicode_Check(a[14]) ? PyUnicode_AsUTF8(a[14]) : nullptr;
+  c.tiled = layout != nullptr && !strcmp(layout, "tiled");
+  if (!c.tiled && (layout == nullptr || strcmp(layout, "linear") != 0)) {
+    PyErr_Format(PyExc_ValueError, "sf_layout must be 'linear' or 'tiled', got %R", a[14]);
+    throw PyErrorSet();
+  }
+  c.variant = (int)integer_of(a[15]);
+  c.num_splits = integer_of(a[16]);
+  c.win = resolve_window(truth_of(a[10]), a[17], a[18]);
+  c.sink = optional_tensor(a[19], "learnable_sink");
+  if (!is_none(a[20])) c.softcap = number_of(a[20]);
+  c.used = optional_tensor(a[21], "seqused_k");
+  c.table = optional_tensor(a[22], "page_table");
+  if (c.q.is_cuda()) c.status = status_word(c.q.device());
+  {
+    NoGil nogil;
+    run(c);
+  }
+  return pair_of(a[12], c.out, a[13], c.lse);
 }
 
 // ---- flash_attn_varlen_fp4_func -------------------------------------------------------------------
-at::Tensor offsets_of(PyObject* o, const char* name, const at::Device& device) {
-  if (is_none(o)) return {};
-  const at::Tensor& t = tensor_of(o, name);
+at::Tensor offsets_of(const at::Tensor& t, const char* name, const at::Device& device) {
+  if (!t.defined()) return {};
   FA4_ASSERT(t.dim() == 1, "%s must be one-dimensional", name);
   if (t.device() == device && t.scalar_type() == at::kInt && t.is_contiguous()) return t;
   return t.to(device, at::kInt).contiguous();
@@ -519,9 +587,14 @@ int64_t longest_of(const at::Tensor& cu) { return cu.diff().max().item<int64_t>(
 
 // q k v q_sf k_sf v_sf q_scale k_scale v_scale cu_q cu_k seqused_k cu_v max_q max_k softmax_scale causal
 // window_left window_right learnable_sink softcap return_lse
-PyObject* varlen_fwd(PyObject* const* a) {
-  at::Tensor q = as_u8(a[0], "q"), k = as_u8(a[1], "k"), v = as_u8(a[2], "v");
-  at::Tensor q_sf = as_u8(a[3], "q_sf"), k_sf = as_u8(a[4], "k_sf"), v_sf = as_u8(a[5], "v_sf");
+struct VarlenCall : Call {
+  at::Tensor cu_q, cu_k, cu_v;
+  bool known = false;              // max_q and max_k are given
+  int64_t max_q = 0, max_k = 0;
+};
+
+void run_varlen(VarlenCall& c) {
+  at::Tensor &q = c.q, &k = c.k, &v = c.v, &q_sf = c.q_sf, &k_sf = c.k_sf, &v_sf = c.v_sf, &out = c.out, &lse = c.lse;
   FA4_ASSERT(q.dim() == 3 && k.dim() == 3 && v.dim() == 3, "packed operands are 3-D");
   FA4_ASSERT(q.is_cuda() && k.is_cuda() && v.is_cuda(), "inputs must be on CUDA");
   q = inner_contiguous(std::move(q));
@@ -536,7 +609,7 @@ PyObject* varlen_fwd(PyObject* const* a) {
   v_sf = v_sf.contiguous();
   const int64_t total_q = q.size(0), Hq = q.size(1), D = 2 * q.size(2);
   const int64_t total_k = k.size(0), Hkv = k.size(1), Dv = v.size(1);
-  const bool has_cu_v = !is_none(a[12]);
+  const bool has_cu_v = c.cu_v.defined();
   const int64_t total_kp = has_cu_v ? 2 * v.size(2) : cdiv(total_k, 32) * 32;
   FA4_ASSERT(2 * k.size(2) == D && v.size(0) == Hkv && Hkv > 0 && Hq % Hkv == 0,
              "head counts / head dims of q, k, v do not fit");
@@ -549,33 +622,32 @@ PyObject* varlen_fwd(PyObject* const* a) {
              "scale factors must be the packed linear layouts");
   if (!head_dims_built(D, Dv))
     fail(PyExc_NotImplementedError, "head dims (D=%lld, Dv=%lld) not built", (long long)D, (long long)Dv);
-  const at::Tensor cu_q = offsets_of(a[9], "cu_seqlens_q", device), cu_k = offsets_of(a[10], "cu_seqlens_k", device);
+  const at::Tensor cu_q = offsets_of(c.cu_q, "cu_seqlens_q", device), cu_k = offsets_of(c.cu_k, "cu_seqlens_k", device);
   FA4_ASSERT(cu_q.numel() == cu_k.numel() && cu_q.numel() >= 2, "cu_seqlens_q / cu_seqlens_k describe different batches");
   const int64_t seqs = cu_q.numel() - 1;
-  const at::Tensor cu_v = offsets_of(a[12], "cu_seqlens_v", device), used = offsets_of(a[11], "seqused_k", device);
+  const at::Tensor cu_v = offsets_of(c.cu_v, "cu_seqlens_v", device), used = offsets_of(c.used, "seqused_k", device);
   FA4_ASSERT(!cu_v.defined() || cu_v.numel() == seqs + 1, "cu_seqlens_v has another batch size");
   FA4_ASSERT(!used.defined() || used.numel() == seqs, "seqused_k has another batch size");
   // without both maxima one synchronising read; pass them to stay asynchronous, as the reference's callers do
-  const bool known = !is_none(a[13]) && !is_none(a[14]);
-  int64_t max_q = known ? integer_of(a[13]) : longest_of(cu_q), max_k = known ? integer_of(a[14]) : longest_of(cu_k);
+  int64_t max_q = c.known ? c.max_q : longest_of(cu_q), max_k = c.known ? c.max_k : longest_of(cu_k);
   max_q = std::min(std::max<int64_t>(1, max_q), total_q);
   max_k = std::min(std::max<int64_t>(1, max_k), total_k);
-  const double softmax_scale = is_none(a[15]) ? 1.0 / std::sqrt((double)D) : number_of(a[15]);
-  const Window win = resolve_window(truth_of(a[16]), a[17], a[18]);
-  const at::Tensor sink = sink_of(a[19], Hq, device);
+  const double softmax_scale = c.default_softmax_scale ? 1.0 / std::sqrt((double)D) : c.softmax_scale;
+  const Window win = c.win;
+  const at::Tensor sink = sink_of(c.sink, Hq, device);
 
   // per-sequence tiles of the packed scales, padded to the longest sequence
-  const int64_t c = D / 16, ckp = total_kp / 16;
-  fa4_nvfp4_sf_job jobs[3] = {sf_job(q_sf, seqs, Hq, max_q, c, 0, c, Hq * c, 1),
-                              sf_job(k_sf, seqs, Hkv, max_k, c, 0, c, Hkv * c, 1),
+  const int64_t cols = D / 16, ckp = total_kp / 16;
+  fa4_nvfp4_sf_job jobs[3] = {sf_job(q_sf, seqs, Hq, max_q, cols, 0, cols, Hq * cols, 1),
+                              sf_job(k_sf, seqs, Hkv, max_k, cols, 0, cols, Hkv * cols, 1),
                               sf_job(v_sf, seqs, Hkv, Dv, cdiv(max_k, 16), 0, Dv * ckp, ckp, 2)};
   jobs[0].cu_seqlens = cu_q.data_ptr<int32_t>();
   jobs[1].cu_seqlens = cu_k.data_ptr<int32_t>();
   jobs[2].cu_seqlens = (cu_v.defined() ? cu_v : cu_k).data_ptr<int32_t>();
   jobs[0].packed_rows = jobs[1].packed_rows = 1;
   const c10::DataPtr tiles = tile_scales(jobs, stream);
-  at::Tensor out = new_tensor({total_q, Hq, Dv}, at::kBFloat16, device), lse;
-  if (truth_of(a[21])) lse = new_tensor({Hq, total_q}, at::kFloat, device);
+  out = new_tensor({total_q, Hq, Dv}, at::kBFloat16, device);
+  if (c.want_lse) lse = new_tensor({Hq, total_q}, at::kFloat, device);
 
   fa4_nvfp4_params p = {};
   p.struct_size = sizeof p;
@@ -583,7 +655,7 @@ PyObject* varlen_fwd(PyObject* const* a) {
   p.q_sf = jobs[0].dst; p.k_sf = jobs[1].dst; p.v_sf = jobs[2].dst;
   p.out = out.data_ptr();
   p.lse = lse.defined() ? lse.data_ptr<float>() : nullptr;
-  p.status = status_word(device);
+  p.status = c.status;
   p.q_stride_s = q.stride(0); p.q_stride_h = q.stride(1); p.q_stride_b = q.stride(0) * std::max<int64_t>(1, total_q);
   p.k_stride_s = k.stride(0); p.k_stride_h = k.stride(1); p.k_stride_b = k.stride(0) * std::max<int64_t>(1, total_k);
   p.v_stride_h = v.stride(0); p.v_stride_d = v.stride(1); p.v_stride_b = v.stride(0) * Hkv;
@@ -591,9 +663,9 @@ PyObject* varlen_fwd(PyObject* const* a) {
   p.B = (int32_t)seqs; p.Sq = (int32_t)max_q; p.Sk = (int32_t)max_k; p.Hq = (int32_t)Hq; p.Hkv = (int32_t)Hkv;
   p.D = (int32_t)D; p.Dv = (int32_t)Dv;
   p.causal = win.causal ? 1 : 0;
-  p.q_scale = scalar_of(a[6], "q_scale");
-  p.k_scale = scalar_of(a[7], "k_scale");
-  p.v_scale = scalar_of(a[8], "v_scale");
+  p.q_scale = c.scale[0].value("q_scale");
+  p.k_scale = c.scale[1].value("k_scale");
+  p.v_scale = c.scale[2].value("v_scale");
   p.softmax_scale = (float)softmax_scale;
 
   fa4_nvfp4_varlen x = {};
@@ -609,25 +681,47 @@ PyObject* varlen_fwd(PyObject* const* a) {
   x.window_left = win.left;
   x.window_right = win.right;
   x.sink = sink.defined() ? sink.data_ptr<float>() : nullptr;
-  x.softcap = is_none(a[20]) ? 0.f : (float)number_of(a[20]);
+  x.softcap = (float)c.softcap;
   x.cu_seqlens_v = cu_v.defined() ? cu_v.data_ptr<int32_t>() : nullptr;
   x.total_v = cu_v.defined() ? (int32_t)total_kp : 0;
   check_rc(fa4_nvfp4_fwd_varlen(&p, &x, stream), "fa4_nvfp4_fwd_varlen");
-  return pair_of(nullptr, out, nullptr, lse);
+}
+
+PyObject* varlen_fwd(PyObject* const* a) {
+  VarlenCall c;
+  c.q = as_u8(a[0], "q"), c.k = as_u8(a[1], "k"), c.v = as_u8(a[2], "v");
+  c.q_sf = as_u8(a[3], "q_sf"), c.k_sf = as_u8(a[4], "k_sf"), c.v_sf = as_u8(a[5], "v_sf");
+  for (int i = 0; i < 3; ++i) c.scale[i] = scale_of(a[6 + i]);
+  c.cu_q = tensor_of(a[9], "cu_seqlens_q");
+  c.cu_k = tensor_of(a[10], "cu_seqlens_k");
+  c.used = optional_tensor(a[11], "seqused_k");
+  c.cu_v = optional_tensor(a[12], "cu_seqlens_v");
+  c.known = !is_none(a[13]) && !is_none(a[14]);
+  if (c.known) c.max_q = integer_of(a[13]), c.max_k = integer_of(a[14]);
+  c.default_softmax_scale = is_none(a[15]);
+  if (!c.default_softmax_scale) c.softmax_scale = number_of(a[15]);
+  c.win = resolve_window(truth_of(a[16]), a[17], a[18]);
+  c.sink = optional_tensor(a[19], "learnable_sink");
+  if (!is_none(a[20])) c.softcap = number_of(a[20]);
+  c.want_lse = truth_of(a[21]);
+  if (c.q.is_cuda()) c.status = status_word(c.q.device());
+  {
+    NoGil nogil;
+    run_varlen(c);
+  }
+  return pair_of(nullptr, c.out, nullptr, c.lse);
 }
 
 // ---- quantize_qkv_fused ----------------------------------------------------------------------------
-// q k v linear_sf -> (packed, linear scales or None, tiled scales, LazyScale) x 3
-PyObject* quantize_qkv(PyObject* const* a) {
-  static const char* names[3] = {"q", "k", "v"};
-  const bool linear = truth_of(a[3]);
-  const at::Device device = tensor_of(a[0], "q").device();
+// Allocates the results and launches; no Python.
+void quantize(const at::Tensor (&in)[3], bool linear, at::Tensor (&packed)[3], at::Tensor (&lin)[3],
+              at::Tensor (&tiled)[3], ScaleState& state) {
+  const at::Device device = in[0].device();
   fa4_nvfp4_quant_job jobs[3] = {};
-  at::Tensor packed[3], lin[3], tiled[3];
   c10::DataPtr scratch, scales;
   c10::cuda::OptionalCUDAGuard guard;
   for (int i = 0; i < 3; ++i) {
-    const at::Tensor& x = tensor_of(a[i], names[i]);
+    const at::Tensor& x = in[i];
     FA4_ASSERT(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 4 && x.stride(-1) == 1 &&
                    x.device() == device,
                "quantize_qkv_fused takes CUDA bf16 (B, S, H, D) tensors, last dim contiguous");
@@ -661,9 +755,21 @@ PyObject* quantize_qkv(PyObject* const* a) {
   }
   const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream(device.index());
   check_rc(fa4_nvfp4_quantize_jobs_bf16(jobs, 3, static_cast<float*>(scratch.get()), stream.stream()), "fa4_nvfp4_quantize_jobs_bf16");
+  state.device = std::move(scales);
+  state.stream = stream.stream();
+}
+
+// q k v linear_sf -> (packed, linear scales or None, tiled scales, LazyScale) x 3
+PyObject* quantize_qkv(PyObject* const* a) {
+  static const char* names[3] = {"q", "k", "v"};
+  const bool linear = truth_of(a[3]);
+  at::Tensor in[3], packed[3], lin[3], tiled[3];
+  for (int i = 0; i < 3; ++i) in[i] = tensor_of(a[i], names[i]);
   auto state = std::make_shared<ScaleState>();
-  state->device = std::move(scales);
-  state->stream = stream.stream();
+  {
+    NoGil nogil;
+    quantize(in, linear, packed, lin, tiled, *state);
+  }
   PyObject* res = PyTuple_New(3);
   for (int i = 0; i < 3; ++i) {
     PyObject* t = PyTuple_New(4);
@@ -696,7 +802,7 @@ struct Event {
   }
 };
 
-PyObject* host_pieces(PyObject* const* a) {
+void issue_pieces(PyObject* const* a) {
   at::Tensor host[6], dev[6];
   static const char* names[6] = {"q", "k", "v", "q_sf", "k_sf", "v_sf"};
   for (int i = 0; i < 6; ++i) {
@@ -707,7 +813,19 @@ PyObject* host_pieces(PyObject* const* a) {
   at::Tensor lse_host;
   if (!is_none(a[15])) lse_host = tensor_of(a[15], "lse_host");
   const bool causal = truth_of(a[20]);
-  const auto device = dev[0].device();
+  const at::Device device = dev[0].device();
+  Call call;                       // what the pieces share
+  for (int i = 0; i < 3; ++i) call.scale[i] = scale_of(a[16 + i]);
+  call.default_softmax_scale = is_none(a[19]);
+  if (!call.default_softmax_scale) call.softmax_scale = number_of(a[19]);
+  call.win = resolve_window(causal, nullptr, nullptr);
+  call.status = status_word(device);
+  std::vector<std::pair<int64_t, int64_t>> ranges;
+  for (Py_ssize_t n = 0; n < PyList_GET_SIZE(a[21]); ++n) {
+    PyObject* r = PyList_GET_ITEM(a[21], n);
+    const int64_t s0 = integer_of(PyTuple_GET_ITEM(r, 0)), s1 = integer_of(PyTuple_GET_ITEM(r, 1));
+    ranges.emplace_back(s0, s1);
+  }
   cudaStream_t raw[3];
   for (int i = 0; i < 3; ++i) {
     raw[i] = static_cast<cudaStream_t>(PyLong_AsVoidPtr(a[22 + i]));
@@ -717,15 +835,9 @@ PyObject* host_pieces(PyObject* const* a) {
                               s_compute = c10::cuda::getStreamFromExternal(raw[1], device.index()),
                               s_out = c10::cuda::getStreamFromExternal(raw[2], device.index());
   const int64_t B = dev[0].size(0), Sq = dev[0].size(1), Hq = dev[0].size(2), Sk = dev[1].size(1), skp = 2 * dev[2].size(3);
-  PyObject* ranges = a[21];
+  NoGil nogil;                     // (copies from and to pageable memory wait for themselves and for what is before them)
   c10::cuda::CUDAGuard device_guard(device);
   Event in_done, compute_done;
-  PyObject* linear = PyUnicode_FromString("linear");
-  PyObject *zero = PyLong_FromLong(0), *one = PyLong_FromLong(1);
-  struct Refs {
-    PyObject* o[3];
-    ~Refs() { for (PyObject* x : o) Py_XDECREF(x); }
-  } refs{{linear, zero, one}};
   // rows [r0, r1) of batch entry b (contiguous byte tensors, both sides)
   auto load = [&](int i, int64_t b, int64_t r0, int64_t r1) {
     const int64_t row = dev[i].stride(1), at_byte = b * dev[i].stride(0) + r0 * row;
@@ -749,9 +861,7 @@ PyObject* host_pieces(PyObject* const* a) {
     // The query rows of the first entry come by range, so that its first piece starts early.
     for (int i : {3, 4, 5, 1, 2}) load(i, b, 0, dev[i].size(1));
     if (b > 0) load(0, b, 0, Sq);
-    for (Py_ssize_t n = 0; n < PyList_GET_SIZE(ranges); ++n) {
-      PyObject* r = PyList_GET_ITEM(ranges, n);
-      const int64_t s0 = integer_of(PyTuple_GET_ITEM(r, 0)), s1 = integer_of(PyTuple_GET_ITEM(r, 1));
+    for (const auto& [s0, s1] : ranges) {
       const int64_t sk = causal ? s1 : Sk;     // s1 is a multiple of 128, or Sq == Sk for the last range
       if (b == 0) load(0, b, s0, s1);
       in_done.order(raw[0], raw[1]);
@@ -761,33 +871,20 @@ PyObject* host_pieces(PyObject* const* a) {
         c10::cuda::CUDAStreamGuard g(s_compute);
         const bool whole = s1 - s0 == Sq;
         const int64_t kp = cdiv(sk, 32) * 32;
-        const at::Tensor t[8] = {dev[0].narrow(0, b, 1).narrow(1, s0, s1 - s0), dev[1].narrow(0, b, 1).narrow(1, 0, sk),
-                                 dev[2].narrow(0, b, 1).narrow(3, 0, kp / 2),   dev[3].narrow(0, b, 1).narrow(1, s0, s1 - s0),
-                                 dev[4].narrow(0, b, 1).narrow(1, 0, sk),       dev[5].narrow(0, b, 1).narrow(3, 0, kp / 16),
-                                 out.narrow(0, b, 1).narrow(1, s0, s1 - s0),    lse.narrow(0, b, 1)};
-        PyObject* w[8];
-        for (int i = 0; i < 8; ++i) w[i] = THPVariable_Wrap(t[i]);
-        PyObject* args[23] = {w[0], w[1], w[2], w[3], w[4], w[5], a[16], a[17], a[18], a[19], a[20], Py_True, w[6],
-                              whole ? w[7] : Py_None, linear, zero, one, Py_None, Py_None, Py_None, zero, Py_None, Py_None};
-        PyObject* res = nullptr;
-        try {
-          res = fwd(args);
-        } catch (...) {
-          for (PyObject* x : w) Py_DECREF(x);
-          throw;
-        }
+        Call c = call;
+        c.q = dev[0].narrow(0, b, 1).narrow(1, s0, s1 - s0);
+        c.k = dev[1].narrow(0, b, 1).narrow(1, 0, sk);
+        c.v = dev[2].narrow(0, b, 1).narrow(3, 0, kp / 2);
+        c.q_sf = dev[3].narrow(0, b, 1).narrow(1, s0, s1 - s0);
+        c.k_sf = dev[4].narrow(0, b, 1).narrow(1, 0, sk);
+        c.v_sf = dev[5].narrow(0, b, 1).narrow(3, 0, kp / 16);
+        c.out = out.narrow(0, b, 1).narrow(1, s0, s1 - s0);
+        if (whole) c.lse = lse.narrow(0, b, 1);
+        run(c);
         if (!whole) {
-          const at::Tensor& piece = THPVariable_Unpack(PyTuple_GET_ITEM(res, 1));
-          float* dst = lse.data_ptr<float>() + b * Hq * Sq + s0;
-          const cudaError_t e = cudaMemcpy2DAsync(dst, Sq * 4, piece.data_ptr<float>(), (s1 - s0) * 4, (s1 - s0) * 4, Hq,
-                                                  cudaMemcpyDeviceToDevice, raw[1]);
-          Py_DECREF(res);
-          res = nullptr;
-          for (PyObject*& x : w) Py_CLEAR(x);
-          C10_CUDA_CHECK(e);
+          C10_CUDA_CHECK(cudaMemcpy2DAsync(lse.data_ptr<float>() + b * Hq * Sq + s0, Sq * 4, c.lse.data_ptr<float>(),
+                                           (s1 - s0) * 4, (s1 - s0) * 4, Hq, cudaMemcpyDeviceToDevice, raw[1]));
         }
-        Py_XDECREF(res);
-        for (PyObject* x : w) Py_XDECREF(x);
       }
       compute_done.order(raw[1], raw[2]);
       store(out_host, out, b, s0, s1);
@@ -801,6 +898,10 @@ PyObject* host_pieces(PyObject* const* a) {
   for (const at::Tensor& t : host) keep(t, s_in);
   keep(out_host, s_out);
   if (lse_host.defined()) keep(lse_host, s_out);
+}
+
+PyObject* host_pieces(PyObject* const* a) {
+  issue_pieces(a);
   Py_RETURN_NONE;
 }
 
@@ -822,6 +923,15 @@ PyObject* window_of(PyObject* const* a) {
   return res;
 }
 
+// Sets the exception _lib.check raises for a return code of the C ABI.
+void raise_for(const CallFailed& f) {
+  PyObject* mod = PyImport_ImportModule("flash_attention_b200._lib");
+  if (mod == nullptr) return;
+  PyObject* r = PyObject_CallMethod(mod, "check", "is", f.rc, f.what);
+  Py_DECREF(mod);
+  Py_XDECREF(r);
+}
+
 template <PyObject* (*fn)(PyObject* const*), int kArgs>
 PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (n != kArgs) {
@@ -832,6 +942,12 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
   try {
     return fn(args);
   } catch (const PyErrorSet&) {
+    return nullptr;
+  } catch (const Failure& f) {
+    PyErr_SetString(f.type, f.message.c_str());
+    return nullptr;
+  } catch (const CallFailed& f) {
+    raise_for(f);
     return nullptr;
   }
   END_HANDLE_TH_ERRORS

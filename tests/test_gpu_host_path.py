@@ -1,0 +1,72 @@
+"""The native host path beside other Python threads and beside the operands a caller may pass: what waits for
+the GPU waits without the interpreter lock, what is not bytes is not read as bytes, and a call that fails
+half-way leaves the buffers of the next one in order."""
+import threading
+import time
+
+import pytest
+import torch
+
+import flash_attention_b200 as fa
+from tests.helpers import make_qkv
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(device, B=1, S=256, Hq=4, Hkv=2, seed=31):
+    q, k, v = make_qkv(B, S, S, Hq, Hkv, 128, seed=seed, device=device)
+    return tuple(fa.NVFP4Tensor(t.data.to(device), t.sf.to(device), t.scale, is_v=t.is_v) for t in fa.quantize_qkv(q, k, v))
+
+
+def _largest_gap(call, device, busy_s=0.5):
+    """Runs `call` behind a kernel that keeps the stream busy; returns (its duration, the longest time another
+    Python thread stood still meanwhile)."""
+    gaps, stop = [], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    torch.cuda.synchronize(device)
+    t = threading.Thread(target=tick)
+    t.start()
+    try:
+        time.sleep(0.05)
+        torch.cuda._sleep(int(busy_s * 1.9e9))
+        t0 = time.perf_counter()
+        call()
+        took = time.perf_counter() - t0
+    finally:
+        stop.set()
+        t.join()
+        torch.cuda.synchronize(device)
+    return took, max(gaps)
+
+
+@pytest.mark.parametrize("waits_for", ["scale", "sink", "longest", "pageable operands"])
+def test_a_call_that_waits_lets_other_threads_run(cuda_device, waits_for):
+    Q, K, V = _operands(cuda_device)
+    ops = (Q.data, K.data, V.data, Q.sf, K.sf, V.sf)
+    if waits_for == "scale":
+        s = [torch.tensor([t.scale], device=cuda_device) for t in (Q, K, V)]
+        call = lambda: fa.flash_attn_fp4_func(*ops, *s, causal=True)
+    elif waits_for == "sink":
+        sink = torch.zeros(4)
+        call = lambda: fa.flash_attn_fp4_func(*ops, Q.scale, K.scale, V.scale, learnable_sink=sink)
+    elif waits_for == "longest":
+        cu = torch.tensor([0, 128, 256], dtype=torch.int32, device=cuda_device)
+        call = lambda: fa.flash_attn_varlen_fp4_func(*(t[0] for t in ops), Q.scale, K.scale, V.scale, cu, cu)
+    else:
+        pipe = fa.HostPipeline(1, 256, 256, 4, 2, device=cuda_device)
+        host = [t.cpu() for t in ops]
+        out = torch.empty(1, 256, 4, 128, dtype=torch.bfloat16)
+        call = lambda: pipe.run(*host, Q.scale, K.scale, V.scale, out, causal=True)
+    call()                                       # allocations and module loading
+    took, gap = _largest_gap(call, cuda_device)
+    assert took > 0.2, f"the call did not wait ({took:.3f} s): nothing was tested"
+    assert gap < 0.5 * took, f"another thread stood still for {gap:.3f} s of {took:.3f} s"
+    fa.check_status(cuda_device)
