@@ -808,6 +808,9 @@ void issue_pieces(PyObject* const* a) {
   for (int i = 0; i < 6; ++i) {
     host[i] = tensor_of(a[i], names[i]);
     dev[i] = tensor_of(a[6 + i], names[i]);
+    FA4_ASSERT(host[i].element_size() == 1 && host[i].is_cpu() && host[i].is_contiguous() && dev[i].is_contiguous() &&
+                   host[i].sizes() == dev[i].sizes(),
+               "%s: packed bytes in a contiguous CPU tensor of the pipeline's shape expected", names[i]);
   }
   const at::Tensor out = tensor_of(a[12], "out"), lse = tensor_of(a[13], "lse"), out_host = tensor_of(a[14], "out_host");
   at::Tensor lse_host;

@@ -21,6 +21,8 @@ import torch
 from . import _lib
 from .interface import check_status
 
+_PACKED = (torch.uint8, torch.float8_e4m3fn, torch.float4_e2m1fn_x2)
+
 
 class HostPipeline:
     """Reusable device staging buffers and streams for one problem shape on one GPU.
@@ -72,6 +74,8 @@ class HostPipeline:
                        (v_sf, self.v_sf)):
             assert not t.is_cuda and tuple(t.shape) == tuple(ref.shape) and t.is_contiguous(), \
                 "host operands must be contiguous CPU tensors of the pipeline's shape"
+        # packed bytes are copied as they are; other types hold byte VALUES and are converted to them
+        q, k, v, q_sf, k_sf, v_sf = (t if t.dtype in _PACKED else t.to(torch.uint8) for t in (q, k, v, q_sf, k_sf, v_sf))
         assert tuple(out_host.shape) == tuple(self.out.shape) and out_host.dtype == torch.bfloat16
         if causal and Sq != Sk:
             raise NotImplementedError("HostPipeline splits causal problems only for Sq == Sk")

@@ -70,3 +70,18 @@ def test_a_call_that_waits_lets_other_threads_run(cuda_device, waits_for):
     assert took > 0.2, f"the call did not wait ({took:.3f} s): nothing was tested"
     assert gap < 0.5 * took, f"another thread stood still for {gap:.3f} s of {took:.3f} s"
     fa.check_status(cuda_device)
+
+
+def test_host_operands_of_wider_types_are_converted_to_bytes(cuda_device):
+    Q, K, V = _operands(cuda_device)
+    want, want_lse = fa.flash_attn_func(Q, K, V, causal=True, return_lse=True)
+    host = [t.cpu() for t in (Q.data, K.data, V.data, Q.sf, K.sf, V.sf)]
+    pipe = fa.HostPipeline(1, 256, 256, 4, 2, device=cuda_device)
+    for given in ([t.to(torch.int32) for t in host],                    # byte values in a wider type
+                  host[:3] + [t.view(torch.float8_e4m3fn) for t in host[3:]],   # scale bytes under their own type
+                  [host[0], host[1].to(torch.int64)] + host[2:]):
+        out = torch.zeros(1, 256, 4, 128, dtype=torch.bfloat16).pin_memory()
+        lse = torch.zeros(1, 4, 256).pin_memory()
+        pipe.run(*given, Q.scale, K.scale, V.scale, out, lse, causal=True)
+        pipe.wait()
+        assert torch.equal(out, want.cpu()) and torch.equal(lse, want_lse.cpu()), [t.dtype for t in given]
