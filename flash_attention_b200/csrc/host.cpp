@@ -849,7 +849,7 @@ void issue_pieces(PyObject* const* a) {
                                    cudaMemcpyHostToDevice, raw[0]));
   };
   auto store = [&](const at::Tensor& to, const at::Tensor& from, int64_t b, int64_t r0, int64_t r1) {
-    if (to.is_cpu() && to.is_contiguous() && to.scalar_type() == from.scalar_type() && to.sizes() == from.sizes()) {
+    if (to.is_contiguous() && to.scalar_type() == from.scalar_type() && to.sizes() == from.sizes()) {
       const int64_t size = from.element_size(), row = from.stride(1) * size, at_byte = b * from.stride(0) * size + r0 * row;
       C10_CUDA_CHECK(cudaMemcpyAsync(static_cast<uint8_t*>(to.data_ptr()) + at_byte,
                                      static_cast<const uint8_t*>(from.data_ptr()) + at_byte, (r1 - r0) * row,
