@@ -859,48 +859,59 @@ void issue_pieces(PyObject* const* a) {
       to.select(0, b).narrow(0, r0, r1 - r0).copy_(from.select(0, b).narrow(0, r0, r1 - r0), /*non_blocking=*/true);
     }
   };
-  for (int64_t b = 0; b < B; ++b) {
-    // Few, large loads: while a copy-out runs, PCIe lets about 16 GB/s in, and each copy waits its turn.
-    // The query rows of the first entry come by range, so that its first piece starts early.
-    for (int i : {3, 4, 5, 1, 2}) load(i, b, 0, dev[i].size(1));
-    if (b > 0) load(0, b, 0, Sq);
-    for (const auto& [s0, s1] : ranges) {
-      const int64_t sk = causal ? s1 : Sk;     // s1 is a multiple of 128, or Sq == Sk for the last range
-      if (b == 0) load(0, b, s0, s1);
-      in_done.order(raw[0], raw[1]);
-      {
-        // one range of query rows against its keys, through the same entry as any other call.  The LSE of
-        // a partial range is a strided slice of (Hq, Sq): written compactly, then moved into place
-        c10::cuda::CUDAStreamGuard g(s_compute);
-        const bool whole = s1 - s0 == Sq;
-        const int64_t kp = cdiv(sk, 32) * 32;
-        Call c = call;
-        c.q = dev[0].narrow(0, b, 1).narrow(1, s0, s1 - s0);
-        c.k = dev[1].narrow(0, b, 1).narrow(1, 0, sk);
-        c.v = dev[2].narrow(0, b, 1).narrow(3, 0, kp / 2);
-        c.q_sf = dev[3].narrow(0, b, 1).narrow(1, s0, s1 - s0);
-        c.k_sf = dev[4].narrow(0, b, 1).narrow(1, 0, sk);
-        c.v_sf = dev[5].narrow(0, b, 1).narrow(3, 0, kp / 16);
-        c.out = out.narrow(0, b, 1).narrow(1, s0, s1 - s0);
-        if (whole) c.lse = lse.narrow(0, b, 1);
-        run(c);
-        if (!whole) {
-          C10_CUDA_CHECK(cudaMemcpy2DAsync(lse.data_ptr<float>() + b * Hq * Sq + s0, Sq * 4, c.lse.data_ptr<float>(),
-                                           (s1 - s0) * 4, (s1 - s0) * 4, Hq, cudaMemcpyDeviceToDevice, raw[1]));
-        }
-      }
-      compute_done.order(raw[1], raw[2]);
-      store(out_host, out, b, s0, s1);
-    }
-    if (lse_host.defined()) store(lse_host, lse, b, 0, Hq);
-  }
-  // pinned blocks go back to their pool no earlier than these copies have run
+  // pinned blocks go back to their pool no earlier than the copies issued here have run, also after an error
   auto keep = [](const at::Tensor& t, const c10::cuda::CUDAStream& s) {
     if (t.is_pinned()) at::getHostAllocator(at::kCUDA)->record_event(t.data_ptr(), t.storage().data_ptr().get_context(), s.unwrap());
   };
-  for (const at::Tensor& t : host) keep(t, s_in);
-  keep(out_host, s_out);
-  if (lse_host.defined()) keep(lse_host, s_out);
+  auto keep_all = [&] {
+    for (const at::Tensor& t : host) keep(t, s_in);
+    keep(out_host, s_out);
+    if (lse_host.defined()) keep(lse_host, s_out);
+  };
+  try {
+    for (int64_t b = 0; b < B; ++b) {
+      // Few, large loads: while a copy-out runs, PCIe lets about 16 GB/s in, and each copy waits its turn.
+      // The query rows of the first entry come by range, so that its first piece starts early.
+      for (int i : {3, 4, 5, 1, 2}) load(i, b, 0, dev[i].size(1));
+      if (b > 0) load(0, b, 0, Sq);
+      for (const auto& [s0, s1] : ranges) {
+        const int64_t sk = causal ? s1 : Sk;     // s1 is a multiple of 128, or Sq == Sk for the last range
+        if (b == 0) load(0, b, s0, s1);
+        in_done.order(raw[0], raw[1]);
+        {
+          // one range of query rows against its keys, through the same entry as any other call.  The LSE of
+          // a partial range is a strided slice of (Hq, Sq): written compactly, then moved into place
+          c10::cuda::CUDAStreamGuard g(s_compute);
+          const bool whole = s1 - s0 == Sq;
+          const int64_t kp = cdiv(sk, 32) * 32;
+          Call c = call;
+          c.q = dev[0].narrow(0, b, 1).narrow(1, s0, s1 - s0);
+          c.k = dev[1].narrow(0, b, 1).narrow(1, 0, sk);
+          c.v = dev[2].narrow(0, b, 1).narrow(3, 0, kp / 2);
+          c.q_sf = dev[3].narrow(0, b, 1).narrow(1, s0, s1 - s0);
+          c.k_sf = dev[4].narrow(0, b, 1).narrow(1, 0, sk);
+          c.v_sf = dev[5].narrow(0, b, 1).narrow(3, 0, kp / 16);
+          c.out = out.narrow(0, b, 1).narrow(1, s0, s1 - s0);
+          if (whole) c.lse = lse.narrow(0, b, 1);
+          run(c);
+          if (!whole) {
+            C10_CUDA_CHECK(cudaMemcpy2DAsync(lse.data_ptr<float>() + b * Hq * Sq + s0, Sq * 4, c.lse.data_ptr<float>(),
+                                             (s1 - s0) * 4, (s1 - s0) * 4, Hq, cudaMemcpyDeviceToDevice, raw[1]));
+          }
+        }
+        compute_done.order(raw[1], raw[2]);
+        store(out_host, out, b, s0, s1);
+      }
+      if (lse_host.defined()) store(lse_host, lse, b, 0, Hq);
+    }
+  } catch (...) {
+    try {
+      keep_all();
+    } catch (const std::exception&) {      // (the first error is the one to report)
+    }
+    throw;
+  }
+  keep_all();
 }
 
 PyObject* host_pieces(PyObject* const* a) {

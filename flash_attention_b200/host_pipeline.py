@@ -87,14 +87,22 @@ class HostPipeline:
             self.s_in.wait_event(self.inputs_free)
         if self.outputs_free is not None:
             self.s_compute.wait_event(self.outputs_free)
-        _lib.host().host_pieces(q, k, v, q_sf, k_sf, v_sf, self.q, self.k, self.v, self.q_sf, self.k_sf, self.v_sf,
-                                self.out, self.lse, out_host, lse_host, q_scale, k_scale, v_scale, softmax_scale, causal,
-                                self.ranges, self.s_in.cuda_stream, self.s_compute.cuda_stream, self.s_out.cuda_stream)
-        self.inputs_free = torch.cuda.Event()
-        self.inputs_free.record(self.s_compute)
-        self.outputs_free = torch.cuda.Event()
-        self.outputs_free.record(self.s_out)
-        self.done = self.outputs_free
+        try:
+            _lib.host().host_pieces(q, k, v, q_sf, k_sf, v_sf, self.q, self.k, self.v, self.q_sf, self.k_sf, self.v_sf,
+                                    self.out, self.lse, out_host, lse_host, q_scale, k_scale, v_scale, softmax_scale,
+                                    causal, self.ranges, self.s_in.cuda_stream, self.s_compute.cuda_stream,
+                                    self.s_out.cuda_stream)
+        except BaseException:
+            # what was issued before the error still runs: the next call and wait() come after it
+            self.s_out.wait_stream(self.s_in)
+            self.s_out.wait_stream(self.s_compute)
+            raise
+        finally:
+            self.inputs_free = torch.cuda.Event()
+            self.inputs_free.record(self.s_compute)
+            self.outputs_free = torch.cuda.Event()
+            self.outputs_free.record(self.s_out)
+            self.done = self.outputs_free
         return self.done
 
     def wait(self):

@@ -85,3 +85,33 @@ def test_host_operands_of_wider_types_are_converted_to_bytes(cuda_device):
         pipe.run(*given, Q.scale, K.scale, V.scale, out, lse, causal=True)
         pipe.wait()
         assert torch.equal(out, want.cpu()) and torch.equal(lse, want_lse.cpu()), [t.dtype for t in given]
+
+
+def test_a_failed_call_keeps_its_buffers_until_its_copies_have_run(cuda_device):
+    """An error behind the first copies: the pinned operands must not go back to their pool while those copies
+    are on their way, wait() waits for them, and the next call is right."""
+    Q, K, V = _operands(cuda_device)
+    want = fa.flash_attn_func(Q, K, V, causal=True)[0]
+    ops = (Q.data, K.data, V.data, Q.sf, K.sf, V.sf)
+    pipe = fa.HostPipeline(1, 256, 256, 4, 2, device=cuda_device)
+    out = torch.zeros(1, 256, 4, 128, dtype=torch.bfloat16).pin_memory()
+    good = [t.cpu().pin_memory() for t in ops]
+    pipe.run(*good, Q.scale, K.scale, V.scale, out, causal=True)          # allocations and module loading
+    pipe.wait()
+    cpu = [t.cpu() for t in ops]
+    host = [t.pin_memory() for t in cpu]
+    where = {t.data_ptr() for t in host}
+    torch.cuda._sleep(int(0.5 * 1.9e9))
+    with pytest.raises(ValueError):
+        pipe.run(*host, 0.0, K.scale, V.scale, out, causal=True)          # refused when the first piece is launched
+    assert not pipe.done.query()
+    del host
+    again = [t.pin_memory() for t in cpu]
+    reused = where & {t.data_ptr() for t in again}
+    still_copying = not pipe.done.query()
+    pipe.wait()
+    assert still_copying and not reused
+    out.zero_()
+    pipe.run(*again, Q.scale, K.scale, V.scale, out, causal=True)
+    pipe.wait()
+    assert torch.equal(out, want.cpu())
