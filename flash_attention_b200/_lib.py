@@ -26,6 +26,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libfa4_nvfp4.so")
 CSRC = os.path.join(_HERE, "csrc")
 HOST_PATH = os.path.join(_HERE, "_host.so")
+HOST_ABI_PATH = HOST_PATH + ".abi"
 LOCK_PATH = os.path.join(_HERE, ".build.lock")
 SOURCES = ["api.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -105,8 +106,24 @@ def _needs_build() -> bool:
     return _stale(LIB_PATH, _dependencies())
 
 
+def _host_abi() -> str:
+    """What the host extension is compiled against: it uses C++ classes of torch and the C API of Python,
+    so it works with exactly these."""
+    return (f"python {sysconfig.get_config_var('SOABI')}, torch {torch.__version__} {torch.version.git_version}, "
+            f"cxx11 abi {int(torch._C._GLIBCXX_USE_CXX11_ABI)}\n")
+
+
+def _host_built_for() -> str:
+    """What HOST_PATH was compiled against, as written down beside it ("" if nothing is known)."""
+    try:
+        with open(HOST_ABI_PATH) as f:
+            return f.read()
+    except FileNotFoundError:
+        return ""
+
+
 def _host_needs_build() -> bool:
-    return _stale(HOST_PATH, _host_dependencies())
+    return _stale(HOST_PATH, _host_dependencies()) or _host_built_for() != _host_abi()
 
 
 class _BuildLock:
@@ -155,6 +172,10 @@ def _compile_host(verbose: bool) -> None:
                   [f"-I{i}" for i in includes] + [os.path.join(CSRC, "host.cpp"), f"-L{libs}", "-ltorch_python",
                    "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", LIB_PATH, f"-Wl,-rpath,{libs}",
                    "-Wl,-rpath,$ORIGIN"], HOST_PATH, verbose)
+    tmp = f"{HOST_ABI_PATH}.{os.getpid()}.tmp"
+    with open(tmp, "w") as f:
+        f.write(_host_abi())
+    os.replace(tmp, HOST_ABI_PATH)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -246,8 +267,10 @@ def host():
                     if _host_needs_build():
                         if shutil.which("g++"):
                             _compile_host(False)
-                        elif not os.path.exists(HOST_PATH):
-                            raise RuntimeError(f"{HOST_PATH} is missing and g++ is not available; "
+                        elif _host_built_for() != _host_abi() or not os.path.exists(HOST_PATH):
+                            raise RuntimeError(f"{HOST_PATH} is missing or was built for another installation "
+                                               f"(it: {_host_built_for().strip() or 'unknown'}; here: "
+                                               f"{_host_abi().strip()}) and g++ is not available; "
                                                "run flash_attention_b200.build() first")
                     name = __package__ + "._host"
                     loader = importlib.machinery.ExtensionFileLoader(name, HOST_PATH)
