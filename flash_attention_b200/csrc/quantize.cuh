@@ -105,10 +105,11 @@ __device__ __forceinline__ void quantize_block16(const float (&x)[16], float bma
   const float denom = block_scale_of(bmax, ts, sf_byte);
   // The element codes are those of the correctly rounded quotients x / denom.  One residual step is
   // enough for them: only quotients within a few ulp of a rounding boundary of e2m1 (.25 .75 1.25
-  // 1.75 2.5 3.5 5) matter, x has eight significand bits, and for all 2^23 significands of denom and
-  // the values of x next to a boundary the steps below land on the same side of it (or on it) as
-  // the correctly rounded quotient (checked exhaustively on the GPU; without the step 257
-  // denominators fail).  Three instructions a pair where correctly rounded quotients take five.
+  // 1.75 2.5 3.5 5) matter, x has eight significand bits, and for every significand of denom but the
+  // largest (which no bf16 maximum gives) and every reciprocal within one ulp the steps below put the values
+  // of x next to a boundary on the side of it that the correctly rounded quotient is on
+  // (tests/test_quantiser_rounding_cpu.py goes through them; without the step 257 denominators fail).
+  // Three instructions a pair where correctly rounded quotients take five.
   if (denom >= 1e-30f) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(denom));

@@ -103,3 +103,32 @@ def test_fused_quantiser_feeds_the_attention_kernel(cuda_device):
     Q3, K3, V3 = fa.quantize_qkv_fused(q, k, v, linear_sf=False)
     o3, _ = fa.flash_attn_func(Q3, K3, V3, causal=True, return_lse=True)
     assert torch.equal(o1, o3)
+
+
+def test_values_next_to_every_rounding_boundary(cuda_device):
+    """Every denominator significand that a bf16 maximum and an e4m3 block scale can give (128 x 8), and for each
+    the four bf16 values next to each of the seven rounding boundaries of e2m1: the oracle's bytes."""
+    mids = np.array([.25, .75, 1.25, 1.75, 2.5, 3.5, 5.0])
+    for a in range(128, 256):
+        amax = 16.0 * a                                  # tensor scales around one
+        g = np.float32(np.float32(amax) / np.float32(2688))
+        x = np.zeros((5, 4, 16), dtype=np.float32)
+        x[4, 0, 0] = amax
+        for m in range(8, 16):
+            denom = float(np.float32(m / 8) * g)
+            frac, e = np.frexp(mids * denom)
+            below = np.floor(np.ldexp(frac, 8))
+            for half, (lo, hi) in enumerate(((0, 1), (-1, 2))):
+                block = x[(m - 8) // 2, 2 * (m % 2) + half]
+                for col, j in ((0, lo), (7, hi)):
+                    n = below + j
+                    n = np.where(n > 256, 2 * n - 256, np.where(n < 128, 64 + n / 2, n))      # eight bits
+                    block[col:col + 7] = np.ldexp(n, e - 8) * (1 - 2 * (m % 2))
+                block[14] = torch.tensor(6 * denom).bfloat16().float().item()
+        x = torch.from_numpy(x.reshape(1, 5, 1, 64))
+        assert torch.equal(x.bfloat16().float(), x)
+        want = orc.quantize_nvfp4(x.numpy())
+        assert np.array_equal(want.sf[0, :4, 0], 0x38 + np.repeat(np.arange(8), 2).reshape(4, 4))   # 1, 1.125 .. 1.875
+        q = fa.quantize_qkv_fused(*(x.bfloat16().to(cuda_device),) * 3)[0]
+        assert q.scale == want.scale
+        assert np.array_equal(q.sf.cpu().numpy(), want.sf) and np.array_equal(q.data.cpu().numpy(), want.data), a

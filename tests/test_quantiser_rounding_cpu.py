@@ -1,0 +1,53 @@
+"""The element codes of the quantiser rest on quotients x / denom that are one residual step from the correctly
+rounded ones.  That is enough if every bf16 x next to a rounding boundary of e2m1 falls on the same side of it, for
+every denominator.  Powers of two change nothing, so all 2^23 significands in [1, 2) are all denominators."""
+import os
+import subprocess
+import tempfile
+
+import numpy as np
+
+SRC = r'''
+#include <math.h>
+#include <stdio.h>
+static int side(float y, float b) { return (y > b) - (y < b); }
+int main(void) {
+  const float bounds[7] = {.25f, .75f, 1.25f, 1.75f, 2.5f, 3.5f, 5.f};
+  const int reps[3] = {-1, 0, 1};
+  long bad = 0;
+#pragma omp parallel for reduction(+ : bad)
+  for (int m = 0; m < (1 << 23) - 1; ++m) {     /* the largest one: see the test */
+    const float d = 1.f + (float)m * 0x1p-23f;
+    for (int u = 0; u < 3; ++u) {
+      float r = 1.f / d;                                   /* rcp.approx.ftz: within one ulp of this */
+      if (reps[u]) r = nextafterf(r, reps[u] > 0 ? 2.f : 0.f);
+      r = fmaf(fmaf(-d, r, 1.f), r, r);
+      for (int k = 0; k < 7; ++k) {
+        int e;
+        const double t = (double)bounds[k] * d;            /* exact */
+        const double s = floor(ldexp(frexp(t, &e), 8));
+        for (int j = -1; j <= 2; ++j) {                    /* two bf16 values on either side of the boundary */
+          const double n = s + j, n8 = n > 256 ? 2 * n - 256 : n < 128 ? 64 + n / 2 : n;    /* eight bits */
+          const float x = (float)ldexp(n8, e - 8), y0 = x * r;
+          const float y = fmaf(fmaf(y0, -d, x), r, y0);
+          bad += side(y, bounds[k]) != side(x / d, bounds[k]);
+        }
+      }
+    }
+  }
+  printf("%ld\n", bad);
+  return 0;
+}'''
+
+
+def test_one_residual_step_keeps_every_quotient_on_its_side():
+    """With any reciprocal that is within one ulp.  Left out: 2 - 2^-23, where a reciprocal one ulp too small puts
+    the quotient of .5 on the boundary instead of above it; no bf16 maximum gives that denominator."""
+    reachable = {float(np.frexp(np.float32(m / 8) * (np.float32(a) / np.float32(2688)))[0])
+                 for a in range(128, 256) for m in range(8, 16)}
+    assert 1 - 2 ** -24 not in reachable
+    with tempfile.TemporaryDirectory() as d:
+        c, exe = os.path.join(d, "t.c"), os.path.join(d, "t")
+        open(c, "w").write(SRC)
+        subprocess.run(["gcc", "-O2", "-fopenmp", "-mfma", "-ffp-contract=off", c, "-o", exe, "-lm"], check=True)
+        assert int(subprocess.run([exe], capture_output=True, text=True, check=True).stdout) == 0
