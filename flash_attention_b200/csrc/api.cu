@@ -20,6 +20,9 @@ namespace {
 using namespace fa4;
 
 constexpr uint64_t kDefaultBudgetNs = 2000ull * 1000 * 1000;
+// SMs of a B200, for rules that must give one answer on the host alone (the size of a workspace is asked for
+// without a device) and for the shares of the streaming kernels; persistent grids ask the device.
+constexpr int64_t kSms = 148;
 
 PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -187,7 +190,7 @@ namespace {
 // Sk=777, 24 CTAs: 8.8 and 7.7).  A single split needs neither.
 bool decode_in_cluster(const fa4_nvfp4_params* p, int num_splits) {
   const int64_t ctas = (int64_t)num_splits * p->Hkv * p->B;
-  const int64_t resident = 148 * (p->Sq * (p->Hq / p->Hkv) <= 16 ? 3 : 2);
+  const int64_t resident = kSms * (p->Sq * (p->Hq / p->Hkv) <= 16 ? 3 : 2);
   return num_splits == 1 || (num_splits <= dec::kMaxCluster && ctas <= resident);
 }
 int64_t splitkv_bytes(const fa4_nvfp4_params* p, int num_splits) {
@@ -561,7 +564,7 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     // then run on with few CTAs beside them, bound by the latency of their loads (paged batch of 16,
     // longest 8192: 23.9 -> 21.6 us).  Even lengths keep HBM busy with three tiles, and the room beside two
     // shallow CTAs lets the next call's start early (B=4, Sk=32768: 32.9 us shallow, 34.7 deep).
-    const bool deep = cache.seqused_k != nullptr && p->B >= 4 && (int64_t)num_splits * p->Hkv * p->B <= 2 * 148;
+    const bool deep = cache.seqused_k != nullptr && p->B >= 4 && (int64_t)num_splits * p->Hkv * p->B <= 2 * kSms;
 #define FA4_DEC(rows, depth)                                                                             \
   (merge ? launch_dec(attn_decode_kernel<rows, true, depth>, rows, dec::Smem<depth>::kRequest)          \
          : launch_dec(attn_decode_kernel<rows, false, depth>, rows, dec::Smem<depth>::kRequest))
@@ -650,7 +653,7 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
   if ((num_splits > 1 || decode) && !merged) {
     const int64_t items = (int64_t)p->B * p->Sq * p->Hq * (p->Dv / 4);
     int64_t blocks = (items + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
+    if (blocks > kSms * 16) blocks = kSms * 16;
     return launch_pdl(combine_splits_kernel, dim3((unsigned)blocks), 256, 0, stream, kp.o_partial, kp.lse_partial, kp.out,
                       kp.lse, num_splits, p->B, p->Sq, p->Hq, p->Dv, kp.o_stride_b, kp.o_stride_s, kp.o_stride_h);
   }
@@ -738,7 +741,7 @@ int describe_outputs(QuantJob* j, bool is_v, int64_t s_out, void* packed, void* 
     j->rt = (j->S + 127) / 128;
     items = (int64_t)j->B * j->rt * 32 * j->nb;
     // four rows per item once that gives every SM its CTAs
-    j->single = items < 148 * kQuantizeCtas * 256;
+    j->single = items < kSms * kQuantizeCtas * 256;
     if (j->single) items *= 4;
     j->div_nb = make_fastdiv((uint32_t)j->nb);
     j->div_h = make_fastdiv((uint32_t)(j->D / 16));
@@ -756,7 +759,7 @@ int launch_amax(QuantJobs& q, cudaStream_t stream) {
   for (int i = 0; i < q.n; ++i) {
     QuantJob& j = q.job[i];
     j.amax_block0 = blocks;
-    j.amax_blocks = share_of(148 * kAmaxCtas, j.units, total, kAmaxThreads);
+    j.amax_blocks = share_of(kSms * kAmaxCtas, j.units, total, kAmaxThreads);
     j.parts = q.parts + blocks;
     j.num_parts = j.amax_blocks;
     blocks += j.amax_blocks;
@@ -772,7 +775,7 @@ int launch_quantize(QuantJobs& q, cudaStream_t stream) {
   for (int i = 0; i < q.n; ++i) {
     QuantJob& j = q.job[i];
     const int64_t most = j.is_v ? j.items : ((int64_t)j.items + 255) / 256;
-    int64_t ctas = 148 * kQuantizeCtas * weight(j) / total;
+    int64_t ctas = kSms * kQuantizeCtas * weight(j) / total;
     if (ctas < 1) ctas = 1;
     if (ctas > most || j.single) ctas = most;
     j.block0 = (int)blocks;

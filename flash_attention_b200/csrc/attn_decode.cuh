@@ -313,7 +313,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       const bool is_k = warp == 4;
       // (a K stage is free once its scores are in tensor memory, a V stage once its product is in O: no
       // commits of their own)
-            const uint32_t full0 = is_k ? L::kKFull : L::kVFull, free0 = is_k ? L::kSFull : L::kPvDone;
+      const uint32_t full0 = is_k ? L::kKFull : L::kVFull, free0 = is_k ? L::kSFull : L::kPvDone;
       const uint32_t tile0 = base + (is_k ? L::kOffK : L::kOffV), sf0 = base + (is_k ? L::kOffSFK : L::kOffSFV);
       const uint8_t* sf_src = is_k ? p.k_sf + hk * p.ksf_stride_h : p.v_sf + hk * p.vsf_stride_h;
       const int64_t sf_stride_b = is_k ? p.ksf_stride_b : p.vsf_stride_b;
@@ -442,21 +442,21 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     //      P^T tiles and scale chunks (rows past R are never written again)
     ok = true;
     if (wg == 0) {
-    for (uint32_t i = tid; i < (L::kOffRed - L::kOffQ) / 16; i += 128) {
-      *reinterpret_cast<uint4*>(gbase + L::kOffQ + i * 16) = make_uint4(0u, 0u, 0u, 0u);  // Q, SFQ, P, SFP are contiguous
-    }
-    FA4_DEC_SYNC()
-    if (ok) {
-      const int r = tid >> 2, ch = tid & 3;
-      if (r < R) *reinterpret_cast<uint4*>(gbase + L::kOffQ + sw64_offset(r, ch)) = q_pref;
-    }
-    if (ok && tid < 64) {
-      // scale bytes of row r: two words (one per 64-element step) of the tiled layout
-      const int r = tid >> 1, ks = tid & 1;
-      if (r < R) *reinterpret_cast<uint32_t*>(gbase + L::kOffSFQ + 512 * ks + r * 16) = qsf_pref;
-    }
-    fence_proxy_async_smem();
-    mbar_arrive(bar(L::kQReady));
+      for (uint32_t i = tid; i < (L::kOffRed - L::kOffQ) / 16; i += 128) {
+        *reinterpret_cast<uint4*>(gbase + L::kOffQ + i * 16) = make_uint4(0u, 0u, 0u, 0u);  // Q, SFQ, P, SFP are contiguous
+      }
+      FA4_DEC_SYNC()
+      if (ok) {
+        const int r = tid >> 2, ch = tid & 3;
+        if (r < R) *reinterpret_cast<uint4*>(gbase + L::kOffQ + sw64_offset(r, ch)) = q_pref;
+      }
+      if (ok && tid < 64) {
+        // scale bytes of row r: two words (one per 64-element step) of the tiled layout
+        const int r = tid >> 1, ks = tid & 1;
+        if (r < R) *reinterpret_cast<uint32_t*>(gbase + L::kOffSFQ + 512 * ks + r * 16) = qsf_pref;
+      }
+      fence_proxy_async_smem();
+      mbar_arrive(bar(L::kQReady));
     }
 
     // After the transpose below a thread owns ONE query row (row = lane % kR) with kR neighbouring

@@ -1,5 +1,5 @@
-// Warp-specialised kernel with 64-key sub-blocks and FOUR score buffers (split-KV and KV-cache views
-// stay with attn_ws.cuh).
+// Warp-specialised kernel with 64-key sub-blocks and FOUR score buffers: every prefill call but split-KV,
+// which stays with attn_ws.cuh.
 //
 // The kernel of attn_ws.cuh keeps two 128-column S buffers in tensor memory and lets two pairs of
 // softmax warpgroups alternate over the 128-key blocks, a thread owning half a row.  The two
