@@ -137,7 +137,7 @@ bool truth_of(PyObject* o) {
 // ---- per-tensor scales that are still on their way ------------------------------------------------
 // What quantize_qkv hands out for a scale: the quantiser leaves it on the device, and an attention call
 // on the quantiser's stream reads it there, so quantising and attending never wait on the host.
-// float(scale) copies all three back and waits for the stream, once.
+// float(scale) copies all three back and waits for the stream, once; calls after that take the values.
 struct ScaleState {
   c10::DataPtr device;              // three floats
   cudaStream_t stream;
@@ -215,10 +215,11 @@ Scale scale_of(PyObject* o) {
   }
   return s;
 }
-// The device copies of three scales for a call on `stream`; false: take their values instead.
+// The device copies of three scales for a call on `stream`; false: take their values instead (they are known,
+// or have to be fetched).
 bool device_scales(const Scale (&s)[3], const at::Device& device, cudaStream_t stream, const float** ptr) {
   for (int i = 0; i < 3; ++i) {
-    if (!s[i].lazy || s[i].lazy->stream != stream || s[i].lazy->device.device() != device) return false;
+    if (!s[i].lazy || s[i].lazy->known || s[i].lazy->stream != stream || s[i].lazy->device.device() != device) return false;
     ptr[i] = s[i].lazy->ptr(s[i].which);
   }
   return true;

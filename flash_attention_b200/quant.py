@@ -125,7 +125,8 @@ class NVFP4Tensor:
 def _get_scale(t: NVFP4Tensor) -> float:
     s = t._scale
     if _lib._host is not None and isinstance(s, _lib._host.LazyScale):
-        s = t._scale = float(s)
+        # (``_scale`` stays: a captured call may read the scale on the device, where it lives as long as this)
+        return float(s)
     return s
 
 
@@ -139,8 +140,7 @@ NVFP4Tensor.scale = property(_get_scale, _set_scale)
 
 
 def _getstate(t: NVFP4Tensor) -> dict:
-    t.scale                                  # a copy or a pickle carries the number
-    return t.__dict__
+    return {**t.__dict__, "_scale": t.scale}     # a copy or a pickle carries the number
 
 
 NVFP4Tensor.__getstate__ = _getstate

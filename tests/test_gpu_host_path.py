@@ -1,6 +1,7 @@
 """The native host path beside other Python threads and beside the operands a caller may pass: what waits for
 the GPU waits without the interpreter lock, what is not bytes is not read as bytes, and a call that fails
 half-way leaves the buffers of the next one in order."""
+import copy
 import threading
 import time
 
@@ -115,3 +116,24 @@ def test_a_failed_call_keeps_its_buffers_until_its_copies_have_run(cuda_device):
     pipe.run(*again, Q.scale, K.scale, V.scale, out, causal=True)
     pipe.wait()
     assert torch.equal(out, want.cpu())
+
+
+def test_a_captured_call_may_read_scales_on_the_device(cuda_device):
+    """A capture on the quantiser's own stream takes the scales from the device.  They live as long as the
+    operands, also when their values are read before the graph is replayed."""
+    q, k, v = make_qkv(1, 256, 256, 4, 2, 128, seed=41, device=cuda_device)
+    want = fa.flash_attn_func(*fa.quantize_qkv_fused(q, k, v), causal=True)[0]
+    stream = torch.cuda.Stream(cuda_device)
+    stream.wait_stream(torch.cuda.current_stream(cuda_device))
+    with torch.cuda.stream(stream):
+        ops = fa.quantize_qkv_fused(q, k, v)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            out = fa.flash_attn_func(*ops, causal=True)[0]
+        assert all(t.scale > 0 for t in ops) and copy.copy(ops[0]).scale == ops[0].scale
+        reused = [torch.full((128,), 3.0, device=cuda_device) for _ in range(64)]     # small blocks of the same stream
+        graph.replay()
+        stream.synchronize()
+    assert torch.equal(out, want) and len(reused) == 64
+    fa.check_status(cuda_device)
