@@ -21,6 +21,7 @@
 #include <ATen/cuda/CachingHostAllocator.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Device.h>
@@ -150,6 +151,8 @@ struct ScaleState {
     std::lock_guard<std::mutex> lock(fetching);
     if (known) return;
     c10::cuda::CUDAGuard guard(device.device().index());
+    // another stream may be capturing (a call outside of this one's stream takes the values)
+    c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
     float v[3];
     C10_CUDA_CHECK(cudaMemcpyAsync(v, device.get(), sizeof v, cudaMemcpyDeviceToHost, stream));
     C10_CUDA_CHECK(cudaStreamSynchronize(stream));

@@ -137,3 +137,17 @@ def test_a_captured_call_may_read_scales_on_the_device(cuda_device):
         stream.synchronize()
     assert torch.equal(out, want) and len(reused) == 64
     fa.check_status(cuda_device)
+
+
+def test_scales_may_be_fetched_while_another_stream_captures(cuda_device):
+    q, k, v = make_qkv(1, 256, 256, 4, 2, 128, seed=42, device=cuda_device)
+    want = fa.flash_attn_func(*fa.quantize_qkv_fused(q, k, v), causal=True)[0]
+    ops = fa.quantize_qkv_fused(q, k, v)         # its scales are read by nobody before the capture
+    torch.cuda.synchronize(cuda_device)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = fa.flash_attn_func(*ops, causal=True)[0]
+    graph.replay()
+    torch.cuda.synchronize(cuda_device)
+    assert torch.equal(out, want)
+    fa.check_status(cuda_device)
