@@ -153,8 +153,8 @@ __device__ __forceinline__ bool mbar_wait_relaxed(uint32_t bar, uint32_t parity,
 // A wait of the softmax warps: no call (they hold a row of scores in registers, some of them still on
 // their way from tensor memory) and no clock of its own, only the CTA's abort flag.  It is bounded all
 // the same: for every copy and product that such a wait depends on, or for what comes of it, an issuer or a
-// loader waits with a clock (the P V issuer for its own last product, before it leaves), and the first of
-// those waits to run out raises the flag.
+// loader waits with a clock (one of them, before it leaves, for the last product), and the first of those
+// waits to run out raises the flag.
 __device__ __forceinline__ bool mbar_wait_flag(uint32_t bar, uint32_t parity, const volatile uint32_t* s_abort) {
   for (;;) {
 #pragma unroll 1
