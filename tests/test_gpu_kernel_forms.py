@@ -1,6 +1,7 @@
 """The branches of the dispatch and of the host path at the sizes where they can go wrong: the edge between
 the narrow and the wide window form, more tiles than CTAs with tiles that have no rows between them, tile
-lists longer than a CTA's table, and the quantiser's small, unaligned and strided inputs."""
+lists longer than a CTA's table, the decode kernel's ring depths and the two ways its splits are merged, and
+the quantiser's small, unaligned and strided inputs."""
 import numpy as np
 import pytest
 import torch
@@ -96,3 +97,53 @@ def test_scales_on_the_device_give_the_bits_of_scales_on_the_host(cuda_device):
         assert all(isinstance(t.scale, float) for t in ops)
         known = fa.flash_attn_func(*ops, return_lse=True, **kw)
         assert torch.equal(lazy[0], known[0]) and torch.equal(lazy[1], known[1]), kw
+
+
+@pytest.mark.parametrize("Sq", [1, 2, 4])
+@pytest.mark.parametrize("B,splits", [(8, 1), (8, 2), (8, 8), (8, 9), (8, 19), (120, 2)],
+                         ids=["deep", "deep2", "deep8", "deep9combined", "shallow19", "clusters_do_not_fit"])
+def test_decode_ring_depths_and_merges(cuda_device, B, splits, Sq):
+    """Ragged entries with none, one, and odd and even numbers of key blocks (the two softmax warpgroups take
+    them in turn), in the deep ring (at least four entries, up to two CTAs an SM) and the shallow one, merged
+    inside a cluster (up to eight splits that fit at once) or by the combine kernel: the bits of the entry
+    alone, which runs the shallow ring, and the oracle's values."""
+    lens = [0, 1, 128, 129, 300, 640, 641, 1500] * (B // 8)
+    q, k, v = make_qkv(B, Sq, 1536, 8, 2, 128, seed=8, device=cuda_device)
+    Q, K, V = fa.quantize_qkv_fused(q, k, v)
+    used = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+
+    def run(b0, b1):
+        return fa.flash_attn_fp4_func(*(t.data[b0:b1] for t in (Q, K, V)), *(t.sf[b0:b1] for t in (Q, K, V)), Q.scale,
+                                      K.scale, V.scale, causal=True, return_lse=True, seqused_k=used[b0:b1],
+                                      num_splits=splits)
+
+    out, lse = run(0, B)
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    for b in list(range(8)) + [B - 1]:
+        o, l = run(b, b + 1)
+        assert torch.equal(out[b:b + 1], o) and torch.equal(lse[b:b + 1], l), lens[b]
+    n = lens[7]
+    ops = [fa.NVFP4Tensor(Q.data[7:8], Q.sf[7:8], Q.scale), fa.NVFP4Tensor(K.data[7:8, :n], K.sf[7:8, :n], K.scale),
+           fa.NVFP4Tensor(V.data[7:8, ..., :(n + 31) // 32 * 16], V.sf[7:8, ..., :(n + 31) // 32 * 2], V.scale, is_v=True)]
+    assert_parity(out[7:8], lse[7:8], *oracles(*ops, True, num_splits=splits, variant=fa.VARIANT_DECODE))
+
+
+@pytest.mark.parametrize("Sq,Sk,splits", [(1, 2048, 4), (1, 2048, 9), (100, 2048, 4), (100, 4096, 9)],
+                         ids=["decode_cluster", "decode_combine", "prefill_cluster", "prefill_combine"])
+def test_split_calls_replay_from_a_cuda_graph(cuda_device, Sq, Sk, splits):
+    q, k, v = make_qkv(2, Sq, Sk, 8, 2, 128, seed=9, device=cuda_device)
+    Q, K, V = fa.quantize_qkv_fused(q, k, v)
+    call = lambda: fa.flash_attn_fp4_func(Q.data, K.data, V.data, Q.sf, K.sf, V.sf, Q.scale, K.scale, V.scale, causal=True,
+                                          return_lse=True, num_splits=splits)
+    first = [t.clone() for t in call()]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out, lse = call()
+    Q.data.bitwise_xor_(0x88)                       # other operands in the same buffers: every sign of q
+    second = call()
+    assert not torch.equal(first[0], second[0])
+    graph.replay()
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    assert torch.equal(out, second[0]) and torch.equal(lse, second[1])
