@@ -45,8 +45,8 @@ class DeviceStatus:
         idx = device.index if device.index is not None else torch.cuda.current_device()
         w = cls._words.get(idx)
         if w is None:
-            w = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
-            cls._words[idx] = w
+            # one word per device also when several threads make their first call at once: its address is kept
+            w = cls._words.setdefault(idx, torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx)))
         return w
 
 

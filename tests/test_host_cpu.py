@@ -322,3 +322,24 @@ def test_padded_key_offsets_of_a_packed_batch():
     cu = torch.tensor([0, 70, 199, 200, 533, 533], dtype=torch.int32)
     assert fa.padded_key_offsets(cu).tolist() == [0, 96, 256, 288, 640, 640]
     assert fa.padded_key_offsets(torch.tensor([0, 64, 128], dtype=torch.int32)).tolist() == [0, 64, 128]
+
+
+def test_first_calls_of_two_threads_share_one_status_word(monkeypatch):
+    """The kernels keep the address of the word they were given first; check_status must read that one."""
+    import threading
+    from flash_attention_b200 import interface
+    both = threading.Barrier(2, timeout=10)
+
+    def zeros(*args, **kw):              # as the real one, it lets other threads run
+        both.wait()
+        return object()
+
+    monkeypatch.setattr(interface.torch, "zeros", zeros)
+    monkeypatch.setattr(interface.DeviceStatus, "_words", {})
+    got = []
+    threads = [threading.Thread(target=lambda: got.append(interface.DeviceStatus.word(torch.device("cuda", 0)))) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(got) == 2 and got[0] is got[1] is interface.DeviceStatus._words[0]
