@@ -155,7 +155,7 @@ __device__ __forceinline__ bool wait_probed(bool probed, uint32_t bar, uint32_t 
 // moved by more than the lazy threshold).  A rolled loop, but in line, like the masks below: no row of
 // scores is live at either place, and a call from the softmax loop costs the registers of its calling
 // convention there (64-key kernel, us: long context with outlier channels 12530 -> 12180, 127-key
-// window 134 -> 113; non-causal S = 4096, where corrections are rare, moves less than boxes differ).
+// window 134 -> 113; non-causal S = 4096, where corrections are rare, moves less than one GPU differs from the next).
 __device__ __forceinline__ void rescale_accumulator(uint32_t taddr, float f, int nchunks) {
 #pragma unroll 1
   for (int c = 0; c < nchunks; ++c) {

@@ -3,7 +3,7 @@
 // include/fa4_nvfp4.h.
 //
 // Why it exists: a decode step is 5-10 us of GPU time, and the same checks, attribute reads and
-// ctypes assignments written in Python took 35-60 us per call (B200 box, 76 us per pass of a
+// ctypes assignments written in Python took 35-60 us per call (B200, 76 us per pass of a
 // one-token call with linear scales), so the GPU waited for the host.  Here they take 5-8 us.
 //
 // The functions take their arguments positionally (METH_FASTCALL); interface.py and varlen.py own

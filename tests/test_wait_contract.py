@@ -1,5 +1,5 @@
-"""The no-hang contract of the prefill kernels, read from their source (a lost completion cannot be staged
-on a shared GPU): a wait without a clock of its own ends only when another role raises the abort flag, so
+"""The no-hang contract of the prefill kernels, read from their source (a completion that never comes is
+nothing a test can stage without hanging a kernel): a wait without a clock of its own ends only when another role raises the abort flag, so
 behind each completion that such a wait depends on some role must wait with a clock."""
 import os
 import re
