@@ -10,9 +10,9 @@
 // the signatures, defaults and documentation.  Each reads its Python arguments into plain values first and
 // then works without the interpreter lock: allocations, launches, reads of a value that is still on the
 // device and copies of pageable memory may all wait for the GPU, and other Python threads run meanwhile.
-// Error types and messages are those of the
-// reference's host code (flash_attn/cute/interface.py:231-236, 384-398): AssertionError for
-// malformed tensors, NotImplementedError for what is not built, ValueError for bad numbers.
+// Error types and messages are those of the reference's host code (flash_attn/cute/interface.py:231-236,
+// 384-398): AssertionError for malformed tensors, NotImplementedError for what is not built, ValueError
+// for bad numbers.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -841,7 +841,7 @@ void issue_pieces(PyObject* const* a) {
   const c10::cuda::CUDAStream s_in = c10::cuda::getStreamFromExternal(raw[0], device.index()),
                               s_compute = c10::cuda::getStreamFromExternal(raw[1], device.index()),
                               s_out = c10::cuda::getStreamFromExternal(raw[2], device.index());
-  const int64_t B = dev[0].size(0), Sq = dev[0].size(1), Hq = dev[0].size(2), Sk = dev[1].size(1), skp = 2 * dev[2].size(3);
+  const int64_t B = dev[0].size(0), Sq = dev[0].size(1), Hq = dev[0].size(2), Sk = dev[1].size(1);
   NoGil nogil;                     // (copies from and to pageable memory wait for themselves and for what is before them)
   c10::cuda::CUDAGuard device_guard(device);
   Event in_done, compute_done;
