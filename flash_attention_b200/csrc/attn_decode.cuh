@@ -228,7 +228,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   constexpr int kN = kR <= 16 ? 16 : 32;
   using TM = Tm<kN, kDepth>;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
   WaitCtx& wc = *reinterpret_cast<WaitCtx*>(gbase + L::kOffMisc + 16);
   const int R = p.Sq * p.group;  // live query rows (<= kR)
@@ -309,7 +309,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     // issuing K and V in turn tied the K stream to the P V products: K of block i + 1 went out
     // only when P V of block i - 3 had freed a V stage, one block time before Q K^T needs it, and
     // the kernel ran at one block per memory latency.)
-    if (lane == 0) {
+    if (elect_one()) {
       const bool is_k = warp == 4;
       // (a K stage is free once its scores are in tensor memory, a V stage once its product is in O: no
       // commits of their own)
@@ -354,7 +354,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     // ============================================ K . Q^T issuer ===============================
     // (One thread that issued both products paced the kernel: the copies, products and commits of a
     // block are fourteen tcgen05 instructions, about 100 clocks of issue each.)
-    if (lane == 0 && n > 0) {
+    if (elect_one() && n > 0) {
       ok = mbar_wait(bar(L::kQReady), 0, wc, kDQReady);
       uint64_t dq[2];
       if (ok) {
@@ -393,7 +393,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
   } else if (warp == 7) {
     // ============================================ V^T . P^T issuer =============================
-    if (lane == 0) {
+    if (elect_one()) {
       for (int li = 0; ok && li < n; ++li) {
         const uint32_t st = li % kDepth, slot = li % kDepth;
         ok = mbar_wait(bar(L::kVFull + st), (li / kDepth) & 1, wc, kDVFull);

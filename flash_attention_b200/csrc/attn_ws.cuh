@@ -317,7 +317,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
   volatile float* s_fin = reinterpret_cast<volatile float*>(gbase + kOffFin);    // [2][4][128][2]
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = warp_index();
   const int lane = tid & 31;
   WaitCtx& wc = *reinterpret_cast<WaitCtx*>(gbase + kOffMisc + 16);
   const int num_tiles = p.num_m_blocks * p.Hq * p.B * (kGeneral ? p.num_splits : 1);
@@ -381,7 +381,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
 
   if (warp >= kProducerWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
-    if (warp == kProducerWarp && lane == 0) {
+    if (warp == kProducerWarp && elect_one()) {
       // ========================================= TMA producer ===================================
       uint32_t issued_k = 0, issued_v = 0, issued_q = 0;
       FA4_FOR_EACH_TILE {
@@ -477,7 +477,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
           while (!mbar_try_wait(bars.at(Bars::kQFull + (i & 1)), (i >> 1) & 1) && globaltimer_ns() - t0 < lim) {}
         }
       }
-    } else if (warp == kIssuerWarp && lane == 0) {
+    } else if (warp == kIssuerWarp && elect_one()) {
       // ========================================= QK^T issuer ====================================
       FA4_FOR_EACH_TILE {
         const Tile t = decode_tile<kGeneral>(p, tile);
@@ -530,7 +530,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         tc_commit(bars.at(Bars::kDrain));
         while (!mbar_try_wait(bars.at(Bars::kDrain), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
       }
-    } else if (warp == kPvIssuerWarp && lane == 0) {
+    } else if (warp == kPvIssuerWarp && elect_one()) {
       // ========================================= PV issuer ======================================
       FA4_FOR_EACH_TILE {
         const Tile t = decode_tile<kGeneral>(p, tile);
@@ -585,7 +585,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         tc_commit(bars.at(Bars::kDrain + 1));
         while (!mbar_try_wait(bars.at(Bars::kDrain + 1), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
       }
-    } else if (warp == kStoreWarp && lane == 0) {
+    } else if (warp == kStoreWarp && elect_one()) {
       // ========================================= output store ===================================
       // (the split-KV path writes fp32 partial outputs directly and does not use this role)
       if (!(kGeneral && p.num_splits > 1)) {

@@ -290,7 +290,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   volatile float* s_fin = reinterpret_cast<volatile float*>(gbase + kOffFin);    // [2][4][128][2]
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = warp_index();
   const int lane = tid & 31;
   WaitCtx& wc = *reinterpret_cast<WaitCtx*>(gbase + kOffMisc + 16);
   const int ncta = gridDim.x, cta = blockIdx.x;
@@ -515,7 +515,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     if (lane == 0) bulk_wait_group0();
   } else if (warp >= kLoadKWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kD == 192 ? kRegsEven : kRegsOther));
-    if ((warp == kLoadKWarp || warp == kLoadVWarp) && lane == 0) {
+    if ((warp == kLoadKWarp || warp == kLoadVWarp) && elect_one()) {
       // ========================================= TMA loaders ====================================
       // One warp streams Q and K, the other V, each as far ahead as its own ring allows: what Q K^T of
       // the next tile needs never queues behind a V stage that P V has yet to free.
@@ -635,7 +635,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
         while (!mbar_try_wait(bars.at(Bars::kDrain + (is_k ? 2 : 3)), 0) && globaltimer_ns() - t0 < lim) {}
       }
-    } else if (warp == kIssuerWarp && lane == 0) {
+    } else if (warp == kIssuerWarp && elect_one()) {
       // ========================================= QK^T issuer ====================================
       FA4_FOR_EACH_TILE {
         const TileRec t = s_tiles[it];
@@ -691,7 +691,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         tc_commit(bars.at(Bars::kDrain));
         while (!mbar_try_wait(bars.at(Bars::kDrain), 0) && globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
       }
-    } else if (warp == kPvIssuerWarp && lane == 0) {
+    } else if (warp == kPvIssuerWarp && elect_one()) {
       // ========================================= P V issuer =====================================
       FA4_FOR_EACH_TILE {
         const TileRec t = s_tiles[it];
