@@ -489,6 +489,7 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
   kp.div_hq = make_fastdiv((uint32_t)p->Hq);
   kp.div_group = make_fastdiv((uint32_t)kp.group);
   kp.div_splits = make_fastdiv((uint32_t)num_splits);
+  kp.div_page = make_fastdiv(cache.page_table != nullptr ? (uint32_t)(cache.page_size / kBlockN) : 1u);
   kp.num_m_blocks = (p->Sq + kBlockM - 1) / kBlockM;
   kp.num_n_blocks = (p->Sk + kBlockN - 1) / kBlockN;
   kp.causal = win_right >= 0 ? 1 : 0;
@@ -555,9 +556,9 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     dp.o_partial = kp.o_partial;
     dp.lse_partial = kp.lse_partial;
     const bool merge = decode_in_cluster(p, num_splits);
-    auto launch_dec = [&](auto kernel, int rows, uint32_t smem) -> int {
+    auto launch_dec = [&](auto kernel, int threads, uint32_t smem) -> int {
       return launch_pdl_cluster(merge ? (unsigned)num_splits : 1u, kernel,
-                                dim3((unsigned)num_splits, (unsigned)p->Hkv, (unsigned)p->B), dec::threads_of(rows), smem,
+                                dim3((unsigned)num_splits, (unsigned)p->Hkv, (unsigned)p->B), threads, smem,
                                 stream, tm_k, tm_v, kp, dp);
     };
     // The deep form where several entries have lengths of their own and no third CTA per SM waits: the long entries
@@ -566,8 +567,8 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     // shallow CTAs lets the next call's start early (B=4, Sk=32768: 32.9 us shallow, 34.7 deep).
     const bool deep = cache.seqused_k != nullptr && p->B >= 4 && (int64_t)num_splits * p->Hkv * p->B <= 2 * kSms;
 #define FA4_DEC(rows, depth)                                                                             \
-  (merge ? launch_dec(attn_decode_kernel<rows, true, depth>, rows, dec::Smem<depth>::kRequest)          \
-         : launch_dec(attn_decode_kernel<rows, false, depth>, rows, dec::Smem<depth>::kRequest))
+  (merge ? launch_dec(attn_decode_kernel<rows, true, depth>, dec::threads_of(rows, depth), dec::form<rows, depth>::kRequest)          \
+         : launch_dec(attn_decode_kernel<rows, false, depth>, dec::threads_of(rows, depth), dec::form<rows, depth>::kRequest))
     const int rc = dec_rows <= 4    ? (deep ? FA4_DEC(4, 5) : FA4_DEC(4, 3))
                    : dec_rows <= 8  ? (deep ? FA4_DEC(8, 5) : FA4_DEC(8, 3))
                    : dec_rows <= 16 ? (deep ? FA4_DEC(16, 5) : FA4_DEC(16, 3))
@@ -651,11 +652,13 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     if (rc != 0) return rc;
   }
   if ((num_splits > 1 || decode) && !merged) {
-    const int64_t items = (int64_t)p->B * p->Sq * p->Hq * (p->Dv / 4);
-    int64_t blocks = (items + 255) / 256;
+    // (fewer than 2^31 rows: the workspace holds at least 512 bytes of each)
+    const uint32_t rows = (uint32_t)p->B * p->Sq * p->Hq, per_block = num_splits > kCombineBatch ? 1u : kCombineWarps;
+    uint32_t blocks = (rows + per_block - 1) / per_block;
     if (blocks > kSms * 16) blocks = kSms * 16;
-    return launch_pdl(combine_splits_kernel, dim3((unsigned)blocks), 256, 0, stream, kp.o_partial, kp.lse_partial, kp.out,
-                      kp.lse, num_splits, p->B, p->Sq, p->Hq, p->Dv, kp.o_stride_b, kp.o_stride_s, kp.o_stride_h);
+    return launch_pdl(combine_splits_kernel, dim3(blocks), kCombineWarps * 32, 0, stream, kp.o_partial, kp.lse_partial,
+                      kp.out, kp.lse, num_splits, rows, (int)(kCombineWarps / per_block), kp.div_hq,
+                      make_fastdiv((uint32_t)p->Sq), p->Sq, p->Hq, p->Dv, kp.o_stride_b, kp.o_stride_s, kp.o_stride_h);
   }
   return 0;
 }

@@ -41,6 +41,7 @@ struct KernelParams {
   // divisors of the tile-list arithmetic, as multiply-high + shift: every warp decodes every tile
   FastDiv div_tiles_per_m;   // Hq * B
   FastDiv div_hq, div_group, div_splits;
+  FastDiv div_page;          // blocks of a page (cache views with a page table)
   int num_m_blocks, num_n_blocks;
   int compact_tiles;         // packed batch whose slots are mostly empty: deal the existing tiles (64-key kernel)
   int tile_begin, tile_end;  // the part of the tile list this launch works on (64-key kernel)

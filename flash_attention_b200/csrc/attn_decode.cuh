@@ -25,12 +25,20 @@
 // attn_ws.cuh.  Grid = (splits, Hkv, B).
 //   warps 0-3  softmax / correction / epilogue (thread = key lane, after the transpose a row; in the
 //              correction and the epilogue a dv lane)
-//   warps 8-11 up to eight rows: a second softmax warpgroup, which takes the odd blocks
+//   warps 8-11 up to eight rows: a second softmax warpgroup, which takes the odd blocks; in the deep form
+//              warps 8-19: three more, the blocks dealt in turn
 //   warp 4     TMA producer of K (ring of three tiles, through the page table if there is one)
 //   warp 5     issuer of K . Q^T (owns tensor memory)
 //   warp 6     TMA producer of V (its own ring, independent of K's)
 //   warp 7     issuer of V^T . P^T
 // Every wait is bounded, like everywhere else.
+//
+// Most calls are over in 6-20 us, and whatever runs once per CTA -- set-up, epilogue, merge -- runs from cold
+// instruction memory: its length in code, not in work, is its time.  So what is the same for all lanes of a row is
+// done by the lanes of that row at once instead of row after row in unrolled code, divisions are multiplications, and
+// the merge takes a row a warp.  us, code unrolled over the rows -> this: 32 rows (GQA 4, eight tokens), 2 entries of up
+// to 16384 keys 42.2 -> 26.2; 16 rows, 4 x 8192 21.6 -> 18.0; 4 rows, paged batch of 16 up to 8192 20.7 -> 18.7 (with
+// combine_splits_kernel written the same way 21.9, 16.6, 18.7).
 #pragma once
 #include "attn_common.cuh"
 #include "softmax.cuh"
@@ -44,15 +52,21 @@ namespace dec {
 // trip, so five are better whenever no third CTA is there to run.
 constexpr int kMaxCluster = 8;  // splits that are merged inside a cluster (portable cluster size)
 constexpr int kMaxRows = 32; // query rows per kv head: Sq * group
-// Softmax warpgroups: two up to eight rows, one above (registers: three CTAs of twelve warps per SM
-// leave 56 per thread).  With two, even blocks go to one and odd ones to the other.
-__host__ __device__ constexpr int softmax_wgs(int rows) { return rows <= 8 ? 2 : 1; }
-__host__ __device__ constexpr int threads_of(int rows) { return softmax_wgs(rows) == 2 ? 384 : 256; }
+// Softmax warpgroups: one above eight rows; up to eight, two in the shallow form (registers: three CTAs of
+// twelve warps per SM leave 56 per thread) and four in the deep one, whose long entries run on with few CTAs
+// beside them: a block is a chain of some 1700 clocks in its warpgroup, and only the reference is handed
+// from block to block.  Blocks are dealt in turn.  us, two warpgroups -> four: 32 paged sequences up to 16384
+// 66.6 -> 61.0, 16 up to 8192 20.25 -> 20.23 (there the loads of a CTA pace it).
+__host__ __device__ constexpr int softmax_wgs(int rows, int depth) {
+  return rows > 8 ? 1 : (depth == 5 ? 4 : 2);
+}
+__host__ __device__ constexpr int strands_of(int rows) { return rows <= 8 ? 4 : 1; }
+__host__ __device__ constexpr int threads_of(int rows, int depth) { return 128 + 128 * softmax_wgs(rows, depth); }
 
-constexpr uint32_t kQBytes = kMaxRows * 64;                // Q^T / P^T operand: up to 32 rows x 64 bytes
-// shared memory
-template <int kDepth>
+// shared memory of the form with kN rows per operand and kWgs softmax warpgroups
+template <int kDepth, int kN, int kWgs>
 struct Smem {
+  static constexpr uint32_t kQBytes = kN * 64;                      // Q^T / P^T operand: rows of 64 bytes
   static constexpr uint32_t kOffK = 0;
   static constexpr uint32_t kOffV = kOffK + kDepth * kTileBytes;
   static constexpr uint32_t kOffSFK = kOffV + kDepth * kTileBytes;
@@ -61,21 +75,24 @@ struct Smem {
   static constexpr uint32_t kOffSFQ = kOffQ + kQBytes;              // two 512-byte chunks
   static constexpr uint32_t kOffP = kOffSFQ + 1024;                 // kDepth x kQBytes
   static constexpr uint32_t kOffSFP = kOffP + kDepth * kQBytes;     // kDepth x 2 chunks x 512
-  static constexpr uint32_t kOffRed = kOffSFP + kDepth * 1024;      // 2 WGs x 2 x 4 warps x 32 floats
-  static constexpr uint32_t kOffHand = kOffRed + 2 * 2 * 4 * kMaxRows * 4;   // 2 WGs x 4 warps x 32 references
-  static constexpr uint32_t kOffBar = kOffHand + 2 * 4 * kMaxRows * 4;
+  static constexpr uint32_t kOffRed = kOffSFP + kDepth * 1024;      // WGs x 2 x 4 warps x kN floats
+  static constexpr uint32_t kOffHand = kOffRed + kWgs * 2 * 4 * kN * 4;   // WGs x 4 warps x kN references
+  static constexpr uint32_t kOffSum = kOffHand + kWgs * 4 * kN * 4;       // kWgs = 2: 2 x 256 (row sum, its reference)
+  static constexpr uint32_t kOffOld = kOffSum + (kWgs == 2 ? 2 * 256 * 8 : 0);   // kWgs = 2: WGs x (4 warps' sums, 1 reference) x kN
+  static constexpr uint32_t kOffBar = kOffOld + (kWgs == 2 ? kWgs * 5 * kN * 4 : 0);
   // barriers
   static constexpr uint32_t kKFull = 0, kVFull = kKFull + kDepth, kSFull = kVFull + kDepth, kSFree = kSFull + kDepth,
                             kPFull = kSFree + kDepth, kPvDone = kPFull + kDepth, kQReady = kPvDone + kDepth,
-                            kSync = kQReady + 1 /* 2 */, kHand = kSync + 2 /* 2 x 4 */, kFin = kHand + 8,
+                            kSync = kQReady + 1 /* WGs */, kHand = kSync + kWgs /* WGs x 4 */, kFin = kHand + 4 * kWgs,
                             kDrain = kFin + 1 /* 2 */, kCount = kDrain + 2;
-  static constexpr uint32_t kOffMisc = kOffBar + 8 * kCount;
+  static constexpr uint32_t kOffMisc = (kOffBar + 8 * kCount + 15) / 16 * 16;
   static constexpr uint32_t kRequest = kOffMisc + 16 + sizeof(WaitCtx) + 1024;
+  // (1 KB per CTA is the system's)
+  static_assert((kDepth == 3 ? 3 : 2) * (kRequest + 1024) <= 228 * 1024, "decode kernel shared memory");
 };
-// (1 KB per CTA is the system's)
-static_assert(3 * (Smem<3>::kRequest + 1024) <= 228 * 1024 && 2 * (Smem<5>::kRequest + 1024) <= 228 * 1024,
-              "decode kernel shared memory");
-static_assert(Smem<5>::kOffMisc % 8 == 0 && Smem<3>::kOffMisc % 8 == 0, "the wait context is 8-byte aligned");
+
+template <int kRows, int kDepth>
+using form = Smem<kDepth, (kRows <= 16 ? 16 : 32), softmax_wgs(kRows, kDepth)>;   // of the kernel's form
 
 // tensor memory of the form with N columns per operand: S^T buffers, O^T, scale factors.  The K / V / P
 // scale slots alternate between two copies: the copy and the product that reads it are issued by one
@@ -184,7 +201,7 @@ __device__ __forceinline__ void lane_group_transpose(float (&x)[T], int lane) {
 __device__ __forceinline__ void block_exponent1(float bm, float m_ref, float sl2, float& noff,
                                                 uint32_t& ue) {
   constexpr float kMagic = 12582912.f + 127.f;
-  const float msc = (m_ref == kNegInf) ? 0.f : m_ref * sl2;
+  const float msc = (m_ref == kNegInf) ? 0.f : __fmul_rn(m_ref, sl2);   // (not contracted: one result in all forms)
   const float c_t = static_cast<float>(kShift) - kLog2Of6 + 0.4999995f - msc;
   const float c_off = static_cast<float>(kShift) - msc;
   float t = fmaf(bm, sl2, c_t);
@@ -211,22 +228,24 @@ struct DecodeParams {
 // kMerge: the splits of a (kv head, batch entry) are one cluster, which merges their partials through
 // distributed shared memory and writes the result; otherwise they go to o_partial / lse_partial.
 template <int kR, bool kMerge, int kDepth>
-__global__ void __launch_bounds__(dec::threads_of(kR), kDepth == 3 ? 3 : 2)
+__global__ void __launch_bounds__(dec::threads_of(kR, kDepth), kDepth == 3 ? 3 : 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const KernelParams p, const DecodeParams d) {
   using namespace dec;
-  using L = Smem<kDepth>;
+  constexpr int kWgs = softmax_wgs(kR, kDepth);
+  constexpr int kN = kR <= 16 ? 16 : 32, kMaxRows = kN;   // (stride of the arrays per row)
+  using L = form<kR, kDepth>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - smem_u32(smem_raw));
   auto bar = [&](uint32_t idx) -> uint32_t { return base + L::kOffBar + 8u * idx; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + L::kOffMisc);
   volatile uint32_t* s_abort = reinterpret_cast<volatile uint32_t*>(gbase + L::kOffMisc + 4);
-  volatile float* s_red = reinterpret_cast<volatile float*>(gbase + L::kOffRed);    // [2][2][4][32]
-  volatile float* s_hand = reinterpret_cast<volatile float*>(gbase + L::kOffHand);  // [2][4][32]
-  constexpr int kWgs = softmax_wgs(kR);
-  constexpr int kN = kR <= 16 ? 16 : 32;
+  volatile float* s_red = reinterpret_cast<volatile float*>(gbase + L::kOffRed);    // [WGs][2][4][rows]
+  volatile float* s_old = reinterpret_cast<volatile float*>(gbase + L::kOffOld);
+  volatile float* s_hand = reinterpret_cast<volatile float*>(gbase + L::kOffHand);  // [WGs][4][rows]
   using TM = Tm<kN, kDepth>;
+  constexpr int kStrands = strands_of(kR), kOwn = kStrands / kWgs;   // partial row sums; of a warpgroup
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
   const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
@@ -245,9 +264,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       mbar_init(bar(L::kPvDone + s), 1);
     }
     mbar_init(bar(L::kQReady), 128);
-    for (int w = 0; w < 2; ++w) mbar_init(bar(L::kSync + w), 128);
-    for (int w = 0; w < 8; ++w) mbar_init(bar(L::kHand + w), 32);
-    mbar_init(bar(L::kFin), 128);
+    for (int w = 0; w < kWgs; ++w) mbar_init(bar(L::kSync + w), 128);
+    for (int w = 0; w < 4 * kWgs; ++w) mbar_init(bar(L::kHand + w), 32);
+    mbar_init(bar(L::kFin), 128 * (kWgs > 1 ? kWgs - 1 : 1));
     for (int w = 0; w < 2; ++w) mbar_init(bar(L::kDrain + w), 1);
     fence_barrier_init();
   }
@@ -268,7 +287,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   if (tid < 128) {
     const int r = tid >> 2, ch = tid & 3;
     if (r < R) {
-      const int s = r / p.group, h = hk * p.group + r % p.group;
+      const int s = fast_div(r, p.div_group), h = hk * p.group + r - s * p.group;
       q_pref = *reinterpret_cast<const uint4*>(d.q + b * d.q_stride_b + s * d.q_stride_s + h * d.q_stride_h +
                                                ch * 16);
     }
@@ -276,7 +295,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   if (tid < 64) {
     const int r = tid >> 1, ks = tid & 1;
     if (r < R) {
-      const int s = r / p.group, h = hk * p.group + r % p.group;
+      const int s = fast_div(r, p.div_group), h = hk * p.group + r - s * p.group;
       const uint8_t* chunk = d.q_sf + b * p.qsf_stride_b + h * p.qsf_stride_h + ((int64_t)(s / 128) * 2 + ks) * 512;
       const int rr = s % 128;
       qsf_pref = *reinterpret_cast<const uint32_t*>(chunk + (rr % 32) * 16 + (rr / 32) * 4);
@@ -291,10 +310,22 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     sk = used < 0 ? 0 : (used < p.Sk ? used : p.Sk);
   }
   const int n_total = (sk + kBlockN - 1) / kBlockN;
-  const int per = (n_total + d.num_splits - 1) / d.num_splits;
+  const int per = fast_div(n_total + d.num_splits - 1, p.div_splits);
   const int i0 = split * per < n_total ? split * per : n_total;
   const int i1 = i0 + per < n_total ? i0 + per : n_total;
   const int n = i1 - i0;
+  // (producers) lane l: where the CTA's block li + l lies: batch coordinate, block inside it
+  auto locate = [&](int li) -> int2 {
+    int2 r = make_int2(b, i0 + li + lane);
+    if (p.page_table != nullptr && li + lane < n) {
+      const int pg = fast_div(r.y, p.div_page);
+      r.x = p.page_table[(int64_t)b * p.pages_per_seq + pg];
+      r.y -= pg * (p.page_size / kBlockN);
+    }
+    return r;
+  };
+  int2 at = make_int2(0, 0);
+  if (warp == 4 || warp == 6) at = locate(0);
   __syncthreads();
   tc_fence_after_sync();
   pdl_trigger();
@@ -309,45 +340,44 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     // issuing K and V in turn tied the K stream to the P V products: K of block i + 1 went out
     // only when P V of block i - 3 had freed a V stage, one block time before Q K^T needs it, and
     // the kernel ran at one block per memory latency.)
-    if (elect_one()) {
-      const bool is_k = warp == 4;
-      // (a K stage is free once its scores are in tensor memory, a V stage once its product is in O: no
-      // commits of their own)
-      const uint32_t full0 = is_k ? L::kKFull : L::kVFull, free0 = is_k ? L::kSFull : L::kPvDone;
-      const uint32_t tile0 = base + (is_k ? L::kOffK : L::kOffV), sf0 = base + (is_k ? L::kOffSFK : L::kOffSFV);
-      const uint8_t* sf_src = is_k ? p.k_sf + hk * p.ksf_stride_h : p.v_sf + hk * p.vsf_stride_h;
-      const int64_t sf_stride_b = is_k ? p.ksf_stride_b : p.vsf_stride_b;
-      uint32_t issued = 0;
-      for (int li = 0; ok && li < n; ++li) {
-        const int nb = i0 + li;
-        const uint32_t st = li % kDepth;
-        int kb = b, nbl = nb;   // batch coordinate and block inside it (a page of the pool)
-        if (p.page_table != nullptr) {
-          const int key0 = nb * kBlockN, pg = key0 / p.page_size;
-          kb = p.page_table[(int64_t)b * p.pages_per_seq + pg];
-          nbl = (key0 - pg * p.page_size) / kBlockN;
+    // Where the blocks lie (a page of the pool and the block in it) is looked up by the whole warp, a block a
+    // lane and 32 blocks at a time, the first ones before the CTA's set-up is over: read one by one in front of each
+    // load, the table held the K stream to a block per latency, 700 clocks, which four softmax warpgroups outrun.
+    const bool is_k = warp == 4;
+    // (a K stage is free once its scores are in tensor memory, a V stage once its product is in O: no
+    // commits of their own)
+    const uint32_t full0 = is_k ? L::kKFull : L::kVFull, free0 = is_k ? L::kSFull : L::kPvDone;
+    const uint32_t tile0 = base + (is_k ? L::kOffK : L::kOffV), sf0 = base + (is_k ? L::kOffSFK : L::kOffSFV);
+    const uint8_t* sf_src = is_k ? p.k_sf + hk * p.ksf_stride_h : p.v_sf + hk * p.vsf_stride_h;
+    const int64_t sf_stride_b = is_k ? p.ksf_stride_b : p.vsf_stride_b;
+    int li = 0;
+    for (; li < n; ++li) {
+      if ((li & 31) == 0 && li > 0) at = locate(li);
+      const uint32_t st = li % kDepth;
+      const int kb = __shfl_sync(0xffffffffu, at.x, li & 31), nbl = __shfl_sync(0xffffffffu, at.y, li & 31);
+      if (elect_one()) {
+        if (li >= kDepth) ok = mbar_wait(bar(free0 + st), ((li - kDepth) / kDepth) & 1, wc, is_k ? kDKFree : kDVFree);
+        if (ok) {
+          mbar_arrive_expect_tx(bar(full0 + st), kTileBytes + kSfBytes);
+          if (is_k) {
+            tma_load_4d(tile0 + st * kTileBytes, &tm_k, bar(full0 + st), 0, hk, nbl * kBlockN, kb);
+          } else {
+            tma_load_4d(tile0 + st * kTileBytes, &tm_v, bar(full0 + st), nbl * (kBlockN / 2), 0, hk, kb);
+          }
+          bulk_load(sf0 + st * kSfBytes, sf_src + kb * sf_stride_b + (int64_t)nbl * kSfBytes, kSfBytes,
+                    bar(full0 + st));
         }
-        if (li >= kDepth) {
-          ok = mbar_wait(bar(free0 + st), ((li - kDepth) / kDepth) & 1, wc, is_k ? kDKFree : kDVFree);
-          if (!ok) break;
-        }
-        mbar_arrive_expect_tx(bar(full0 + st), kTileBytes + kSfBytes);
-        if (is_k) {
-          tma_load_4d(tile0 + st * kTileBytes, &tm_k, bar(full0 + st), 0, hk, nbl * kBlockN, kb);
-        } else {
-          tma_load_4d(tile0 + st * kTileBytes, &tm_v, bar(full0 + st), nbl * (kBlockN / 2), 0, hk, kb);
-        }
-        bulk_load(sf0 + st * kSfBytes, sf_src + kb * sf_stride_b + (int64_t)nbl * kSfBytes, kSfBytes,
-                  bar(full0 + st));
-        issued = li + 1;
       }
-      if (!ok) {
-        // bounded drain: let the copies already issued land before the CTA's memory is released
-        const uint64_t t0 = globaltimer_ns();
-        for (uint32_t i = issued > kDepth ? issued - kDepth : 0; i < issued; ++i) {
-          while (!mbar_try_wait(bar(full0 + (i % kDepth)), (i / kDepth) & 1) &&
-                 globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
-        }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+    }
+    if (!ok && lane == 0) {
+      // bounded drain: let the copies already issued (those of the blocks before li) land before the CTA's memory
+      // is released
+      const uint64_t t0 = globaltimer_ns();
+      for (int i = li > kDepth ? li - kDepth : 0; i < li; ++i) {
+        while (!mbar_try_wait(bar(full0 + (i % kDepth)), (i / kDepth) & 1) &&
+               globaltimer_ns() - t0 < 50ull * 1000 * 1000) {}
       }
     }
   } else if (warp == 5) {
@@ -401,7 +431,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         tc_fence_after_sync();
         const uint32_t sfv = tmem + TM::kSFV + 8 * (li & 1), sfp = tmem + TM::kSFP + 8 * (li & 1);
         const uint32_t vt = base + L::kOffV + st * kTileBytes, vsf = base + L::kOffSFV + st * kSfBytes;
-        const uint32_t pt = base + L::kOffP + slot * kQBytes, psf = base + L::kOffSFP + slot * 1024;
+        const uint32_t pt = base + L::kOffP + slot * L::kQBytes, psf = base + L::kOffSFP + slot * 1024;
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) tc_cp_sf(sfv + 4 * ks, vsf + 512 * ks);
         ok = mbar_wait(bar(L::kPFull + slot), (li / kDepth) & 1, wc, kDPFull);
@@ -428,7 +458,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     // and writes the result.  What a block hands to the next one is the reference maximum of its rows,
     // from warp wq of one warpgroup to warp wq of the other (every warp knows all rows); everything
     // else of a block -- about 1000 clocks of latencies -- then runs beside the neighbouring block's.
-    const int wg = warp >> 3, wq = warp & 3;
+    const int wg = warp < 4 ? 0 : (warp >> 2) - 1, wq = warp & 3;
     const uint32_t lane_addr = tmem + (static_cast<uint32_t>(wq * 32) << 16);
     s_red += wg * (2 * 4 * kMaxRows);
     uint32_t sync_phase = 0;
@@ -465,12 +495,17 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     // thread that kept "its key, all rows" ran it kR times.
     const int my_row = lane & (kR - 1), grp = lane / kR;
     const int key_in_blk = wq * 32 + grp * kR;   // first of this thread's kR keys inside the block
+    // Row sums: kStrands of them, that of block li in strand li % kStrands, each relative to the reference of its own
+    // last block; so a row's sum is the same bits with two warpgroups and with four.  With two, a thread has two,
+    // of which shared memory keeps the one that is not in use.
     float m_ref = kNegInf, l_sum = 0.f;
+    float2* strands = reinterpret_cast<float2*>(gbase + L::kOffSum) + wg * 128 + (tid & 127);    // [2][256]
+    if (kOwn == 2) strands[0] = strands[256] = make_float2(0.f, kNegInf);
     // last visible key of the row (causal: bottom-right aligned on the entry's key count); rows
     // past R see nothing
     int lim = -1;
     if (my_row < R) {
-      const int c = sk - p.Sq + my_row / p.group;
+      const int c = sk - p.Sq + fast_div(my_row, p.div_group);
       lim = (p.causal && c < sk - 1) ? c : sk - 1;
     }
 
@@ -520,15 +555,16 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       const float m_loc = fmaxf(fmaxf(red[my_row], red[kMaxRows + my_row]),
                                 fmaxf(red[2 * kMaxRows + my_row], red[3 * kMaxRows + my_row]));
       float m_prev = m_ref;
-      if (kWgs == 2 && li > 0) {
+      if (kWgs > 1 && li > 0) {
+        const int before = (wg + kWgs - 1) % kWgs;
         // the reference after block li - 1 (the unbroken chain also orders the reuse of the slots: block
         // li + 1 overwrites this one's source only after it has read what this block hands on)
-        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kHand + 4 * (wg ^ 1) + wq), ((li - 1) >> 1) & 1, wc, kDHand));
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kHand + 4 * before + wq), ((li - 1) / kWgs) & 1, wc, kDHand));
         if (!ok) break;
-        m_prev = s_hand[((wg ^ 1) * 4 + wq) * kMaxRows + my_row];
+        m_prev = s_hand[(before * 4 + wq) * kMaxRows + my_row];
       }
       const float m_new = next_reference(m_prev, m_loc, sc.sl2);
-      if (kWgs == 2) {
+      if (kWgs > 1) {
         if (lane < kR) s_hand[(wg * 4 + wq) * kMaxRows + my_row] = m_new;
         mbar_arrive(bar(L::kHand + 4 * wg + wq));
       }
@@ -538,7 +574,12 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         fac = reference_factor(m_prev, m_new, sc.sl2);
         moved_row = m_prev != kNegInf;
       }
-      // this warpgroup's share of the row sum follows the reference (kWgs = 1: by the same factor)
+      // the row sum of this block's strand follows the reference (kWgs = 1: by the same factor)
+      if constexpr (kOwn == 2) {
+        const float2 strand = strands[128 * (li & 2)];
+        l_sum = strand.x;
+        m_ref = strand.y;
+      }
       if (m_new != m_ref) {
         l_sum *= kWgs == 1 ? fac : reference_factor(m_ref, m_new, sc.sl2);
         m_ref = m_new;
@@ -566,10 +607,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           }
           l_sum = fmaf(psum, __uint_as_float(ue[q] << 23), l_sum);
         }
+        if (kOwn == 2) strands[128 * (li & 2)] = make_float2(l_sum, m_ref);
         if (my_row < R) {   // rows past R stay zero (written once at set-up)
           // kR keys = kR / 2 bytes of the row's 64, inside one 16-byte chunk of the swizzled tile
           const uint32_t col = static_cast<uint32_t>(key_in_blk) >> 1;
-          uint8_t* dst = gbase + L::kOffP + slot * kQBytes + sw64_offset(my_row, col >> 4) + (col & 15);
+          uint8_t* dst = gbase + L::kOffP + slot * L::kQBytes + sw64_offset(my_row, col >> 4) + (col & 15);
           // scale byte of 16-key block blk = key_in_blk / 16: chunk blk / 4, the row's word, byte blk % 4
           uint8_t* sf_dst = gbase + L::kOffSFP + slot * 1024 + 512 * (key_in_blk >> 6) + my_row * 16 +
                             ((key_in_blk >> 4) & 3);
@@ -624,16 +666,29 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 
     // ---- epilogue: row sums over the 128 key lanes, then thread = dv lane of O^T --------------
     if (ok) {
-      float v = l_sum;   // this thread's share of its row; the lanes of one row are kR apart
+      // this thread's share of its row; the lanes of one row are kR apart
+      float v = l_sum;
 #pragma unroll
       for (int o = kR; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if constexpr (kOwn == 2) {
+        // the strand that is not the last block's (its index: that of the block before, two warpgroups ago)
+        const int c = (n + kWgs - 1 - wg) / kWgs;
+        const float2 other = strands[256 * (c & 1)];
+        float v_old = other.x;
+#pragma unroll
+        for (int o = kR; o < 32; o <<= 1) v_old += __shfl_xor_sync(0xffffffffu, v_old, o);
+        if (lane < kR) {
+          s_old[(wg * 5 + wq) * kN + lane] = v_old;
+          if (wq == 0) s_old[(wg * 5 + 4) * kN + lane] = other.y;
+        }
+      }
       // (the buffer of the exchange after the last one)
       volatile float* red = s_red + (((n + kWgs - 1 - wg) / kWgs) & 1) * (4 * kMaxRows);
       if (lane < kR) red[wq * kMaxRows + lane] = v;
-      if (kWgs == 2 && wg == 1) {
-        // the second warpgroup leaves its sums and their reference to the first and is done (the reference in this
+      if (kWgs > 1 && wg > 0) {
+        // the other warpgroups leave their sums and the references to the first and are done (the last reference in this
         // warp's own slot: what its last block handed on there, or -inf if it had none.  Another warp's slot
-        // may not have been read yet: a warp of the first warpgroup can be a block behind this one)
+        // may not have been read yet: a warp of the next warpgroup can be a block behind this one)
         if (wq == 0 && lane < kR) s_hand[(wg * 4 + wq) * kMaxRows + lane] = m_ref;
         mbar_arrive(bar(L::kFin));
       } else {
@@ -641,12 +696,32 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       }
     }
     if (ok && wg == 0) {
-      volatile float* red = s_red + (((n + kWgs - 1) / kWgs) & 1) * (4 * kMaxRows);
-      volatile float* red_b = s_red + 2 * 4 * kMaxRows + ((n / 2) & 1) * (4 * kMaxRows);
+      if (kWgs > 1) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kFin), 0, wc, kDFin));
+      // Per row, the lanes of a row alike: the sum over the warps in a fixed order (it does not depend on
+      // timing), brought to the last reference of the row; the factor of the output; the LSE
+      float scale = 0.f, lse = kNegInf;
+      if (ok) {
+        float m_s[kStrands], l_s[kStrands], m_fin = kNegInf, l_tot = 0.f;
+#pragma unroll
+        for (int i = 0; i < kStrands; ++i) {
+          // strand i is one of warpgroup w, which did c blocks: that of its last block, with the sums in the buffer of
+          // the exchange after the last one, or the other one
+          const int w = i % kWgs, c = (n + kWgs - 1 - w) / kWgs;
+          const bool last = kOwn == 1 || ((c + 1) & 1) == i / kWgs;
+          volatile float* sum = (last ? s_red + (2 * w + (c & 1)) * (4 * kN) : s_old + w * (5 * kN)) + my_row;
+          l_s[i] = ((sum[0] + sum[kN]) + sum[2 * kN]) + sum[3 * kN];
+          const float handed = s_hand[w * 4 * kN + my_row];
+          m_s[i] = !last ? s_old[(w * 5 + 4) * kN + my_row] : (w == 0 ? m_ref : handed);
+          m_fin = fmaxf(m_fin, m_s[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < kStrands; ++i) l_tot = fmaf(l_s[i], reference_factor(m_s[i], m_fin, sc.sl2), l_tot);
+        if (l_tot > 0.f && n > 0) scale = sc.out_scale / l_tot;
+        lse = finish_lse(m_fin, l_tot, sc.sl2);
+      }
       float o[kR];
 #pragma unroll
       for (int r = 0; r < kR; ++r) o[r] = 0.f;
-      if (kWgs == 2) ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kFin), 0, wc, kDFin));
       if (ok && n > 0) {
         ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kPvDone + ((n - 1) % kDepth)),
                                                ((n - 1) / kDepth) & 1, wc, kDPvDone));
@@ -657,29 +732,31 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         }
       }
       if (ok) {
+        // (kMerge: the K and V rings are free, every product has completed)
+        float* dst = reinterpret_cast<float*>(gbase + L::kOffK) + tid;
+        constexpr int step = 128;
+        if constexpr (!kMerge) {
+          // row r = s * group + (head in the group): the rows of one token are neighbours
+          dst = d.o_partial + ((((int64_t)split * p.B + b) * p.Sq) * p.Hq + hk * p.group) * 128 + tid;
+        }
+        int in_group = 0;
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
-          if (r < R) {
-            // fixed order over the warps: the sum of a row does not depend on timing
-            float l_tot = ((red[r] + red[kMaxRows + r]) + red[2 * kMaxRows + r]) + red[3 * kMaxRows + r];
-            float m_fin = __shfl_sync(0xffffffffu, m_ref, r);      // lane r of every warp owns row r
-            if (kWgs == 2) {
-              const float m_a = m_fin, m_b = s_hand[4 * kMaxRows + r];
-              m_fin = fmaxf(m_a, m_b);
-              const float l_b = ((red_b[r] + red_b[kMaxRows + r]) + red_b[2 * kMaxRows + r]) + red_b[3 * kMaxRows + r];
-              l_tot = l_tot * reference_factor(m_a, m_fin, sc.sl2) + l_b * reference_factor(m_b, m_fin, sc.sl2);
+          if (r < R) *dst = o[r] * __shfl_sync(0xffffffffu, scale, r);   // lane r of every warp owns row r
+          dst += step;
+          if constexpr (!kMerge) {
+            if (++in_group == p.group) {
+              in_group = 0;
+              dst += (int64_t)(p.Hq - p.group) * 128;
             }
-            const int s = r / p.group, h = hk * p.group + r % p.group;
-            const float scale = (l_tot > 0.f && n > 0) ? sc.out_scale / l_tot : 0.f;
-            const float lse = finish_lse(m_fin, l_tot, sc.sl2);
-            if constexpr (kMerge) {
-              // (the K ring is free: every product has completed)
-              reinterpret_cast<float*>(gbase + L::kOffK)[r * 128 + tid] = o[r] * scale;
-              if (tid == r) reinterpret_cast<float*>(gbase + L::kOffV)[r] = lse;
-            } else {
-              d.o_partial[((((int64_t)split * p.B + b) * p.Sq + s) * p.Hq + h) * 128 + tid] = o[r] * scale;
-              if (tid == r) d.lse_partial[(((int64_t)split * p.B + b) * p.Hq + h) * p.Sq + s] = lse;
-            }
+          }
+        }
+        if (tid < R) {
+          if constexpr (kMerge) {
+            reinterpret_cast<float*>(gbase + L::kOffV)[tid] = lse;
+          } else {
+            const int s = fast_div(tid, p.div_group), h = hk * p.group + tid - s * p.group;
+            d.lse_partial[(((int64_t)split * p.B + b) * p.Hq + h) * p.Sq + s] = lse;
           }
         }
       }
@@ -688,36 +765,48 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   }
 
   if constexpr (kMerge) {
-    // Merge (the arithmetic of combine_splits_kernel): row r by CTA r % splits, thread = dv.  A launch of
+    // Merge (the arithmetic of combine_splits_kernel): row r by CTA r % splits, a warp a row, four dv a lane.  A launch of
     // its own for it costs 2-3 us behind a kernel of 6.  Every thread of every CTA comes here, also
     // after a wait that ran out (then nothing is written).
     cluster_sync();
     if (warp < 4) {
       const uint32_t ns = d.num_splits;
-      uint32_t gave_up = 0;
-      for (uint32_t i = 0; i < ns; ++i) gave_up |= ld_cluster_u32(base + L::kOffMisc + 4, i);
-      for (int r = split; r < R && gave_up == 0; r += ns) {
-        float l[kMaxCluster], v[kMaxCluster], m = kNegInf;
+      const uint32_t gave_up = lane < ns ? ld_cluster_u32(base + L::kOffMisc + 4, lane) : 0u;
+      const bool whole = !__any_sync(0xffffffffu, gave_up != 0u);
+#pragma unroll 1
+      for (int r = split + warp * ns; r < R && whole; r += 4 * ns) {
+        float l[kMaxCluster], m = kNegInf;
+        float4 v[kMaxCluster];
 #pragma unroll
         for (uint32_t i = 0; i < kMaxCluster; ++i) {
-          l[i] = i < ns ? __uint_as_float(ld_cluster_u32(base + L::kOffV + 4 * r, i)) : kNegInf;
-          v[i] = i < ns ? __uint_as_float(ld_cluster_u32(base + L::kOffK + 4 * (r * 128 + tid), i)) : 0.f;
+          l[i] = kNegInf;
+          v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (i < ns) {
+            l[i] = __uint_as_float(ld_cluster_u32(base + L::kOffV + 4 * r, i));
+            v[i] = ld_cluster_f4(base + L::kOffK + 16 * (r * 32 + lane), i);
+          }
         }
 #pragma unroll
         for (int i = 0; i < kMaxCluster; ++i) m = fmaxf(m, l[i]);
-        float acc = 0.f, sum = 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        float sum = 0.f;
         if (m != kNegInf) {
 #pragma unroll
           for (int i = 0; i < kMaxCluster; ++i) {
             const float w = __expf(l[i] - m);
             sum += w;
-            acc = fmaf(w, v[i], acc);
+            acc.x = fmaf(w, v[i].x, acc.x);
+            acc.y = fmaf(w, v[i].y, acc.y);
+            acc.z = fmaf(w, v[i].z, acc.z);
+            acc.w = fmaf(w, v[i].w, acc.w);
           }
-          acc *= 1.f / sum;
+          const float inv = 1.f / sum;
+          acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
         }
-        const int s = r / p.group, h = hk * p.group + r % p.group;
-        p.out[b * p.o_stride_b + s * p.o_stride_s + h * p.o_stride_h + tid] = __float2bfloat16_rn(acc);
-        if (tid == 0 && p.lse != nullptr)
+        const int s = fast_div(r, p.div_group), h = hk * p.group + r - s * p.group;
+        *reinterpret_cast<uint2*>(p.out + b * p.o_stride_b + s * p.o_stride_s + h * p.o_stride_h + 4 * lane) =
+            make_uint2(pack_bf16x2(acc.x, acc.y), pack_bf16x2(acc.z, acc.w));
+        if (lane == 0 && p.lse != nullptr)
           p.lse[((int64_t)b * p.Hq + h) * p.Sq + s] = m == kNegInf ? kNegInf : m + __logf(sum);
       }
     }

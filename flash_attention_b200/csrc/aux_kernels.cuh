@@ -192,53 +192,59 @@ qk_tile_probe_kernel(const __grid_constant__ CUtensorMap tm_q,
 // Split-KV combine (the reference's flash_fwd_combine.py; math of
 // tests/cute/test_flash_attn_fast.py:295-300): per output row
 //   lse = log sum_i exp(lse_i),   out = sum_i exp(lse_i - lse) * out_i
-// over the splits' normalised fp32 partial outputs.  One thread = four neighbouring columns of
-// one (batch, query, head) row; HBM-bound: reads num_splits * (Dv + 1) floats, writes Dv bf16.
+// over the splits' normalised fp32 partial outputs.  A row by one warp (lane = four columns), or, above
+// kCombineBatch splits, by the four warps of the block, which take every fourth split each: all loads of a row
+// are then in flight at once, where batches one after the other cost a trip to L2 each.
+// It reads num_splits * (Dv + 1) floats a row, but behind a decode kernel of 10-30 us its own time is that of
+// its code, run once from cold instruction memory: short, no 64-bit division.  us per call, four columns a thread in
+// batches of eight splits with 64-bit index arithmetic -> this: 3 entries of 7301 keys, 37 splits 11.5 -> 7.5; 65536
+// keys, 37 splits 25.6 -> 19.4; 4 x 32768, 9 splits 33.0 -> 31.2.
 // ---------------------------------------------------------------------------------------------
-__global__ void combine_splits_kernel(const float* __restrict__ o_partial,
-                                      const float* __restrict__ lse_partial,
-                                      __nv_bfloat16* __restrict__ out, float* __restrict__ lse,
-                                      int num_splits, int B, int Sq, int Hq, int Dv,
-                                      int64_t o_stride_b, int64_t o_stride_s, int64_t o_stride_h) {
-  const int per_row = Dv / 4;
-  const int64_t rows = (int64_t)B * Sq * Hq;
-  const int64_t split_o = rows * Dv, split_l = rows;
+constexpr int kCombineWarps = 4, kCombineBatch = 8;
+__global__ void __launch_bounds__(kCombineWarps * 32)
+combine_splits_kernel(const float* __restrict__ o_partial, const float* __restrict__ lse_partial,
+                      __nv_bfloat16* __restrict__ out, float* __restrict__ lse, int num_splits, uint32_t rows,
+                      int warps_per_row, FastDiv div_hq, FastDiv div_sq, int Sq, int Hq, int Dv, int64_t o_stride_b,
+                      int64_t o_stride_s, int64_t o_stride_h) {
+  __shared__ float4 s_acc[kCombineWarps][32];
+  __shared__ float s_max[kCombineWarps], s_sum[kCombineWarps];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool alone = warps_per_row == 1;
+  const int first = alone ? 0 : warp, per_block = alone ? kCombineWarps : 1;
+  const bool mine = 4 * lane < Dv;
   pdl_wait();
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < rows * per_row;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(idx % per_row);
-    const int64_t r = idx / per_row;  // (b, s, h) in the partial layout
-    const int h = (int)(r % Hq);
-    const int64_t bs = r / Hq;
-    const int s = (int)(bs % Sq), b = (int)(bs / Sq);
+  for (uint32_t r0 = blockIdx.x * per_block; r0 < rows; r0 += gridDim.x * per_block) {
+    const uint32_t r = r0 + (alone ? warp : 0);      // (b, s, h) in the partial layout
+    const bool live = r < rows;
+    const int bs = fast_div((int)r, div_hq), h = (int)r - bs * Hq, b = fast_div(bs, div_sq), s = bs - b * Sq;
     const int64_t l_idx = ((int64_t)b * Hq + h) * Sq + s;
-    // loads in batches of eight, all in flight before the first is used: the partials come from L2
-    // (the kernel before wrote them) and a chain of dependent round trips would set the pace
-    constexpr int kBatch = 8;
-    float m = -INFINITY;
-    for (int i0 = 0; i0 < num_splits; i0 += kBatch) {
-      float l[kBatch];
-#pragma unroll
-      for (int j = 0; j < kBatch; ++j) l[j] = (i0 + j < num_splits) ? lse_partial[(i0 + j) * split_l + l_idx] : -INFINITY;
-#pragma unroll
-      for (int j = 0; j < kBatch; ++j) m = fmaxf(m, l[j]);
-    }
+    float m = -INFINITY, sum = 0.f;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    float sum = 0.f;
-    if (m != -INFINITY) {
-      for (int i0 = 0; i0 < num_splits; i0 += kBatch) {
-        float l[kBatch];
-        float4 v[kBatch];
+    if (live) {
+#pragma unroll 1
+      for (int i0 = first; i0 < num_splits; i0 += kCombineBatch * warps_per_row) {
+        float l[kCombineBatch], top = m;
+        float4 v[kCombineBatch];
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {
-          const bool live = i0 + j < num_splits;
-          l[j] = live ? lse_partial[(i0 + j) * split_l + l_idx] : -INFINITY;
-          v[j] = live ? *reinterpret_cast<const float4*>(o_partial + (i0 + j) * split_o + r * Dv + 4 * c)
-                      : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < kCombineBatch; ++j) {
+          const int i = i0 + j * warps_per_row;
+          l[j] = -INFINITY;
+          v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (i < num_splits) {
+            l[j] = lse_partial[(int64_t)i * rows + l_idx];
+            if (mine) v[j] = *reinterpret_cast<const float4*>(o_partial + ((int64_t)i * rows + r) * Dv + 4 * lane);
+          }
         }
 #pragma unroll
-        for (int j = 0; j < kBatch; ++j) {   // ascending split order, as before
-          const float w = __expf(l[j] - m);  // exp(-inf) = 0 for the padding of the last batch
+        for (int j = 0; j < kCombineBatch; ++j) top = fmaxf(top, l[j]);
+        if (top == -INFINITY) continue;
+        const float keep = __expf(m - top);    // (0 before the first split with a key)
+        sum *= keep;
+        acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+        m = top;
+#pragma unroll
+        for (int j = 0; j < kCombineBatch; ++j) {
+          const float w = __expf(l[j] - m);    // exp(-inf) = 0 past the last split
           sum += w;
           acc.x = fmaf(w, v[j].x, acc.x);
           acc.y = fmaf(w, v[j].y, acc.y);
@@ -246,15 +252,43 @@ __global__ void combine_splits_kernel(const float* __restrict__ o_partial,
           acc.w = fmaf(w, v[j].w, acc.w);
         }
       }
-      const float inv = 1.f / sum;
-      acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
     }
-    __nv_bfloat16* dst = out + b * o_stride_b + (int64_t)s * o_stride_s + h * o_stride_h + 4 * c;
-    uint2 pk;
-    pk.x = pack_bf16x2(acc.x, acc.y);
-    pk.y = pack_bf16x2(acc.z, acc.w);
-    *reinterpret_cast<uint2*>(dst) = pk;
-    if (c == 0 && lse != nullptr) lse[l_idx] = (m == -INFINITY) ? -INFINITY : m + __logf(sum);
+    if (!alone) {
+      s_acc[warp][lane] = acc;
+      if (lane == 0) {
+        s_max[warp] = m;
+        s_sum[warp] = sum;
+      }
+      __syncthreads();
+      if (warp == 0) {
+        const float m0 = m;
+#pragma unroll
+        for (int w = 1; w < kCombineWarps; ++w) m = fmaxf(m, s_max[w]);
+        if (m != -INFINITY) {
+          const float keep = __expf(m0 - m);
+          sum *= keep;
+          acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+#pragma unroll
+          for (int w = 1; w < kCombineWarps; ++w) {
+            const float f = __expf(s_max[w] - m);
+            const float4 a = s_acc[w][lane];
+            sum += f * s_sum[w];
+            acc.x = fmaf(f, a.x, acc.x);
+            acc.y = fmaf(f, a.y, acc.y);
+            acc.z = fmaf(f, a.z, acc.z);
+            acc.w = fmaf(f, a.w, acc.w);
+          }
+        }
+      }
+      __syncthreads();                         // (the slots are read out before the next row's)
+    }
+    if (live && (alone || warp == 0)) {
+      const float inv = m == -INFINITY ? 0.f : 1.f / sum;
+      if (mine)
+        *reinterpret_cast<uint2*>(out + b * o_stride_b + (int64_t)s * o_stride_s + h * o_stride_h + 4 * lane) =
+            make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
+      if (lane == 0 && lse != nullptr) lse[l_idx] = m == -INFINITY ? -INFINITY : m + __logf(sum);
+    }
   }
 }
 
