@@ -842,7 +842,10 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         scale = (l_tot > 0.f) ? sc.out_scale / l_tot : 0.f;
       }
       // warpgroup k stores output columns [32 k, 32 k + 32); with kD = 64 two of them only arrive
-      if (kGeneral && p.num_splits > 1 && (kD == 128 || wg < kD / 32)) {
+      if (kGeneral && p.num_splits > 1 && kD != 128 && wg >= kD / 32) {
+        // (without the staging tile's barriers: no store warp answers them on this path)
+        stage_accumulator_chunk<false>(0u, gbase + kOffOut, row, wg, 0.f, n > 0 ? bars.at(Bars::kOFree) : 0u);
+      } else if (kGeneral && p.num_splits > 1) {
         // (merged in the cluster: into the K and V rings, which are free -- every product has completed)
         float* prow = p.merge_splits
                           ? reinterpret_cast<float*>(gbase + kOffK) + row * kD

@@ -147,3 +147,21 @@ def test_split_calls_replay_from_a_cuda_graph(cuda_device, Sq, Sk, splits):
     torch.cuda.synchronize()
     fa.check_status(cuda_device)
     assert torch.equal(out, second[0]) and torch.equal(lse, second[1])
+
+
+def _attend(Q, K, V, **kw):
+    out, lse = fa.flash_attn_fp4_func(Q.data, K.data, V.data, Q.sf, K.sf, V.sf, Q.scale, K.scale, V.scale, return_lse=True, **kw)
+    torch.cuda.synchronize()
+    fa.check_status(Q.data.device)
+    return out, lse
+
+
+@pytest.mark.parametrize("B,Sq,Sk,Hq,D,splits", [(1, 3, 1300, 3, 64, 9), (1, 130, 1300, 2, 64, 10), (2, 200, 700, 40, 64, 2),
+                                                 (1, 129, 1300, 3, 128, 11), (1, 5, 4200, 1, 128, 33)])
+def test_combine_by_one_and_by_four_warps(cuda_device, B, Sq, Sk, Hq, D, splits):
+    """Up to eight splits a row is a warp's, above it is four warps'; head dim 64 fills half a warp; 2 x 40 x 2 tiles
+    of two splits are more than are merged inside clusters."""
+    q, k, v = make_qkv(B, Sq, Sk, Hq, Hq, D, seed=13, device=cuda_device)
+    Q, K, V = fa.quantize_qkv_fused(q, k, v)
+    out, lse = _attend(Q, K, V, causal=True, num_splits=splits, variant=fa.VARIANT_WS)
+    assert_parity(out, lse, *oracles(Q, K, V, True, num_splits=splits, variant=fa.VARIANT_WS))
