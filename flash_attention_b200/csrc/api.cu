@@ -618,26 +618,24 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
       // Hq=32, Hkv=8, causal, wide form / narrow form, D = 64 and 128: 128 keys 59/50, 65/59; 256 keys 74/61,
       // 77/72; 384 keys 71/69, 73/77; 512 keys 82/82, 83/89.
       const bool narrow = win_left >= 0 && win_right >= 0 && (int64_t)win_left + win_right <= 256;
-      if (general && local && narrow) {
-        rc = p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, true, true, true, true>)
-                         : (p->D == 64 ? launch64(attn_fwd_ws64_kernel<64, true, true, true, true>)
-                                       : launch64(attn_fwd_ws64_kernel<192, true, true, true, true>));
-      } else if (general && local) {   // window (with or without sink / softcap / cache view)
-        rc = p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, true>)
-                         : (p->D == 64 ? launch64(attn_fwd_ws64_kernel<64, true>)
-                                       : launch64(attn_fwd_ws64_kernel<192, true>));
-      } else if (general && cached) {   // KV-cache view without a window
-        rc = p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, true, false, true>)
-                         : (p->D == 64 ? launch64(attn_fwd_ws64_kernel<64, true, false, true>)
-                                       : launch64(attn_fwd_ws64_kernel<192, true, false, true>));
-      } else if (general) {     // sink / softcap only: plain tile geometry
-        rc = p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, true, false>)
-                         : (p->D == 64 ? launch64(attn_fwd_ws64_kernel<64, true, false>)
-                                       : launch64(attn_fwd_ws64_kernel<192, true, false>));
-      } else {
-        rc = p->D == 128 ? launch64(attn_fwd_ws64_kernel<128>)
-                         : (p->D == 64 ? launch64(attn_fwd_ws64_kernel<64>) : launch64(attn_fwd_ws64_kernel<192>));
-      }
+#define FA4_WS64(...)                                                                                     \
+  (p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, __VA_ARGS__>)                                        \
+               : (p->D == 64 ? launch64(attn_fwd_ws64_kernel<64, __VA_ARGS__>) : launch64(attn_fwd_ws64_kernel<192, __VA_ARGS__>)))
+      // The soft cap has its own instantiations: 64 tanh and selects in the middle of the loop are 6 KB of code, a
+      // fifth of what an SM's instruction cache holds (24 packed sequences up to 2048, no cap: 174 us with the code in
+      // the kernel, 168 without).
+      const bool cap = softcap > 0.f;
+      if (general && local && narrow)           // window (with or without sink / cache view)
+        rc = cap ? FA4_WS64(true, true, true, true, true) : FA4_WS64(true, true, true, true);
+      else if (general && local)
+        rc = cap ? FA4_WS64(true, true, true, false, true) : FA4_WS64(true);
+      else if (general && cached)               // KV-cache view without a window
+        rc = cap ? FA4_WS64(true, false, true, false, true) : FA4_WS64(true, false, true);
+      else if (general)                         // sink / soft cap only: plain tile geometry
+        rc = cap ? FA4_WS64(true, false, false, false, true) : FA4_WS64(true, false);
+      else
+        rc = FA4_WS64(false);
+#undef FA4_WS64
     } else if (p->D == 128) {
       rc = !general ? launch(attn_fwd_ws_kernel<128, false>)
                     : (local ? launch(attn_fwd_ws_kernel<128, true>)

@@ -156,6 +156,40 @@ def _attend(Q, K, V, **kw):
     return out, lse
 
 
+@pytest.mark.parametrize("D", [64, 128, 192])
+@pytest.mark.parametrize("Sq,Sk", [(300, 200), (130, 515), (64, 65), (257, 257), (97, 64)])
+def test_steps_in_which_a_warp_sees_no_key(cuda_device, Sq, Sk, D):
+    """The cache form leaves the work of such steps out, the plain one masks it: the same bits, also for rows that
+    see nothing at all (Sq > Sk)."""
+    q, k, v = make_qkv(2, max(Sq, Sk), max(Sq, Sk), 4, 2, D, seed=11, device=cuda_device)
+    Q, K, V = fa.quantize_qkv_fused(q[:, :Sq], k[:, :Sk], v[:, :Sk, :, :min(D, 128)])
+    plain = _attend(Q, K, V, causal=True, variant=fa.VARIANT_WS64)
+    used = torch.full((2,), Sk, dtype=torch.int32, device=cuda_device)
+    cached = _attend(Q, K, V, causal=True, variant=fa.VARIANT_WS64, seqused_k=used)
+    assert torch.equal(plain[0], cached[0]) and torch.equal(plain[1], cached[1])
+
+
+@pytest.mark.parametrize("D", [64, 128, 192])
+@pytest.mark.parametrize("window", [(None, None), (100, 0), (300, 0)], ids=["none", "narrow", "wide"])
+@pytest.mark.parametrize("used", [None, 333], ids=["dense", "cache"])
+def test_soft_cap_in_every_form(cuda_device, used, window, D):
+    """Bound: the hardware tanh moves a score by up to softcap log2(e) 2^-11 in the exponent, and with it P values
+    over rounding boundaries of the model (rel-RMS 0.05, as in the parity tests of the cap)."""
+    q, k, v = make_qkv(1, 400, 400, 4, 2, D, seed=12, device=cuda_device)
+    Q, K, V = fa.quantize_qkv_fused(q * 2.0, k * 2.0, v[..., :min(D, 128)])
+    kw = {} if used is None else {"seqused_k": torch.tensor([used], dtype=torch.int32, device=cuda_device)}
+    out, lse = _attend(Q, K, V, causal=True, softcap=2.0, window_size=window, **kw)
+    n = 400 if used is None else used
+    part = [Q, fa.NVFP4Tensor(K.data[:, :n], K.sf[:, :n], K.scale),
+            fa.NVFP4Tensor(V.data[..., :(n + 31) // 32 * 16], V.sf[..., :(n + 31) // 32 * 2], V.scale, is_v=True)]
+    oa, la, ob, lb = oracles(*part, True, softcap=2.0, window=window)
+    o = out.float().cpu()
+    assert torch.isfinite(o).all() and orc.error_metrics(o, ob)["rel_rms"] <= 0.05
+    assert torch.equal(torch.isinf(lse.cpu()), torch.isinf(la))
+    fin = torch.isfinite(la)
+    assert (lse.cpu()[fin] - la[fin]).abs().max().item() <= 2e-3 * max(1.0, la[fin].abs().max().item())
+
+
 @pytest.mark.parametrize("B,Sq,Sk,Hq,D,splits", [(1, 3, 1300, 3, 64, 9), (1, 130, 1300, 2, 64, 10), (2, 200, 700, 40, 64, 2),
                                                  (1, 129, 1300, 3, 128, 11), (1, 5, 4200, 1, 128, 33)])
 def test_combine_by_one_and_by_four_warps(cuda_device, B, Sq, Sk, Hq, D, splits):
