@@ -286,7 +286,8 @@ EXPORTS = ["fa4_nvfp4_fwd", "fa4_nvfp4_sf_linear_to_tiled", "fa4_nvfp4_query",
            "fa4_nvfp4_debug_ex2_rate", "fa4_nvfp4_fwd_varlen", "fa4_nvfp4_sf_linear_to_tiled_packed",
            "fa4_nvfp4_fwd_linear_sf_noalloc", "fa4_nvfp4_amax_bf16", "fa4_nvfp4_quantize_qk_bf16",
            "fa4_nvfp4_quantize_v_bf16", "fa4_nvfp4_splitkv_workspace_bytes", "fa4_nvfp4_fwd_splitkv",
-           "fa4_nvfp4_fwd_ex", "fa4_nvfp4_sf_tile_jobs", "fa4_nvfp4_quantize_jobs_bf16", "fa4_nvfp4_fwd_device_scales"]
+           "fa4_nvfp4_fwd_ex", "fa4_nvfp4_sf_tile_jobs", "fa4_nvfp4_quantize_jobs_bf16", "fa4_nvfp4_fwd_device_scales",
+           "fa4_nvfp4_fwd_decode_linear_sf"]
 
 
 def check(rc: int, what: str) -> None:

@@ -210,7 +210,7 @@ struct CacheView {
 };
 int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint64_t workspace_bytes,
                int win_left, int win_right, const float* sink, float softcap, const CacheView& cache,
-               void* cuda_stream, const float* const* scales = nullptr);
+               void* cuda_stream, const float* const* scales = nullptr, const fa4_nvfp4_linear_sf* linear = nullptr);
 }  // namespace
 
 extern "C" int fa4_nvfp4_fwd(const fa4_nvfp4_params* p, void* cuda_stream) {
@@ -218,7 +218,8 @@ extern "C" int fa4_nvfp4_fwd(const fa4_nvfp4_params* p, void* cuda_stream) {
 }
 
 namespace {
-int fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, const float* const* scales, void* cuda_stream) {
+int fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, const float* const* scales, void* cuda_stream,
+           const fa4_nvfp4_linear_sf* linear = nullptr) {
   if (x == nullptr) return -FA4_E_NULL;
   if (x->struct_size != sizeof(fa4_nvfp4_ext)) return -FA4_E_STRUCT;
   const int splits = x->num_splits == 0 ? 1 : x->num_splits;
@@ -237,7 +238,7 @@ int fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, const float* const
     cache.num_pages = x->num_pages;
   }
   return launch_fwd(p, splits, x->workspace, x->workspace_bytes, x->window_left, x->window_right,
-                    x->sink, x->softcap, cache, cuda_stream, scales);
+                    x->sink, x->softcap, cache, cuda_stream, scales, linear);
 }
 }  // namespace
 
@@ -252,6 +253,20 @@ extern "C" int fa4_nvfp4_fwd_device_scales(const fa4_nvfp4_params* p, const fa4_
   q.q_scale = q.k_scale = q.v_scale = 1.f;      // not read
   const float* const scales[3] = {q_scale, k_scale, v_scale};
   return fwd_ex(&q, x, scales, cuda_stream);
+}
+
+extern "C" int fa4_nvfp4_fwd_decode_linear_sf(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x,
+                                              const fa4_nvfp4_linear_sf* sf, void* cuda_stream) {
+  if (p == nullptr || sf == nullptr) return -FA4_E_NULL;
+  if (sf->struct_size != sizeof(fa4_nvfp4_linear_sf) || sf->reserved != 0u) return -FA4_E_STRUCT;
+  if (p->variant != FA4_VARIANT_DECODE) return -FA4_E_VARIANT;
+  if (sf->q_scale == nullptr && sf->k_scale == nullptr && sf->v_scale == nullptr)
+    return fwd_ex(p, x, nullptr, cuda_stream, sf);
+  if (!sf->q_scale || !sf->k_scale || !sf->v_scale) return -FA4_E_NULL;
+  fa4_nvfp4_params q = *p;
+  q.q_scale = q.k_scale = q.v_scale = 1.f;      // not read
+  const float* const scales[3] = {sf->q_scale, sf->k_scale, sf->v_scale};
+  return fwd_ex(&q, x, scales, cuda_stream, sf);
 }
 
 extern "C" int fa4_nvfp4_fwd_varlen(const fa4_nvfp4_params* p, const fa4_nvfp4_varlen* v, void* cuda_stream) {
@@ -430,10 +445,10 @@ int validate_fwd(const fa4_nvfp4_params* p, int num_splits, const void* workspac
 
 int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint64_t workspace_bytes,
                int win_left, int win_right, const float* sink, float softcap, const CacheView& cache,
-               void* cuda_stream, const float* const* scales) {
+               void* cuda_stream, const float* const* scales, const fa4_nvfp4_linear_sf* linear) {
   FwdPlan plan;
   if (int e = validate_fwd(p, num_splits, workspace, workspace_bytes, win_left, win_right, sink, softcap, cache,
-                           false, &plan))
+                           linear != nullptr, &plan))
     return e;
   const int variant = plan.variant;
   const bool decode = plan.decode, local = plan.local, general = plan.general, cached = plan.cached;
@@ -555,6 +570,13 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     dp.num_splits = num_splits;
     dp.o_partial = kp.o_partial;
     dp.lse_partial = kp.lse_partial;
+    dp.lin = LinearScales{};
+    if (linear != nullptr) {
+      const int rows = cache.page_table ? cache.page_size : p->Sk;
+      dp.lin = LinearScales{kp.q_sf, kp.k_sf, kp.v_sf, linear->q_stride_b, linear->q_stride_s, linear->q_stride_h,
+                            linear->k_stride_b, linear->k_stride_s, linear->k_stride_h, linear->v_stride_b,
+                            linear->v_stride_h, linear->v_stride_d, rows, (rows + 31) / 32 * 2};
+    }
     const bool merge = decode_in_cluster(p, num_splits);
     auto launch_dec = [&](auto kernel, int threads, uint32_t smem) -> int {
       return launch_pdl_cluster(merge ? (unsigned)num_splits : 1u, kernel,
@@ -566,14 +588,17 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     // longest 8192: 23.9 -> 21.6 us).  Even lengths keep HBM busy with three tiles, and the room beside two
     // shallow CTAs lets the next call's start early (B=4, Sk=32768: 32.9 us shallow, 34.7 deep).
     const bool deep = cache.seqused_k != nullptr && p->B >= 4 && (int64_t)num_splits * p->Hkv * p->B <= 2 * kSms;
-#define FA4_DEC(rows, depth)                                                                             \
-  (merge ? launch_dec(attn_decode_kernel<rows, true, depth>, dec::threads_of(rows, depth), dec::form<rows, depth>::kRequest)          \
-         : launch_dec(attn_decode_kernel<rows, false, depth>, dec::threads_of(rows, depth), dec::form<rows, depth>::kRequest))
+#define FA4_DEC_FORM(rows, merge, depth, linear)                                                      \
+  launch_dec(attn_decode_kernel<rows, merge, depth, linear>, dec::threads_of(rows, depth), dec::form<rows, depth>::kRequest)
+#define FA4_DEC(rows, depth)                                                                            \
+  (linear != nullptr ? (merge ? FA4_DEC_FORM(rows, true, depth, true) : FA4_DEC_FORM(rows, false, depth, true)) \
+                     : (merge ? FA4_DEC_FORM(rows, true, depth, false) : FA4_DEC_FORM(rows, false, depth, false)))
     const int rc = dec_rows <= 4    ? (deep ? FA4_DEC(4, 5) : FA4_DEC(4, 3))
                    : dec_rows <= 8  ? (deep ? FA4_DEC(8, 5) : FA4_DEC(8, 3))
                    : dec_rows <= 16 ? (deep ? FA4_DEC(16, 5) : FA4_DEC(16, 3))
                                     : FA4_DEC(32, 5);
 #undef FA4_DEC
+#undef FA4_DEC_FORM
     if (rc != 0 || merge) return rc;
   } else {
     // persistent: one CTA per SM walks the tile list

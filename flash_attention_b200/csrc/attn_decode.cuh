@@ -213,6 +213,14 @@ __device__ __forceinline__ void block_exponent1(float bm, float m_ref, float sl2
 
 }  // namespace dec
 
+// Linear scale factors as a caller's cache holds them: q (B, Sq, Hq, 8), k (B, Sk, Hkv, 8), v (B, Hkv, 128, columns)
+// bytes, any strides in the outer dimensions and any alignment.
+struct LinearScales {
+  const uint8_t *q, *k, *v;
+  int64_t q_b, q_s, q_h, k_b, k_s, k_h, v_b, v_h, v_d;
+  int k_rows, v_cols;    // rows of k and columns of v of an entry (of a page)
+};
+
 struct DecodeParams {
   const uint8_t* q;      // (B, Sq, Hq, 64) packed e2m1
   const uint8_t* q_sf;   // tiled (B, Hq, ceil(Sq/128), 2, 512)
@@ -220,6 +228,7 @@ struct DecodeParams {
   int num_splits;
   float* o_partial;      // (splits, B, Sq, Hq, 128) fp32
   float* lse_partial;    // (splits, B, Hq, Sq) fp32
+  LinearScales lin;      // kLinear
 };
 
 // kR: query rows the softmax code is built for (4, 8, 16 or 32 >= Sq * group): the size of the
@@ -227,7 +236,11 @@ struct DecodeParams {
 // columns of an S^T buffer) is 16 up to sixteen rows and 32 above.
 // kMerge: the splits of a (kv head, batch entry) are one cluster, which merges their partials through
 // distributed shared memory and writes the result; otherwise they go to o_partial / lse_partial.
-template <int kR, bool kMerge, int kDepth>
+// kLinear: the scales come in the caller's linear layouts, and the producers put them into tiles on the way: a lane
+// reads the eight bytes of four rows, two blocks at a time and ahead of the ones it stores.  For short calls, of which
+// the launch that tiles the scales is a third; with many keys the reads, a 32-byte sector for eight bytes,
+// take longer than that launch (the line lies in host.cpp).
+template <int kR, bool kMerge, int kDepth, bool kLinear>
 __global__ void __launch_bounds__(dec::threads_of(kR, kDepth), kDepth == 3 ? 3 : 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const KernelParams p, const DecodeParams d) {
@@ -296,9 +309,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const int r = tid >> 1, ks = tid & 1;
     if (r < R) {
       const int s = fast_div(r, p.div_group), h = hk * p.group + r - s * p.group;
-      const uint8_t* chunk = d.q_sf + b * p.qsf_stride_b + h * p.qsf_stride_h + ((int64_t)(s / 128) * 2 + ks) * 512;
-      const int rr = s % 128;
-      qsf_pref = *reinterpret_cast<const uint32_t*>(chunk + (rr % 32) * 16 + (rr / 32) * 4);
+      if constexpr (kLinear) {
+        const uint8_t* src = d.lin.q + b * d.lin.q_b + s * d.lin.q_s + h * d.lin.q_h + 4 * ks;
+        qsf_pref = src[0] | (uint32_t)src[1] << 8 | (uint32_t)src[2] << 16 | (uint32_t)src[3] << 24;
+      } else {
+        const uint8_t* chunk = d.q_sf + b * p.qsf_stride_b + h * p.qsf_stride_h + ((int64_t)(s / 128) * 2 + ks) * 512;
+        const int rr = s % 128;
+        qsf_pref = *reinterpret_cast<const uint32_t*>(chunk + (rr % 32) * 16 + (rr / 32) * 4);
+      }
     }
   }
 
@@ -325,7 +343,42 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     return r;
   };
   int2 at = make_int2(0, 0);
-  if (warp == 4 || warp == 6) at = locate(0);
+  // kLinear: the scale words of blocks fetched, fetched + 1: rows l, l + 32, l + 64, l + 96 of lane l, three aligned words
+  // around the eight bytes of a row, which start `shift` bits into the first one (the same in the four rows, 32 strides
+  // apart).  Words without a byte of the tensor are not read.
+  uint32_t words[kLinear ? 2 : 1][4][3], shift[2] = {0u, 0u};
+  auto fetch = [&](int li0) {
+    if constexpr (kLinear) {
+      const bool is_k = warp == 4;
+      const int64_t row_stride = is_k ? d.lin.k_s : d.lin.v_d;
+      const uint8_t* head = is_k ? d.lin.k + hk * d.lin.k_h : d.lin.v + hk * d.lin.v_h;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int li = li0 + u;
+        const int kb = __shfl_sync(0xffffffffu, at.x, li & 31), nbl = __shfl_sync(0xffffffffu, at.y, li & 31);
+        if (li < n) {
+          const int left = is_k ? d.lin.k_rows - nbl * kBlockN : d.lin.v_cols - nbl * 8;   // rows, bytes of a row
+          const uint8_t* src = head + kb * (is_k ? d.lin.k_b : d.lin.v_b) + (is_k ? nbl * kBlockN * row_stride : nbl * 8) +
+                               lane * row_stride;
+          const uint32_t skew = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 3u);
+          const uint32_t end = skew + (is_k || left > 8 ? 8u : (uint32_t)left);
+          shift[u] = 8u * skew;
+          src -= skew;
+#pragma unroll
+          for (int c = 0; c < 4; ++c, src += 32 * row_stride) {
+            const bool row_ok = !is_k || c * 32 + lane < left;
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+              words[u][c][x] = row_ok && 4u * x < end ? *reinterpret_cast<const uint32_t*>(src + 4 * x) : 0u;
+          }
+        }
+      }
+    }
+  };
+  if (warp == 4 || warp == 6) {
+    at = locate(0);
+    if (kLinear) fetch(0);
+  }
   __syncthreads();
   tc_fence_after_sync();
   pdl_trigger();
@@ -350,26 +403,56 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     const uint32_t tile0 = base + (is_k ? L::kOffK : L::kOffV), sf0 = base + (is_k ? L::kOffSFK : L::kOffSFV);
     const uint8_t* sf_src = is_k ? p.k_sf + hk * p.ksf_stride_h : p.v_sf + hk * p.vsf_stride_h;
     const int64_t sf_stride_b = is_k ? p.ksf_stride_b : p.vsf_stride_b;
+    auto load_tile = [&](int st, int kb, int nbl) {
+      if (is_k) tma_load_4d(tile0 + st * kTileBytes, &tm_k, bar(full0 + st), 0, hk, nbl * kBlockN, kb);
+      else tma_load_4d(tile0 + st * kTileBytes, &tm_v, bar(full0 + st), nbl * (kBlockN / 2), 0, hk, kb);
+    };
     int li = 0;
     for (; li < n; ++li) {
-      if ((li & 31) == 0 && li > 0) at = locate(li);
+      if ((li & 31) == 0 && li > 0 && !kLinear) at = locate(li);
       const uint32_t st = li % kDepth;
       const int kb = __shfl_sync(0xffffffffu, at.x, li & 31), nbl = __shfl_sync(0xffffffffu, at.y, li & 31);
-      if (elect_one()) {
+      const bool lead = elect_one();
+      if (lead) {
         if (li >= kDepth) ok = mbar_wait(bar(free0 + st), ((li - kDepth) / kDepth) & 1, wc, is_k ? kDKFree : kDVFree);
         if (ok) {
-          mbar_arrive_expect_tx(bar(full0 + st), kTileBytes + kSfBytes);
-          if (is_k) {
-            tma_load_4d(tile0 + st * kTileBytes, &tm_k, bar(full0 + st), 0, hk, nbl * kBlockN, kb);
-          } else {
-            tma_load_4d(tile0 + st * kTileBytes, &tm_v, bar(full0 + st), nbl * (kBlockN / 2), 0, hk, kb);
-          }
-          bulk_load(sf0 + st * kSfBytes, sf_src + kb * sf_stride_b + (int64_t)nbl * kSfBytes, kSfBytes,
-                    bar(full0 + st));
+          if constexpr (kLinear) mbar_expect_tx(bar(full0 + st), kTileBytes);
+          else mbar_arrive_expect_tx(bar(full0 + st), kTileBytes + kSfBytes);
+          load_tile(st, kb, nbl);
+          if constexpr (!kLinear)
+            bulk_load(sf0 + st * kSfBytes, sf_src + kb * sf_stride_b + (int64_t)nbl * kSfBytes, kSfBytes, bar(full0 + st));
         }
       }
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
+      if constexpr (kLinear) {
+        // the stage is free (its leader waited): both chunks of the block, 16 bytes a lane; the tile's barrier
+        // completes with the copy and with this arrival
+        const int u = li & 1;
+        const int left = is_k ? 8 : d.lin.v_cols - nbl * 8;
+        uint32_t lo[4], hi[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t w0 = u ? words[1][c][0] : words[0][c][0], w1 = u ? words[1][c][1] : words[0][c][1],
+                         w2 = u ? words[1][c][2] : words[0][c][2], sh = u ? shift[1] : shift[0];
+          lo[c] = __funnelshift_r(w0, w1, sh);
+          hi[c] = __funnelshift_r(w1, w2, sh);
+          if (left < 8) {                       // (bytes past the row's end are zero)
+            lo[c] &= left < 4 ? (1u << (8 * left)) - 1u : 0xffffffffu;
+            hi[c] &= left <= 4 ? 0u : (1u << (8 * (left - 4))) - 1u;
+          }
+        }
+        uint8_t* dst = gbase + (is_k ? L::kOffSFK : L::kOffSFV) + st * kSfBytes + lane * 16;
+        *reinterpret_cast<uint4*>(dst) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<uint4*>(dst + 512) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lead) mbar_arrive(bar(full0 + st));
+        if (u == 1) {
+          if (((li + 1) & 31) == 0) at = locate(li + 1);
+          fetch(li + 1);
+        }
+      }
     }
     if (!ok && lane == 0) {
       // bounded drain: let the copies already issued (those of the blocks before li) land before the CTA's memory

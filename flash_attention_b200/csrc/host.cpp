@@ -301,6 +301,12 @@ int64_t prefill_splits(int64_t B, int64_t Sq, int64_t Sk, int64_t Hq, int64_t sm
   return best;
 }
 
+// Up to this many keys (times kv heads, over the batch) a decode call reads linear scales itself instead of having
+// them tiled by a launch of their own; the results are the same bits.  us, tiled first / read linear, 8 kv heads of 4
+// query heads, one token: 8192 keys 13.9 / 9.2, 4 x 4096 15.7 / 11.4, 16 x 1024 12.3 / 11.5, 32 x 512 11.4 / 10.3; but
+// 16 x 2048 16.9 / 20.3, 32 x 1024 15.9 / 17.6, 4 x 8192 17.2 / 17.1, 32 x 2048 23.8 / 30.9.
+constexpr int64_t kLinearKeys = 160 * 1024;
+
 int64_t sm_count(const at::Device& d) { return at::cuda::getDeviceProperties(d.index())->multiProcessorCount; }
 
 bool head_dims_built(int64_t D, int64_t Dv) {
@@ -431,8 +437,17 @@ void run(Call& c) {
   if (device.index() != c10::cuda::current_device()) guard.set_device(device);
   void* stream = c10::cuda::getCurrentCUDAStream(device.index()).stream();
 
+  const Window win = c.win;
+  const double softcap = c.softcap;
+  // A handful of query rows per kv head (decode, append): the transposed kernel, which always
+  // splits the keys over CTAs and merges with the combine kernel.
+  const bool decode_ok = D == 128 && Dv == 128 && Sq * (Hq / Hkv) <= 32 && win.left < 0 && win.right <= 0 &&
+                         !c.sink.defined() && softcap == 0.0;
+  const bool decode = c.variant == FA4_VARIANT_DECODE || (c.variant == FA4_VARIANT_AUTO && decode_ok);
+
   c10::DataPtr tiles;                     // scratch for tiled copies of linear scales
   const void* sf_ptr[3];
+  fa4_nvfp4_linear_sf linear = {};
   if (!c.tiled) {
     validate(q_sf, "q_sf", {B, Sq, Hq, D / 16}, at::kByte, device);
     validate(k_sf, "k_sf", {B_kv, Sk_kv, Hkv, D / 16}, at::kByte, device);
@@ -440,9 +455,19 @@ void run(Call& c) {
     q_sf = inner_contiguous(std::move(q_sf));
     k_sf = inner_contiguous(std::move(k_sf));
     v_sf = inner_contiguous(std::move(v_sf));
-    fa4_nvfp4_sf_job jobs[3] = {sf_job(q_sf, 1, 2, 1), sf_job(k_sf, 1, 2, 1), sf_job(v_sf, 2, 1, 2)};
-    tiles = tile_scales(jobs, stream);
-    for (int i = 0; i < 3; ++i) sf_ptr[i] = jobs[i].dst;
+    if (decode && decode_ok && B * Hkv * Sk <= kLinearKeys) {     // the decode kernel reads them as they are
+      linear.struct_size = sizeof linear;
+      linear.q_stride_b = q_sf.stride(0); linear.q_stride_s = q_sf.stride(1); linear.q_stride_h = q_sf.stride(2);
+      linear.k_stride_b = k_sf.stride(0); linear.k_stride_s = k_sf.stride(1); linear.k_stride_h = k_sf.stride(2);
+      linear.v_stride_b = v_sf.stride(0); linear.v_stride_h = v_sf.stride(1); linear.v_stride_d = v_sf.stride(2);
+      sf_ptr[0] = q_sf.data_ptr();
+      sf_ptr[1] = k_sf.data_ptr();
+      sf_ptr[2] = v_sf.data_ptr();
+    } else {
+      fa4_nvfp4_sf_job jobs[3] = {sf_job(q_sf, 1, 2, 1), sf_job(k_sf, 1, 2, 1), sf_job(v_sf, 2, 1, 2)};
+      tiles = tile_scales(jobs, stream);
+      for (int i = 0; i < 3; ++i) sf_ptr[i] = jobs[i].dst;
+    }
   } else {
     validate(q_sf, "q_sf", {B, Hq, cdiv(Sq, 128), D / 64, 512}, at::kByte, device);
     validate(k_sf, "k_sf", {B_kv, Hkv, cdiv(Sk_kv, 128), D / 64, 512}, at::kByte, device);
@@ -497,20 +522,13 @@ void run(Call& c) {
   long num_splits = c.num_splits;
   if (num_splits < 0 || num_splits > 128) fail(PyExc_ValueError, "num_splits must be in 0..128");
   const bool auto_splits = num_splits == 0;
-  const Window win = c.win;
   p.causal = win.causal ? 1 : 0;
-  const double softcap = c.softcap;
   if (!(softcap >= 0.0) || !std::isfinite(softcap)) fail(PyExc_ValueError, "softcap must be a finite number >= 0");
   const at::Tensor sink = sink_of(c.sink, Hq, device);
-  // A handful of query rows per kv head (decode, append): the transposed kernel, which always
-  // splits the keys over CTAs and merges with the combine kernel.
-  const bool decode_ok = D == 128 && Dv == 128 && Sq * (Hq / Hkv) <= 32 && win.left < 0 && win.right <= 0 &&
-                         !sink.defined() && softcap == 0.0;
   if (p.variant == FA4_VARIANT_DECODE && !decode_ok)
     fail(PyExc_NotImplementedError,
          "the decode kernel takes D = Dv = 128, Sq * (Hq / Hkv) <= 32, no window / sink / softcap");
-  if (p.variant == FA4_VARIANT_AUTO && decode_ok) p.variant = FA4_VARIANT_DECODE;
-  const bool decode = p.variant == FA4_VARIANT_DECODE;
+  if (decode) p.variant = FA4_VARIANT_DECODE;
   if (auto_splits)
     num_splits = decode ? decode_splits(B, Hkv, Sk, sm_count(device)) : prefill_splits(B, Sq, Sk, Hq, sm_count(device));
 
@@ -540,7 +558,10 @@ void run(Call& c) {
       x.workspace = workspace.get();
       x.workspace_bytes = (uint64_t)bytes;
     }
-    if (lazy)
+    if (linear.struct_size != 0) {
+      if (lazy) linear.q_scale = scales[0], linear.k_scale = scales[1], linear.v_scale = scales[2];
+      check_rc(fa4_nvfp4_fwd_decode_linear_sf(&p, &x, &linear, stream), "fa4_nvfp4_fwd_decode_linear_sf");
+    } else if (lazy)
       check_rc(fa4_nvfp4_fwd_device_scales(&p, &x, scales[0], scales[1], scales[2], stream), "fa4_nvfp4_fwd_device_scales");
     else
       check_rc(fa4_nvfp4_fwd_ex(&p, &x, stream), "fa4_nvfp4_fwd_ex");

@@ -203,6 +203,25 @@ int fa4_nvfp4_fwd_device_scales(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* 
                                 const float* k_scale, const float* v_scale, void* cuda_stream);
 
 /*
+ * fa4_nvfp4_fwd_ex of the decode kernel (p->variant FA4_VARIANT_DECODE) with LINEAR scale factors: p->q_sf
+ * (B, Sq, Hq, D/16), p->k_sf (B, Sk, Hkv, D/16) and p->v_sf (B, Hkv, Dv, Skp/16), Skp = Sk rounded up to a
+ * multiple of 32 (with a page table: per page of page_size keys), the last dimension contiguous, no
+ * alignment asked for.  One launch, no scratch for tiled copies; same bits as with tiled scales.
+ */
+typedef struct fa4_nvfp4_linear_sf {
+  uint32_t struct_size;     /* sizeof(fa4_nvfp4_linear_sf) */
+  uint32_t reserved;        /* 0 */
+  int64_t q_stride_b, q_stride_s, q_stride_h; /* bytes */
+  int64_t k_stride_b, k_stride_s, k_stride_h;
+  int64_t v_stride_b, v_stride_h, v_stride_d;
+  const float* q_scale;     /* all NULL, or the per-tensor scales in device memory */
+  const float* k_scale;     /* (see fa4_nvfp4_fwd_device_scales) */
+  const float* v_scale;
+} fa4_nvfp4_linear_sf;
+int fa4_nvfp4_fwd_decode_linear_sf(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, const fa4_nvfp4_linear_sf* sf,
+                                   void* cuda_stream);
+
+/*
  * Packed variable-length batches in ONE launch: the reference's flash_attn_varlen_func
  * (flash_attn/cute/interface.py:1795-1840; its persistent varlen scheduler is
  * flash_attn/cute/tile_scheduler.py:755-1087).  q, k, v, out of `p` have no batch dimension:

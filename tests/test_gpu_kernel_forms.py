@@ -199,3 +199,40 @@ def test_combine_by_one_and_by_four_warps(cuda_device, B, Sq, Sk, Hq, D, splits)
     Q, K, V = fa.quantize_qkv_fused(q, k, v)
     out, lse = _attend(Q, K, V, causal=True, num_splits=splits, variant=fa.VARIANT_WS)
     assert_parity(out, lse, *oracles(Q, K, V, True, num_splits=splits, variant=fa.VARIANT_WS))
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,splits,paged", [(1, 1, 1, 4, 1, 1, False), (1, 1, 777, 32, 8, 0, False), (2, 2, 800, 8, 2, 3, False),
+                                                         (1, 8, 4230, 8, 2, 1, False), (3, 1, 1000, 16, 1, 2, False),
+                                                         (5, 1, 700, 8, 2, 2, False), (2, 1, 33, 8, 8, 1, False),
+                                                         (2, 4, 768, 8, 2, 9, True), (1, 1, 9000, 4, 1, 2, True)])
+def test_decode_reads_linear_scales(cuda_device, B, Sq, Sk, Hq, Hkv, splits, paged, offset):
+    """The decode kernel's own reading of linear scales -- one key, ragged key counts (a row of V's scales is then 2 or 6
+    bytes more than a multiple of 8), more than 32 blocks a CTA, pages, every base alignment, outer strides with
+    holes -- against the tiled ones: the same bits."""
+    rows, slots = (B * -(-Sk // 256), 256) if paged else (B, Sk)
+    g = torch.Generator(device=cuda_device).manual_seed(14)
+    q, k, v = (torch.randn(b, S, H, 128, generator=g, device=cuda_device, dtype=torch.bfloat16)
+               for b, S, H in ((B, Sq, Hq), (rows, slots, Hkv), (rows, slots, Hkv)))
+    Q, K, V = fa.quantize_qkv_fused(q, k, v)
+
+    def moved(t):        # the same bytes `offset` into an allocation, a head more in the (possibly) strided dimension
+        wide = torch.full((*t.shape[:-2], t.shape[-2] + 1, t.shape[-1]), 0x7f, dtype=torch.uint8, device=cuda_device)
+        wide[..., :-1, :] = t
+        buf = torch.empty(wide.numel() + 8, dtype=torch.uint8, device=cuda_device)
+        at = buf[offset:offset + wide.numel()].view(wide.shape)
+        at.copy_(wide)
+        return at[..., :-1, :]
+
+    kw = {"causal": True, "num_splits": splits, "return_lse": True, "variant": fa.VARIANT_DECODE}
+    if paged:
+        kw["page_table"] = torch.randperm(rows, generator=g, device=cuda_device).to(torch.int32).view(B, -1)
+        kw["seqused_k"] = torch.full((B,), Sk, dtype=torch.int32, device=cuda_device)
+    elif B == 5:
+        kw["seqused_k"] = torch.tensor([0, 1, 700, 129, 300], dtype=torch.int32, device=cuda_device)
+    scales = (Q.scale, K.scale, V.scale)
+    want = fa.flash_attn_fp4_func(Q.data, K.data, V.data, *(t.tiled_sf() for t in (Q, K, V)), *scales, sf_layout="tiled", **kw)
+    got = fa.flash_attn_fp4_func(Q.data, K.data, V.data, *(moved(t.sf) for t in (Q, K, V)), *scales, sf_layout="linear", **kw)
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
