@@ -388,7 +388,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         const Tile t = decode_tile<kGeneral>(p, tile);
         const int n = t.n_blocks;
         if (n == 0) continue;
-        if (status_poisoned(p.status, p.epoch)) {
+        if (it > 0 && status_poisoned(p.status, p.epoch)) {
           *s_abort = 1u;  // another CTA failed: stop this one quickly
           break;
         }
@@ -411,9 +411,9 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
           nbl = nb;
           if constexpr (kGeneral) {
             if (p.page_table != nullptr) {
-              const int key0 = nb * kBlockN, pg = key0 / p.page_size;
+              const int pg = fast_div(nb, p.div_page);
               kb = p.page_table[(int64_t)t.b * p.pages_per_seq + pg];
-              nbl = (key0 - pg * p.page_size) / kBlockN;
+              nbl = nb - pg * (p.page_size / kBlockN);
             }
           }
         };
@@ -483,7 +483,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         const Tile t = decode_tile<kGeneral>(p, tile);
         const int n = t.n_blocks;
         if (n == 0) continue;
-        if (status_poisoned(p.status, p.epoch)) {
+        if (it > 0 && status_poisoned(p.status, p.epoch)) {
           *s_abort = 1u;  // another CTA failed: stop this one quickly
           break;
         }
@@ -536,7 +536,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         const Tile t = decode_tile<kGeneral>(p, tile);
         const int n = t.n_blocks;
         if (n == 0) continue;
-        if (status_poisoned(p.status, p.epoch)) {
+        if (it > 0 && status_poisoned(p.status, p.epoch)) {
           *s_abort = 1u;  // another CTA failed: stop this one quickly
           break;
         }
@@ -622,7 +622,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
       const Tile t = decode_tile<kGeneral>(p, tile);
       const int n = t.n_blocks;
       if (n == 0) continue;
-      if (status_poisoned(p.status, p.epoch)) {
+      if (it > 0 && status_poisoned(p.status, p.epoch)) {
           *s_abort = 1u;  // another CTA failed: stop this one quickly
           break;
         }
@@ -711,9 +711,7 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
     FA4_FOR_EACH_TILE {
       const Tile t = decode_tile<kGeneral>(p, tile);
       const int n = t.n_blocks;
-      const bool poisoned =
-          status_poisoned(p.status, p.epoch);
-      if (poisoned) {
+      if (it > 0 && status_poisoned(p.status, p.epoch)) {
         *s_abort = 1u;
         break;
       }
@@ -895,9 +893,9 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         {
           const Tile t = decode_tile<true>(p, cta);     // one work item per CTA; its split is its rank
           const uint32_t ns = p.num_splits;
-          uint32_t gave_up = 0;
-          for (uint32_t i = 0; i < ns; ++i) gave_up |= ld_cluster_u32(base + kOffMisc + 4, i);
-          for (uint32_t r = warp * ns + t.split; r < 128 && gave_up == 0; r += kStatsWarp0 * ns) {
+          const uint32_t gave_up = lane < ns ? ld_cluster_u32(base + kOffMisc + 4, lane) : 0u;
+          const bool whole = !__any_sync(0xffffffffu, gave_up != 0u);
+          for (uint32_t r = warp * ns + t.split; r < 128 && whole; r += kStatsWarp0 * ns) {
             const int q_idx = t.m_blk * kBlockM + r;
             if (q_idx >= p.Sq) break;
             const uint32_t o_addr = base + kOffK + r * (kD * 4) + ((lane ^ (r & (kD / 4 - 1))) << 4);

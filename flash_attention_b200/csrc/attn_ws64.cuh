@@ -350,7 +350,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     tmem_relinquish();
   }
   tc_fence_before_sync();
-  pdl_wait();
+  if constexpr (kWindow || kCache) pdl_wait();     // (their tiles depend on lengths in memory)
   // this CTA's tiles: p.tile_begin + tile_of_round(0), (1), ... below tile_end
   int tile_end = p.tile_end;
   {
@@ -367,6 +367,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
     }
     if (tile < list_end) s_tiles[tid] = make_tile_rec<kWindow || kCache>(p, tile);
   }
+  if constexpr (!(kWindow || kCache)) pdl_wait();
   __syncthreads();
   tc_fence_after_sync();
   pdl_trigger();
@@ -543,10 +544,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         int k0 = 0;      // first key of the sequence inside the packed tensor
         if (packed) k0 = !is_k && p.cu_seqlens_v != nullptr ? p.cu_seqlens_v[t.b] : p.cu_seqlens_k[t.b];
         if (is_k) {
-          if (status_poisoned(p.status, p.epoch)) {
+          if (it > 0 && status_poisoned(p.status, p.epoch)) {
             // another CTA of this launch failed: stop this one quickly.  Only this role polls the
-            // status word (a global load at every tile start); the others see the abort flag in
-            // their next wait, when the tiles stop coming
+            // status word (a global load at every tile start but the first, whose loads it would hold up by its
+            // latency); the others see the abort flag in their next wait, when the tiles stop coming
             *s_abort = 1u;
             break;
           }
