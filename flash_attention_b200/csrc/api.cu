@@ -585,8 +585,9 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     };
     // The deep form where several entries have lengths of their own and no third CTA per SM waits: the long entries
     // then run on with few CTAs beside them, bound by the latency of their loads (paged batch of 16,
-    // longest 8192: 23.9 -> 21.6 us).  Even lengths keep HBM busy with three tiles, and the room beside two
-    // shallow CTAs lets the next call's start early (B=4, Sk=32768: 32.9 us shallow, 34.7 deep).
+    // longest 8192: 23.9 -> 21.6 us before its four warpgroups, 18.6 with them).  Even lengths keep HBM busy with three
+    // tiles, and the room beside two shallow CTAs lets the next call's start early (B=4, Sk=32768: 33.0 us shallow, 40.3
+    // deep).
     const bool deep = cache.seqused_k != nullptr && p->B >= 4 && (int64_t)num_splits * p->Hkv * p->B <= 2 * kSms;
 #define FA4_DEC_FORM(rows, merge, depth, linear)                                                      \
   launch_dec(attn_decode_kernel<rows, merge, depth, linear>, dec::threads_of(rows, depth), dec::form<rows, depth>::kRequest)
