@@ -260,6 +260,11 @@ extern "C" int fa4_nvfp4_fwd_decode_linear_sf(const fa4_nvfp4_params* p, const f
   if (p == nullptr || sf == nullptr) return -FA4_E_NULL;
   if (sf->struct_size != sizeof(fa4_nvfp4_linear_sf) || sf->reserved != 0u) return -FA4_E_STRUCT;
   if (p->variant != FA4_VARIANT_DECODE) return -FA4_E_VARIANT;
+  // the producers walk upwards from the pointers they are given, as for the data; 0 repeats a row
+  const int64_t strides[] = {sf->q_stride_b, sf->q_stride_s, sf->q_stride_h, sf->k_stride_b, sf->k_stride_s,
+                             sf->k_stride_h, sf->v_stride_b, sf->v_stride_h, sf->v_stride_d};
+  for (int64_t s : strides)
+    if (s < 0) return -FA4_E_STRIDE;
   if (sf->q_scale == nullptr && sf->k_scale == nullptr && sf->v_scale == nullptr)
     return fwd_ex(p, x, nullptr, cuda_stream, sf);
   if (!sf->q_scale || !sf->k_scale || !sf->v_scale) return -FA4_E_NULL;

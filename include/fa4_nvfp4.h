@@ -211,7 +211,7 @@ int fa4_nvfp4_fwd_device_scales(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* 
 typedef struct fa4_nvfp4_linear_sf {
   uint32_t struct_size;     /* sizeof(fa4_nvfp4_linear_sf) */
   uint32_t reserved;        /* 0 */
-  int64_t q_stride_b, q_stride_s, q_stride_h; /* bytes */
+  int64_t q_stride_b, q_stride_s, q_stride_h; /* bytes, >= 0 */
   int64_t k_stride_b, k_stride_s, k_stride_h;
   int64_t v_stride_b, v_stride_h, v_stride_d;
   const float* q_scale;     /* all NULL, or the per-tensor scales in device memory */

@@ -236,3 +236,22 @@ def test_decode_reads_linear_scales(cuda_device, B, Sq, Sk, Hq, Hkv, splits, pag
     torch.cuda.synchronize()
     fa.check_status(cuda_device)
     assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+def test_linear_decode_takes_device_scales_and_repeated_rows(cuda_device):
+    """Per-tensor scales that have not left the device, and one head's scales for all heads (stride 0)."""
+    q, k, v = make_qkv(2, 1, 700, 8, 2, 128, seed=15, device=cuda_device)
+    kw = {"causal": True, "return_lse": True}
+    known = fa.quantize_qkv_fused(q, k, v)
+    scales = tuple(t.scale for t in known)
+    data = [t.data for t in known]
+    Q, K, V = fa.quantize_qkv_fused(q, k, v)
+    want = fa.flash_attn_fp4_func(*data, *(t.sf for t in known), *scales, **kw)
+    got = fa.flash_attn_fp4_func(Q.data, K.data, V.data, Q.sf, K.sf, V.sf, Q._scale, K._scale, V._scale, **kw)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+    one = [Q.sf[:, :, :1].expand(-1, -1, 8, -1), K.sf[:, :, :1].expand(-1, -1, 2, -1), V.sf[:, :1].expand(-1, 2, -1, -1)]
+    want = fa.flash_attn_fp4_func(*data, *(t.contiguous() for t in one), *scales, **kw)
+    got = fa.flash_attn_fp4_func(*data, *one, *scales, **kw)
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])

@@ -318,6 +318,39 @@ def test_varlen_entry_point_checks_its_arguments_on_the_host():
     assert call(varlen()) == -5
 
 
+class _LinearSf(ctypes.Structure):
+    """Mirror of ``fa4_nvfp4_linear_sf``."""
+    _fields_ = [("struct_size", ctypes.c_uint32), ("reserved", ctypes.c_uint32)] + \
+               [(f"{t}_stride_{d}", ctypes.c_int64) for t, ds in (("q", "bsh"), ("k", "bsh"), ("v", "bhd")) for d in ds] + \
+               [(f"{t}_scale", ctypes.c_void_p) for t in "qkv"]
+
+
+@pytest.mark.parametrize("mutate,code", [
+    (lambda p, x, s: setattr(s, "struct_size", 8), 7),
+    (lambda p, x, s: setattr(s, "reserved", 1), 7),
+    (lambda p, x, s: setattr(p, "variant", 0), 5),                      # the decode kernel has to be named
+    (lambda p, x, s: setattr(p, "variant", 3), 5),
+    (lambda p, x, s: setattr(s, "k_scale", 0x1000), 1),                 # one scale on the device, two on the host
+    (lambda p, x, s: (setattr(s, "q_scale", 0x1000), setattr(s, "v_scale", 0x1000)), 1),
+    (lambda p, x, s: setattr(p, "k_sf", None), 1),
+    (lambda p, x, s: setattr(p, "Sq", 17), 2),                          # more query rows than the kernel holds
+    (lambda p, x, s: setattr(x, "window_left", 5), 2),
+] + [(lambda p, x, s, name=name: setattr(s, name, -8), 3) for name, _ in _LinearSf._fields_[2:11]])
+def test_decode_entry_for_linear_scales_checks_its_arguments_on_the_host(mutate, code):
+    """fa4_nvfp4_fwd_decode_linear_sf: every rejection comes before any CUDA call."""
+    L = fa.lib()
+    p, x, s = _good_params(), _lib.Ext(), _LinearSf()
+    p.Sq, p.variant = 1, 4
+    x.struct_size, x.num_splits, x.window_left, x.window_right = ctypes.sizeof(_lib.Ext), 1, -1, -1
+    s.struct_size = ctypes.sizeof(_LinearSf)
+    for name, _ in _LinearSf._fields_[2:11]:
+        setattr(s, name, 8)
+    call = lambda *a: L.fa4_nvfp4_fwd_decode_linear_sf(*(ctypes.byref(t) if t is not None else None for t in a), None)
+    assert call(None, x, s) == -1 and call(p, x, None) == -1 and call(p, None, s) == -1
+    mutate(p, x, s)
+    assert call(p, x, s) == -code
+
+
 def test_padded_key_offsets_of_a_packed_batch():
     cu = torch.tensor([0, 70, 199, 200, 533, 533], dtype=torch.int32)
     assert fa.padded_key_offsets(cu).tolist() == [0, 96, 256, 288, 640, 640]
