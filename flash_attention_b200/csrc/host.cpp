@@ -302,10 +302,30 @@ int64_t prefill_splits(int64_t B, int64_t Sq, int64_t Sk, int64_t Hq, int64_t sm
 }
 
 // Up to this many keys (times kv heads, over the batch) a decode call reads linear scales itself instead of having
-// them tiled by a launch of their own; the results are the same bits.  us, tiled first / read linear, 8 kv heads of 4
-// query heads, one token: 8192 keys 13.9 / 9.2, 4 x 4096 15.7 / 11.4, 16 x 1024 12.3 / 11.5, 32 x 512 11.4 / 10.3; but
-// 16 x 2048 16.9 / 20.3, 32 x 1024 15.9 / 17.6, 4 x 8192 17.2 / 17.1, 32 x 2048 23.8 / 30.9.
-constexpr int64_t kLinearKeys = 160 * 1024;
+// them tiled by a launch of their own; the results are the same bits.  A lane fetches the eight bytes of a row, 32
+// bytes of a sector, so the line depends on how far apart the rows of K are (`row_stride` bytes; V's, whose
+// neighbouring blocks share the sector, cost the same in every shape):
+//  * up to 16 bytes (one or two kv heads) two to four rows share a sector and reading is faster at any length -- but
+//    for five to eight query rows, whose instantiations have no registers to spare (`tight`);
+//  * from 256 bytes on (32 kv heads; `tight`: 128) the line is 128 k keys, between those 160 k.
+// Tiling goes over the whole of a page pool, reading only over the pages in use: a pool of two or three times the keys
+// of the table (`pool_ratio`) moves the line fourfold each time, beyond that reading is always faster.
+// us, tiled first / read linear, one token, inputs from HBM (kv heads x query heads each):
+//   8 x 4, 160 k keys x heads as 1, 4, 16, 32 entries 15.1 / 14.4, 14.7 / 13.9, 15.1 / 14.4, 14.0 / 13.1; 256 k 17.6 /
+//     17.1, 17.3 / 17.2, 17.1 / 20.4, 16.0 / 17.6; 1 M 43.5 / 43.7, 43.3 / 44.0, 42.8 / 54.6, 42.2 / 54.9
+//   32 x 1, 128 k, 1, 4, 16 entries 13.5 / 13.1, 13.8 / 13.6, 15.7 / 16.2, 160 k 14.6 / 14.7, 15.1 / 15.7, 18.0 / 18.3
+//   16 x 1, 8 tokens, 128 k, 1, 8, 32 entries 15.1 / 15.8, 14.7 / 14.3, 17.4 / 17.8, 160 k 16.6 / 18.1, 15.9 / 16.7,
+//     19.8 / 19.9; 16 x 4, 4 tokens, 160 k 17.5 / 17.4, 17.0 / 17.3, 22.1 / 20.7
+//   2 x 4, 1 M, 4, 16, 32 entries 46.5 / 41.3, 46.1 / 41.7, 45.2 / 45.4; 1 x 16, 1 M, 8 entries 56.1 / 43.5
+//   1 x 8, 384 k, 4, 16, 32 entries 26.4 / 27.1, 27.8 / 28.3, 25.2 / 25.4; 2 x 8, 1 M, 8 entries 47.7 / 52.0
+//   pool of 2, 3 times the table, 8 x 4, 512 k 28.3 / 24.6, 32.9 / 24.7; 16 ragged entries 24.8 / 24.0, 28.2 / 23.8;
+//     1 M 39.7 / 43.6, 47.9 / 43.8; of 16 times, 1 x 8, 256 k 122 / 19
+int64_t linear_keys_limit(int64_t rows, int64_t row_stride, int64_t pool_ratio) {
+  const bool tight = rows > 4 && rows <= 8;
+  if (pool_ratio > 3 || (row_stride <= 16 && !tight)) return INT64_MAX;
+  const int64_t line = row_stride >= (tight ? 128 : 256) ? 128 * 1024 : 160 * 1024;
+  return line << (2 * (std::max<int64_t>(pool_ratio, 1) - 1));
+}
 
 int64_t sm_count(const at::Device& d) { return at::cuda::getDeviceProperties(d.index())->multiProcessorCount; }
 
@@ -455,7 +475,9 @@ void run(Call& c) {
     q_sf = inner_contiguous(std::move(q_sf));
     k_sf = inner_contiguous(std::move(k_sf));
     v_sf = inner_contiguous(std::move(v_sf));
-    if (decode && decode_ok && B * Hkv * Sk <= kLinearKeys) {     // the decode kernel reads them as they are
+    const int64_t pool_ratio = paged ? B_kv * Sk_kv / std::max<int64_t>(1, B * Sk) : 1;
+    if (decode && decode_ok && B * Hkv * Sk <= linear_keys_limit(Sq * (Hq / Hkv), k_sf.stride(1), pool_ratio)) {
+      // the decode kernel reads them as they are
       linear.struct_size = sizeof linear;
       linear.q_stride_b = q_sf.stride(0); linear.q_stride_s = q_sf.stride(1); linear.q_stride_h = q_sf.stride(2);
       linear.k_stride_b = k_sf.stride(0); linear.k_stride_s = k_sf.stride(1); linear.k_stride_h = k_sf.stride(2);
@@ -952,6 +974,9 @@ PyObject* choose_num_splits(PyObject* const* a) {
   return PyLong_FromLongLong(
       prefill_splits(integer_of(a[0]), integer_of(a[1]), integer_of(a[2]), integer_of(a[3]), integer_of(a[4])));
 }
+PyObject* choose_linear_keys(PyObject* const* a) {
+  return PyLong_FromLongLong(linear_keys_limit(integer_of(a[0]), integer_of(a[1]), integer_of(a[2])));
+}
 PyObject* window_of(PyObject* const* a) {
   const Window w = resolve_window(truth_of(a[0]), a[1], a[2]);
   PyObject *t = w.causal ? Py_True : Py_False, *l = w.left < 0 ? nullptr : PyLong_FromLong(w.left),
@@ -999,6 +1024,7 @@ PyMethodDef methods[] = {method<fwd, 23>("fwd"),
                          method<varlen_fwd, 22>("varlen_fwd"),
                          method<choose_decode_splits, 4>("choose_decode_splits"),
                          method<choose_num_splits, 5>("choose_num_splits"),
+                         method<choose_linear_keys, 3>("choose_linear_keys"),
                          method<quantize_qkv, 4>("quantize_qkv"),
                          method<host_pieces, 25>("host_pieces"),
                          method<window_of, 3>("resolve_window"),

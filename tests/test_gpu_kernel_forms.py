@@ -205,10 +205,11 @@ def test_combine_by_one_and_by_four_warps(cuda_device, B, Sq, Sk, Hq, D, splits)
 @pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,splits,paged", [(1, 1, 1, 4, 1, 1, False), (1, 1, 777, 32, 8, 0, False), (2, 2, 800, 8, 2, 3, False),
                                                          (1, 8, 4230, 8, 2, 1, False), (3, 1, 1000, 16, 1, 2, False),
                                                          (5, 1, 700, 8, 2, 2, False), (2, 1, 33, 8, 8, 1, False),
-                                                         (2, 4, 768, 8, 2, 9, True), (1, 1, 9000, 4, 1, 2, True)])
+                                                         (2, 4, 768, 8, 2, 9, True), (1, 1, 9000, 4, 1, 2, True),
+                                                         (1, 1, 170001, 16, 1, 0, False), (1, 1, 270080, 4, 1, 9, True)])
 def test_decode_reads_linear_scales(cuda_device, B, Sq, Sk, Hq, Hkv, splits, paged, offset):
     """The decode kernel's own reading of linear scales -- one key, ragged key counts (a row of V's scales is then 2 or 6
-    bytes more than a multiple of 8), more than 32 blocks a CTA, pages, every base alignment, outer strides with
+    bytes more than a multiple of 8), more than 32 blocks a CTA, keys past the general line, pages, every base alignment, outer strides with
     holes -- against the tiled ones: the same bits."""
     rows, slots = (B * -(-Sk // 256), 256) if paged else (B, Sk)
     g = torch.Generator(device=cuda_device).manual_seed(14)
@@ -252,6 +253,35 @@ def test_linear_decode_takes_device_scales_and_repeated_rows(cuda_device):
     one = [Q.sf[:, :, :1].expand(-1, -1, 8, -1), K.sf[:, :, :1].expand(-1, -1, 2, -1), V.sf[:, :1].expand(-1, 2, -1, -1)]
     want = fa.flash_attn_fp4_func(*data, *(t.contiguous() for t in one), *scales, **kw)
     got = fa.flash_attn_fp4_func(*data, *one, *scales, **kw)
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+@pytest.mark.parametrize("spare", [0, 3, 37], ids=["full", "line_moved", "no_line"])
+def test_decode_from_a_pool_larger_than_the_table(cuda_device, spare):
+    """Linear scales of a pool that other sequences share: the pages in use are read where they are, or the whole pool
+    is tiled; either way the bits of the entry in a pool of its own."""
+    rows, B, Sk = 12, 2, 6 * 256
+    g = torch.Generator(device=cuda_device).manual_seed(16)
+    q, k, v = (torch.randn(b, S, H, 128, generator=g, device=cuda_device, dtype=torch.bfloat16)
+               for b, S, H in ((B, 1, 8), (rows, 256, 2), (rows, 256, 2)))
+    Q, K, V = fa.quantize_qkv_fused(q, k, v)
+    table = torch.randperm(rows, generator=g, device=cuda_device).view(B, -1)
+    used = torch.tensor([Sk, 700], dtype=torch.int32, device=cuda_device)
+    at = torch.randperm(rows + spare, generator=g, device=cuda_device)[:rows]       # where the pages went
+
+    def pool(t):
+        other = torch.full((rows + spare, *t.shape[1:]), 0x7f, dtype=torch.uint8, device=cuda_device)   # NaN scales
+        other[at] = t
+        return other
+
+    def run(ops, where):
+        return fa.flash_attn_fp4_func(Q.data, ops[0], ops[1], Q.sf, ops[2], ops[3], Q.scale, K.scale, V.scale, causal=True,
+                                      return_lse=True, seqused_k=used, page_table=where.to(torch.int32).contiguous())
+
+    ops = (K.data, V.data, K.sf, V.sf)
+    want, got = run(ops, table), run([pool(t) for t in ops], at[table])
     torch.cuda.synchronize()
     fa.check_status(cuda_device)
     assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])

@@ -230,6 +230,20 @@ def test_decode_split_choice_and_oracle_model_selection():
     assert kernel_model(128, rows=4, variant=2) == {"step_keys": 128, "ascending": False}
 
 
+def test_where_decode_reads_linear_scales_itself():
+    """The line in keys x kv heads: further out (or nowhere) where scale rows share sectors and where the pool that
+    would have to be tiled is larger than what the table covers."""
+    limit = _lib.host().choose_linear_keys                     # rows, bytes between K's scale rows, pool / table
+    assert limit(4, 64, 1) == limit(8, 64, 1) == limit(32, 32, 1) == 160 * 1024
+    assert limit(5, 128, 1) == limit(16, 256, 1) == limit(4, 256, 1) == 128 * 1024 and limit(9, 128, 1) == 160 * 1024
+    assert limit(4, 64, 0) == 160 * 1024                       # entries that share pages
+    assert limit(4, 64, 2) == 640 * 1024 and limit(4, 64, 3) == 2560 * 1024
+    forever = 2 ** 63 - 1
+    assert limit(4, 64, 4) == limit(8, 8, 100) == forever
+    assert [limit(rows, 16, 1) == forever for rows in (1, 4, 5, 8, 9, 32)] == [True, True, False, False, True, True]
+    assert limit(4, 24, 1) == 160 * 1024
+
+
 def test_oracle_split_model_matches_unsplit_statistics():
     from oracle import nvfp4_oracle as orc
     from tests.helpers import make_qkv, oracles
