@@ -682,11 +682,13 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
   }
   if ((num_splits > 1 || decode) && !merged) {
     // (fewer than 2^31 rows: the workspace holds at least 512 bytes of each)
-    const uint32_t rows = (uint32_t)p->B * p->Sq * p->Hq, per_block = num_splits > kCombineBatch ? 1u : kCombineWarps;
+    const uint32_t rows = (uint32_t)p->B * p->Sq * p->Hq;
+    const bool shared_rows = num_splits > kCombineBatch && rows <= kCombineSharedRows;
+    const uint32_t per_block = shared_rows ? 1u : kCombineWarps * 128u / (uint32_t)p->Dv;
     uint32_t blocks = (rows + per_block - 1) / per_block;
-    if (blocks > kSms * 16) blocks = kSms * 16;
+    if (blocks > kSms * kCombineBlocksPerSm) blocks = kSms * kCombineBlocksPerSm;
     return launch_pdl(combine_splits_kernel, dim3(blocks), kCombineWarps * 32, 0, stream, kp.o_partial, kp.lse_partial,
-                      kp.out, kp.lse, num_splits, rows, (int)(kCombineWarps / per_block), kp.div_hq,
+                      kp.out, kp.lse, num_splits, rows, shared_rows ? kCombineWarps : 1, kp.div_hq,
                       make_fastdiv((uint32_t)p->Sq), p->Sq, p->Hq, p->Dv, kp.o_stride_b, kp.o_stride_s, kp.o_stride_h);
   }
   return 0;

@@ -192,15 +192,24 @@ qk_tile_probe_kernel(const __grid_constant__ CUtensorMap tm_q,
 // Split-KV combine (the reference's flash_fwd_combine.py; math of
 // tests/cute/test_flash_attn_fast.py:295-300): per output row
 //   lse = log sum_i exp(lse_i),   out = sum_i exp(lse_i - lse) * out_i
-// over the splits' normalised fp32 partial outputs.  A row by one warp (lane = four columns), or, above
-// kCombineBatch splits, by the four warps of the block, which take every fourth split each: all loads of a row
-// are then in flight at once, where batches one after the other cost a trip to L2 each.
+// over the splits' normalised fp32 partial outputs.  A row by one warp, lane = four columns (head dim 64: by half
+// a warp); or, above kCombineBatch splits and up to kCombineSharedRows rows, by the four warps of the block, which take
+// every fourth split each: all loads of a row are then in flight at once, where batches one after the other
+// cost a trip to L2 each.  With more rows the warps of the other rows cover those trips (2048 rows are 14 warps an
+// SM), and a block a row only adds its two barriers.
 // It reads num_splits * (Dv + 1) floats a row, but behind a decode kernel of 10-30 us its own time is that of
 // its code, run once from cold instruction memory: short, no 64-bit division.  us per call, four columns a thread in
-// batches of eight splits with 64-bit index arithmetic -> this: 3 entries of 7301 keys, 37 splits 11.5 -> 7.5; 65536
-// keys, 37 splits 25.6 -> 19.4; 4 x 32768, 9 splits 33.0 -> 31.2.
+// batches of eight splits with 64-bit index arithmetic -> this: 3 entries of 7301 keys, 37 splits 22.7 -> 17.3; 65536
+// keys, 37 splits 25.8 -> 19.6; 4 x 32768, 9 splits 33.1 -> 31.5.
+// One warp a row / four, us per call, head dim 128 (64): 1024 rows of 9 splits 25.8 / 25.7 (23.5 / 23.6), 24 splits
+// 32.8 / 29.2 (28.5 / 25.0); 2048 rows of 9 splits 28.4 / 29.0 (25.9 / 26.7), 24 splits 42.7 / 41.3 (36.2 / 34.8);
+// 4096 rows of 9 splits 45.0 / 48.2 (40.5 / 43.6), 24 splits 72.3 / 73.8 (59.7 / 61.4); 131072 rows of 9 splits 513 /
+// 618 (340 / 496).  Head dim 64 in half warps instead of half-empty ones: 131072 rows of 2, 9 splits 184 -> 160,
+// 371 -> 340.  kCombineBlocksPerSm 16 -> 64: 131072 rows of 9, 24 splits 522 -> 513, 1175 -> 1153.  (With that many rows of
+// 16 and more splits the form before was 2-3 % faster: 796 -> 816 with 16, 1116 -> 1153 with 24.)
 // ---------------------------------------------------------------------------------------------
 constexpr int kCombineWarps = 4, kCombineBatch = 8;
+constexpr uint32_t kCombineSharedRows = 2048, kCombineBlocksPerSm = 64;
 __global__ void __launch_bounds__(kCombineWarps * 32)
 combine_splits_kernel(const float* __restrict__ o_partial, const float* __restrict__ lse_partial,
                       __nv_bfloat16* __restrict__ out, float* __restrict__ lse, int num_splits, uint32_t rows,
@@ -209,12 +218,15 @@ combine_splits_kernel(const float* __restrict__ o_partial, const float* __restri
   __shared__ float4 s_acc[kCombineWarps][32];
   __shared__ float s_max[kCombineWarps], s_sum[kCombineWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // lanes_per_row lanes have a row's columns: alone, both halves of a warp have a row each at head dim 64
   const bool alone = warps_per_row == 1;
-  const int first = alone ? 0 : warp, per_block = alone ? kCombineWarps : 1;
-  const bool mine = 4 * lane < Dv;
+  const int lanes_per_row = alone ? Dv / 4 : 32, rows_per_warp = 32 / lanes_per_row;
+  const int first = alone ? 0 : warp, per_block = alone ? kCombineWarps * rows_per_warp : 1;
+  const int row = alone ? warp * rows_per_warp + lane / lanes_per_row : 0, col = 4 * (lane & (lanes_per_row - 1));
+  const bool mine = col < Dv;
   pdl_wait();
   for (uint32_t r0 = blockIdx.x * per_block; r0 < rows; r0 += gridDim.x * per_block) {
-    const uint32_t r = r0 + (alone ? warp : 0);      // (b, s, h) in the partial layout
+    const uint32_t r = r0 + row;                       // (b, s, h) in the partial layout
     const bool live = r < rows;
     const int bs = fast_div((int)r, div_hq), h = (int)r - bs * Hq, b = fast_div(bs, div_sq), s = bs - b * Sq;
     const int64_t l_idx = ((int64_t)b * Hq + h) * Sq + s;
@@ -232,7 +244,7 @@ combine_splits_kernel(const float* __restrict__ o_partial, const float* __restri
           v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
           if (i < num_splits) {
             l[j] = lse_partial[(int64_t)i * rows + l_idx];
-            if (mine) v[j] = *reinterpret_cast<const float4*>(o_partial + ((int64_t)i * rows + r) * Dv + 4 * lane);
+            if (mine) v[j] = *reinterpret_cast<const float4*>(o_partial + ((int64_t)i * rows + r) * Dv + col);
           }
         }
 #pragma unroll
@@ -285,9 +297,9 @@ combine_splits_kernel(const float* __restrict__ o_partial, const float* __restri
     if (live && (alone || warp == 0)) {
       const float inv = m == -INFINITY ? 0.f : 1.f / sum;
       if (mine)
-        *reinterpret_cast<uint2*>(out + b * o_stride_b + (int64_t)s * o_stride_s + h * o_stride_h + 4 * lane) =
+        *reinterpret_cast<uint2*>(out + b * o_stride_b + (int64_t)s * o_stride_s + h * o_stride_h + col) =
             make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
-      if (lane == 0 && lse != nullptr) lse[l_idx] = m == -INFINITY ? -INFINITY : m + __logf(sum);
+      if (col == 0 && lse != nullptr) lse[l_idx] = m == -INFINITY ? -INFINITY : m + __logf(sum);
     }
   }
 }

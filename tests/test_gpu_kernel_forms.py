@@ -191,10 +191,11 @@ def test_soft_cap_in_every_form(cuda_device, used, window, D):
 
 
 @pytest.mark.parametrize("B,Sq,Sk,Hq,D,splits", [(1, 3, 1300, 3, 64, 9), (1, 130, 1300, 2, 64, 10), (2, 200, 700, 40, 64, 2),
-                                                 (1, 129, 1300, 3, 128, 11), (1, 5, 4200, 1, 128, 33)])
+                                                 (1, 129, 1300, 3, 128, 11), (1, 5, 4200, 1, 128, 33),
+                                                 (1, 2048, 1300, 1, 64, 9), (1, 2049, 1300, 1, 64, 9), (1, 683, 1300, 3, 128, 9)])
 def test_combine_by_one_and_by_four_warps(cuda_device, B, Sq, Sk, Hq, D, splits):
-    """Up to eight splits a row is a warp's, above it is four warps'; head dim 64 fills half a warp; 2 x 40 x 2 tiles
-    of two splits are more than are merged inside clusters."""
+    """Up to eight splits, or with more than 2048 rows, a row is a warp's, else it is four warps'; at head dim 64 two rows are
+    a warp's, the last of an odd number alone; 2 x 40 x 2 tiles of two splits are more than are merged inside clusters."""
     q, k, v = make_qkv(B, Sq, Sk, Hq, Hq, D, seed=13, device=cuda_device)
     Q, K, V = fa.quantize_qkv_fused(q, k, v)
     out, lse = _attend(Q, K, V, causal=True, num_splits=splits, variant=fa.VARIANT_WS)
