@@ -99,23 +99,26 @@ def test_scales_on_the_device_give_the_bits_of_scales_on_the_host(cuda_device):
         assert torch.equal(lazy[0], known[0]) and torch.equal(lazy[1], known[1]), kw
 
 
-@pytest.mark.parametrize("Sq", [1, 2, 4])
+@pytest.mark.parametrize("layout", ["linear", "tiled"])
+@pytest.mark.parametrize("Sq", [1, 2, 4, 8])
 @pytest.mark.parametrize("B,splits", [(8, 1), (8, 2), (8, 8), (8, 9), (8, 19), (120, 2)],
                          ids=["deep", "deep2", "deep8", "deep9combined", "shallow19", "clusters_do_not_fit"])
-def test_decode_ring_depths_and_merges(cuda_device, B, splits, Sq):
-    """Ragged entries with none, one, and odd and even numbers of key blocks (the two softmax warpgroups take
+def test_decode_ring_depths_and_merges(cuda_device, B, splits, Sq, layout):
+    """Ragged entries with none, one, and odd and even numbers of key blocks (the two or four softmax warpgroups take
     them in turn), in the deep ring (at least four entries, up to two CTAs an SM) and the shallow one, merged
-    inside a cluster (up to eight splits that fit at once) or by the combine kernel: the bits of the entry
-    alone, which runs the shallow ring, and the oracle's values."""
+    inside a cluster (up to eight splits that fit at once) or by the combine kernel, with 4, 8, 16 and 32 rows, from
+    scales that the kernel tiles itself and from tiled ones: the bits of the entry alone, which runs the shallow
+    ring, and the oracle's values."""
     lens = [0, 1, 128, 129, 300, 640, 641, 1500] * (B // 8)
     q, k, v = make_qkv(B, Sq, 1536, 8, 2, 128, seed=8, device=cuda_device)
     Q, K, V = fa.quantize_qkv_fused(q, k, v)
     used = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+    sf = [t.tiled_sf() if layout == "tiled" else t.sf for t in (Q, K, V)]
 
     def run(b0, b1):
-        return fa.flash_attn_fp4_func(*(t.data[b0:b1] for t in (Q, K, V)), *(t.sf[b0:b1] for t in (Q, K, V)), Q.scale,
+        return fa.flash_attn_fp4_func(*(t.data[b0:b1] for t in (Q, K, V)), *(t[b0:b1] for t in sf), Q.scale,
                                       K.scale, V.scale, causal=True, return_lse=True, seqused_k=used[b0:b1],
-                                      num_splits=splits)
+                                      num_splits=splits, sf_layout=layout)
 
     out, lse = run(0, B)
     torch.cuda.synchronize()
@@ -127,6 +130,43 @@ def test_decode_ring_depths_and_merges(cuda_device, B, splits, Sq):
     ops = [fa.NVFP4Tensor(Q.data[7:8], Q.sf[7:8], Q.scale), fa.NVFP4Tensor(K.data[7:8, :n], K.sf[7:8, :n], K.scale),
            fa.NVFP4Tensor(V.data[7:8, ..., :(n + 31) // 32 * 16], V.sf[7:8, ..., :(n + 31) // 32 * 2], V.scale, is_v=True)]
     assert_parity(out[7:8], lse[7:8], *oracles(*ops, True, num_splits=splits, variant=fa.VARIANT_DECODE))
+
+
+@pytest.mark.parametrize("Sq", [1, 2, 4, 8])
+@pytest.mark.parametrize("splits", [0, 1, 3, 9], ids=["chosen", "one", "cluster", "combine"])
+def test_decode_of_a_paged_batch_with_tiled_scales(cuda_device, splits, Sq):
+    """A serving cache: five entries of unequal lengths in a shuffled pool whose scales are kept tiled, 4 to 32 rows: the
+    bits of a contiguous cache, and every entry against the oracle on its own keys."""
+    lens, page, Sk = [700, 1, 1536, 129, 900], 256, 1536
+    B, pages = len(lens), Sk // 256
+    q, k, v = make_qkv(B, Sq, Sk, 8, 2, 128, seed=17, device=cuda_device)
+    Q, K, V = fa.quantize_qkv_fused(q, k, v)
+    used = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+    g = torch.Generator().manual_seed(18)
+    table = torch.randperm(B * pages + 2, generator=g)[:B * pages].reshape(B, pages)
+    pool = [torch.full((B * pages + 2, *shape), fill, dtype=torch.uint8, device=cuda_device)
+            for shape, fill in (((page, 2, 64), 0x77), ((2, 128, page // 2), 0x77), ((2, page // 128, 2, 512), 0x7f),
+                                ((2, 1, 2 * (page // 128), 512), 0x7f))]
+    for b in range(B):
+        for j in range(pages):
+            at, k0, t0 = int(table[b, j]), j * page, j * (page // 128)
+            pool[0][at] = K.data[b, k0:k0 + page]
+            pool[1][at] = V.data[b, ..., k0 // 2:(k0 + page) // 2]
+            pool[2][at] = K.tiled_sf()[b, :, t0:t0 + page // 128]
+            pool[3][at] = V.tiled_sf()[b, :, :, 2 * t0:2 * (t0 + page // 128)]
+    kw = {"causal": True, "return_lse": True, "seqused_k": used, "num_splits": splits, "sf_layout": "tiled"}
+    scales = (Q.scale, K.scale, V.scale)
+    out, lse = fa.flash_attn_fp4_func(Q.data, pool[0], pool[1], Q.tiled_sf(), pool[2], pool[3], *scales,
+                                      page_table=table.to(torch.int32).to(cuda_device), **kw)
+    flat = fa.flash_attn_fp4_func(Q.data, K.data, V.data, Q.tiled_sf(), K.tiled_sf(), V.tiled_sf(), *scales, **kw)
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    assert torch.equal(out, flat[0]) and torch.equal(lse, flat[1])
+    n_splits = splits or fa.interface.choose_decode_splits(B, 2, Sk, cuda_device)
+    for b, n in enumerate(lens):
+        ops = [fa.NVFP4Tensor(Q.data[b:b + 1], Q.sf[b:b + 1], Q.scale), fa.NVFP4Tensor(K.data[b:b + 1, :n], K.sf[b:b + 1, :n], K.scale),
+               fa.NVFP4Tensor(V.data[b:b + 1, ..., :(n + 31) // 32 * 16], V.sf[b:b + 1, ..., :(n + 31) // 32 * 2], V.scale, is_v=True)]
+        assert_parity(out[b:b + 1], lse[b:b + 1], *oracles(*ops, True, num_splits=n_splits, variant=fa.VARIANT_DECODE))
 
 
 @pytest.mark.parametrize("Sq,Sk,splits", [(1, 2048, 4), (1, 2048, 9), (100, 2048, 4), (100, 4096, 9)],

@@ -637,18 +637,20 @@ def test_softcap_parity(cuda_device, case):
     ("twenty_four_rows_of_thirty_two_noncausal", 1, 3, 700, 8, 1, False, 2),
     ("seventeen_rows_mha", 1, 17, 400, 2, 2, True, 1),
 ], ids=lambda c: c[0])
-def test_decode_kernel_parity(cuda_device, case):
+@pytest.mark.parametrize("layout", ["linear", "tiled"])
+def test_decode_kernel_parity(cuda_device, case, layout):
     """The transposed decode kernel (keys on the lanes, the Sq * Hq / Hkv <= 32 query rows of a kv
     head on the N side), which the automatic choice runs for these shapes: against the oracle's
     model of it (128-key steps upwards, contiguous shares of the blocks per split) at the usual
-    tolerances, and deterministic."""
+    tolerances, and deterministic; from linear scales, which it tiles itself, and from tiled ones."""
     _, B, Sq, Sk, Hq, Hkv, causal, splits = case
     q, k, v = make_qkv(B, Sq, Sk, Hq, Hkv, 128, seed=13, device=cuda_device)
     Q, K, V = fa.quantize_qkv(q, k, v)
-    out, lse = run(Q, K, V, causal, num_splits=splits)
+    ops = [fa.NVFP4Tensor(t.data, t.tiled_sf(), t.scale, tiled=True, is_v=t.is_v) for t in (Q, K, V)] if layout == "tiled" else (Q, K, V)
+    out, lse = run(*ops, causal, num_splits=splits)
     n = splits if splits else fa.interface.choose_decode_splits(B, Hkv, Sk, cuda_device)
     assert_parity(out, lse, *oracles(Q, K, V, causal, num_splits=n))
-    out2, lse2 = run(Q, K, V, causal, fa.VARIANT_DECODE, num_splits=splits)
+    out2, lse2 = run(*ops, causal, fa.VARIANT_DECODE, num_splits=splits)
     assert torch.equal(out, out2) and torch.equal(lse, lse2)
     # the prefill kernel on the same problem: another grouping of the same 4-bit P
     out_w, lse_w = run(Q, K, V, causal, fa.VARIANT_WS)
