@@ -646,8 +646,10 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
         return 0;
       };
       // Windows of up to two blocks' worth of keys run the narrow form of the kernel.  us at B=2, S=4096,
-      // Hq=32, Hkv=8, causal, wide form / narrow form, D = 64 and 128: 128 keys 59/50, 65/59; 256 keys 74/61,
-      // 77/72; 384 keys 71/69, 73/77; 512 keys 82/82, 83/89.
+      // Hq=32, Hkv=8, causal, wide form / narrow form, D = 128: 64 keys 51.7/45.4, 128 54.1/49.2, 192 57.5/57.8, 256
+      // 59.6/58.1, 288 67.6/68.2, 384 63.8/64.7, 512 72.7/74.1.  D = 64: 128 44.8/40.4, 256 51.4/49.6, 384 59.2/55.8, 512
+      // 68.0/66.0; D = 192: 57.2/50.7, 63.3/57.7, 65.2/61.2, 73.4/70.9 (there the narrow form is ahead beyond the line too,
+      // by 3-6 %).
       const bool narrow = win_left >= 0 && win_right >= 0 && (int64_t)win_left + win_right <= 256;
 #define FA4_WS64(...)                                                                                     \
   (p->D == 128 ? launch64(attn_fwd_ws64_kernel<128, __VA_ARGS__>)                                        \

@@ -50,6 +50,11 @@ namespace dec {
 // kDepth of each.  Three let THREE CTAs share an SM (70 KB of shared memory, 128 tensor-memory columns),
 // five let two (115 KB, 256 columns).  A CTA's loads are bound by their latency, kDepth x 18 KB per round
 // trip, so five are better whenever no third CTA is there to run.
+// (Registers: three CTAs of 384 threads leave 56, two of 640 leave 48, and up to eight rows the kernel wants more.  Bytes
+// of spill stores, merging / not: shallow 4 / 28, with linear scales 96 / 112-136; deep, four rows 48 / 84, 176 / 100;
+// eight rows 100 / 40, 212 / 136.  None above eight rows.  With them the deep form is still the faster one for ragged
+// batches, see softmax_wgs, and reading linear scales faster than a launch of its own, see linear_keys_limit in
+// host.cpp, whose line is nearer for five to eight rows.)
 constexpr int kMaxCluster = 8;  // splits that are merged inside a cluster (portable cluster size)
 constexpr int kMaxRows = 32; // query rows per kv head: Sq * group
 // Softmax warpgroups: one above eight rows; up to eight, two in the shallow form (registers: three CTAs of
@@ -465,8 +470,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
   } else if (warp == 5) {
     // ============================================ K . Q^T issuer ===============================
-    // (One thread that issued both products paced the kernel: the copies, products and commits of a
-    // block are fourteen tcgen05 instructions, about 100 clocks of issue each.)
+    // (One thread that issued both products paced the kernel while an issuing thread took 100 clocks for each of a
+    // block's fourteen copies, products and commits, see elect_one.  Two threads stay: the second product's waits would
+    // hold up the first.)
     if (elect_one() && n > 0) {
       ok = mbar_wait(bar(L::kQReady), 0, wc, kDQReady);
       uint64_t dq[2];

@@ -17,7 +17,7 @@
 //   warp 22     PV issuer: tcgen05.cp of the P/V scale factors and tcgen05.mma for O += P V
 //   warp 23     output store: sends the staged bf16 O tile of every query tile with TMA
 //
-// Why this shape (measured on B200, see the timeline facility below):
+// Why this shape (measured on B200):
 //  * The exponentials of a block cost 1024 clocks of the XU pipe per SM (16 ex2/clk), far more
 //    than its tensor-core time (256 clocks), so the kernel is organised around keeping the XU
 //    pipe busy.
@@ -28,8 +28,8 @@
 //    memory), roughly as long as the exponentials themselves.  Two warps per scheduler could not
 //    hide it; with the maxima gone a thread no longer needs the whole row in registers, so the
 //    row is split in two halves and four softmax warps per scheduler overlap each other.
-//  * One thread needs on the order of 100 clocks per tcgen05 instruction or barrier wait next to
-//    the busy softmax warps and a block needs 18 of them: two issuing threads.
+//  * A block needs 18 tcgen05 instructions and barrier waits, in two chains that wait for different
+//    things (K and a free S buffer; V, P and O): two issuing threads, so that neither holds up the other.
 //  * Prologue and epilogue of a tile (first loads, last PV, O to global memory) were a fifth of
 //    a tile's time: the CTA is persistent, the producer and the QK^T issuer run ahead into the
 //    next tile while the softmax warps finish the current one (Q is double buffered; only

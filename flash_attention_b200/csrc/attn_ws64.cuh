@@ -67,9 +67,11 @@ static_assert((kThreads / 128) * 32 * kRegsLaunch <= 16384, "register file of a 
 // tensor memory: S[4] x 64 columns, O 128, scale factors
 // (O at column 256 and Q scales at 384 as in the 128-key kernel); K and V scales have one slot of
 // columns per shared-memory stage, written by the issuer in front of the first product that reads it (one
-// thread, one pipe: no barrier.  By the loaders, with a barrier, while an issuing thread still took 100 clocks an
-// instruction; us, loaders -> issuers: 127-key window 81.5 -> 78.7, 24 packed sequences 174 -> 168, D = 192 111.6 ->
-// 110.4, causal GQA 1312 -> 1315)
+// thread, one pipe: no barrier).  us, copied by the loaders behind a barrier of their own -> by the issuers: 127-key
+// window 81.5 -> 78.7, 24 packed sequences 174 -> 168.  In the plain form, both measured on the same day: 54 sequences
+// of 300 45.5 -> 44.5 causal, 57.9 -> 55.6 not; 16 of 1024 62.3 -> 60.9; head dim 64, S = 16384 1277 -> 1270; but long tiles of
+// head dim 128 lose 0.1-0.2 % (causal GQA 1310.5 -> 1312.2, S = 32768 10094 -> 10110), for which a second way of
+// feeding the issuers is not kept.
 // (sized for head dim 192: three 64-element steps, 12 scale columns per Q / K tile)
 constexpr uint32_t kTmS64 = 0, kTmSFQ64 = 384 /* 12 */, kTmSFK64 = 396 /* 4 x 12 */, kTmSFV64 = 444 /* 4 x 8 */,
                    kTmSFP64 = 476 /* 4 x 4 */;
@@ -278,8 +280,8 @@ __device__ __forceinline__ uint32_t sw32_offset(uint32_t row, uint32_t chunk) {
 // steps.  Masks go to the scores in registers instead of through tensor memory, and the Q K^T issuer
 // waits for the P slot of a step before it issues the step's scores, one wait instead of 512.  Both
 // shorten the chain of a short tile and cost a long one: the branch sits in the hot loop, and Q K^T no
-// longer runs ahead of P V.  us, wide form -> this one: 127-key window, D = 64 114 -> 93; 1023 keys, D = 128
-// 143 -> 161.
+// longer runs ahead of P V.  us, wide form -> this one: 127-key window, D = 64 83.6 -> 75.1; 1023 keys, D = 128
+// 106.5 -> 108.5 (the line lies in api.cu).
 template <int kD, bool kGeneral = false, bool kWindow = kGeneral, bool kCache = kWindow, bool kNarrow = false,
           bool kCap = false>
 __global__ void __launch_bounds__(ws64::kThreads, 1)
@@ -765,9 +767,13 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         if constexpr (kWindow || kCache) {
           // None of the warp's 32 rows sees any of the 64 keys (the limits grow by one from row to row): P is zero, its
           // scales are the smallest, and the reference goes on as it came -- what the steps below would give.  A
-          // quarter of the steps of a 127-key window, an eighth of those of a one-block causal tile.  us: 127-key window
-          // 75.4 -> 72.4; 24 packed sequences up to 2048 173.2 -> 170.9.  (In the plain form, whose tiles are long, the
-          // code costs more than it saves: causal GQA 1313 -> 1327.)
+          // quarter of the steps of a 127-key window, an eighth of those of a one-block causal tile.  us, masked -> left
+          // out: 127-key window 75.4 -> 72.4; packed, 512 sequences of 128 242 -> 228, 64 of 512 175.0 -> 172.7, 4 of 8192
+          // 1397 -> 1398; S = 8192, windows of 512, 1024, 4096 keys 152 -> 143, 229 -> 219, 576 -> 565; a chunk of 2048
+          // against 32768 keys of a cache 746 -> 744.  Head dim 64 gains as much where tiles are short (143 -> 135, 217 -> 211;
+          // 256 packed of 128 100.5 -> 98.0) and loses 0.5-0.9 % where they are long (window of 4096 552 -> 555, the
+          // chunk 724 -> 728, 4 x 4096 through a cache 357 -> 359.5), one of 16384 keys 1.5 %.  (In the plain form, whose
+          // tiles are long, the code costs more than it saves: causal GQA 1313 -> 1327.)
           const int r0 = (warp & 3) * 32;
           if (cut && (upper_key<kWindow>(p, t, r0 + 31, nb) < 64 * h64 ||
                       (kWindow && lower_key(p, t, r0, nb) > 64 * h64 + 63))) {

@@ -55,12 +55,12 @@ __device__ __forceinline__ void report_status(const WaitCtx& w, uint32_t code, u
 // Exactly one lane of a converged warp, for the roles of one thread that issue copies and products.
 // Their operands (addresses, descriptors, coordinates, tensor-memory columns) are uniform-register operands of
 // the instructions.  Behind elect.sync the compiler knows that one thread runs the branch and keeps them
-// there; behind `lane == 0` it does not, and each such instruction paid for the way there: an issuer took about
-// 100 clocks an instruction, and its share of the scheduler's issue slots came out of the softmax warps'.  The
+// there; behind `lane == 0` it does not, and each such instruction paid for the way there: an issuer then takes
+// about 100 clocks an instruction, and its share of the scheduler's issue slots comes out of the softmax warps'.  The
 // warp's index goes through warp_index() for the same reason.
-// us, lane == 0 -> elected: causal GQA, S = 8192 1433 -> 1318; non-causal, S = 4096 715 -> 675; a 127-key
-// window, D = 64 90 -> 81; D = 192, S = 2048 123 -> 112; 24 packed sequences up to 2048 187 -> 178; split-KV,
-// 128 rows against 16384 keys 40.6 -> 39.0.
+// us, lane == 0 -> elected, the rest of the kernels as they are: causal GQA, S = 8192 1514 -> 1311; non-causal, S = 4096
+// 755 -> 670; S = 32768 12855 -> 10835; a 127-key window, D = 64 101 -> 74.5; D = 192, S = 2048 120 -> 110; 24 packed
+// sequences up to 2048 182 -> 166; split-KV, 128 rows against 16384 keys 45.0 -> 39.1.
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
 __device__ __forceinline__ bool elect_one() {
   uint32_t ok;
