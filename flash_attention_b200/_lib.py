@@ -209,6 +209,10 @@ def lib() -> ctypes.CDLL:
             L.fa4_nvfp4_fwd.restype = ctypes.c_int
             L.fa4_nvfp4_splitkv_workspace_bytes.argtypes = [ctypes.POINTER(Params), ctypes.c_int32]
             L.fa4_nvfp4_splitkv_workspace_bytes.restype = ctypes.c_int64
+            L.fa4_nvfp4_fwd_ex_workspace_bytes.argtypes = [ctypes.POINTER(Params), ctypes.POINTER(Ext)]
+            L.fa4_nvfp4_fwd_ex_workspace_bytes.restype = ctypes.c_int64
+            L.fa4_nvfp4_decode_is_balanced.argtypes = [ctypes.c_int32] * 5
+            L.fa4_nvfp4_decode_is_balanced.restype = ctypes.c_int
             L.fa4_nvfp4_fwd_splitkv.argtypes = [ctypes.POINTER(Params), ctypes.c_int32, ctypes.c_void_p,
                                                 ctypes.c_uint64, ctypes.c_void_p]
             L.fa4_nvfp4_fwd_splitkv.restype = ctypes.c_int
@@ -285,7 +289,8 @@ EXPORTS = ["fa4_nvfp4_fwd", "fa4_nvfp4_sf_linear_to_tiled", "fa4_nvfp4_query",
            "fa4_nvfp4_debug_qk_tile", "fa4_nvfp4_debug_wait_expiry", "fa4_nvfp4_debug_mma_rate",
            "fa4_nvfp4_debug_ex2_rate", "fa4_nvfp4_fwd_varlen", "fa4_nvfp4_sf_linear_to_tiled_packed",
            "fa4_nvfp4_fwd_linear_sf_noalloc", "fa4_nvfp4_amax_bf16", "fa4_nvfp4_quantize_qk_bf16",
-           "fa4_nvfp4_quantize_v_bf16", "fa4_nvfp4_splitkv_workspace_bytes", "fa4_nvfp4_fwd_splitkv",
+           "fa4_nvfp4_quantize_v_bf16", "fa4_nvfp4_splitkv_workspace_bytes", "fa4_nvfp4_fwd_ex_workspace_bytes",
+           "fa4_nvfp4_decode_is_balanced", "fa4_nvfp4_fwd_splitkv",
            "fa4_nvfp4_fwd_ex", "fa4_nvfp4_sf_tile_jobs", "fa4_nvfp4_quantize_jobs_bf16", "fa4_nvfp4_fwd_device_scales",
            "fa4_nvfp4_fwd_decode_linear_sf"]
 

@@ -10,6 +10,7 @@
 #include "quantize.cuh"
 
 #include <cudaTypedefs.h>
+#include <algorithm>
 #include <atomic>
 #include <map>
 #include <mutex>
@@ -193,6 +194,42 @@ bool decode_in_cluster(const fa4_nvfp4_params* p, int num_splits) {
   const int64_t resident = kSms * (p->Sq * (p->Hq / p->Hkv) <= 16 ? 3 : 2);
   return num_splits == 1 || (num_splits <= dec::kMaxCluster && ctas <= resident);
 }
+// The balanced form of a decode call (entries of unequal lengths, see balance() in attn_decode.cuh).
+constexpr int kSortedUnits = 200;       // units from which on entries come by length
+int balanced_slots(const fa4_nvfp4_params* p) { return (int)kSms * (p->Sq * (p->Hq / p->Hkv) <= 16 ? 3 : 2); }
+// One CTA a place and piece; or, with (nearly) as many units as places, what the units need and a quarter more to cut the
+// long ones.  (Half and a tenth as many more: 64 entries up to 8192 keys, 8 heads 41.3, 39.9 us, with a quarter 38.6.)
+int balanced_ctas(const fa4_nvfp4_params* p) {
+  const int units = p->B * p->Hkv, slots = balanced_slots(p);
+  return units + slots / 16 <= slots ? slots : units + slots / 4;
+}
+int64_t balanced_bytes(const fa4_nvfp4_params* p) {
+  // partial O and LSE of a CTA, then the table of pieces
+  const int64_t rows = (int64_t)balanced_ctas(p) * p->Sq * (p->Hq / p->Hkv);
+  return rows * 129 * 4 + 16 + (int64_t)p->B * p->Hkv * 8;
+}
+// Whether a decode call with key counts in memory is dealt by the lengths.  The host knows the longest possible length
+// alone.  Dealing costs 3 us (1.3 in front of the first load, the rest the second launch), so it takes that many blocks
+// (times kv heads, over the batch) for the unevenness to cost more.  us, splits of equal number / dealt, lengths
+// spread over the logarithm down to a 64th of the longest, GQA 4:
+//   one token, 2048 blocks: 5, 8, 16, 32 entries of 8 heads 9.5 / 10.6, 9.9 / 10.6, 8.8 / 9.3, 8.9 / 11.3; 4096: 14.4 / 14.5, 15.2 /
+//     14.8, 11.5 / 10.5, 11.2 / 11.7, 3 entries 17.1 / 18.9; 8192: 25.1 / 23.1, 21.0 / 16.6, 18.5 / 14.6, 20.0 / 15.8, 3
+//     entries 21.6 / 21.1, 48 entries 19.7 / 18.8, 64 entries (more units than places) 21.9 / 22.9; 16384: 38.7 / 34.6,
+//     39.9 / 30.3, 34.8 / 26.9, 33.8 / 23.3; 3, 48, 64 entries 36.4 / 33.0, 31.7 / 24.4, 29.6 / 30.3; 32768: 64 entries
+//     41.2 / 38.6; two entries never gain (16384: 43.1 / 43.4)
+//   32 heads, 8 entries, 4096, 8192, 32768 blocks 13.0 / 13.8, 20.8 / 17.3, 58.6 / 33.5; 24 entries 13.7 / 17.6, 17.5 / 21.8,
+//     38.5 / 36.5; 40 entries, 32768, 81920 41.2 / 49.8, 81 / 81
+//   four tokens (16 rows), 1024 blocks: 6, 16 entries 9.9 / 11.0, 9.7 / 10.9; 2048: 13.8 / 12.3, 12.4 / 10.5; 4096: 21.8 / 18.1,
+//     19.2 / 12.5; eight (32 rows): 1024: 16.4 / 13.6, 13.3 / 13.9; 2048: 18.3 / 16.2, 16.7 / 12.5; 4096: 30.4 / 23.8, 26.7 / 16.4
+// (Above eight rows a block takes one softmax warpgroup longer, so a long entry costs more.)
+bool decode_balanced(const fa4_nvfp4_params* p, const int32_t* seqused_k) {
+  if (seqused_k == nullptr || p->B < 3 || p->B > dec::kMaxBalanced || p->Sk > dec::kMaxBalancedKeys) return false;
+  const int64_t units = (int64_t)p->B * p->Hkv, blocks = units * ((p->Sk + kBlockN - 1) / kBlockN);
+  const int slots = balanced_slots(p);
+  if (units > 2 * slots || balanced_ctas(p) > dec::kMaxBalancedCtas || blocks > dec::kMaxBalancedBlocks) return false;
+  if (units > slots) return blocks >= 40 * units;
+  return blocks >= std::max<int64_t>(p->Sq * (p->Hq / p->Hkv) > 8 ? 2048 : (units < 40 ? 6144 : 4096), 24 * units);
+}
 int64_t splitkv_bytes(const fa4_nvfp4_params* p, int num_splits) {
   // partial O (num_splits, B, Sq, Hq, Dv) fp32, then partial LSE (num_splits, B, Hq, Sq) fp32
   return (int64_t)num_splits * p->B * p->Sq * p->Hq * ((int64_t)p->Dv + 1) * 4;
@@ -363,6 +400,22 @@ extern "C" int64_t fa4_nvfp4_splitkv_workspace_bytes(const fa4_nvfp4_params* p, 
   return num_splits == 1 ? 0 : splitkv_bytes(p, num_splits);
 }
 
+extern "C" int fa4_nvfp4_decode_is_balanced(int32_t B, int32_t Sq, int32_t Sk, int32_t Hq, int32_t Hkv) {
+  fa4_nvfp4_params p = {};
+  p.B = B; p.Sq = Sq; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv;
+  const int32_t any = 0;      // (only whether there are counts matters)
+  return B > 0 && Sq > 0 && Sk > 0 && Hkv > 0 && Hq >= Hkv && decode_balanced(&p, &any) ? 1 : 0;
+}
+
+extern "C" int64_t fa4_nvfp4_fwd_ex_workspace_bytes(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x) {
+  if (x == nullptr) return -FA4_E_NULL;
+  if (x->struct_size != sizeof(fa4_nvfp4_ext)) return -FA4_E_STRUCT;
+  const int64_t bytes = fa4_nvfp4_splitkv_workspace_bytes(p, x->num_splits == 0 ? 1 : x->num_splits);
+  if (bytes < 0 || p->variant != FA4_VARIANT_DECODE || p->Hkv <= 0 || p->Hq < p->Hkv || !decode_balanced(p, x->seqused_k))
+    return bytes;
+  return std::max(bytes, balanced_bytes(p));
+}
+
 extern "C" int fa4_nvfp4_fwd_splitkv(const fa4_nvfp4_params* p, int32_t num_splits, void* workspace,
                                      uint64_t workspace_bytes, void* cuda_stream) {
   if (num_splits < 1 || num_splits > 128) return -FA4_E_SHAPE;
@@ -374,7 +427,7 @@ namespace {
 struct FwdPlan {
   int variant = 0;
   int win_left = -1, win_right = -1;
-  bool decode = false, d192 = false, local = false, general = false, cached = false;
+  bool decode = false, balanced = false, d192 = false, local = false, general = false, cached = false;
   int dec_rows = 0;
 };
 
@@ -419,7 +472,9 @@ int validate_fwd(const fa4_nvfp4_params* p, int num_splits, const void* workspac
     // a handful of query rows per kv head, head dim 128, causal or unmasked
     if (p->D != 128 || p->Dv != 128 || (int64_t)p->Sq * (p->Hq / p->Hkv) > dec::kMaxRows) return -FA4_E_SHAPE;
     if (win_left >= 0 || win_right > 0 || sink != nullptr || softcap > 0.f) return -FA4_E_SHAPE;
-    if (!decode_in_cluster(p, num_splits)) {
+    plan->balanced = workspace != nullptr && aligned16(workspace) && decode_balanced(p, cache.seqused_k) &&
+                     workspace_bytes >= (uint64_t)balanced_bytes(p);
+    if (!plan->balanced && !decode_in_cluster(p, num_splits)) {
       if (workspace == nullptr || !aligned16(workspace)) return -FA4_E_NULL;
       if (workspace_bytes < (uint64_t)splitkv_bytes(p, num_splits)) return -FA4_E_TOO_LARGE;
     }
@@ -583,6 +638,30 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
                             linear->v_stride_h, linear->v_stride_d, rows, (rows + 31) / 32 * 2};
     }
     const bool merge = decode_in_cluster(p, num_splits);
+    dp.balance = Balance{};
+    if (plan.balanced) {
+      const int units = p->B * p->Hkv, slots = balanced_slots(p), ctas = balanced_ctas(p);
+      dp.o_partial = static_cast<float*>(workspace);
+      dp.lse_partial = dp.o_partial + (int64_t)ctas * dec_rows * 128;
+      dp.balance = Balance{ctas, slots, dec::kMinBlocks, units >= kSortedUnits ? 6 : 1, 1.f / (float)slots,
+                           1.f / (float)(ctas - units),
+                           reinterpret_cast<int2*>(dp.lse_partial + ((int64_t)ctas * dec_rows + 3) / 4 * 4)};
+      auto launch_bal = [&](auto kernel, int threads, uint32_t smem) -> int {
+        return launch_pdl(kernel, dim3((unsigned)ctas), threads, smem, stream, tm_k, tm_v, kp, dp);
+      };
+#define FA4_DEC(rows, depth)                                                                                            \
+  (linear != nullptr                                                                                                    \
+       ? launch_bal(attn_decode_kernel<rows, kBalanced, depth, true>, dec::threads_of(rows, depth), dec::form<rows, depth>::kRequest) \
+       : launch_bal(attn_decode_kernel<rows, kBalanced, depth, false>, dec::threads_of(rows, depth), dec::form<rows, depth>::kRequest))
+      const int rc = dec_rows <= 4 ? FA4_DEC(4, 3) : dec_rows <= 8 ? FA4_DEC(8, 3) : dec_rows <= 16 ? FA4_DEC(16, 3) : FA4_DEC(32, 5);
+#undef FA4_DEC
+      if (rc != 0) return rc;
+      const uint32_t rows = (uint32_t)(units * dec_rows);
+      return launch_pdl(combine_pieces_kernel, dim3((rows + kCombineWarps - 1) / kCombineWarps), kCombineWarps * 32, 0, stream,
+                        dp.o_partial, dp.lse_partial, dp.balance.pieces, kp.out, kp.lse, rows, dec_rows,
+                        make_fastdiv((uint32_t)dec_rows), make_fastdiv((uint32_t)p->Hkv), kp.div_group, kp.Sq, kp.Hq, kp.Hkv, kp.group,
+                        kp.o_stride_b, kp.o_stride_s, kp.o_stride_h);
+    }
     auto launch_dec = [&](auto kernel, int threads, uint32_t smem) -> int {
       return launch_pdl_cluster(merge ? (unsigned)num_splits : 1u, kernel,
                                 dim3((unsigned)num_splits, (unsigned)p->Hkv, (unsigned)p->B), threads, smem,
@@ -593,12 +672,16 @@ int launch_fwd(const fa4_nvfp4_params* p, int num_splits, void* workspace, uint6
     // longest 8192: 23.9 -> 21.6 us before its four warpgroups, 18.6 with them).  Even lengths keep HBM busy with three
     // tiles, and the room beside two shallow CTAs lets the next call's start early (B=4, Sk=32768: 33.0 us shallow, 40.3
     // deep).
-    const bool deep = cache.seqused_k != nullptr && p->B >= 4 && (int64_t)num_splits * p->Hkv * p->B <= 2 * kSms;
+    // Not for clusters of three, five, six or seven, of which an SM's two places leave too few at once (one token, up to
+    // 6528 keys, 8 heads: 5 entries in clusters of seven 12.8 us deep, 9.5 shallow; 6 in clusters of six 13.1, 10.3; 12 in
+    // clusters of three 12.8, 9.9; but 16 entries of 2048 in pairs 8.8, 9.5).
+    const bool deep = cache.seqused_k != nullptr && p->B >= 4 && (int64_t)num_splits * p->Hkv * p->B <= 2 * kSms &&
+                      (!merge || (num_splits & (num_splits - 1)) == 0);
 #define FA4_DEC_FORM(rows, merge, depth, linear)                                                      \
   launch_dec(attn_decode_kernel<rows, merge, depth, linear>, dec::threads_of(rows, depth), dec::form<rows, depth>::kRequest)
 #define FA4_DEC(rows, depth)                                                                            \
-  (linear != nullptr ? (merge ? FA4_DEC_FORM(rows, true, depth, true) : FA4_DEC_FORM(rows, false, depth, true)) \
-                     : (merge ? FA4_DEC_FORM(rows, true, depth, false) : FA4_DEC_FORM(rows, false, depth, false)))
+  (linear != nullptr ? (merge ? FA4_DEC_FORM(rows, kCluster, depth, true) : FA4_DEC_FORM(rows, kWorkspace, depth, true)) \
+                     : (merge ? FA4_DEC_FORM(rows, kCluster, depth, false) : FA4_DEC_FORM(rows, kWorkspace, depth, false)))
     const int rc = dec_rows <= 4    ? (deep ? FA4_DEC(4, 5) : FA4_DEC(4, 3))
                    : dec_rows <= 8  ? (deep ? FA4_DEC(8, 5) : FA4_DEC(8, 3))
                    : dec_rows <= 16 ? (deep ? FA4_DEC(16, 5) : FA4_DEC(16, 3))

@@ -22,7 +22,11 @@
 // One CTA = one (split, kv head, batch entry): a contiguous share of the entry's 128-key blocks,
 // visited in ascending order; its normalised fp32 partial O and partial LSE are merged inside the
 // cluster of an entry's splits (up to eight), or by combine_splits_kernel as on the split-KV path of
-// attn_ws.cuh.  Grid = (splits, Hkv, B).
+// attn_ws.cuh.  Grid = (splits, Hkv, B).  Batches whose entries have key counts in memory and many keys are dealt to the
+// CTAs by those counts instead (kBalanced): equal splits leave a batch of lengths spread over the logarithm waiting
+// for the longest entry's CTAs with four fifths of the GPU idle.  us, 16 entries up to 8192 keys, 8 heads, GQA 4 18.5 ->
+// 14.4, four tokens 34.1 -> 17.7; 32 up to 16384 57.3 -> 33.2 (143 MB of keys: 22 us at the copy bandwidth); 5 up to
+// 51200, 32 heads 131 -> 65.
 //   warps 0-3  softmax / correction / epilogue (thread = key lane, after the transpose a row; in the
 //              correction and the epilogue a dv lane)
 //   warps 8-11 up to eight rows: a second softmax warpgroup, which takes the odd blocks; in the deep form
@@ -52,11 +56,17 @@ namespace dec {
 // trip, so five are better whenever no third CTA is there to run.
 // (Registers: three CTAs of 384 threads leave 56, two of 640 leave 48, and up to eight rows the kernel wants more.  Bytes
 // of spill stores, merging / not: shallow 4 / 28, with linear scales 96 / 112-136; deep, four rows 48 / 84, 176 / 100;
-// eight rows 100 / 40, 212 / 136.  None above eight rows.  With them the deep form is still the faster one for ragged
+// eight rows 100 / 40, 212 / 136.  None above eight rows.  Balanced, shallow: 12-20, with linear scales 132.  With them the deep form is still the faster one for ragged
 // batches, see softmax_wgs, and reading linear scales faster than a launch of its own, see linear_keys_limit in
 // host.cpp, whose line is nearer for five to eight rows.)
 constexpr int kMaxCluster = 8;  // splits that are merged inside a cluster (portable cluster size)
 constexpr int kMaxRows = 32; // query rows per kv head: Sq * group
+// Limits of a balanced call (see balance(), which counts in floats): entries; keys of one, blocks of all, CTAs.
+constexpr int kMaxBalanced = 128, kMaxBalancedKeys = 1 << 26, kMaxBalancedBlocks = (1 << 20) - 8192, kMaxBalancedCtas = 4095;
+// Blocks below which a unit is not cut further.  (Two, three, four: one token, 48 entries up to 4096 keys of one head 10.7,
+// 10.6, 10.7 us; four tokens, 6 entries up to 2048 of 8 heads 9.6, 9.8, 11.0.)
+constexpr int kMinBlocks = 3;
+constexpr float kResetLimit = 6.f;       // log2 units a reference may fall by where a split starts inside of a CTA
 // Softmax warpgroups: one above eight rows; up to eight, two in the shallow form (registers: three CTAs of
 // twelve warps per SM leave 56 per thread) and four in the deep one, whose long entries run on with few CTAs
 // beside them: a block is a chain of some 1700 clocks in its warpgroup, and only the reference is handed
@@ -91,7 +101,8 @@ struct Smem {
                             kSync = kQReady + 1 /* WGs */, kHand = kSync + kWgs /* WGs x 4 */, kFin = kHand + 4 * kWgs,
                             kDrain = kFin + 1 /* 2 */, kCount = kDrain + 2;
   static constexpr uint32_t kOffMisc = (kOffBar + 8 * kCount + 15) / 16 * 16;
-  static constexpr uint32_t kRequest = kOffMisc + 16 + sizeof(WaitCtx) + 1024;
+  static constexpr uint32_t kOffWork = (kOffMisc + 16 + sizeof(WaitCtx) + 15) / 16 * 16;   // DecodeWork
+  static constexpr uint32_t kRequest = kOffWork + 48 + 1024;
   // (1 KB per CTA is the system's)
   static_assert((kDepth == 3 ? 3 : 2) * (kRequest + 1024) <= 228 * 1024, "decode kernel shared memory");
 };
@@ -226,6 +237,15 @@ struct LinearScales {
   int k_rows, v_cols;    // rows of k and columns of v of an entry (of a page)
 };
 
+// How the CTAs of the balanced form are dealt, see balance().  Its partials: ctas x (Sq * group) x 128 floats in
+// o_partial, as many LSEs in lse_partial.
+struct Balance {
+  int ctas, slots;       // of the grid; at once on the GPU
+  int min_per, rounds;
+  float inv_slots, inv_extra;   // 1 / slots, 1 / (ctas - B * Hkv)
+  int2* pieces;          // (B, Hkv): first CTA and number of CTAs
+};
+
 struct DecodeParams {
   const uint8_t* q;      // (B, Sq, Hq, 64) packed e2m1
   const uint8_t* q_sf;   // tiled (B, Hq, ceil(Sq/128), 2, 512)
@@ -234,7 +254,105 @@ struct DecodeParams {
   float* o_partial;      // (splits, B, Sq, Hq, 128) fp32
   float* lse_partial;    // (splits, B, Hq, Sq) fp32
   LinearScales lin;      // kLinear
+  Balance balance;       // kBalanced
 };
+
+// How the splits of a (kv head, batch entry) become one result.
+enum DecodeMerge {
+  kWorkspace,   // partials to o_partial / lse_partial, merged by combine_splits_kernel
+  kCluster,     // the splits are one cluster, which merges them through distributed shared memory
+  kBalanced     // entries of unequal lengths, CTAs dealt by the lengths: see balance()
+};
+
+// What a CTA of the balanced form works on: blocks i0 .. i0 + n - 1 of kv head hk of entry b, the `piece`-th of `pieces`.
+struct alignas(16) DecodeWork {
+  int b, hk, piece, pieces;   // b < 0: nothing
+  int i0, n, share, into;     // share: blocks of a split; into: those of i0's split before i0
+  int sk, pad[3];             // keys of the entry
+};
+
+// Whole quotient of numbers below 2^20 (the exact one is off the next integer by more than the reciprocal's error).
+__device__ __forceinline__ int small_div(int n, float inv) { return (int)(((float)n + 0.5f) * inv); }
+static_assert(sizeof(DecodeWork) == 48, "its place in shared memory");
+// Entries of unequal lengths (key counts in memory): the grid is dealt by the lengths.  A unit (kv head, entry) is cut
+// into the fewest pieces of at most `per` blocks, and `per` is the smallest number, from the mean of a resident CTA on,
+// for which the grid has the CTAs.  With more CTAs than fit at once (d.balance.rounds > 1) entries come by length, the
+// longest first, to within a factor of two.  Run by one warp; `len`: B words of shared memory.
+__device__ __forceinline__ DecodeWork balance(const KernelParams& p, const DecodeParams& d, int lane, int* len) {
+  const int cid = blockIdx.x;
+  int longest = 0, total = 0;
+#pragma unroll 1
+  for (int e = lane; e < p.B; e += 32) {
+    const int used = p.seqused_k[e];
+    const int sk = used < 0 ? 0 : (used < p.Sk ? used : p.Sk);
+    const int n = (sk + kBlockN - 1) / kBlockN;
+    len[e] = sk;
+    longest = max(longest, n);
+    total += n;
+  }
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  total = __reduce_add_sync(0xffffffffu, total) * p.Hkv;
+  __syncwarp();
+  auto pieces_of = [&](int e, int per, float inv) -> int {
+    return max(1, small_div((len[e] + kBlockN - 1) / kBlockN + per - 1, inv));
+  };
+  // (as many pieces as units, and what the whole list has of `hi`: always enough)
+  int lo = max(d.balance.min_per, small_div(total + d.balance.slots - 1, d.balance.inv_slots));
+  int hi = max(lo, min(longest, small_div(total, d.balance.inv_extra) + 1));
+#pragma unroll 1
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    const float inv = __frcp_rn((float)mid);
+    int c = 0;
+#pragma unroll 1
+    for (int e = lane; e < p.B; e += 32) c += pieces_of(e, mid, inv);
+    if (__reduce_add_sync(0xffffffffu, c) * p.Hkv <= d.balance.ctas) hi = mid; else lo = mid + 1;
+  }
+  const float inv = __frcp_rn((float)lo);
+  DecodeWork w;
+  w.b = -1; w.hk = 0; w.piece = 0; w.pieces = 1; w.i0 = 0; w.n = 0; w.share = 1; w.into = 0; w.sk = 0;
+  int at = cid;           // less the CTAs of the entries passed so far
+#pragma unroll 1
+  for (int round = 0; round < d.balance.rounds && w.b < 0; ++round) {
+    const int top = longest >> round, bottom = round + 1 < d.balance.rounds ? top >> 1 : -1;
+#pragma unroll 1
+    for (int e0 = 0; e0 < p.B; e0 += 32) {
+      int mine = 0;
+      if (e0 + lane < p.B) {
+        const int n = (len[e0 + lane] + kBlockN - 1) / kBlockN;
+        if (n <= top && n > bottom) mine = max(1, small_div(n + lo - 1, inv));
+      }
+      int upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, at < upto * p.Hkv);
+      if (hit != 0u) {
+        const int l = __ffs(hit) - 1;
+        w.b = e0 + l;
+        w.pieces = __shfl_sync(0xffffffffu, mine, l);
+        at -= (__shfl_sync(0xffffffffu, upto, l) - w.pieces) * p.Hkv;
+        break;
+      }
+      at -= __shfl_sync(0xffffffffu, upto, 31) * p.Hkv;
+    }
+  }
+  if (w.b >= 0) {
+    const float inv_pieces = __frcp_rn((float)w.pieces);
+    w.hk = small_div(at, inv_pieces);
+    w.piece = at - w.hk * w.pieces;
+    w.sk = len[w.b];
+    const int n = (w.sk + kBlockN - 1) / kBlockN, each = small_div(n + w.pieces - 1, inv_pieces);
+    w.share = max(1, fast_div(n + d.num_splits - 1, p.div_splits));
+    w.i0 = min(n, w.piece * each);
+    w.n = min(n - w.i0, each);
+    w.into = w.i0 - w.share * small_div(w.i0, __frcp_rn((float)w.share));
+    if (lane == 0 && w.piece == 0) d.balance.pieces[w.b * p.Hkv + w.hk] = make_int2(cid, w.pieces);
+  }
+  return w;
+}
 
 // kR: query rows the softmax code is built for (4, 8, 16 or 32 >= Sq * group): the size of the
 // lane-group transpose and the number of keys a thread owns afterwards.  N (the MMA's N, the
@@ -245,11 +363,12 @@ struct DecodeParams {
 // reads the eight bytes of four rows, two blocks at a time and ahead of the ones it stores.  For short calls, of which
 // the launch that tiles the scales is a third; with many keys the reads, a 32-byte sector for eight bytes,
 // take longer than that launch (the line lies in host.cpp).
-template <int kR, bool kMerge, int kDepth, bool kLinear>
+template <int kR, DecodeMerge kHow, int kDepth, bool kLinear>
 __global__ void __launch_bounds__(dec::threads_of(kR, kDepth), kDepth == 3 ? 3 : 2)
 attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const KernelParams p, const DecodeParams d) {
   using namespace dec;
+  constexpr bool kBal = kHow == kBalanced, kMerge = kHow == kCluster;
   constexpr int kWgs = softmax_wgs(kR, kDepth);
   constexpr int kN = kR <= 16 ? 16 : 32, kMaxRows = kN;   // (stride of the arrays per row)
   using L = form<kR, kDepth>;
@@ -266,7 +385,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   constexpr int kStrands = strands_of(kR), kOwn = kStrands / kWgs;   // partial row sums; of a warpgroup
 
   const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
-  const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+  const int split = kBal ? 0 : blockIdx.x;
+  int hk = blockIdx.y, b = blockIdx.z;
   WaitCtx& wc = *reinterpret_cast<WaitCtx*>(gbase + L::kOffMisc + 16);
   const int R = p.Sq * p.group;  // live query rows (<= kR)
 
@@ -296,6 +416,25 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   }
   tc_fence_before_sync();
   pdl_wait();
+  DecodeWork work;
+  if constexpr (kBal) {
+    // (the memory of the softmax warps' exchanges is free until the first scores)
+    static_assert(L::kOffBar - L::kOffRed >= 4 * kMaxBalanced, "scratch");
+    DecodeWork* slot = reinterpret_cast<DecodeWork*>(gbase + L::kOffWork);
+    if (warp == 0) {
+      const DecodeWork w = balance(p, d, lane, reinterpret_cast<int*>(gbase + L::kOffRed));
+      if (lane == 0) *slot = w;
+    }
+    __syncthreads();
+    work = *slot;
+    tc_fence_after_sync();
+    if (work.b < 0) {
+      if (warp == 5) tmem_dealloc(*tmem_slot, TM::kCols);
+      return;
+    }
+    hk = work.hk;
+    b = work.b;
+  }
   // The query rows and their scale words go to registers before anything else is read: their
   // latency (a trip to HBM while every CTA of the grid starts its K / V stream) then overlaps the
   // rendezvous below.  Threads 0-127: row tid / 4, 16-byte chunk tid % 4; threads 0-63
@@ -328,18 +467,32 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   // this CTA's share of the entry's K/V blocks (ascending, contiguous, ceil division like the
   // split-KV path of the prefill kernel)
   int sk = p.Sk;
-  if (p.seqused_k != nullptr) {
+  if constexpr (kBal) {
+    sk = work.sk;
+  } else if (p.seqused_k != nullptr) {
     const int used = p.seqused_k[b];
     sk = used < 0 ? 0 : (used < p.Sk ? used : p.Sk);
   }
-  const int n_total = (sk + kBlockN - 1) / kBlockN;
-  const int per = fast_div(n_total + d.num_splits - 1, p.div_splits);
-  const int i0 = split * per < n_total ? split * per : n_total;
-  const int i1 = i0 + per < n_total ? i0 + per : n_total;
-  const int n = i1 - i0;
+  int i0, n;
+  // kBalanced: the references of the rows follow the splits, not the CTAs, so that how P is rounded does not depend on
+  // how many CTAs there are.  A reference starts anew with every split (at li = next_start), and a CTA that begins
+  // inside of one visits that one's first block before its own (pre = 1), for the reference alone.
+  int pre = 0, next_start = 1 << 30;
+  if constexpr (kBal) {
+    pre = work.n > 0 && work.into > 0 ? 1 : 0;
+    i0 = work.i0 - pre;
+    n = work.n + pre;
+    next_start = pre + work.share - work.into;
+  } else {
+    const int n_total = (sk + kBlockN - 1) / kBlockN;
+    const int per = fast_div(n_total + d.num_splits - 1, p.div_splits);
+    i0 = split * per < n_total ? split * per : n_total;
+    n = (i0 + per < n_total ? i0 + per : n_total) - i0;
+  }
   // (producers) lane l: where the CTA's block li + l lies: batch coordinate, block inside it
   auto locate = [&](int li) -> int2 {
     int2 r = make_int2(b, i0 + li + lane);
+    if (kBal && pre != 0 && li + lane == 0) r.y = work.i0 - work.into;
     if (p.page_table != nullptr && li + lane < n) {
       const int pg = fast_div(r.y, p.div_page);
       r.x = p.page_table[(int64_t)b * p.pages_per_seq + pg];
@@ -384,8 +537,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     at = locate(0);
     if (kLinear) fetch(0);
   }
-  __syncthreads();
-  tc_fence_after_sync();
+  if constexpr (!kBal) {
+    __syncthreads();
+    tc_fence_after_sync();
+  }
   pdl_trigger();
   const uint32_t tmem = *tmem_slot;
   const ScoreScales sc = score_scales(p);
@@ -599,7 +754,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     }
 
     for (int li = wg; ok && li < n; li += kWgs) {
-      const int nb = i0 + li;
+      const int nb = kBal && pre != 0 && li == 0 ? work.i0 - work.into : i0 + li;
       const uint32_t buf = li % kDepth, slot = li % kDepth;
       ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kSFull + buf), (li / kDepth) & 1, wc, kDSFull));
       if (!ok) break;
@@ -652,7 +807,20 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         if (!ok) break;
         m_prev = s_hand[(before * 4 + wq) * kMaxRows + my_row];
       }
-      const float m_new = next_reference(m_prev, m_loc, sc.sl2);
+      float m_new = next_reference(m_prev, m_loc, sc.sl2);
+      if constexpr (kBal) {
+        while (next_start < li) next_start += work.share;
+        if (next_start == li) {
+          // A split starts: its reference is the maximum of this block.  Not where that lies far below the one
+          // before (or where the row sees no key): what the split adds is then nothing beside what is there, and the
+          // factors stay finite.
+          m_new = m_prev == kNegInf || (m_prev - m_loc) * sc.sl2 <= kResetLimit ? m_loc : m_prev;
+        }
+        if (pre != 0 && li == 0) {
+#pragma unroll
+          for (int j = 0; j < kR; ++j) x[j] = kNegInf;
+        }
+      }
       if (kWgs > 1) {
         if (lane < kR) s_hand[(wg * 4 + wq) * kMaxRows + my_row] = m_new;
         mbar_arrive(bar(L::kHand + 4 * wg + wq));
@@ -801,7 +969,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           l_s[i] = ((sum[0] + sum[kN]) + sum[2 * kN]) + sum[3 * kN];
           const float handed = s_hand[w * 4 * kN + my_row];
           m_s[i] = !last ? s_old[(w * 5 + 4) * kN + my_row] : (w == 0 ? m_ref : handed);
-          m_fin = fmaxf(m_fin, m_s[i]);
+          // (of the last block; the references of a CTA only grow, but for those of a new split)
+          if constexpr (kBal) m_fin = i == (n - 1) % kStrands ? m_s[i] : m_fin;
+          else m_fin = fmaxf(m_fin, m_s[i]);
         }
 #pragma unroll
         for (int i = 0; i < kStrands; ++i) l_tot = fmaf(l_s[i], reference_factor(m_s[i], m_fin, sc.sl2), l_tot);
@@ -824,16 +994,32 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         // (kMerge: the K and V rings are free, every product has completed)
         float* dst = reinterpret_cast<float*>(gbase + L::kOffK) + tid;
         constexpr int step = 128;
-        if constexpr (!kMerge) {
+        if constexpr (kBal) {
+          dst = d.o_partial + (int64_t)blockIdx.x * R * 128 + tid;
+        } else if constexpr (!kMerge) {
           // row r = s * group + (head in the group): the rows of one token are neighbours
           dst = d.o_partial + ((((int64_t)split * p.B + b) * p.Sq) * p.Hq + hk * p.group) * 128 + tid;
         }
         int in_group = 0;
+        if (kBal && work.pieces == 1) {
+          // the result itself
+          __nv_bfloat16* res = p.out + b * p.o_stride_b + (int64_t)hk * p.group * p.o_stride_h + tid;
+#pragma unroll
+          for (int r = 0; r < kR; ++r) {
+            const float v = o[r] * __shfl_sync(0xffffffffu, scale, r);
+            if (r < R) *res = __float2bfloat16_rn(v);
+            res += p.o_stride_h;
+            if (++in_group == p.group) {
+              in_group = 0;
+              res += p.o_stride_s - (int64_t)p.group * p.o_stride_h;
+            }
+          }
+        } else
 #pragma unroll
         for (int r = 0; r < kR; ++r) {
           if (r < R) *dst = o[r] * __shfl_sync(0xffffffffu, scale, r);   // lane r of every warp owns row r
           dst += step;
-          if constexpr (!kMerge) {
+          if constexpr (!kMerge && !kBal) {
             if (++in_group == p.group) {
               in_group = 0;
               dst += (int64_t)(p.Hq - p.group) * 128;
@@ -845,7 +1031,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             reinterpret_cast<float*>(gbase + L::kOffV)[tid] = lse;
           } else {
             const int s = fast_div(tid, p.div_group), h = hk * p.group + tid - s * p.group;
-            d.lse_partial[(((int64_t)split * p.B + b) * p.Hq + h) * p.Sq + s] = lse;
+            if (kBal && work.pieces > 1) d.lse_partial[(int64_t)blockIdx.x * R + tid] = lse;
+            else if (!kBal) d.lse_partial[(((int64_t)split * p.B + b) * p.Hq + h) * p.Sq + s] = lse;
+            else if (p.lse != nullptr) p.lse[((int64_t)b * p.Hq + h) * p.Sq + s] = lse;
           }
         }
       }

@@ -210,6 +210,27 @@ qk_tile_probe_kernel(const __grid_constant__ CUtensorMap tm_q,
 // ---------------------------------------------------------------------------------------------
 constexpr int kCombineWarps = 4, kCombineBatch = 8;
 constexpr uint32_t kCombineSharedRows = 2048, kCombineBlocksPerSm = 64;
+// Partials (lse, normalised O) of a batch join a row's merge so far: maximum, sum of weights, weighted sum.
+__device__ __forceinline__ void merge_batch(float& m, float& sum, float4& acc, const float (&l)[kCombineBatch],
+                                            const float4 (&v)[kCombineBatch]) {
+  float top = m;
+#pragma unroll
+  for (int j = 0; j < kCombineBatch; ++j) top = fmaxf(top, l[j]);
+  if (top == -INFINITY) return;
+  const float keep = __expf(m - top);    // (0 before the first split with a key)
+  sum *= keep;
+  acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+  m = top;
+#pragma unroll
+  for (int j = 0; j < kCombineBatch; ++j) {
+    const float w = __expf(l[j] - m);    // exp(-inf) = 0 past the last split
+    sum += w;
+    acc.x = fmaf(w, v[j].x, acc.x);
+    acc.y = fmaf(w, v[j].y, acc.y);
+    acc.z = fmaf(w, v[j].z, acc.z);
+    acc.w = fmaf(w, v[j].w, acc.w);
+  }
+}
 __global__ void __launch_bounds__(kCombineWarps * 32)
 combine_splits_kernel(const float* __restrict__ o_partial, const float* __restrict__ lse_partial,
                       __nv_bfloat16* __restrict__ out, float* __restrict__ lse, int num_splits, uint32_t rows,
@@ -235,7 +256,7 @@ combine_splits_kernel(const float* __restrict__ o_partial, const float* __restri
     if (live) {
 #pragma unroll 1
       for (int i0 = first; i0 < num_splits; i0 += kCombineBatch * warps_per_row) {
-        float l[kCombineBatch], top = m;
+        float l[kCombineBatch];
         float4 v[kCombineBatch];
 #pragma unroll
         for (int j = 0; j < kCombineBatch; ++j) {
@@ -247,22 +268,7 @@ combine_splits_kernel(const float* __restrict__ o_partial, const float* __restri
             if (mine) v[j] = *reinterpret_cast<const float4*>(o_partial + ((int64_t)i * rows + r) * Dv + col);
           }
         }
-#pragma unroll
-        for (int j = 0; j < kCombineBatch; ++j) top = fmaxf(top, l[j]);
-        if (top == -INFINITY) continue;
-        const float keep = __expf(m - top);    // (0 before the first split with a key)
-        sum *= keep;
-        acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
-        m = top;
-#pragma unroll
-        for (int j = 0; j < kCombineBatch; ++j) {
-          const float w = __expf(l[j] - m);    // exp(-inf) = 0 past the last split
-          sum += w;
-          acc.x = fmaf(w, v[j].x, acc.x);
-          acc.y = fmaf(w, v[j].y, acc.y);
-          acc.z = fmaf(w, v[j].z, acc.z);
-          acc.w = fmaf(w, v[j].w, acc.w);
-        }
+        merge_batch(m, sum, acc, l, v);
       }
     }
     if (!alone) {
@@ -302,6 +308,45 @@ combine_splits_kernel(const float* __restrict__ o_partial, const float* __restri
       if (col == 0 && lse != nullptr) lse[l_idx] = m == -INFINITY ? -INFINITY : m + __logf(sum);
     }
   }
+}
+
+// The same for a balanced decode call (attn_decode.cuh), a warp a row: the partials of row r of unit u = (b, hk) are
+// those of CTAs pieces[u].x .. + pieces[u].y - 1, `unit_rows` x 128 each.  Units of one piece are written already.
+__global__ void __launch_bounds__(kCombineWarps * 32)
+combine_pieces_kernel(const float* __restrict__ o_partial, const float* __restrict__ lse_partial,
+                      const int2* __restrict__ pieces, __nv_bfloat16* __restrict__ out, float* __restrict__ lse, uint32_t rows,
+                      int unit_rows, FastDiv div_rows, FastDiv div_hkv, FastDiv div_group, int Sq, int Hq, int Hkv, int group,
+                      int64_t o_stride_b, int64_t o_stride_s, int64_t o_stride_h) {
+  const uint32_t row = blockIdx.x * kCombineWarps + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  pdl_wait();
+  if (row >= rows) return;
+  const int u = fast_div((int)row, div_rows), r = (int)row - u * unit_rows;
+  const int2 mine = pieces[u];
+  if (mine.y == 1) return;
+  float m = -INFINITY, sum = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+  for (int i0 = 0; i0 < mine.y; i0 += kCombineBatch) {
+    float l[kCombineBatch];
+    float4 v[kCombineBatch];
+#pragma unroll
+    for (int j = 0; j < kCombineBatch; ++j) {
+      l[j] = -INFINITY;
+      v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i0 + j < mine.y) {
+        const int64_t at = (int64_t)(mine.x + i0 + j) * unit_rows + r;
+        l[j] = lse_partial[at];
+        v[j] = *reinterpret_cast<const float4*>(o_partial + at * 128 + 4 * lane);
+      }
+    }
+    merge_batch(m, sum, acc, l, v);
+  }
+  const float inv = m == -INFINITY ? 0.f : 1.f / sum;
+  const int b = fast_div(u, div_hkv), hk = u - b * Hkv, s = fast_div(r, div_group), h = hk * group + r - s * group;
+  *reinterpret_cast<uint2*>(out + b * o_stride_b + (int64_t)s * o_stride_s + h * o_stride_h + 4 * lane) =
+      make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
+  if (lane == 0 && lse != nullptr) lse[((int64_t)b * Hq + h) * Sq + s] = m == -INFINITY ? -INFINITY : m + __logf(sum);
 }
 
 // ---------------------------------------------------------------------------------------------

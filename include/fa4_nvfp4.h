@@ -193,6 +193,16 @@ typedef struct fa4_nvfp4_ext {
   int32_t reserved2;        /* 0 */
 } fa4_nvfp4_ext;
 int fa4_nvfp4_fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, void* cuda_stream);
+/*
+ * The workspace that fa4_nvfp4_fwd_ex makes use of (x->workspace and x->workspace_bytes are not read): at least
+ * fa4_nvfp4_splitkv_workspace_bytes(p, splits), which remains enough to run; more for a decode call
+ * (FA4_VARIANT_DECODE) with x->seqused_k over many keys, whose CTAs are then dealt by the lengths of the entries.  The
+ * splits stay what the reference maxima of P follow, so the two ways differ by fp32 rounding (and, where a
+ * reference moves within a split, in how P is rounded behind it).
+ */
+int64_t fa4_nvfp4_fwd_ex_workspace_bytes(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x);
+/* Whether a decode call of this shape with seqused_k and that workspace is dealt by the lengths (1 or 0). */
+int fa4_nvfp4_decode_is_balanced(int32_t B, int32_t Sq, int32_t Sk, int32_t Hq, int32_t Hkv);
 
 /*
  * fa4_nvfp4_fwd_ex with the three per-tensor scales in DEVICE memory (p->q_scale, k_scale, v_scale

@@ -2,6 +2,8 @@
 the narrow and the wide window form, more tiles than CTAs with tiles that have no rows between them, tile
 lists longer than a CTA's table, the decode kernel's ring depths and the two ways its splits are merged, and
 the quantiser's small, unaligned and strided inputs."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -326,3 +328,83 @@ def test_decode_from_a_pool_larger_than_the_table(cuda_device, spare):
     torch.cuda.synchronize()
     fa.check_status(cuda_device)
     assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1])
+
+
+@pytest.mark.parametrize("Sq,Hq,Hkv,Sk,lens,layout,paged,splits", [
+    # one token: an empty entry, single keys, block edges; split and not; more splits than blocks
+    (1, 32, 8, 13312, [13312, 0, 1, 127, 128], "tiled", True, 0),
+    (1, 32, 8, 13312, [13312, 129, 4096, 4097, 1], "linear", False, 0),
+    (1, 32, 8, 13312, [0, 0, 0, 0, 0], "tiled", False, 0),
+    (1, 32, 8, 13312, [13312, 13312, 13311, 13185, 13184], "tiled", True, 3),
+    (1, 32, 8, 13312, [13312, 900, 260, 300, 12000], "tiled", False, 128),
+    (2, 8, 2, 9000, [9000, 1] + [33 * i for i in range(31)], "linear", False, 1),           # two chunks of entries
+    (4, 16, 8, 3200, [3200, 300, 3199, 0, 4, 3] * 6, "tiled", True, 2),                    # eight rows, entries by length
+    (4, 32, 8, 8704, [8704, 3, 130, 8000], "tiled", True, 0),                              # sixteen rows
+    (8, 32, 8, 8704, [8704, 7, 130, 8000], "linear", False, 5),                            # 32 rows
+    (1, 4, 4, 5120, [5120 - 40 * i for i in range(127)] + [0], "tiled", False, 2),  # more units than places, 128 entries
+], ids=str)
+def test_decode_dealt_by_the_lengths(cuda_device, Sq, Hq, Hkv, Sk, lens, layout, paged, splits):
+    """CTAs dealt by the key counts, against each entry alone with the same splits: fp32 partials in another
+    grouping, so bf16 neighbours (2^-8 of a value), and rows whose reference moves inside a split, which may round P anew behind
+    it (two roundings of all of P differ by 0.16 rel-RMS; fewer than one row in 256 does that here)."""
+    B = len(lens)
+    assert fa.lib().fa4_nvfp4_decode_is_balanced(B, Sq, Sk, Hq, Hkv) == 1
+    if splits == 0:
+        splits = fa._lib.host().choose_decode_splits(B, Hkv, Sk, 148)
+    rows, slots = (B * (Sk // 128), 128) if paged else (B, Sk)
+    g = torch.Generator(device=cuda_device).manual_seed(21)
+    q, k, v = (torch.randn(b, S, H, 128, generator=g, device=cuda_device, dtype=torch.bfloat16)
+               for b, S, H in ((B, Sq, Hq), (rows, slots, Hkv), (rows, slots, Hkv)))
+    Q, K, V = fa.quantize_qkv_fused(q, k, v)
+    sf = (lambda t: t.sf) if layout == "linear" else (lambda t: t.tiled_sf())
+    used = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+    table = torch.randperm(rows, generator=g, device=cuda_device).to(torch.int32).view(B, -1) if paged else None
+
+    def call(b0, b1):
+        part = (lambda x: x) if paged else (lambda x: x[b0:b1])
+        return fa.flash_attn_fp4_func(Q.data[b0:b1], part(K.data), part(V.data), sf(Q)[b0:b1], part(sf(K)), part(sf(V)),
+                                      Q.scale, K.scale, V.scale, causal=True, sf_layout=layout, num_splits=splits,
+                                      seqused_k=used[b0:b1], page_table=None if table is None else table[b0:b1],
+                                      return_lse=True)
+
+    out, lse = call(0, B)
+    alone = [call(b, b + 1) for b in range(B)]
+    fa.check_status(cuda_device)
+    ref, ref_lse = (torch.cat([a[i] for a in alone]) for i in (0, 1))
+    assert torch.isfinite(out).all() and torch.equal(torch.isinf(lse), torch.isinf(ref_lse))
+    fin = torch.isfinite(ref_lse)
+    if fin.any():
+        assert (lse[fin] - ref_lse[fin]).abs().max().item() <= 1e-4
+    assert torch.equal(out.isfinite(), ref.isfinite()) and (out.float() - ref.float()).norm() <= 0.01 * ref.float().norm()
+    assert torch.equal(out.permute(0, 2, 1, 3)[~fin], torch.zeros_like(out.permute(0, 2, 1, 3)[~fin]))
+
+
+def test_decode_dealt_by_the_lengths_where_references_move(cuda_device):
+    """Scores that grow and shrink along the keys by up to 40 log2 units, so that references move within splits, fall where one
+    starts, or are kept there (more than kResetLimit below): against exact attention, no further off than the entries
+    alone are (with the quarter that the parity tests allow P's rounding)."""
+    B, Sk, Hq, Hkv = 6, 12288, 8, 8
+    lens = [12288, 5000, 700, 12000, 3000, 129]
+    g = torch.Generator(device=cuda_device).manual_seed(22)
+    q = torch.randn(B, 1, Hq, 128, generator=g, device=cuda_device)
+    k = torch.randn(B, Sk, Hkv, 128, generator=g, device=cuda_device)
+    v = torch.randn(B, Sk, Hkv, 128, generator=g, device=cuda_device)
+    wave = torch.sin(torch.arange(Sk, device=cuda_device) / torch.tensor([2000.0, 300.0, 90.0, 5000.0, 700.0, 40.0],
+                                                                         device=cuda_device)[:, None]) * 14.0
+    k = k + wave[:, :, None, None] * (q / q.norm(dim=-1, keepdim=True))
+    Q, K, V = fa.quantize_qkv_fused(q.bfloat16(), k.bfloat16(), v.bfloat16())
+    used = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+    for splits in (1, 3, 40):
+        kw = dict(causal=True, num_splits=splits, return_lse=True)
+        assert fa.lib().fa4_nvfp4_decode_is_balanced(B, 1, Sk, Hq, Hkv) == 1
+        got, lse = fa.flash_attn_fp4_func(Q.data, K.data, V.data, Q.sf, K.sf, V.sf, Q.scale, K.scale, V.scale, seqused_k=used, **kw)
+        for b, n in enumerate(lens):
+            one = [t[b:b + 1] for t in (Q.data, K.data, V.data, Q.sf, K.sf, V.sf)]
+            alone, _ = fa.flash_attn_fp4_func(*one, Q.scale, K.scale, V.scale, seqused_k=used[b:b + 1], **kw)
+            qd, kd, vd = (t.dequantize()[b:b + 1].float() for t in (Q, K, V))
+            s = torch.einsum("bqhd,bkhd->bhqk", qd, kd[:, :n]) / math.sqrt(128)
+            exact = torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), vd[:, :n])
+            e_got, e_alone = ((x.float() - exact).norm() / exact.norm() for x in (got[b:b + 1], alone))
+            assert e_got <= 1.25 * e_alone + 0.01, (splits, b, e_got, e_alone)
+            assert (lse[b, :, 0] - s.logsumexp(-1)[0, :, 0]).abs().max() <= 1e-3 * s.abs().max()
+    fa.check_status(cuda_device)
