@@ -901,7 +901,7 @@ int launch_quantize(QuantJobs& q, cudaStream_t stream) {
     j.blocks = (int)ctas;
     blocks += ctas;
   }
-  return launch_pdl(quantize_kernel, dim3((unsigned)blocks), 256, 0, stream, q);
+  return launch_pdl(quantize_kernel, dim3((unsigned)blocks), 256, kQuantizeSmem, stream, q);
 }
 }  // namespace
 

@@ -35,24 +35,21 @@ __device__ __forceinline__ float e4m3_value(uint32_t byte) {
   return __half2float(__ushort_as_half(static_cast<unsigned short>(h2 & 0xffffu)));
 }
 
-// Clears the sign of nibbles whose magnitude is zero (the formats agree on "no negative zero").
+// Clears the sign of nibbles whose magnitude is zero (the formats agree on "no negative zero"): a magnitude
+// of 1..7 plus 7 sets bit 3 of its nibble and carries no further.
 __device__ __forceinline__ uint32_t drop_negative_zero(uint32_t n) {
-  const uint32_t mag = n & 0x77777777u;
-  const uint32_t nz = ((mag + 0x77777777u) | mag) & 0x88888888u;
-  return n & (0x77777777u | nz);
+  return n & (((n & 0x77777777u) + 0x77777777u) | 0x77777777u);
 }
 
-// Correctly rounded a / b from the correctly rounded reciprocal rb = RN(1 / b) and nb = -b: the
-// product a rb is within 2 ulp of the quotient, one residual step (the residual a - y b is exact
-// in an FMA) makes it faithful and a second one correctly rounded (Markstein's division theorem).
-// Five FMA-pipe instructions where a library division takes a dozen and a branch.  Needs finite
-// rb and residuals that do not underflow: callers keep operands near the bottom of the fp32
-// range on the library path.
-__device__ __forceinline__ float div_rn_by(float a, float nb, float rb) {
-  const float y0 = __fmul_rn(a, rb);
-  const float y1 = fmaf(fmaf(y0, nb, a), rb, y0);
-  return fmaf(fmaf(y1, nb, a), rb, y1);
-}
+// a / b from 1 / b in two terms, hi + lo (lo = the residual of hi, times hi): the product is within a few
+// 2^-47 of the quotient before its one rounding.  That is not always the correctly rounded quotient, but
+// on the same side of every rounding boundary that matters here, for every a and b that can occur
+// (tests/test_quantiser_rounding_cpu.py goes through all of them).  Two FMA-pipe instructions; needs lo to be no
+// denormal, so callers keep b between 1e-30 and 1e20.
+struct Reciprocal {
+  float hi, lo;
+};
+__device__ __forceinline__ float div_by(float a, const Reciprocal& r) { return fmaf(a, r.hi, __fmul_rn(a, r.lo)); }
 
 // Rare path of quantize_block16 (denominators near the bottom of the fp32 range), out of line so
 // that the hot loop stays small.
@@ -67,33 +64,36 @@ __device__ __noinline__ uint2 quantize_block16_exact(Block16 x, float denom) {
                     pack8_e2m1(y[8], y[9], y[10], y[11], y[12], y[13], y[14], y[15]));
 }
 
-// Per-tensor constants of the quantiser: the tensor scale g, -g, RN(1 / g), and whether g is so
-// small (below 1e-18) that the residual steps above could underflow where it matters: then the
-// block scales take the library division.
+// Per-tensor constants of the quantiser: the tensor scale g, 1 / g, and whether g or a block's scale times g lies
+// where the two-term reciprocals lose bits (`odd`: block scales take the library division; `huge`: the elements
+// as well).
 struct TensorScale {
-  float g, neg_g, rcp_g;
-  bool tiny;
+  float g;
+  Reciprocal rcp;
+  bool odd, huge;
 };
 __device__ __forceinline__ TensorScale make_tensor_scale(float amax) {
   TensorScale t;
   t.g = tensor_scale_of(amax);
-  t.neg_g = -t.g;
-  t.tiny = !(t.g >= 1e-18f);
-  t.rcp_g = t.tiny ? 0.f : __frcp_rn(t.g);
+  t.huge = t.g > 1e17f && t.g < INFINITY;
+  t.odd = !(t.g >= 1e-18f) || t.huge;
+  t.rcp.hi = t.odd ? 0.f : __frcp_rn(t.g);
+  t.rcp.lo = fmaf(-t.g, t.rcp.hi, 1.f) * t.rcp.hi;
   return t;
 }
 
 // Scale byte and its value times g for a block with maximum bmax.
 __device__ __forceinline__ float block_scale_of(float bmax, const TensorScale& ts, uint32_t& sf_byte) {
   // block scale = e4m3_rne(min((bmax / 6) / g, 448)).  With g >= 1e-18 every quotient that can
-  // reach the first rounding boundary of e4m3 (2^-10) has exact residuals; smaller quotients give
+  // reach the first rounding boundary of e4m3 (2^-10) is far from the denormals; smaller quotients give
   // the zero byte whatever their last bits are.
-  constexpr float kRcp6 = 0.16666667163372039794921875f;   // RN(1 / 6)
+  constexpr float kSixth = 0.16666667163372039794921875f;   // RN(1 / 6), and 1 / 6 minus it
+  constexpr Reciprocal kRcp6 = {kSixth, -4.967053731282552e-09f};
   float t;
-  if (ts.tiny) {
+  if (ts.odd) {
     t = __fdiv_rn(__fdiv_rn(bmax, 6.f), ts.g);
   } else {
-    t = div_rn_by(div_rn_by(bmax, -6.f, kRcp6), ts.neg_g, ts.rcp_g);
+    t = div_by(div_by(bmax, kRcp6), ts.rcp);
   }
   sf_byte = e4m3_byte(fminf(t, 448.f));
   return __fmul_rn(e4m3_value(sf_byte), ts.g);
@@ -103,23 +103,21 @@ __device__ __forceinline__ float block_scale_of(float bmax, const TensorScale& t
 __device__ __forceinline__ void quantize_block16(const float (&x)[16], float bmax, const TensorScale& ts,
                                                  uint32_t& lo, uint32_t& hi, uint32_t& sf_byte) {
   const float denom = block_scale_of(bmax, ts, sf_byte);
-  // The element codes are those of the correctly rounded quotients x / denom.  One residual step is
-  // enough for them: only quotients within a few ulp of a rounding boundary of e2m1 (.25 .75 1.25
-  // 1.75 2.5 3.5 5) matter, x has eight significand bits, and for every significand of denom but the
-  // largest (which no bf16 maximum gives) and every reciprocal within one ulp the steps below put the values
-  // of x next to a boundary on the side of it that the correctly rounded quotient is on
-  // (tests/test_quantiser_rounding_cpu.py goes through them; without the step 257 denominators fail).
-  // Three instructions a pair where correctly rounded quotients take five.
-  if (denom >= 1e-30f) {
+  // The element codes are those of the correctly rounded quotients x / denom: only quotients within a few
+  // ulp of a rounding boundary of e2m1 (.25 .75 1.25 1.75 2.5 3.5 5) matter, x has eight significand bits, and
+  // for every significand of denom but the largest (which no bf16 maximum gives) and every reciprocal
+  // within one ulp the products below put the values of x next to a boundary on the side of it that the
+  // correctly rounded quotient is on.  Two instructions a pair where one term and a residual step took three.
+  if (denom >= 1e-30f && !ts.huge) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(denom));
-    r = fmaf(fmaf(-denom, r, 1.f), r, r);
-    const float2 rr = make_float2(r, r), nd = make_float2(-denom, -denom);
+    const float rl = __fmul_rn(fmaf(-denom, r, 1.f), r);
+    const float2 r2 = make_float2(r, r), rl2 = make_float2(rl, rl);
     float2 y[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float2 v = make_float2(x[2 * i], x[2 * i + 1]), y0 = __fmul2_rn(v, rr);
-      y[i] = __ffma2_rn(__ffma2_rn(y0, nd, v), rr, y0);
+      const float2 v = make_float2(x[2 * i], x[2 * i + 1]);
+      y[i] = __ffma2_rn(v, r2, __fmul2_rn(v, rl2));
     }
     lo = pack8_e2m1(y[0].x, y[0].y, y[1].x, y[1].y, y[2].x, y[2].y, y[3].x, y[3].y);
     hi = pack8_e2m1(y[4].x, y[4].y, y[5].x, y[5].y, y[6].x, y[6].y, y[7].x, y[7].y);
@@ -264,7 +262,7 @@ amax_kernel(const __grid_constant__ QuantJobs jobs) {
 //
 // Q / K, blocks along D: a work item is one block of 16 in the rows l, l + 32, l + 64, l + 96 of a
 // 128-row tile: their four scales share a 16-byte piece of the tiled layout.  Neighbouring threads take
-// neighbouring blocks, so a warp's reads (1 KB, the four rows in flight together) and packed writes
+// neighbouring blocks, so a warp's reads (1 KB a row) and packed writes
 // are contiguous.  (A thread with four neighbouring blocks of a row needs no exchange of scale bytes,
 // but its 128-byte stride filled the load/store pipe: 148 instead of 131 us.)
 //   packed (B, S, H, D/2), lin (B, S, H, D/16) or null, tiled (B, H, ceil(S/128), D/64, 512) or null
@@ -275,63 +273,91 @@ amax_kernel(const __grid_constant__ QuantJobs jobs) {
 //   packed (B, H, Dv, s_out/2), lin (B, H, Dv, s_out/16) or null,
 //   tiled (B, H, ceil(Dv/128), 2 ceil(s_out/128), 512) or null
 //
-// Persistent: two CTAs per SM in all, dealt to the tensors in proportion to their bytes, and each
-// keeps the loads of its next item in flight behind the arithmetic of the current one.
+// Persistent: three CTAs per SM in all, dealt to the tensors in proportion to their bytes; a CTA's next item or
+// tile is on its way to shared memory (cp.async, 96 KB per SM) behind the arithmetic of the current one.
 //
-// What bounds it: instruction issue and latency about equally, then HBM.  q, k, v of the sizes above,
-// quantise pass alone: 153 us as three kernels with correctly rounded divisions (274 instructions per
-// block), 117 us here (about 180).
+// What bounds it: instruction issue (68 % of the slots busy, the ALU pipe 58 %), then HBM.  q, k, v of the sizes
+// above, maxima and quantise pass together: 190 us with the loads of an item in registers (two CTAs of 119
+// registers per SM, 175 instructions per block of 16) and one residual step per quotient; 166 us here (157).  In
+// between: three CTAs with two rows in flight in registers 174 (49 KB per SM in flight are too few); cp.async of a
+// thread's own two pieces, half sectors each, 210.  No gain: units of four rows one below the other (168), the
+// low halves unpacked on the FMA pipe (166), hints that keep the end of the tensors in L2 (166; other sizes 2 %).
 // ---------------------------------------------------------------------------------------------
 
-// Where a Q / K work item lies.
+// Where a Q / K work item lies: its first row (k0 = 0), or row k0 of it.
 struct RowsItem {
-  const __nv_bfloat16* src;     // block (b, s0, h, c)
-  int b, rt, l, h, c, s0;
+  int s0;                       // the row
+  uint32_t blk, piece;          // blocks of 16 before it in the tensor; 16-byte pieces of tiled scales before its own
 };
-__device__ __forceinline__ RowsItem rows_item_at(const QuantJob& j, uint32_t item, int k0) {
+// What a thread copies for its warp: the 64 16-byte pieces of 32 neighbouring blocks of a row are copied by
+// lane as they follow in memory (a copy of its own two would take half sectors), pieces l and l + 32 by lane l.
+struct RowsLoad {
+  const __nv_bfloat16 *a, *b;
+  int sa, sb;                   // their rows
+};
+__device__ __forceinline__ RowsItem rows_item_at(const QuantJob& j, uint32_t item, int k0, RowsLoad& ld) {
   RowsItem it;
-  const int rest = fast_div((int)item, j.div_nb), col = (int)item - rest * j.nb, bt = rest >> 5;
-  it.l = rest & 31;
-  it.b = fast_div(bt, j.div_rt);
-  it.rt = bt - it.b * j.rt;
-  it.h = fast_div(col, j.div_h);
-  it.c = col - it.h * (j.D >> 4);
-  it.s0 = it.rt * 128 + k0 * 32 + it.l;
-  it.src = j.x + it.b * j.sb + it.s0 * j.ss + it.h * j.sh + it.c * 16;
+  const int rest = fast_div((int)item, j.div_nb), col = (int)item - rest * j.nb;
+  const int bt = rest >> 5, l = rest & 31;
+  const int b = fast_div(bt, j.div_rt), rt = bt - b * j.rt;
+  const int h = fast_div(col, j.div_h), c = col - h * (j.D >> 4);
+  it.s0 = rt * 128 + k0 * 32 + l;
+  const uint64_t src = reinterpret_cast<uint64_t>(j.x + b * j.sb + it.s0 * j.ss + h * j.sh + c * 16);
+  it.blk = ((uint32_t)b * j.S + it.s0) * (uint32_t)j.nb + col;
+  it.piece = ((((uint32_t)b * j.H + h) * j.rt + rt) * (uint32_t)(j.D >> 6) + (c >> 2)) * 32u + l;
+  const int lane = threadIdx.x & 31;
+  ld.a = reinterpret_cast<const __nv_bfloat16*>(__shfl_sync(0xffffffffu, src, lane >> 1)) + (lane & 1) * 8;
+  ld.b = reinterpret_cast<const __nv_bfloat16*>(__shfl_sync(0xffffffffu, src, 16 + (lane >> 1))) + (lane & 1) * 8;
+  ld.sa = __shfl_sync(0xffffffffu, it.s0, lane >> 1);
+  ld.sb = __shfl_sync(0xffffffffu, it.s0, 16 + (lane >> 1));
   return it;
 }
+// The rows of an item on their way to shared memory as one group of asynchronous copies.  Row k of warp w: 1 KB at
+// 1024 (8 k + w) of `stage`, piece p at place p ^ (p / 8 % 2) (a lane then reads its two pieces without bank conflicts).
+constexpr uint32_t kRowsStage = 4 * 8 * 1024;
+__device__ __forceinline__ uint32_t piece_at(uint32_t p) { return (p ^ ((p >> 3) & 1u)) * 16; }
+template <int kRows>
+__device__ __forceinline__ void load_rows(const QuantJob& j, const RowsLoad& ld, uint32_t stage) {
+  const uint32_t dst = stage + (threadIdx.x >> 5) * 1024 + piece_at(threadIdx.x & 31);
+#pragma unroll
+  for (int k = 0; k < kRows; ++k) {
+    if (ld.sa + 32 * k < j.S)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 8192 * k), "l"(ld.a + 32 * k * j.ss) : "memory");
+    if (ld.sb + 32 * k < j.S)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 8192 * k + 512), "l"(ld.b + 32 * k * j.ss) : "memory");
+  }
+}
+__device__ __forceinline__ void commit_copies() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
 // kRows = 4: the item's four rows; 1: row k0 of them (tensors too small to fill the GPU otherwise).
-// `raw` holds the item's rows; each is refilled with the row of the next item as soon as it has been
-// unpacked, so that its latency passes behind the arithmetic without a second set of registers.
 template <int kRows>
-__device__ __forceinline__ void quantize_rows_item(const QuantJob& j, const RowsItem& it, int k0, Words8 (&raw)[kRows],
-                                                   const RowsItem& next, bool has_next, const TensorScale& ts) {
-  const bool wide = j.wide != 0;
-  const int col = it.h * (j.D >> 4) + it.c;
-  uint8_t* dst = j.packed + (((int64_t)it.b * j.S + it.s0) * j.nb + col) * 8;
+__device__ __forceinline__ void quantize_rows_item(const QuantJob& j, const RowsItem& it, int k0, const uint8_t* stage,
+                                                   const TensorScale& ts) {
   uint32_t bytes = 0u;          // byte k: the scale of row k
 #pragma unroll
   for (int k = 0; k < kRows; ++k) {
+    const uint8_t* row = stage + (8 * k + (threadIdx.x >> 5)) * 1024;
+    const uint4 a = *reinterpret_cast<const uint4*>(row + piece_at(2 * (threadIdx.x & 31)));
+    const uint4 b = *reinterpret_cast<const uint4*>(row + piece_at(2 * (threadIdx.x & 31) + 1));
+    const Words8 raw = {{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
     float v[16];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      v[2 * i] = __uint_as_float(raw[k].w[i] << 16);
-      v[2 * i + 1] = __uint_as_float(raw[k].w[i] & 0xffff0000u);
+      v[2 * i] = __uint_as_float(raw.w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(raw.w[i] & 0xffff0000u);
     }
-    const float bmax = absmax16(raw[k]);
-    if (has_next && next.s0 + 32 * k < j.S) raw[k] = load32(next.src + 32 * k * j.ss, wide);
+    const float bmax = absmax16(raw);
     if (it.s0 + 32 * k < j.S) {
       uint32_t lo, hi, sfb;
       quantize_block16(v, bmax, ts, lo, hi, sfb);
       bytes |= sfb << (8 * k);
-      *reinterpret_cast<uint2*>(dst + (int64_t)(256 * k) * j.nb) = make_uint2(lo, hi);
+      *reinterpret_cast<uint2*>(j.packed + (uint64_t)(it.blk + 32u * k * j.nb) * 8) = make_uint2(lo, hi);
     }
   }
   // Four neighbouring lanes hold the four columns of a scale word.  kRows = 4: transpose the 4 x 4
   // bytes between them, so that lane q ends up with the word of row q and all four store.
-  const int q = it.c & 3;
-  int row = k0;
+  const int q = threadIdx.x & 3;
+  int row = 0;                  // (of the item: k0 stands in s0, blk and the piece's word)
   bool mine = true;
   if (kRows == 4) {
     uint32_t p = __shfl_xor_sync(0xffffffffu, bytes, 1);
@@ -345,12 +371,10 @@ __device__ __forceinline__ void quantize_rows_item(const QuantJob& j, const Rows
     bytes |= __shfl_xor_sync(0xffffffffu, bytes, 2);
     mine = q == 0;
   }
-  const int s = it.rt * 128 + row * 32 + it.l;
-  if (mine && j.lin != nullptr && s < j.S)
-    *reinterpret_cast<uint32_t*>(j.lin + ((int64_t)it.b * j.S + s) * j.nb + (col & ~3)) = bytes;
+  if (mine && j.lin != nullptr && it.s0 + 32 * row < j.S)
+    *reinterpret_cast<uint32_t*>(j.lin + (it.blk & ~3u) + (uint64_t)(32u * row * j.nb)) = bytes;
   if (mine && j.tiled != nullptr)
-    *reinterpret_cast<uint32_t*>(j.tiled + ((((int64_t)it.b * j.H + it.h) * j.rt + it.rt) * (j.D >> 6) + (it.c >> 2)) * 512 +
-                                 it.l * 16 + row * 4) = bytes;
+    *reinterpret_cast<uint32_t*>(j.tiled + (uint64_t)it.piece * 16 + (row + k0) * 4) = bytes;
 }
 
 // Where a V tile lies, and this thread's eight 16-byte pieces of it (128 keys x 16 chunks of 8 d).
@@ -366,27 +390,24 @@ __device__ __forceinline__ VTile v_tile_at(const QuantJob& j, int tile_idx) {
   t.d0 = (t.hd - t.bh * dt) * 128;
   return t;
 }
-__device__ __forceinline__ void load_v_tile(const QuantJob& j, const VTile& t, uint4 (&v)[8]) {
+// Copies the tile into shared memory asynchronously (zeros outside of the tensor) as one group of copies.
+__device__ __forceinline__ void load_v_tile(const QuantJob& j, const VTile& t, uint32_t tile) {
   const int b = fast_div(t.bh, j.div_h), h = t.bh - b * j.H;
   const __nv_bfloat16* src = j.x + b * j.sb + h * j.sh + t.d0;
+  const int ch = threadIdx.x & 15;
 #pragma unroll
   for (int n = 0; n < 8; ++n) {
-    const int i = threadIdx.x + 256 * n, key = t.kb0 * 128 + (i >> 4), ch = i & 15;
-    v[n] = make_uint4(0u, 0u, 0u, 0u);             // zero outside the tensor
-    if (key < j.S && t.d0 + ch * 8 < j.D) v[n] = *reinterpret_cast<const uint4*>(src + (int64_t)key * j.ss + ch * 8);
+    const int row = (threadIdx.x >> 4) + 16 * n, key = t.kb0 * 128 + row;
+    const bool in = key < j.S && t.d0 + ch * 8 < j.D;
+    // (row >> 4 == n)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tile + row * 256 + ((ch ^ n) << 4)),
+                 "l"(in ? src + (int64_t)key * j.ss + ch * 8 : j.x), "r"(in ? 16 : 0)
+                 : "memory");
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
 }
-// `raw` is refilled with the CTA's next tile once it has been stored to shared memory.
-__device__ __forceinline__ void quantize_v_tile(const QuantJob& j, const VTile& t, uint4 (&raw)[8], const VTile& next,
-                                                bool has_next, const TensorScale& ts, uint8_t* tile) {
+__device__ __forceinline__ void quantize_v_tile(const QuantJob& j, const VTile& t, const TensorScale& ts, const uint8_t* tile) {
   const int kt = j.rt, Sk = j.s_out, Dv = j.D, d0 = t.d0, k0 = t.kb0 * 128, tid = threadIdx.x;
-#pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    const int i = tid + 256 * n, key = i >> 4, ch = i & 15;
-    *reinterpret_cast<uint4*>(tile + key * 256 + ((ch ^ (key >> 4)) << 4)) = raw[n];
-  }
-  __syncthreads();
-  if (has_next) load_v_tile(j, next, raw);
   const int n_kb_total = Sk / 16;
 #pragma unroll 1
   for (int item = tid; item < 64 * 8; item += 256) {
@@ -447,11 +468,13 @@ __device__ __forceinline__ void quantize_v_tile(const QuantJob& j, const VTile& 
   }
 }
 
-constexpr int kQuantizeCtas = 2;     // per SM
-constexpr int kQuantizeVWeight = 24; // cost of a byte of V, that of Q and K being 16
+constexpr int kQuantizeCtas = 3;     // per SM
+constexpr uint32_t kQuantizeSmem = 2 * 128 * 256;   // two V tiles, or two items of every thread
+static_assert(kQuantizeSmem == 2 * kRowsStage, "two stages");
+constexpr int kQuantizeVWeight = 28; // cost of a byte of V, that of Q and K being 16
 __global__ void __launch_bounds__(256, kQuantizeCtas)
 quantize_kernel(const __grid_constant__ QuantJobs jobs) {
-  __shared__ __align__(16) uint8_t tile[128 * 256];  // [key][16 chunks of 16 B], chunk ^ (key/16)
+  extern __shared__ __align__(16) uint8_t tiles[];    // V: two of [key][16 chunks of 16 B], chunk ^ (key/16)
   __shared__ float warp_max[8];
   int ji = 0;
   while (ji + 1 < jobs.n && (int)blockIdx.x >= jobs.job[ji + 1].block0) ++ji;
@@ -466,22 +489,30 @@ quantize_kernel(const __grid_constant__ QuantJobs jobs) {
   int k0 = 0;
   VTile vt;
   RowsItem it;
-  union {
-    uint4 v[8];
-    Words8 rows[4];
-  } raw;
+  const uint32_t smem = smem_u32(tiles);
+  RowsLoad ld;
+  RowsItem next;
+  int tn = -1;
   if (j.is_v) {
     vt = v_tile_at(j, t);
-    load_v_tile(j, vt, raw.v);
+    load_v_tile(j, vt, smem);
   } else if (t >= 0) {
     if (j.single) {
       k0 = t / quarter;
-      t -= k0 * quarter;
+      it = rows_item_at(j, t - k0 * quarter, k0, ld);
+      load_rows<1>(j, ld, smem);
+      commit_copies();
+    } else {
+      it = rows_item_at(j, t, 0, ld);
+      load_rows<4>(j, ld, smem);
+      commit_copies();
+      tn = t - per_round;
+      if (tn >= 0) {
+        next = rows_item_at(j, tn, 0, ld);
+        load_rows<4>(j, ld, smem + kRowsStage);
+      }
+      commit_copies();
     }
-    it = rows_item_at(j, t, k0);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if ((k == 0 || !j.single) && it.s0 + 32 * k < j.S) raw.rows[k] = load32(it.src + 32 * k * j.ss, j.wide != 0);
   }
   float m = 0.f;
   for (int i = threadIdx.x; i < j.num_parts; i += 256) m = fmaxf(m, j.parts[i]);
@@ -500,27 +531,43 @@ quantize_kernel(const __grid_constant__ QuantJobs jobs) {
   if (j.scale_out != nullptr && first == 0 && threadIdx.x == 0) *j.scale_out = ts.g;
   if (j.is_v) {
 #pragma unroll 1
-    for (;;) {
-      const int tn = t - j.blocks;
-      const VTile next = v_tile_at(j, tn >= 0 ? tn : t);
-      quantize_v_tile(j, vt, raw.v, next, tn >= 0, ts, tile);
+    for (uint32_t buf = 0;; buf ^= 128 * 256) {
+      tn = t - j.blocks;
+      VTile vn = vt;
+      if (tn >= 0) {
+        vn = v_tile_at(j, tn);
+        load_v_tile(j, vn, smem + (buf ^ (128 * 256)));
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      __syncthreads();
+      quantize_v_tile(j, vt, ts, tiles + buf);
       if (tn < 0) break;
-      __syncthreads();            // the transpose buffer is read out
-      vt = next;
+      __syncthreads();            // the buffer is read out
+      vt = vn;
       t = tn;
     }
   } else if (t >= 0) {            // (items come in whole warps; lanes ascend with the blocks)
     if (j.single) {
-      quantize_rows_item<1>(j, it, k0, *reinterpret_cast<Words8(*)[1]>(&raw.rows[0]), it, false, ts);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncwarp();
+      quantize_rows_item<1>(j, it, k0, tiles, ts);
     } else {
 #pragma unroll 1
-      for (;;) {
-        const int tn = t - per_round;
-        const RowsItem next = rows_item_at(j, tn >= 0 ? tn : t, 0);
-        quantize_rows_item<4>(j, it, 0, raw.rows, next, tn >= 0, ts);
+      for (uint32_t buf = 0;; buf ^= kRowsStage) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        quantize_rows_item<4>(j, it, 0, tiles + buf, ts);
+        __syncwarp();             // (the stage is read out)
         if (tn < 0) break;
         it = next;
-        t = tn;
+        tn -= per_round;
+        if (tn >= 0) {
+          next = rows_item_at(j, tn, 0, ld);
+          load_rows<4>(j, ld, smem + buf);
+        }
+        commit_copies();
       }
     }
   }

@@ -132,3 +132,22 @@ def test_values_next_to_every_rounding_boundary(cuda_device):
         q = fa.quantize_qkv_fused(*(x.bfloat16().to(cuda_device),) * 3)[0]
         assert q.scale == want.scale
         assert np.array_equal(q.sf.cpu().numpy(), want.sf) and np.array_equal(q.data.cpu().numpy(), want.data), a
+
+
+@pytest.mark.parametrize("B,S,Hq,Hkv,D,std", [
+    (1, 130, 1, 1, 64, 1.0),         # four blocks a row: a warp's blocks lie in eight rows, two of them in the last tile
+    (3, 77, 3, 1, 64, 1.0),          # twelve blocks a row
+    (2, 2500, 32, 3, 128, 1.0),      # several items a thread, the last tile of rows not full, several V tiles a CTA
+    (1, 96, 2, 1, 128, 1e25),        # tensor scales beyond the two-term reciprocals
+    (1, 96, 2, 1, 128, 2.5e20),      # and just below that line: denominators near 1e20
+])
+def test_loads_in_stages_and_scales_at_the_ends(cuda_device, B, S, Hq, Hkv, D, std):
+    g = torch.Generator().manual_seed(B * S)
+    q, k, v = ((torch.randn(B, S, H, D, generator=g) * std).bfloat16() for H in (Hq, Hkv, Hkv))
+    Q, K, V = fa.quantize_qkv_fused(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device))
+    for got, want, mult in ((Q, _oracle_qk(q), 1), (K, _oracle_qk(k), 1), (V, _oracle_v(v), 2)):
+        assert got.scale == want.scale
+        assert np.array_equal(got.sf.cpu().numpy(), want.sf)
+        assert np.array_equal(got.data.cpu().numpy(), want.data)
+        lin = want.sf if got.is_v else np.transpose(want.sf, (0, 2, 1, 3))
+        assert np.array_equal(got.sf_tiled.cpu().numpy(), _tiled(lin, mult))

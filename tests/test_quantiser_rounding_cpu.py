@@ -51,3 +51,63 @@ def test_one_residual_step_keeps_every_quotient_on_its_side():
         open(c, "w").write(SRC)
         subprocess.run(["gcc", "-O2", "-fopenmp", "-mfma", "-ffp-contract=off", c, "-o", exe, "-lm"], check=True)
         assert int(subprocess.run([exe], capture_output=True, text=True, check=True).stdout) == 0
+
+
+TWO_TERMS = r'''
+#include <math.h>
+#include <stdio.h>
+static int side(float y, float b) { return (y > b) - (y < b); }
+static int e4m3(float t) {                     /* round to nearest even, saturating: an index of the value */
+  int e;
+  if (t > 448.f) t = 448.f;
+  if (t < 0x1p-6f) return (int)nearbyintf(t * 512.f);
+  const float m = nearbyintf(frexpf(t, &e) * 16.f);
+  return (e + 100) * 8 + (int)m;
+}
+int main(void) {
+  const float bounds[7] = {.25f, .75f, 1.25f, 1.75f, 2.5f, 3.5f, 5.f};
+  long bad = 0;
+  /* elements: x / d from 1 / d in two terms */
+#pragma omp parallel for reduction(+ : bad)
+  for (int m = 0; m < (1 << 23) - 1; ++m) {     /* the largest one: see the test */
+    const float d = 1.f + (float)m * 0x1p-23f;
+    for (int u = -1; u < 2; ++u) {
+      float r = 1.f / d;                                   /* rcp.approx.ftz: within one ulp of this */
+      if (u) r = nextafterf(r, u > 0 ? 2.f : 0.f);
+      const float rl = fmaf(-d, r, 1.f) * r;
+      for (int k = 0; k < 7; ++k) {
+        int e;
+        const double t = (double)bounds[k] * d;            /* exact */
+        const double s = floor(ldexp(frexp(t, &e), 8));
+        for (int j = -1; j <= 2; ++j) {                    /* two bf16 values on either side of the boundary */
+          const double n = s + j, n8 = n > 256 ? 2 * n - 256 : n < 128 ? 64 + n / 2 : n;    /* eight bits */
+          const float x = (float)ldexp(n8, e - 8);
+          bad += side(fmaf(x, r, x * rl), bounds[k]) != side(x / d, bounds[k]);
+        }
+      }
+    }
+  }
+  /* block scales: every block maximum and tensor maximum, their ratios down to scales that round to zero */
+  const float h6 = 1.f / 6.f, l6 = -4.967053731282552e-09f;
+  for (int ae = -20; ae <= 20; ae += 8)
+    for (int a = 128; a < 256; ++a) {
+      const float g = ldexpf(a, ae) / 2688.f, r = 1.f / g, rl = fmaf(-g, r, 1.f) * r;
+      for (int be = ae - 22; be <= ae; ++be)
+        for (int b = 128; b < 256; ++b) {
+          const float x = ldexpf(b, be), t = fmaf(x, h6, x * l6);
+          bad += e4m3(fmaf(t, r, t * rl)) != e4m3((x / 6.f) / g);
+        }
+    }
+  printf("%ld\n", bad);
+  return 0;
+}'''
+
+
+def test_reciprocals_in_two_terms_keep_every_code_and_block_scale():
+    """hi + lo of 1 / denom, 1 / 6 and 1 / g: the same e2m1 codes and e4m3 scales as correctly rounded quotients.  Left
+    out as above: the denominator 2 - 2^-23."""
+    with tempfile.TemporaryDirectory() as d:
+        c, exe = os.path.join(d, "t.c"), os.path.join(d, "t")
+        open(c, "w").write(TWO_TERMS)
+        subprocess.run(["gcc", "-O2", "-fopenmp", "-mfma", "-ffp-contract=off", c, "-o", exe, "-lm"], check=True)
+        assert int(subprocess.run([exe], capture_output=True, text=True, check=True).stdout) == 0
