@@ -107,7 +107,7 @@ struct Bars {
                             kSFull = kVFree + kStagesV, kSFree = kSFull + kSBufs,
                             kHand = kSFree + kSBufs, kPFull = kHand + 4 * kSBufs, kPvDone = kPFull + kPSlots,
                             kFin = kPvDone + kPSlots, kFinFree = kFin + 2, kOFree = kFinFree + 2,
-                            kDrain = kOFree + 1, kCount = kDrain + 2;
+                            kDrain = kOFree + 1, kOFree2 = kDrain + 2, kOFull = kOFree2 + 1, kCount = kOFull + 2;
   __device__ explicit Bars(uint32_t b) : base(b) {}
   __device__ __forceinline__ uint32_t at(uint32_t idx) const { return base + 8u * idx; }
 };
@@ -281,7 +281,8 @@ __device__ __forceinline__ uint32_t sw32_offset(uint32_t row, uint32_t chunk) {
 // waits for the P slot of a step before it issues the step's scores, one wait instead of 512.  Both
 // shorten the chain of a short tile and cost a long one: the branch sits in the hot loop, and Q K^T no
 // longer runs ahead of P V.  us, wide form -> this one: 127-key window, D = 64 83.6 -> 75.1; 1023 keys, D = 128
-// 106.5 -> 108.5 (the line lies in api.cu).
+// 106.5 -> 108.5 (the line lies in api.cu).  Of the 75, by masks that pass over the 32-key halves a warp sees whole and a
+// second accumulator, 69.6 are left.
 template <int kD, bool kGeneral = false, bool kWindow = kGeneral, bool kCache = kWindow, bool kNarrow = false,
           bool kCap = false>
 __global__ void __launch_bounds__(ws64::kThreads, 1)
@@ -340,6 +341,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       mbar_init(bars.at(Bars::kFinFree + b), 128);  // the epilogue warpgroup
     }
     mbar_init(bars.at(Bars::kOFree), 128);
+    if constexpr (kD == 64 && kNarrow) {            // two accumulators
+      mbar_init(bars.at(Bars::kOFree2), 128);
+      for (int b = 0; b < 2; ++b) mbar_init(bars.at(Bars::kOFull + b), 1);
+    }
     fence_barrier_init();
   }
   if (warp == kLoadKWarp && lane == 0) {
@@ -379,6 +384,11 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   constexpr int kDv = kD == 192 ? 128 : kD;            // head dim of V and O
   constexpr uint32_t idesc_qk = make_idesc_nvf4(128, 128);
   constexpr uint32_t idesc_pv = make_idesc_nvf4(128, kDv);
+  // Narrow windows at head dim 64 have tensor memory for two accumulators: P V of a tile, a handful of steps, does not
+  // wait for the one before to be read out.  us, one -> two: 127-key window 72.1 -> 69.6.
+  constexpr uint32_t kOBufs = kD == 64 && kNarrow ? 2 : 1;
+  auto o_column = [&](uint32_t tile) -> uint32_t { return kTmO + 64 * (tile % kOBufs); };
+  auto o_free = [&](uint32_t tile) -> uint32_t { return bars.at(tile % kOBufs ? Bars::kOFree2 : Bars::kOFree); };
   constexpr int kSteps = kD / 64;                      // 64-element steps of Q K^T
   constexpr uint32_t kQkBytes = 128u * kD / 2;         // bytes of a Q or K tile
   constexpr uint32_t kQkSfBytes = kSteps * 512u;       // its scale chunks (128 rows x kD / 16)
@@ -452,8 +462,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           }
         }
         const uint32_t Jl = 2 * gb + 2 * n - 1;
-        ok = __all_sync(0xffffffffu,
-                        mbar_wait_flag(bars.at(Bars::kPvDone + (Jl % kPSlots)), (Jl / kPSlots) & 1, s_abort));
+        // (with two accumulators the product that comes next to this P slot may be done before this wait begins, and
+        // its barrier a phase further: the accumulator has one of its own)
+        const uint32_t bar_o = kOBufs > 1 ? Bars::kOFull + ti % kOBufs : Bars::kPvDone + (Jl % kPSlots);
+        ok = __all_sync(0xffffffffu, mbar_wait_flag(bars.at(bar_o), (kOBufs > 1 ? ti / kOBufs : Jl / kPSlots) & 1, s_abort));
         if (!ok) break;
         tc_fence_after_sync();
         scale = (l_tot > 0.f) ? sc.out_scale / l_tot : 0.f;
@@ -468,11 +480,11 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
       for (int c = 0; c < (n > 0 ? kDv / 32 : 0); ++c) {
         uint8_t* box_row = out_row + (c >> 1) * (16 * 1024);
         uint32_t o[32];
-        tmem_ld32(lane_addr + kTmO + 32 * c, o);
+        tmem_ld32(lane_addr + o_column(ti) + 32 * c, o);
         tc_wait_ld();
         if (c == kDv / 32 - 1) {
           tc_fence_before_sync();
-          mbar_arrive(bars.at(Bars::kOFree));  // the P V issuer may start the next tile
+          mbar_arrive(o_free(ti));  // the P V issuer may start the next tile
         }
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -697,15 +709,15 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
             const uint32_t h64 = s;
             ok = mbar_wait(bars.at(Bars::kPFull + slot), (J / kPSlots) & 1, wc, kS64PFull);
             if (!ok) break;
-            if (i == 0 && s == 0 && ti >= 1) {
-              // O of the previous tile must have been copied out of tensor memory
-              ok = mbar_wait(bars.at(Bars::kOFree), (ti - 1) & 1, wc, kS64OFree);
+            if (i == 0 && s == 0 && ti >= kOBufs) {
+              // O of the tile before (the one before that) must have been copied out of tensor memory
+              ok = mbar_wait(o_free(ti), ((ti - kOBufs) / kOBufs) & 1, wc, kS64OFree);
               if (!ok) break;
             }
             tc_fence_after_sync();
             const uint32_t sfp = tmem + kTmSFP64 + 4 * tb, sfv = tmem + kTmSFV64 + 8 * st + 4 * h64;
             tc_cp_sf(sfp, base + kOffSFP + slot * 512);
-            mma_nvf4(tmem + kTmO, make_desc_sw32(base + kOffP + slot * kPTileBytes),
+            mma_nvf4(tmem + o_column(ti), make_desc_sw32(base + kOffP + slot * kPTileBytes),
                      make_desc_sw64(vt + 32 * h64), idesc_pv, sfp, sfv, (i > 0 || s > 0) ? 1u : 0u);
             tc_commit(bars.at(Bars::kPvDone + slot));
           }
@@ -713,6 +725,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           tc_commit(bars.at(Bars::kVFree + st));
         }
         if (!ok) break;
+        if (kOBufs > 1) tc_commit(bars.at(Bars::kOFull + ti % kOBufs));
         gb += n;
         ti += 1;
       }
@@ -828,7 +841,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         mbar_arrive(bars.at(Bars::kSFree + wg));
         if constexpr (kNarrow) {
           if (cut)
-            mask_scores64(s, lower_key(p, t, row, nb) - 64 * h64, upper_key<true>(p, t, row, nb) - 64 * h64);
+            // (D = 192, whose registers are scarcer here, loses by the skip: 37.6 -> 38.1 us)
+            mask_scores64<kD != 192>(s, lower_key(p, t, row, nb) - 64 * h64, upper_key<true>(p, t, row, nb) - 64 * h64,
+                                     lower_key(p, t, (warp & 3) * 32 + 31, nb) - 64 * h64,
+                                     upper_key<true>(p, t, (warp & 3) * 32, nb) - 64 * h64);
         }
         if constexpr (kCap) {
 #pragma unroll
@@ -910,7 +926,7 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           if (!ok) break;
           tc_fence_after_sync();
           const float f = fix ? reference_factor(m_prev, m_new, sc.sl2) : 1.f;
-          rescale_accumulator(lane_addr + kTmO, f, kDv / 32);
+          rescale_accumulator(lane_addr + o_column(ti), f, kDv / 32);
           tc_wait_st();
         }
         fence_proxy_async_smem();

@@ -28,6 +28,19 @@ def test_window_forms_over_several_tiles_per_cta(cuda_device, window, D):
     assert_parity(out, lse, *oracles(Q, K, V, False, window=window))
 
 
+@pytest.mark.parametrize("Sk", [900, 500])       # 500: the first tiles see nothing and take no accumulator
+@pytest.mark.parametrize("window", [(0, 0), (127, 0), (255, 1)])
+def test_two_accumulators_in_turn(cuda_device, window, Sk):
+    """Head dim 64, narrow windows, more than three tiles of one to eight steps per CTA; windows whose limits cut a warp's
+    halves of 32 keys and others that leave them whole."""
+    q, k, v = make_qkv(1, 900, Sk, 64, 4, 64, seed=6, device=cuda_device)
+    Q, K, V = fa.quantize_qkv(q, k, v)
+    out, lse = fa.flash_attn_func(Q, K, V, window_size=window, return_lse=True)
+    torch.cuda.synchronize()
+    fa.check_status(cuda_device)
+    assert_parity(out, lse, *oracles(Q, K, V, False, window=window))
+
+
 @pytest.mark.parametrize("causal", [True, False])
 @pytest.mark.parametrize("lens", [[700, 1, 130, 390, 5, 700, 64, 257, 129, 31],      # a slot per row block of the longest
                                   [1025, 1, 130, 1300, 5, 128, 64, 257, 129, 31, 0, 897],   # only the tiles that exist
