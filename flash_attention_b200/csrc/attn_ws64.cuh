@@ -277,12 +277,10 @@ __device__ __forceinline__ uint32_t sw32_offset(uint32_t row, uint32_t chunk) {
 // which measured 16 % faster than carrying the window arithmetic along.)
 // kCache: per-entry key counts and page tables without the window arithmetic.
 // kNarrow (windows of a few blocks): most visited blocks are masked and a tile is over after a handful of
-// steps.  Masks go to the scores in registers instead of through tensor memory, and the Q K^T issuer
-// waits for the P slot of a step before it issues the step's scores, one wait instead of 512.  Both
-// shorten the chain of a short tile and cost a long one: the branch sits in the hot loop, and Q K^T no
-// longer runs ahead of P V.  us, wide form -> this one: 127-key window, D = 64 83.6 -> 75.1; 1023 keys, D = 128
-// 106.5 -> 108.5 (the line lies in api.cu).  Of the 75, by masks that pass over the 32-key halves a warp sees whole and a
-// second accumulator, 69.6 are left.
+// steps.  Masks go to the scores in registers instead of through tensor memory, which shortens the chain of a short
+// tile and costs a long one, since the branch sits in the hot loop.  us, wide form -> this one: 127-key window, D = 64
+// 83.6 -> 75.1; 1023 keys, D = 128 106.5 -> 108.5 (the line lies in api.cu).  Of the 75, by masks that pass over the
+// 32-key halves a warp sees whole and a second accumulator, 69 are left.
 template <int kD, bool kGeneral = false, bool kWindow = kGeneral, bool kCache = kWindow, bool kNarrow = false,
           bool kCap = false>
 __global__ void __launch_bounds__(ws64::kThreads, 1)
@@ -389,6 +387,22 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   constexpr uint32_t kOBufs = kD == 64 && kNarrow ? 2 : 1;
   auto o_column = [&](uint32_t tile) -> uint32_t { return kTmO + 64 * (tile % kOBufs); };
   auto o_free = [&](uint32_t tile) -> uint32_t { return bars.at(tile % kOBufs ? Bars::kOFree2 : Bars::kOFree); };
+  // Where the softmax step is cut for the compiler's scheduler.  Left as one piece, exponentials of a step can move up
+  // among its maxima and hand-over, which the next warpgroup waits for; what kept them apart was a wait for
+  // the P slot between the two, which now is the Q K^T issuer's.  Which cut pays differs by form.  us, wait / no cut /
+  // in front of the exponentials / of the maxima / both:
+  //   plain: causal GQA, B=2, S=8192 660 / 699 / 646 / 728 / 640, at D = 64 656 / 689 / 638 / 727 / 633
+  //   D = 128: 24 packed sequences 166.6 / 163.9 / 166.1 / 215.5 / 167.6; 512 tokens against 32768 keys of a cache 199.5 / 196.0 /
+  //     199.6 / 296 / 199.5; windows of 1023, 4096 keys 219.4 / 217.7 / 219.2 / 295 / 231.5, 565.9 / 564.8 / 567.7 / 844 / 578
+  //   D = 64: 100 packed sequences 154.2 / 158.3 / 153.2 / 158.1 / 155.0, 8 long ones 168.2 / 182.5 / 165.6 / 177.0 / 166.6; windows
+  //     of 1023, 16383 keys 212.0 / 208.8 / 207.5 / 220.8 / 212.7, 1388 / 1376 / 1352 / 1544 / 1387
+  //   D = 192: 20 packed sequences 126.3 / 134.4 / 124.9 / 129.9 / 124.1, 60 short ones 72.5 / 74.4 / 72.0 / 73.9 / 72.8
+  // Further cuts in the plain form: in front of the reference 643, between the maxima 643, in front of the last
+  // stores 645, between the 16-key blocks 656 and 680.
+  constexpr bool kPlain = !(kWindow || kCache);
+  // The soft cap's forms (its 64 tanh stand in front of the maxima) take the first cut alone: plain, wait / first cut / both
+  // 358 / 352 / 362, at D = 64 355 / 348 / 356, window of 1023 keys, wait / none / first 182 / 196 / 181.
+  constexpr bool kCutExp = !kNarrow && (kPlain || kD != 128 || kCap), kCutMax = kPlain && !kCap;
   constexpr int kSteps = kD / 64;                      // 64-element steps of Q K^T
   constexpr uint32_t kQkBytes = 128u * kD / 2;         // bytes of a Q or K tile
   constexpr uint32_t kQkSfBytes = kSteps * 512u;       // its scale chunks (128 rows x kD / 16)
@@ -659,7 +673,8 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           // (keys 0-63 and 64-127 of the tile): half the tcgen05 instructions of two N = 64
           // products, and the in-order issue slots of this thread are scarce
           const uint32_t J0 = 2 * G, b0 = J0 % kSBufs;  // 0 or 2
-          if (kNarrow && J0 >= kPSlots) {
+          // P of step J0 + 1 goes where P of step J0 + 1 - kPSlots is (and the softmax warps have no wait of their own for it)
+          if (J0 >= kPSlots) {
             ok = mbar_wait(bars.at(Bars::kPvDone + ((J0 + 1) % kPSlots)), ((J0 + 1 - kPSlots) / kPSlots) & 1, wc, kS64PvDone);
             if (!ok) break;
           }
@@ -769,8 +784,6 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         const int nb = kWindow ? window_visit_block(j >> 1, t) : (j >> 1);
         const int h64 = j & 1;
         const uint32_t bar_s = bars.at(Bars::kSFull + (wg & 2)), par_s = (J / kSBufs) & 1;
-        const uint32_t bar_p = bars.at(Bars::kPvDone + slot), par_p = ((J - kPSlots) / kPSlots) & 1;
-        const bool r_p = (kNarrow || J < kPSlots) ? true : mbar_test(bar_p, par_p);
 
         // 1. the scores of this sub-block: the whole 64-key row of this thread
         ok = __all_sync(0xffffffffu, mbar_test(bar_s, par_s)) || __all_sync(0xffffffffu, mbar_wait_flag(bar_s, par_s, s_abort));
@@ -798,10 +811,6 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
             mbar_arrive(bars.at(Bars::kHand + 4 * wg + (warp & 3)));
             if (m_prev != m_ref) l_sum *= reference_factor(m_ref, m_prev, sc.sl2);
             m_ref = m_prev;
-            if constexpr (!kNarrow) {
-              ok = __all_sync(0xffffffffu, r_p) || __all_sync(0xffffffffu, mbar_wait_flag(bar_p, par_p, s_abort));
-              if (!ok) break;
-            }
             uint8_t* p_tile = gbase + kOffP + slot * kPTileBytes;
             *reinterpret_cast<uint4*>(p_tile + sw32_offset(row, 0)) = make_uint4(0u, 0u, 0u, 0u);
             *reinterpret_cast<uint4*>(p_tile + sw32_offset(row, 1)) = make_uint4(0u, 0u, 0u, 0u);
@@ -852,6 +861,10 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         }
 
         // 2. maxima of the four 16-key blocks, then the new reference
+        if constexpr (kCutMax) {
+          ok = code_boundary(slot + 2);
+          if (!ok) break;
+        }
         float bm4[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -874,6 +887,8 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
           ok = receive(J, j, m_prev);
           if (!ok) break;
         }
+        // (a seam for the compiler's scheduler here: 127-key window 90 -> 86.5 us, at D = 64 69.7 -> 69.0)
+        if constexpr (kNarrow) __syncwarp();
         const float m_new = next_reference(m_prev, m_loc, sc.sl2);
         s_hand[wg * 128 + row] = m_new;
         mbar_arrive(bars.at(Bars::kHand + 4 * wg + (warp & 3)));
@@ -894,9 +909,9 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
         if (m_new != m_ref) l_sum *= reference_factor(m_ref, m_new, sc.sl2);
         m_ref = m_new;
 
-        // 3. exponentials and quantisation; P slot J % 8 is free once P V of sub-block J - 8 has run
-        if constexpr (!kNarrow) {
-          ok = __all_sync(0xffffffffu, r_p) || __all_sync(0xffffffffu, mbar_wait_flag(bar_p, par_p, s_abort));
+        // 3. exponentials and quantisation; P slot J % 8 is free: P V of sub-block J - 8 had run before these scores were made
+        if constexpr (kCutExp) {
+          ok = code_boundary(slot + 1);
           if (!ok) break;
         }
         uint8_t* p_tile = gbase + kOffP + slot * kPTileBytes;

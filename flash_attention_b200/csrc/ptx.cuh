@@ -74,6 +74,22 @@ __device__ __forceinline__ bool elect_one() {
   return ok != 0;
 }
 
+// True, for any `nonzero` that is not zero, by way of a vote that the compiler cannot foresee: code behind a branch on
+// it is not moved in front of it.
+__device__ __forceinline__ bool code_boundary(uint32_t nonzero) {
+  uint32_t all;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 p, %1, 0;\n"
+      "vote.sync.all.pred q, p, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, q;\n"
+      "}\n"
+      : "=r"(all)
+      : "r"(nonzero));
+  return all != 0;
+}
+
 // ---------------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------------
