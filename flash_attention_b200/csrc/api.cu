@@ -222,13 +222,25 @@ int64_t balanced_bytes(const fa4_nvfp4_params* p) {
 //   four tokens (16 rows), 1024 blocks: 6, 16 entries 9.9 / 11.0, 9.7 / 10.9; 2048: 13.8 / 12.3, 12.4 / 10.5; 4096: 21.8 / 18.1,
 //     19.2 / 12.5; eight (32 rows): 1024: 16.4 / 13.6, 13.3 / 13.9; 2048: 18.3 / 16.2, 16.7 / 12.5; 4096: 30.4 / 23.8, 26.7 / 16.4
 // (Above eight rows a block takes one softmax warpgroup longer, so a long entry costs more.)
+// A batch of few units is cut into the more pieces each (444 places), and the second launch merges them row by
+// row: the line rises as the units become fewer.  us, equal / dealt, one kv head unless two are given, last equal and first
+// faster one:
+//   8 rows: 5 units 20000 blocks 43.5 / 47.5, 32000 71.3 / 67.5; 8: 13000 31.3 / 33.2, 20000 40.8 / 38.1; 16: 6500 20.0 /
+//     20.6, 9000 23.0 / 21.5; 32: 6500 19.7 / 17.6; 4 rows, two heads, 10: 13000 30.5 / 30.9, 20000 45.6 / 41.3
+//   16 rows: 3: 16000 62.4 / 66.9, 24000 77.7 / 64.1; 4: 2200 14.2 / 23.5, 12000 49.0 / 49.5, 16000 57.5 / 49.0; 8: 6500 25.5 /
+//     26.7, 9000 36.2 / 30.4; 16, two heads: 3200 17.1 / 17.7, 4500 21.3 / 20.2; 20: 3300 16.1 /
+//     16.8; 32: 2200 14.0 / 12.4
+//   32 rows: 4: 6500 42.9 / 45.6, 9000 46.4 / 41.7; 8: 2200 19.2 / 19.5, 3200 24.8 / 23.1; 16: 2200 17.5 / 15.4
 bool decode_balanced(const fa4_nvfp4_params* p, const int32_t* seqused_k) {
   if (seqused_k == nullptr || p->B < 3 || p->B > dec::kMaxBalanced || p->Sk > dec::kMaxBalancedKeys) return false;
   const int64_t units = (int64_t)p->B * p->Hkv, blocks = units * ((p->Sk + kBlockN - 1) / kBlockN);
   const int slots = balanced_slots(p);
   if (units > 2 * slots || balanced_ctas(p) > dec::kMaxBalancedCtas || blocks > dec::kMaxBalancedBlocks) return false;
   if (units > slots) return blocks >= 40 * units;
-  return blocks >= std::max<int64_t>(p->Sq * (p->Hq / p->Hkv) > 8 ? 2048 : (units < 40 ? 6144 : 4096), 24 * units);
+  const int rows = p->Sq * (p->Hq / p->Hkv);
+  const int64_t least = rows > 8 ? 2048 : (units < 40 ? 6144 : 4096);
+  const int64_t few = units >= 32 ? 0 : (rows > 16 ? 32000 : (rows > 8 ? 72000 : 144000)) / units;
+  return blocks >= std::max({least, few, 24 * units});
 }
 int64_t splitkv_bytes(const fa4_nvfp4_params* p, int num_splits) {
   // partial O (num_splits, B, Sq, Hq, Dv) fp32, then partial LSE (num_splits, B, Hq, Sq) fp32
