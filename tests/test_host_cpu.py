@@ -394,7 +394,7 @@ def test_first_calls_of_two_threads_share_one_status_word(monkeypatch):
 
 @pytest.mark.parametrize("args,dealt", [
     # B, Sq, Sk, Hq, Hkv: few units are dealt from the more blocks on the fewer they are
-    ((4, 2, 70400, 8, 1), 0), ((4, 2, 512000, 8, 1), 1), ((8, 2, 51200, 8, 1), 0), ((16, 2, 35968, 8, 1), 1),
+    ((4, 2, 70400, 8, 1), 0), ((4, 2, 600000, 8, 1), 1), ((8, 2, 51200, 8, 1), 0), ((16, 2, 40000, 8, 1), 1),
     ((4, 4, 102400, 8, 1), 0), ((8, 4, 71936, 8, 1), 1), ((5, 1, 409600, 8, 1), 0), ((16, 1, 80000, 8, 1), 1), ((20, 2, 21004, 8, 1), 0), ((32, 2, 8704, 8, 1), 1),
     ((16, 1, 8192, 32, 8), 1), ((2, 1, 1 << 20, 32, 8), 0)], ids=str)
 def test_which_decode_calls_are_dealt_by_the_lengths(args, dealt):
