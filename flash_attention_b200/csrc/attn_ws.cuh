@@ -777,6 +777,8 @@ attn_fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q,
         l_sum += quantize_pair(&s[0], noff4[0], noff4[1],
                                __byte_perm(ue, 0u, 0x4440u), __byte_perm(ue, 0u, 0x4441u), sc.sl2, chunk);
         *reinterpret_cast<uint4*>(p_tile + sw64_offset(row, 2 * half)) = chunk;
+        ok = code_boundary(b + 2);       // (see quantize_pair)
+        if (!ok) break;
         l_sum += quantize_pair(&s[32], noff4[2], noff4[3],
                                __byte_perm(ue, 0u, 0x4442u), __byte_perm(ue, 0u, 0x4443u), sc.sl2, chunk);
         *reinterpret_cast<uint4*>(p_tile + sw64_offset(row, 2 * half + 1)) = chunk;
