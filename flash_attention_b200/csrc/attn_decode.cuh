@@ -56,7 +56,7 @@ namespace dec {
 // trip, so five are better whenever no third CTA is there to run.
 // (Registers: three CTAs of 384 threads leave 56, two of 640 leave 48, and up to eight rows the kernel wants more.  Bytes
 // of spill stores, merging / not: shallow 4 / 28, with linear scales 96 / 112-136; deep, four rows 48 / 84, 176 / 100;
-// eight rows 100 / 40, 212 / 136.  None above eight rows.  Balanced, shallow: 12-20, with linear scales 132.  With them the deep form is still the faster one for ragged
+// eight rows 100 / 40, 212 / 136.  None above eight rows.  Balanced, shallow: 16-24, with linear scales 76-132.  With them the deep form is still the faster one for ragged
 // batches, see softmax_wgs, and reading linear scales faster than a launch of its own, see linear_keys_limit in
 // host.cpp, whose line is nearer for five to eight rows.)
 constexpr int kMaxCluster = 8;  // splits that are merged inside a cluster (portable cluster size)
@@ -66,7 +66,10 @@ constexpr int kMaxBalanced = 128, kMaxBalancedKeys = 1 << 26, kMaxBalancedBlocks
 // Blocks below which a unit is not cut further.  (Two, three, four: one token, 48 entries up to 4096 keys of one head 10.7,
 // 10.6, 10.7 us; four tokens, 6 entries up to 2048 of 8 heads 9.6, 9.8, 11.0.)
 constexpr int kMinBlocks = 3;
-constexpr float kResetLimit = 6.f;       // log2 units a reference may fall by where a split starts inside of a CTA
+// log2 units by which references may fall, in all, below the highest one that a row has had in its CTA: O and the row sum
+// grow by as much (2^64 on top of the 2^10 of a weight, the 2^12 of a value and the 2^26 of the keys), and what lies further down
+// is nothing beside what is there.
+constexpr float kMaxFall = 64.f;
 // Softmax warpgroups: one above eight rows; up to eight, two in the shallow form (registers: three CTAs of
 // twelve warps per SM leave 56 per thread) and four in the deep one, whose long entries run on with few CTAs
 // beside them: a block is a chain of some 1700 clocks in its warpgroup, and only the reference is handed
@@ -474,9 +477,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     sk = used < 0 ? 0 : (used < p.Sk ? used : p.Sk);
   }
   int i0, n;
-  // kBalanced: the references of the rows follow the splits, not the CTAs, so that how P is rounded does not depend on
-  // how many CTAs there are.  A reference starts anew with every split (at li = next_start), and a CTA that begins
-  // inside of one visits that one's first block before its own (pre = 1), for the reference alone.
+  // kBalanced: the references of the rows follow the splits, not the CTAs: a reference starts anew with every split (at
+  // li = next_start), and a CTA that begins inside of one visits that one's first block before its own (pre = 1), for the
+  // reference alone.  P is then rounded as with a CTA per split, but for rows whose reference moves inside of a split, in blocks
+  // that the CTA passes over.
   int pre = 0, next_start = 1 << 30;
   if constexpr (kBal) {
     pre = work.n > 0 && work.into > 0 ? 1 : 0;
@@ -743,6 +747,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     // last block; so a row's sum is the same bits with two warpgroups and with four.  With two, a thread has two,
     // of which shared memory keeps the one that is not in use.
     float m_ref = kNegInf, l_sum = 0.f;
+    float m_top = kNegInf;       // kBalanced: the highest reference so far (a warpgroup sees its own and those handed to it: all)
+    static_assert(!kBal || kWgs <= 2, "every reference passes through every warpgroup");
     float2* strands = reinterpret_cast<float2*>(gbase + L::kOffSum) + wg * 128 + (tid & 127);    // [2][256]
     if (kOwn == 2) strands[0] = strands[256] = make_float2(0.f, kNegInf);
     // last visible key of the row (causal: bottom-right aligned on the entry's key count); rows
@@ -811,11 +817,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       if constexpr (kBal) {
         while (next_start < li) next_start += work.share;
         if (next_start == li) {
-          // A split starts: its reference is the maximum of this block.  Not where that lies far below the one
-          // before (or where the row sees no key): what the split adds is then nothing beside what is there, and the
-          // factors stay finite.
-          m_new = m_prev == kNegInf || (m_prev - m_loc) * sc.sl2 <= kResetLimit ? m_loc : m_prev;
+          // A split starts: its reference is the maximum of this block, up to kMaxFall below the highest one (further
+          // down, or where the row sees no key, the one before stays).
+          m_new = m_prev == kNegInf || (fmaxf(m_top, m_prev) - m_loc) * sc.sl2 <= kMaxFall ? m_loc : m_prev;
         }
+        m_top = fmaxf(m_top, fmaxf(m_prev, m_new));
         if (pre != 0 && li == 0) {
 #pragma unroll
           for (int j = 0; j < kR; ++j) x[j] = kNegInf;
@@ -957,8 +963,11 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
       // Per row, the lanes of a row alike: the sum over the warps in a fixed order (it does not depend on
       // timing), brought to the last reference of the row; the factor of the output; the LSE
       float scale = 0.f, lse = kNegInf;
+      [[maybe_unused]] float back = 1.f;
+      [[maybe_unused]] bool fell = false;
       if (ok) {
         float m_s[kStrands], l_s[kStrands], m_fin = kNegInf, l_tot = 0.f;
+        [[maybe_unused]] float m_last = kNegInf;       // kBalanced: the last reference, that of O
 #pragma unroll
         for (int i = 0; i < kStrands; ++i) {
           // strand i is one of warpgroup w, which did c blocks: that of its last block, with the sums in the buffer of
@@ -969,9 +978,14 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           l_s[i] = ((sum[0] + sum[kN]) + sum[2 * kN]) + sum[3 * kN];
           const float handed = s_hand[w * 4 * kN + my_row];
           m_s[i] = !last ? s_old[(w * 5 + 4) * kN + my_row] : (w == 0 ? m_ref : handed);
-          // (of the last block; the references of a CTA only grow, but for those of a new split)
-          if constexpr (kBal) m_fin = i == (n - 1) % kStrands ? m_s[i] : m_fin;
-          else m_fin = fmaxf(m_fin, m_s[i]);
+          m_fin = fmaxf(m_fin, m_s[i]);
+          if constexpr (kBal) m_last = i == (n - 1) % kStrands ? m_s[i] : m_last;
+        }
+        if constexpr (kBal) {
+          // the sum goes to the highest reference, where it is of ordinary size; so does O, below
+          m_fin = fmaxf(m_fin, m_top);
+          back = reference_factor(m_last, m_fin, sc.sl2);
+          fell = m_last != m_fin;
         }
 #pragma unroll
         for (int i = 0; i < kStrands; ++i) l_tot = fmaf(l_s[i], reference_factor(m_s[i], m_fin, sc.sl2), l_tot);
@@ -988,6 +1002,10 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
           tc_fence_after_sync();
           tmem_ld_cols<kR>(lane_addr + TM::kO, reinterpret_cast<uint32_t*>(o));
           tc_wait_ld();
+          if (kBal && __any_sync(0xffffffffu, fell)) {
+#pragma unroll
+            for (int r = 0; r < kR; ++r) o[r] *= __shfl_sync(0xffffffffu, back, r);
+          }
         }
       }
       if (ok) {

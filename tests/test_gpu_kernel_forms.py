@@ -394,8 +394,8 @@ def test_decode_dealt_by_the_lengths(cuda_device, Sq, Hq, Hkv, Sk, lens, layout,
 
 def test_decode_dealt_by_the_lengths_where_references_move(cuda_device):
     """Scores that grow and shrink along the keys by up to 40 log2 units, so that references move within splits, fall where one
-    starts, or are kept there (more than kResetLimit below): against exact attention, no further off than the entries
-    alone are (with the quarter that the parity tests allow P's rounding)."""
+    starts: against exact attention, no further off than the entries alone are (with the quarter that the parity tests allow
+    P's rounding)."""
     B, Sk, Hq, Hkv = 6, 12288, 8, 8
     lens = [12288, 5000, 700, 12000, 3000, 129]
     g = torch.Generator(device=cuda_device).manual_seed(22)
@@ -421,3 +421,78 @@ def test_decode_dealt_by_the_lengths_where_references_move(cuda_device):
             assert e_got <= 1.25 * e_alone + 0.01, (splits, b, e_got, e_alone)
             assert (lse[b, :, 0] - s.logsumexp(-1)[0, :, 0]).abs().max() <= 1e-3 * s.abs().max()
     fa.check_status(cuda_device)
+
+
+def _long_beside(device, B, Sq, Sk, Hq, Hkv, lens, level, v_mean, splits):
+    """Decode against a cache in which entry 0 has scores `level[key]` (log2 units, the same for all rows but a few per cent) plus
+    noise, among entries of zeros.  Returns the relative error of entry 0 in the batch and of entry 0 alone (O), and the
+    errors of the LSEs."""
+    g = torch.Generator(device=device).manual_seed(23)
+    n = lens[0]
+    u = (torch.randint(0, 2, (Hkv, 1, 128), generator=g, device=device) * 2 - 1) / math.sqrt(128.0)
+    q = torch.zeros(B, Sq, Hq, 128, device=device)
+    k = torch.zeros(B, Sk, Hkv, 128, device=device, dtype=torch.bfloat16)
+    v = torch.zeros(B, Sk, Hkv, 128, device=device, dtype=torch.bfloat16)
+    # q = 8 u: a score in log2 units is 8 (u . k) / sqrt(128) * log2(e) = 1.0201 (u . k)
+    rise = 1.0 + 0.05 * torch.rand(Sq, Hkv, Hq // Hkv, 1, generator=g, device=device)
+    q[0] = (8.0 * rise * u).reshape(Sq, Hq, 128)
+    # (as a thermometer over the eight scale blocks of a row, whose scales have steps of 6 to 12 %)
+    lev = (level / 1.0201).to(device)
+    top = lev.max() + 1e-3
+    lev = (8.0 * lev[:, None] - top * torch.arange(8, device=device)).clamp(min=0.0).minimum(top).repeat_interleave(16, dim=1)
+    k[0, :n] = (lev[:, None, :] * u[:, 0] + 0.05 * torch.randn(n, Hkv, 128, generator=g, device=device)).bfloat16()
+    v[0, :n] = (v_mean[:, None, None].to(device) + 0.5 * (v_mean != 0)[:, None, None].to(device) *
+                torch.randn(n, Hkv, 128, generator=g, device=device)).bfloat16()
+    Q, K, V = fa.quantize_qkv_fused(q.bfloat16(), k, v)
+    used = torch.tensor(lens, dtype=torch.int32, device=device)
+    T = (Q.data, K.data, V.data, Q.sf, K.sf, V.sf)
+    call = lambda t, u, s: fa.flash_attn_fp4_func(*t, Q.scale, K.scale, V.scale, causal=True, num_splits=s, seqused_k=u,
+                                                  return_lse=True)
+    got, lse = (x[:1] for x in call(T, used, splits))
+    if splits == 0:
+        splits = fa._lib.host().choose_decode_splits(B, Hkv, Sk, 148)
+    alone, lse_alone = call([t[:1] for t in T], used[:1], splits)
+    fa.check_status(device)
+    qd = Q.dequantize()[:1].double()
+    kd = fa.quant.dequantize_lastdim(K.data[:1], K.sf[:1], K.scale)[0, :n].double()
+    vd = fa.quant.dequantize_lastdim(V.data[:1], V.sf[:1], V.scale)[0, :, :, :n].double()
+    qg = qd[0].view(Sq, Hkv, Hq // Hkv, 128)
+    s = torch.einsum("shgd,nhd->hgsn", qg, kd) / math.sqrt(128)
+    s = s.masked_fill(torch.arange(n, device=device)[None, :] > n - Sq + torch.arange(Sq, device=device)[:, None], -math.inf)
+    exact = torch.einsum("hgsn,hdn->shgd", s.softmax(-1), vd).reshape(1, Sq, Hq, 128)
+    exact_lse = s.logsumexp(-1).reshape(1, Hq, Sq)
+    err = lambda x: ((x.double() - exact).norm() / exact.norm()).item()
+    err_lse = lambda x: ((x.double() - exact_lse).abs().max() / max(1.0, exact_lse.abs().max().item())).item()
+    assert torch.isfinite(alone).all()
+    return err(got), err(alone), err_lse(lse), err_lse(lse_alone)
+
+
+@pytest.mark.parametrize("Sq,group", [(1, 4), (1, 8), (4, 4), (8, 4)])
+@pytest.mark.parametrize("fall", [1.0, 2.0, 3.0, 5.0])
+def test_decode_of_maxima_that_fall_from_split_to_split(cuda_device, Sq, group, fall):
+    """128 blocks, a split each, whose maxima fall by 128 to 640 log2 units in all, in an entry of a batch that leaves it to few
+    CTAs: finite, and no further from exact attention than the entry alone (with the quarter that the parity tests allow
+    P's rounding)."""
+    n, B = 16384, 40
+    level = fall * (127 - torch.arange(n) // 128)
+    e, e_alone, l, _ = _long_beside(cuda_device, B, Sq, n, 8 * group, 8, [n] * B, level, torch.ones(n), 128)
+    assert e <= 1.25 * e_alone + 0.01 and l <= 1e-3, (e, e_alone, l)
+
+
+def test_decode_of_maxima_that_fall_with_chosen_splits(cuda_device):
+    n, Sk, B = 4608, 288000, 8
+    level = 4.0 * (35 - torch.arange(n) // 128)
+    e, e_alone, l, _ = _long_beside(cuda_device, B, 1, Sk, 8, 1, [n] + [Sk] * (B - 1), level, torch.ones(n), 0)
+    assert e <= 1.25 * e_alone + 0.01 and l <= 1e-3, (e, e_alone, l)
+
+
+@pytest.mark.parametrize("Sq", [1, 8])
+@pytest.mark.parametrize("height", [10.0, 12.0, 14.0, 16.0, 18.0, 40.0])
+def test_decode_behind_a_first_key_without_a_value(cuda_device, Sq, height):
+    """A first key far above the rest whose V is zero (an attention sink), ten splits of one block each: what the other splits add is
+    the whole result, and is no further off than in the entry alone."""
+    n, Sk, B = 1280, 16384, 40
+    level, v_mean = torch.zeros(n), torch.ones(n)
+    level[0], v_mean[0] = height, 0.0
+    e, e_alone, l, _ = _long_beside(cuda_device, B, Sq, Sk, 32, 8, [n] + [Sk] * (B - 1), level, v_mean, 10)
+    assert e <= 1.25 * e_alone + 0.01 and l <= 1e-3, (e, e_alone, l)
