@@ -246,6 +246,11 @@ int64_t splitkv_bytes(const fa4_nvfp4_params* p, int num_splits) {
   // partial O (num_splits, B, Sq, Hq, Dv) fp32, then partial LSE (num_splits, B, Hq, Sq) fp32
   return (int64_t)num_splits * p->B * p->Sq * p->Hq * ((int64_t)p->Dv + 1) * 4;
 }
+// Workspace with which a call is dealt by the lengths: more than its splits need, so that a caller who has room for those alone
+// gets them, whatever their number.
+int64_t dealt_bytes(const fa4_nvfp4_params* p, int num_splits) {
+  return (decode_in_cluster(p, num_splits) ? 0 : splitkv_bytes(p, num_splits)) + balanced_bytes(p);
+}
 // KV-cache view of K / V: per-entry key counts and / or a page pool (see fa4_nvfp4_ext).
 struct CacheView {
   const int32_t* seqused_k = nullptr;
@@ -425,7 +430,7 @@ extern "C" int64_t fa4_nvfp4_fwd_ex_workspace_bytes(const fa4_nvfp4_params* p, c
   const int64_t bytes = fa4_nvfp4_splitkv_workspace_bytes(p, x->num_splits == 0 ? 1 : x->num_splits);
   if (bytes < 0 || p->variant != FA4_VARIANT_DECODE || p->Hkv <= 0 || p->Hq < p->Hkv || !decode_balanced(p, x->seqused_k))
     return bytes;
-  return std::max(bytes, balanced_bytes(p));
+  return dealt_bytes(p, x->num_splits == 0 ? 1 : x->num_splits);
 }
 
 extern "C" int fa4_nvfp4_fwd_splitkv(const fa4_nvfp4_params* p, int32_t num_splits, void* workspace,
@@ -485,7 +490,7 @@ int validate_fwd(const fa4_nvfp4_params* p, int num_splits, const void* workspac
     if (p->D != 128 || p->Dv != 128 || (int64_t)p->Sq * (p->Hq / p->Hkv) > dec::kMaxRows) return -FA4_E_SHAPE;
     if (win_left >= 0 || win_right > 0 || sink != nullptr || softcap > 0.f) return -FA4_E_SHAPE;
     plan->balanced = workspace != nullptr && aligned16(workspace) && decode_balanced(p, cache.seqused_k) &&
-                     workspace_bytes >= (uint64_t)balanced_bytes(p);
+                     workspace_bytes >= (uint64_t)dealt_bytes(p, num_splits);
     if (!plan->balanced && !decode_in_cluster(p, num_splits)) {
       if (workspace == nullptr || !aligned16(workspace)) return -FA4_E_NULL;
       if (workspace_bytes < (uint64_t)splitkv_bytes(p, num_splits)) return -FA4_E_TOO_LARGE;

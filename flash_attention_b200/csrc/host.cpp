@@ -320,8 +320,8 @@ int64_t prefill_splits(int64_t B, int64_t Sq, int64_t Sk, int64_t Hq, int64_t sm
 //   1 x 8, 384 k, 4, 16, 32 entries 26.4 / 27.1, 27.8 / 28.3, 25.2 / 25.4; 2 x 8, 1 M, 8 entries 47.7 / 52.0
 //   pool of 2, 3 times the table, 8 x 4, 512 k 28.3 / 24.6, 32.9 / 24.7; 16 ragged entries 24.8 / 24.0, 28.2 / 23.8;
 //     1 M 39.7 / 43.6, 47.9 / 43.8; of 16 times, 1 x 8, 256 k 122 / 19
-// A call that is dealt by the lengths of its entries (fa4_nvfp4_decode_is_balanced) reads them at any length: the key
-// counts are on the device, so tiling goes over every slot of the cache.  us, tiled first / read linear, lengths spread over
+// A call that is dealt by the lengths of its entries (fa4_nvfp4_decode_is_balanced, and a split count that is left open) reads them at any
+// length: the key counts are on the device, so tiling goes over every slot of the cache.  us, tiled first / read linear, lengths spread over
 // the logarithm down to a 64th: 8 x 4, 800 k slots x heads as 4, 12 entries 27.9 / 24.8, 32.4 / 27.9; 1.6 M as 4, 12, 40
 //   38.7 / 29.8, 41.1 / 31.9, 36.2 / 27.3; 3.2 M 78.5 / 57.0, 79.8 / 45.2, 63.2 / 43.4; 32 x 1, 800 k as 4 28.8 / 29.4, 1.6 M
 //   as 4, 12 43.9 / 38.8, 43.9 / 42.7, 3.2 M 81.7 / 64.8, 107 / 108; 8 x 4, four tokens, 800 k as 4, 12 31.6 / 27.3, 37.0 / 30.4.
@@ -481,7 +481,7 @@ void run(Call& c) {
     k_sf = inner_contiguous(std::move(k_sf));
     v_sf = inner_contiguous(std::move(v_sf));
     const int64_t pool_ratio = paged ? B_kv * Sk_kv / std::max<int64_t>(1, B * Sk) : 1;
-    const bool dealt = used.defined() && fa4_nvfp4_decode_is_balanced((int32_t)B, (int32_t)Sq, (int32_t)Sk, (int32_t)Hq, (int32_t)Hkv);
+    const bool dealt = c.num_splits == 0 && used.defined() && fa4_nvfp4_decode_is_balanced((int32_t)B, (int32_t)Sq, (int32_t)Sk, (int32_t)Hq, (int32_t)Hkv);
     if (decode && decode_ok && (dealt || B * Hkv * Sk <= linear_keys_limit(Sq * (Hq / Hkv), k_sf.stride(1), pool_ratio))) {
       // the decode kernel reads them as they are
       linear.struct_size = sizeof linear;
@@ -579,8 +579,10 @@ void run(Call& c) {
       x.num_pages = (int32_t)B_kv;
     }
     c10::DataPtr workspace;
-    const int64_t bytes = fa4_nvfp4_fwd_ex_workspace_bytes(&p, &x);
-    if (bytes < 0) check_rc((int)bytes, "fa4_nvfp4_fwd_ex_workspace_bytes");
+    // (a split count that the caller chose is kept to: the result of an entry then does not depend on the others)
+    const int64_t bytes = auto_splits ? fa4_nvfp4_fwd_ex_workspace_bytes(&p, &x)
+                                      : fa4_nvfp4_splitkv_workspace_bytes(&p, (int32_t)num_splits);
+    if (bytes < 0) check_rc((int)bytes, "workspace of fa4_nvfp4_fwd_ex");
     if (bytes > 0) {
       workspace = scratch_bytes(bytes);
       x.workspace = workspace.get();

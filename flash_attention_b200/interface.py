@@ -93,7 +93,9 @@ def flash_attn_fp4_func(
     0 = choose (split only when the query tiles alone leave most SMs idle).  Decode and append
     shapes (D = Dv = 128, Sq * Hq / Hkv <= 32, no window / sink / softcap) run the transposed
     decode kernel (``VARIANT_DECODE``: keys on the tile's lanes, grid = splits x Hkv x B); there
-    ``num_splits=0`` is what a serving loop wants (about two CTAs per SM).
+    ``num_splits=0`` is what a serving loop wants (about two CTAs per SM; with ``seqused_k`` over
+    many keys the CTAs are then dealt by the lengths of the entries, in which an entry's bits depend on
+    the other entries' lengths too).  A chosen count gives the bits of the entry computed alone.
 
     ``window_size=(left, right)``: local attention, query row i sees keys
     ``i + Sk - Sq - left <= j <= i + Sk - Sq + right`` (``None`` = unlimited; ``causal`` is

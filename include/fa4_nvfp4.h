@@ -196,9 +196,11 @@ int fa4_nvfp4_fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, void* cu
 /*
  * The workspace that fa4_nvfp4_fwd_ex makes use of (x->workspace and x->workspace_bytes are not read): at least
  * fa4_nvfp4_splitkv_workspace_bytes(p, splits), which remains enough to run; more for a decode call
- * (FA4_VARIANT_DECODE) with x->seqused_k over many keys, whose CTAs are then dealt by the lengths of the entries.  The
- * splits stay what the reference maxima of P follow, so the two ways differ by fp32 rounding (and, where a
- * reference moves within a split, in how P is rounded behind it).
+ * (FA4_VARIANT_DECODE) with x->seqused_k over many keys, whose CTAs are dealt by the lengths of the entries if
+ * x->workspace_bytes is no less than this.  With less the splits are what runs, and an entry's result is the same bits
+ * whatever the other entries are.  Dealt, the splits stay what the reference maxima of P follow, so the two ways differ
+ * by fp32 rounding (and, where a reference moves within a split, in how P is rounded behind it).  Dealing is
+ * for entries of unequal lengths (up to several times as fast); where all are as long as each other it costs 1 to 5 us a call.
  */
 int64_t fa4_nvfp4_fwd_ex_workspace_bytes(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x);
 /* Whether a decode call of this shape with seqused_k and that workspace is dealt by the lengths (1 or 0). */

@@ -2,6 +2,7 @@
 the narrow and the wide window form, more tiles than CTAs with tiles that have no rows between them, tile
 lists longer than a CTA's table, the decode kernel's ring depths and the two ways its splits are merged, and
 the quantiser's small, unaligned and strided inputs."""
+import ctypes
 import math
 
 import numpy as np
@@ -9,8 +10,11 @@ import pytest
 import torch
 
 import flash_attention_b200 as fa
+from flash_attention_b200 import _lib
+from flash_attention_b200.interface import DeviceStatus
 from oracle import nvfp4_oracle as orc
 from tests.helpers import assert_parity, make_qkv, oracles
+from tests.test_zz_no_alloc import _params
 
 pytestmark = pytest.mark.gpu
 
@@ -423,8 +427,87 @@ def test_decode_dealt_by_the_lengths_where_references_move(cuda_device):
     fa.check_status(cuda_device)
 
 
+def _through_the_c_entry(Q, K, V, used, splits, short=0):
+    """Decode with the workspace that is asked for, which is that of a dealt call, less `short` bytes."""
+    B, Sq, Hq, _ = Q.data.shape
+    Sk, Hkv = K.data.shape[1:3]
+    L, dev = fa.lib(), Q.data.device
+    assert L.fa4_nvfp4_decode_is_balanced(B, Sq, Sk, Hq, Hkv) == 1
+    out = torch.full((B, Sq, Hq, 128), math.nan, dtype=torch.bfloat16, device=dev)
+    lse = torch.full((B, Hq, Sq), math.nan, device=dev)
+    p, x, sf = _params(Q, K, V, out, lse, True, DeviceStatus.word(dev)), _lib.Ext(), [t.tiled_sf() for t in (Q, K, V)]
+    p.variant, (p.q_sf, p.k_sf, p.v_sf) = 4, (t.data_ptr() for t in sf)
+    x.struct_size, x.num_splits, x.window_left, x.window_right = ctypes.sizeof(x), splits, -1, -1
+    x.seqused_k = used.data_ptr()
+    size = L.fa4_nvfp4_fwd_ex_workspace_bytes(ctypes.byref(p), ctypes.byref(x))
+    workspace = torch.empty(size, dtype=torch.uint8, device=dev)
+    x.workspace, x.workspace_bytes = workspace.data_ptr(), size - short
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    assert L.fa4_nvfp4_fwd_ex(ctypes.byref(p), ctypes.byref(x), stream) == 0
+    torch.cuda.synchronize(dev)
+    fa.check_status(dev)
+    return out, lse
+
+
+@pytest.mark.parametrize("Sq,Hq,Hkv,Sk,lens,layout,splits", [
+    (1, 32, 8, 8192, [8192, 300, 4000, 1, 129, 0, 2000, 8191] * 2, "tiled", 2),
+    (1, 32, 8, 13312, [13312, 129, 4096, 4097, 1], "linear", 3),
+    (1, 32, 8, 13312, [13312, 900, 260, 300, 12000], "tiled", 128),
+    (2, 8, 2, 9000, [9000, 1] + [33 * i for i in range(31)], "linear", 1),
+    (8, 32, 8, 8704, [8704, 7, 130, 8000], "tiled", 5),
+], ids=str)
+def test_a_chosen_split_count_gives_the_bits_of_the_entry_alone(cuda_device, Sq, Hq, Hkv, Sk, lens, layout, splits):
+    """Batches that are dealt by the lengths where the split count is left open: with a count, and through the C entry point with
+    a byte less than the workspace of a dealt call, an entry does not depend on its neighbours."""
+    B = len(lens)
+    g = torch.Generator(device=cuda_device).manual_seed(24)
+    Q, K, V = fa.quantize_qkv_fused(*(torch.randn(B, S, H, 128, generator=g, device=cuda_device, dtype=torch.bfloat16)
+                                      for S, H in ((Sq, Hq), (Sk, Hkv), (Sk, Hkv))))
+    used = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+
+    def call(b0, b1):
+        sf = [(t.sf if layout == "linear" else t.tiled_sf())[b0:b1] for t in (Q, K, V)]
+        return fa.flash_attn_fp4_func(*(t.data[b0:b1] for t in (Q, K, V)), *sf, Q.scale, K.scale, V.scale, causal=True,
+                                      sf_layout=layout, num_splits=splits, seqused_k=used[b0:b1], return_lse=True)
+
+    out, lse = call(0, B)
+    short_out, short_lse = _through_the_c_entry(Q, K, V, used, splits, short=1)
+    for b in range(B):
+        o, l = call(b, b + 1)
+        assert torch.equal(out[b:b + 1], o) and torch.equal(lse[b:b + 1], l), lens[b]
+        assert torch.equal(short_out[b:b + 1], o) and torch.equal(short_lse[b:b + 1], l), lens[b]
+    fa.check_status(cuda_device)
+
+
+@pytest.mark.parametrize("Sq,Hq,Hkv,Sk,lens,splits", [
+    (1, 32, 8, 13312, [13312, 13312, 13311, 13185, 13184], 3),
+    (1, 32, 8, 13312, [13312, 900, 260, 300, 12000], 128),
+    (2, 8, 2, 9000, [9000, 1] + [33 * i for i in range(31)], 1),
+    (4, 16, 8, 3200, [3200, 300, 3199, 0, 4, 3] * 6, 2),
+    (8, 32, 8, 8704, [8704, 7, 130, 8000], 5),
+    (1, 4, 4, 5120, [5120 - 40 * i for i in range(127)] + [0], 2),
+], ids=str)
+def test_decode_dealt_with_a_chosen_split_count(cuda_device, Sq, Hq, Hkv, Sk, lens, splits):
+    """Through the C entry point, with the workspace for it: against the splits, within the bounds of
+    test_decode_dealt_by_the_lengths."""
+    B = len(lens)
+    g = torch.Generator(device=cuda_device).manual_seed(25)
+    Q, K, V = fa.quantize_qkv_fused(*(torch.randn(B, S, H, 128, generator=g, device=cuda_device, dtype=torch.bfloat16)
+                                      for S, H in ((Sq, Hq), (Sk, Hkv), (Sk, Hkv))))
+    used = torch.tensor(lens, dtype=torch.int32, device=cuda_device)
+    out, lse = _through_the_c_entry(Q, K, V, used, splits)
+    ref, ref_lse = fa.flash_attn_fp4_func(
+        Q.data, K.data, V.data, Q.sf, K.sf, V.sf, Q.scale, K.scale, V.scale, causal=True, num_splits=splits, seqused_k=used,
+        return_lse=True)
+    fin = torch.isfinite(ref_lse)
+    assert torch.isfinite(out).all() and torch.equal(torch.isinf(lse), torch.isinf(ref_lse))
+    assert (lse[fin] - ref_lse[fin]).abs().max().item() <= 1e-4
+    assert (out.float() - ref.float()).norm() <= 0.01 * ref.float().norm()
+    assert not out.permute(0, 2, 1, 3)[~fin].any()
+
+
 def _long_beside(device, B, Sq, Sk, Hq, Hkv, lens, level, v_mean, splits):
-    """Decode against a cache in which entry 0 has scores `level[key]` (log2 units, the same for all rows but a few per cent) plus
+    """Dealt decode against a cache in which entry 0 has scores `level[key]` (log2 units, the same for all rows but a few per cent) plus
     noise, among entries of zeros.  Returns the relative error of entry 0 in the batch and of entry 0 alone (O), and the
     errors of the LSEs."""
     g = torch.Generator(device=device).manual_seed(23)
@@ -448,7 +531,7 @@ def _long_beside(device, B, Sq, Sk, Hq, Hkv, lens, level, v_mean, splits):
     T = (Q.data, K.data, V.data, Q.sf, K.sf, V.sf)
     call = lambda t, u, s: fa.flash_attn_fp4_func(*t, Q.scale, K.scale, V.scale, causal=True, num_splits=s, seqused_k=u,
                                                   return_lse=True)
-    got, lse = (x[:1] for x in call(T, used, splits))
+    got, lse = (x[:1] for x in (call(T, used, 0) if splits == 0 else _through_the_c_entry(Q, K, V, used, splits)))
     if splits == 0:
         splits = fa._lib.host().choose_decode_splits(B, Hkv, Sk, 148)
     alone, lse_alone = call([t[:1] for t in T], used[:1], splits)
