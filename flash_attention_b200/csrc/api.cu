@@ -209,7 +209,7 @@ int64_t balanced_bytes(const fa4_nvfp4_params* p) {
   return rows * 129 * 4 + 16 + (int64_t)p->B * p->Hkv * 8;
 }
 // Whether a decode call with key counts in memory is dealt by the lengths.  The host knows the longest possible length
-// alone.  Dealing costs 3 us (1.3 in front of the first load, the rest the second launch), so it takes that many blocks
+// alone.  Dealing costs 3 us (1.3 in front of the first load, the rest the second launch, of which 1.2 where nothing is merged), so it takes that many blocks
 // (times kv heads, over the batch) for the unevenness to cost more.  us, splits of equal number / dealt, lengths
 // spread over the logarithm down to a 64th of the longest, GQA 4:
 //   one token, 2048 blocks: 5, 8, 16, 32 entries of 8 heads 9.5 / 10.6, 9.9 / 10.6, 8.8 / 9.3, 8.9 / 11.3; 4096: 14.4 / 14.5, 15.2 /
@@ -231,6 +231,22 @@ int64_t balanced_bytes(const fa4_nvfp4_params* p) {
 //     26.7, 9000 36.2 / 30.4; 16, two heads: 3200 17.1 / 17.7, 4500 21.3 / 20.2; 20: 3300 16.1 /
 //     16.8; 32: 2200 14.0 / 12.4
 //   32 rows: 4: 6500 42.9 / 45.6, 9000 46.4 / 41.7; 8: 2200 19.2 / 19.5, 3200 24.8 / 23.1; 16: 2200 17.5 / 15.4
+// All of these are lengths spread over the logarithm.  Where the lengths do not differ, or are all short, dealing gains nothing, and
+// the call is slower by what it costs; the host cannot tell.  us, equal splits / dealt, GQA 4, 8 kv heads, one token, tiled scales; all
+// entries full, between half and full, uniform, spread as above, one full and the others a 32nd, all a tenth, all 300 keys:
+//   16 x 4096: 18.8 / 21.4, 17.0 / 19.4, 14.9 / 15.1, 11.2 / 10.5, 10.7 / 9.8, 7.4 / 8.7, 7.3 / 8.2
+//   8 x 8192: 18.5 / 21.6, 17.3 / 19.2, 16.3 / 18.1, 15.1 / 14.9, 12.8 / 10.8, 7.3 / 9.6, 6.7 / 8.0
+//   16 x 8192: 32.0 / 35.1, 26.1 / 28.5, 21.4 / 20.1, 16.7 / 13.8, 15.8 / 10.9, 8.1 / 11.5, 7.3 / 8.1
+//   32 x 8192: 55.4 / 55.2, 46.6 / 51.7, 37.8 / 37.9, 33.5 / 20.7, 25.5 / 12.9, 8.8 / 11.4, 6.7 / 8.8
+//   64 x 8192 (more units than places): 108 / 135, 90.4 / 96.8, 68.1 / 68.5, 42.6 / 38.9, 25.6 / 22.1, 31.8 / 21.1, 26.1 / 15.0
+//   16 x 32768: 107 / 113, 78.5 / 79.4, 56.1 / 45.3, 63.9 / 40.2, 46.3 / 18.2, 13.0 / 17.6, 7.3 / 8.2
+//   four tokens, 8 x 4096: 16.5 / 20.0, 14.8 / 17.5, 13.4 / 15.3, 12.3 / 11.9, 11.2 / 11.1, 7.3 / 9.1, 7.3 / 9.3
+//   16 x 8192: 39.7 / 43.0, 38.0 / 33.7, 36.9 / 25.4, 32.7 / 16.6, 31.6 / 12.8, 9.5 / 13.9, 7.7 / 9.5
+//   linear scales, which equal splits have tiled first, 8 x 8192: 24.4 / 30.1, 23.7 / 25.8, 22.1 / 23.5, 21.3 / 19.6, 17.1 / 13.8, 13.6 /
+//     12.6, 12.9 / 10.1; 16 x 8192: 43.9 / 47.9, 37.6 / 38.9, 32.4 / 28.5, 28.2 / 18.4, 27.0 / 13.8, 19.0 / 15.2, 17.6 / 10.2
+// Over the seven and lengths spread down to an eighth, dealing is even in the mean at 8192 blocks (4096 above eight rows), gains up to
+// 39 % beyond (linear scales 56), and at half of that loses 5 to 14 % with tiled scales and gains 3 to 27 % with linear ones: the
+// line stays between the two.  A caller who knows that lengths are even gives a split count, see dealt_bytes().
 bool decode_balanced(const fa4_nvfp4_params* p, const int32_t* seqused_k) {
   if (seqused_k == nullptr || p->B < 3 || p->B > dec::kMaxBalanced || p->Sk > dec::kMaxBalancedKeys) return false;
   const int64_t units = (int64_t)p->B * p->Hkv, blocks = units * ((p->Sk + kBlockN - 1) / kBlockN);

@@ -23,7 +23,7 @@
 // visited in ascending order; its normalised fp32 partial O and partial LSE are merged inside the
 // cluster of an entry's splits (up to eight), or by combine_splits_kernel as on the split-KV path of
 // attn_ws.cuh.  Grid = (splits, Hkv, B).  Batches whose entries have key counts in memory and many keys are dealt to the
-// CTAs by those counts instead (kBalanced): equal splits leave a batch of lengths spread over the logarithm waiting
+// CTAs by those counts instead, where the caller leaves the splits open (kBalanced): equal splits leave a batch of lengths spread over the logarithm waiting
 // for the longest entry's CTAs with four fifths of the GPU idle.  us, 16 entries up to 8192 keys, 8 heads, GQA 4 18.5 ->
 // 14.4, four tokens 34.1 -> 17.7; 32 up to 16384 57.3 -> 33.2 (143 MB of keys: 22 us at the copy bandwidth); 5 up to
 // 51200, 32 heads 131 -> 65.
@@ -56,8 +56,8 @@ namespace dec {
 // trip, so five are better whenever no third CTA is there to run.
 // (Registers: three CTAs of 384 threads leave 56, two of 640 leave 48, and up to eight rows the kernel wants more.  Bytes
 // of spill stores, merging / not: shallow 4 / 28, with linear scales 96 / 112-136; deep, four rows 48 / 84, 176 / 100;
-// eight rows 100 / 40, 212 / 136.  None above eight rows.  Balanced, shallow: 16-24, with linear scales 76-132.  With them the deep form is still the faster one for ragged
-// batches, see softmax_wgs, and reading linear scales faster than a launch of its own, see linear_keys_limit in
+// eight rows 100 / 40, 212 / 136.  None above eight rows.  Balanced, shallow: 16-24, with linear scales 76-132.  With them the deep form is still the faster one for
+// ragged batches, see softmax_wgs, and reading linear scales faster than a launch of its own, see linear_keys_limit in
 // host.cpp, whose line is nearer for five to eight rows.)
 constexpr int kMaxCluster = 8;  // splits that are merged inside a cluster (portable cluster size)
 constexpr int kMaxRows = 32; // query rows per kv head: Sq * group
@@ -479,8 +479,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
   int i0, n;
   // kBalanced: the references of the rows follow the splits, not the CTAs: a reference starts anew with every split (at
   // li = next_start), and a CTA that begins inside of one visits that one's first block before its own (pre = 1), for the
-  // reference alone.  P is then rounded as with a CTA per split, but for rows whose reference moves inside of a split, in blocks
-  // that the CTA passes over.
+  // reference alone.  (It is worked on like the others, with weights of zero.  Without its V tile, P and product: the same bits, and no
+  // faster: 16 entries up to 8192 keys, lengths spread 13.6 -> 13.8 us, a tenth 11.1 -> 11.1.)  P is then rounded as with a CTA per split, but for rows whose
+  // reference moves inside of a split, in blocks that the CTA passes over.
   int pre = 0, next_start = 1 << 30;
   if constexpr (kBal) {
     pre = work.n > 0 && work.into > 0 ? 1 : 0;

@@ -398,7 +398,8 @@ attn_fwd_ws64_kernel(const __grid_constant__ CUtensorMap tm_q,
   //     of 1023, 16383 keys 212.0 / 208.8 / 207.5 / 220.8 / 212.7, 1388 / 1376 / 1352 / 1544 / 1387
   //   D = 192: 20 packed sequences 126.3 / 134.4 / 124.9 / 129.9 / 124.1, 60 short ones 72.5 / 74.4 / 72.0 / 73.9 / 72.8
   // Further cuts in the plain form: in front of the reference 643, between the maxima 643, in front of the last
-  // stores 645, between the 16-key blocks 656 and 680.
+  // stores 645, between the 16-key blocks 656 and 680.  (nvcc 12.9.86: what the scheduler does with a cut is the compiler's, so another one
+  // wants these measured anew.  With the cuts the plain forms spill 12 bytes, at D = 64 20, without 0 and 12.)
   constexpr bool kPlain = !(kWindow || kCache);
   // The soft cap's forms (its 64 tanh stand in front of the maxima) take the first cut alone: plain, wait / first cut / both
   // 358 / 352 / 362, at D = 64 355 / 348 / 356, window of 1023 keys, wait / none / first 182 / 196 / 181.
