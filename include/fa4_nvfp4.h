@@ -200,7 +200,7 @@ int fa4_nvfp4_fwd_ex(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x, void* cu
  * x->workspace_bytes is no less than this.  With less the splits are what runs, and an entry's result is the same bits
  * whatever the other entries are.  Dealt, the splits stay what the reference maxima of P follow, so the two ways differ
  * by fp32 rounding (and, where a reference moves within a split, in how P is rounded behind it).  Dealing is
- * for entries of unequal lengths (up to several times as fast); where all are as long as each other, or short, it costs 1 to 5 us a call,
+ * for entries of unequal lengths (up to several times as fast); where all are as long as each other, or short, it costs 1 to 7 us a call,
  * and up to a quarter of it with more than 444 entries times kv heads.
  */
 int64_t fa4_nvfp4_fwd_ex_workspace_bytes(const fa4_nvfp4_params* p, const fa4_nvfp4_ext* x);
