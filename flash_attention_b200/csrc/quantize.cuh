@@ -65,18 +65,23 @@ __device__ __noinline__ uint2 quantize_block16_exact(Block16 x, float denom) {
 }
 
 // Per-tensor constants of the quantiser: the tensor scale g, 1 / g, and whether g or a block's scale times g lies
-// where the two-term reciprocals lose bits (`odd`: block scales take the library division; `huge`: the elements
-// as well).
+// where the two-term reciprocals lose bits (`odd`: block scales take the library division; `exact`: the elements
+// as well).  That is near the ends of the fp32 range, and where the significand of such a product is all ones: no bf16 maximum
+// gives one, but a caller's own may, and the reciprocal of 2 - 2^-23 is one ulp too small: the quotient of .5 is then on the
+// boundary .25 instead of above it.
 struct TensorScale {
   float g;
   Reciprocal rcp;
-  bool odd, huge;
+  bool odd, exact;
 };
 __device__ __forceinline__ TensorScale make_tensor_scale(float amax) {
   TensorScale t;
   t.g = tensor_scale_of(amax);
-  t.huge = t.g > 1e17f && t.g < INFINITY;
-  t.odd = !(t.g >= 1e-18f) || t.huge;
+  bool ones = false;           // (an e4m3 value has four bits)
+#pragma unroll
+  for (int m = 8; m < 16; ++m) ones |= (~__float_as_uint(__fmul_rn((float)m, t.g)) & 0x7fffffu) == 0u;
+  t.exact = (t.g > 1e17f && t.g < INFINITY) || ones;
+  t.odd = !(t.g >= 1e-18f) || t.exact;
   t.rcp.hi = t.odd ? 0.f : __frcp_rn(t.g);
   t.rcp.lo = fmaf(-t.g, t.rcp.hi, 1.f) * t.rcp.hi;
   return t;
@@ -105,10 +110,10 @@ __device__ __forceinline__ void quantize_block16(const float (&x)[16], float bma
   const float denom = block_scale_of(bmax, ts, sf_byte);
   // The element codes are those of the correctly rounded quotients x / denom: only quotients within a few
   // ulp of a rounding boundary of e2m1 (.25 .75 1.25 1.75 2.5 3.5 5) matter, x has eight significand bits, and
-  // for every significand of denom but the largest (which no bf16 maximum gives) and every reciprocal
+  // for every significand of denom but the largest (which takes the other branch) and every reciprocal
   // within one ulp the products below put the values of x next to a boundary on the side of it that the
   // correctly rounded quotient is on.  Two instructions a pair where one term and a residual step took three.
-  if (denom >= 1e-30f && !ts.huge) {
+  if (denom >= 1e-30f && !ts.exact) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(denom));
     const float rl = __fmul_rn(fmaf(-denom, r, 1.f), r);

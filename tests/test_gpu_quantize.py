@@ -1,4 +1,6 @@
 """GPU parity of the fused NVFP4 quantiser: bit-exact against the CPU oracle's quantiser."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -151,3 +153,37 @@ def test_loads_in_stages_and_scales_at_the_ends(cuda_device, B, S, Hq, Hkv, D, s
         assert np.array_equal(got.data.cpu().numpy(), want.data)
         lin = want.sf if got.is_v else np.transpose(want.sf, (0, 2, 1, 3))
         assert np.array_equal(got.sf_tiled.cpu().numpy(), _tiled(lin, mult))
+
+
+@pytest.mark.parametrize("m", range(9, 16))
+def test_a_maximum_of_the_callers_own_with_significands_of_all_ones(cuda_device, m):
+    """Tensor scales g from a chosen maximum for which m / 8 times g, the denominator of a block, is 2 - 2^-23 (m = 8: no maximum gives
+    that g): the bytes of correctly rounded quotients for the values next to every boundary of e2m1, and for blocks near the
+    smallest scale."""
+    ones = np.float32(2) - np.float32(2) ** -23
+    near = np.float32(float(ones) * 8 / m)
+    g = next(c for c in (near, np.nextafter(near, np.float32(0)), np.nextafter(near, np.float32(9)))
+             if np.float32(m / 8) * c == ones)
+    amax = np.float32(float(g) * 2688)
+    amax = next(c for c in (amax, np.nextafter(amax, np.float32(0)), np.nextafter(amax, np.float32(1e9))) if c / np.float32(2688) == g)
+    x = np.zeros((4, 16), dtype=np.float32)
+    mids = np.array([.25, .75, 1.25, 1.75, 2.5, 3.5, 5.0])
+    for row, (lo, hi) in enumerate(((0, 1), (-1, 2))):
+        frac, e = np.frexp(mids * float(ones))
+        for col, j in ((0, lo), (7, hi)):
+            n = np.floor(np.ldexp(frac, 8)) + j
+            n = np.where(n > 256, 2 * n - 256, np.where(n < 128, 64 + n / 2, n))      # eight bits
+            x[row, col:col + 7] = np.ldexp(n, e - 8)
+        x[row, 14] = 12.0                                  # 6 denominators: the block's scale is m / 8
+    x[2, 0], x[3, 0], x[3, 1] = 1.5 / 128, 1.5 / 64, -1.5 / 256
+    x = torch.from_numpy(x).view(1, 1, 1, 64)
+    assert torch.equal(x.bfloat16().float(), x)
+    data, sf, _ = fa.quant.quantize_lastdim(x, float(g))
+    assert sf.flatten()[0] == sf.flatten()[1] == 0x30 + m
+    xd = x.bfloat16().to(cuda_device)
+    got, got_sf = (torch.full_like(t, 255, device=cuda_device) for t in (data, sf))
+    given = torch.tensor([float(amax)], device=cuda_device)
+    assert fa.lib().fa4_nvfp4_quantize_qk_bf16(xd.data_ptr(), 1, 1, 1, 64, 64, 64, 64, given.data_ptr(), got.data_ptr(),
+                                               got_sf.data_ptr(), None, None,
+                                               ctypes.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)) == 0
+    assert torch.equal(got_sf.cpu(), sf) and torch.equal(got.cpu(), data)
