@@ -72,7 +72,7 @@ __device__ __noinline__ uint2 quantize_block16_exact(Block16 x, float denom) {
 struct TensorScale {
   float g;
   Reciprocal rcp;
-  bool odd, exact;
+  bool odd, exact, finite;
 };
 __device__ __forceinline__ TensorScale make_tensor_scale(float amax) {
   TensorScale t;
@@ -82,6 +82,7 @@ __device__ __forceinline__ TensorScale make_tensor_scale(float amax) {
   for (int m = 8; m < 16; ++m) ones |= (~__float_as_uint(__fmul_rn((float)m, t.g)) & 0x7fffffu) == 0u;
   t.exact = (t.g > 1e17f && t.g < INFINITY) || ones;
   t.odd = !(t.g >= 1e-18f) || t.exact;
+  t.finite = t.g < INFINITY;
   t.rcp.hi = t.odd ? 0.f : __frcp_rn(t.g);
   t.rcp.lo = fmaf(-t.g, t.rcp.hi, 1.f) * t.rcp.hi;
   return t;
@@ -113,7 +114,9 @@ __device__ __forceinline__ void quantize_block16(const float (&x)[16], float bma
   // for every significand of denom but the largest (which takes the other branch) and every reciprocal
   // within one ulp the products below put the values of x next to a boundary on the side of it that the
   // correctly rounded quotient is on.  Two instructions a pair where one term and a residual step took three.
-  if (denom >= 1e-30f && !ts.exact) {
+  // An infinity in front of a residual of either sign would be an infinity or a NaN: with a tensor scale that leaves it a
+  // value (a caller's own), the block takes the quotients.
+  if (denom >= 1e-30f && !ts.exact && (bmax < INFINITY || !ts.finite)) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(denom));
     const float rl = __fmul_rn(fmaf(-denom, r, 1.f), r);

@@ -187,3 +187,19 @@ def test_a_maximum_of_the_callers_own_with_significands_of_all_ones(cuda_device,
                                                got_sf.data_ptr(), None, None,
                                                ctypes.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)) == 0
     assert torch.equal(got_sf.cpu(), sf) and torch.equal(got.cpu(), data)
+
+
+@pytest.mark.parametrize("amax", [1.0, 3.7, 1e-20, 2688.0, 1e30])
+def test_infinities_under_a_maximum_of_the_callers_own(cuda_device, amax):
+    """x / denominator of an infinity is an infinity and takes the largest magnitude with its sign; its neighbours keep theirs."""
+    g = torch.Generator().manual_seed(6)
+    x = (torch.randn(1, 40, 2, 64, generator=g) * (amax / 4)).bfloat16()
+    at = torch.randperm(x.numel(), generator=g)[:60]
+    x.view(-1)[at] = torch.tensor([torch.inf, -torch.inf]).repeat(30).bfloat16()
+    data, sf, _ = fa.quant.quantize_lastdim(x.float(), float(np.float32(amax) / np.float32(2688)))
+    xd, given = x.to(cuda_device), torch.tensor([amax], device=cuda_device)
+    got, got_sf = (torch.full_like(t, 255, device=cuda_device) for t in (data, sf))
+    assert fa.lib().fa4_nvfp4_quantize_qk_bf16(xd.data_ptr(), 1, 40, 2, 64, *xd.stride()[:3], given.data_ptr(), got.data_ptr(),
+                                               got_sf.data_ptr(), None, None,
+                                               ctypes.c_void_p(torch.cuda.current_stream(cuda_device).cuda_stream)) == 0
+    assert torch.equal(got_sf.cpu(), sf) and torch.equal(got.cpu(), data)
