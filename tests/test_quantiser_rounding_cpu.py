@@ -111,3 +111,37 @@ def test_reciprocals_in_two_terms_keep_every_code_and_block_scale():
         open(c, "w").write(TWO_TERMS)
         subprocess.run(["gcc", "-O2", "-fopenmp", "-mfma", "-ffp-contract=off", c, "-o", exe, "-lm"], check=True)
         assert int(subprocess.run([exe], capture_output=True, text=True, check=True).stdout) == 0
+
+
+EVERY_SCALE = r'''
+#include <math.h>
+#include <stdio.h>
+#include <string.h>
+static int on_boundary(float f) { unsigned u; memcpy(&u, &f, 4); return (u & 0x7ffffu) == 0; }    /* five bits at most */
+int main(void) {
+  long bad = 0;
+#pragma omp parallel for reduction(+ : bad)
+  for (int m = 0; m < (1 << 23) - 1; ++m) {     /* the largest one: see the test */
+    const float g = 1.f + (float)m * 0x1p-23f, r = 1.f / g, rl = fmaf(-g, r, 1.f) * r;
+    for (int b = 128; b < 256; ++b) {
+      const float x = (float)b, t = fmaf(x, 1.f / 6.f, x * -4.967053731282552e-09f);
+      const float q = x / 6.f / g, y = fmaf(t, r, t * rl);
+      bad += q != y && (on_boundary(q) || on_boundary(y));
+    }
+  }
+  printf("%ld\n", bad);
+  return 0;
+}'''
+
+
+def test_block_scales_for_every_tensor_scale():
+    """A caller's own maximum can give any g = maximum / 2688 but 2 - 2^-23: the quotient of a block maximum is the correctly rounded one, or both
+    lie between the same two boundaries of e4m3 (which have five bits)."""
+    ones = np.float32(2) - np.float32(2) ** -23
+    near = np.float32(float(ones) * 2688)
+    assert all(c / np.float32(2688) != ones for c in (np.nextafter(near, np.float32(0)), near, np.nextafter(near, np.float32(1e9))))
+    with tempfile.TemporaryDirectory() as d:
+        c, exe = os.path.join(d, "t.c"), os.path.join(d, "t")
+        open(c, "w").write(EVERY_SCALE)
+        subprocess.run(["gcc", "-O2", "-fopenmp", "-mfma", "-ffp-contract=off", c, "-o", exe, "-lm"], check=True)
+        assert int(subprocess.run([exe], capture_output=True, text=True, check=True).stdout) == 0
